@@ -320,6 +320,7 @@ _SIGS = {
     "edg_tridiag_lowest_noalloc": (I32, [P, P, I32, I32, P, P, P]),
     "edg_local_expval": (I32, [P, I64, C.POINTER(SiteDims), I32, P, I32, I64, P, I32, P, P]),
     "edg_local_expval_wide": (I32, [P, I64, I32, C.POINTER(SiteDims), I32, P, I32, I64, P, I32, P, P]),
+    "edg_gauge_apply": (I32, [P, I64, I32, I32, C.POINTER(SiteDims), I32, P, I32, I32, P, I32, I64, P, P]),
     "edg_small_batch_work_elems": (I64, [I64, I32, I32]),
     "edg_lanczos_small_batched": (I32, [C.POINTER(SmallBatch), P, P]),
     "edg_ctx_create": (P, []),

@@ -23,6 +23,8 @@ logger = logging.getLogger(__name__)
 
 __all__ = ["QMB_hamiltonian", "QMB_state"]
 
+_PSI_CODES = {torch.float64: 0, torch.float32: 1, torch.complex128: 2, torch.complex64: 3}
+
 
 class QMB_state:
     """A state vector in the sector basis (host copy made on first access)."""
@@ -208,29 +210,64 @@ class QMB_hamiltonian:
         return self.mat.to_scipy()
 
     # -------------------------------------------------------------- phases
-    def _row_phase(self):
-        """i**e(row) of the real form's gauge transform (None if not used)."""
-        w = self.mat.phase_weights if self.mat is not None else None
+    def _phase_table(self):
+        """Device bytes [n_sites][dmax] of the real form's phase exponents
+        (None if not used); kept on the matrix they belong to."""
+        mat = self.mat
+        w = mat.phase_weights if mat is not None else None
         if w is None:
             return None
-        cfg = torch.from_numpy(self.sector.configs.astype(np.int64)).to(self.sector.device)
-        wt = torch.from_numpy(np.asarray(w, dtype=np.int64)).to(self.sector.device)
-        e = wt[torch.arange(cfg.shape[1], device=cfg.device)[None, :], cfg].sum(dim=1) % 4
-        table = torch.tensor([1, 1j, -1, -1j], dtype=torch.complex128, device=cfg.device)
-        return table[e]
+        if getattr(mat, "_phase_bytes", None) is None:
+            t = np.ascontiguousarray(np.asarray(w, dtype=np.int64) % 4, dtype=np.uint8)
+            mat._phase_bytes = torch.from_numpy(t).to(self.sector.device)
+        return mat._phase_bytes
+
+    def _apply_phase(self, tab, psi, conj):
+        """i**(+-e(row)) psi as complex128 (``edg_gauge_apply``); the phases
+        themselves for psi = None."""
+        import ctypes
+
+        from .. import _lib
+        from .._lib import check, lib, ptr, stream_handle
+
+        sec = self.sector
+        n = len(sec)
+        dims = _lib.SiteDims()
+        for s in range(sec.n_sites):
+            dims.d[s] = int(sec.loc_dims[s])
+        out = torch.empty(n, dtype=torch.complex128, device=sec.device)
+        code = 0 if psi is None else _PSI_CODES[psi.dtype]
+        stride = 1 if psi is None else max(int(psi.stride(0)), 1)
+        check(lib.edg_gauge_apply(ptr(sec.keys), n, sec.key_words, sec.n_hi, ctypes.byref(dims), sec.n_sites,
+                                  ptr(tab), int(tab.shape[1]), 1 if conj else 0, ptr(psi), code, stride, ptr(out),
+                                  stream_handle()), "edg_gauge_apply")
+        return out
+
+    def _row_phase(self):
+        """i**e(row) of the real form's gauge transform (None if not used)."""
+        tab = self._phase_table()
+        return None if tab is None else self._apply_phase(tab, None, False)
+
+    def _with_phase(self, psi, conj):
+        tab = self._phase_table()
+        if tab is None:
+            return psi
+        # one vector over the sector's rows, read in place; anything else (a
+        # stack of states, another dtype or device, autograd) is a product
+        # with the phases
+        if (psi.dim() == 1 and psi.shape[0] == len(self.sector) and psi.stride(0) >= 1 and psi.dtype in _PSI_CODES
+                and psi.device == self.sector.keys.device and not psi.requires_grad and not psi.is_conj()
+                and not psi.is_neg()):
+            return self._apply_phase(tab, psi, conj)
+        ph = self._apply_phase(tab, None, conj)
+        return ph * psi.to(torch.complex128)
 
     def to_original_basis(self, psi: torch.Tensor) -> torch.Tensor:
         """Map a real-form vector back to the reference (complex) basis."""
-        ph = self._row_phase()
-        if ph is None:
-            return psi
-        return ph * psi.to(torch.complex128)
+        return self._with_phase(psi, False)
 
     def from_original_basis(self, psi: torch.Tensor) -> torch.Tensor:
-        ph = self._row_phase()
-        if ph is None:
-            return psi
-        return torch.conj(ph) * psi.to(torch.complex128)
+        return self._with_phase(psi, True)
 
     # -------------------------------------------------------- diagonalize
     def diagonalize(self, n_eigs, format="gpu", loc_dims=None, print_results=False, tol=1e-12, precision="fp64",

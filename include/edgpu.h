@@ -640,6 +640,18 @@ int edg_local_expval_wide(const uint64_t* keys, int64_t n, int32_t n_hi,
                           int64_t psi_stride, const double* diag,
                           int32_t dmax, double* out, cudaStream_t stream);
 
+/* Gauge phases of the real form: out[r] = i^e(r) psi[r * psi_stride]
+ * (complex128), e(r) = sum_s weights[s * dmax + c_s(r)] (weights: device
+ * bytes [n_sites][dmax], exponents 0..3); conj != 0 applies i^-e.  psi: dtype
+ * 0 f64, 1 f32, 2 complex128, 3 complex64; NULL writes the phases.  keys: n
+ * one-word keys, or 2n words split at n_hi (key_words 2).  out must not
+ * overlap psi unless both are complex128 with psi_stride 1. */
+int edg_gauge_apply(const uint64_t* keys, int64_t n, int32_t key_words,
+                    int32_t n_hi, const edg_site_dims* dims, int32_t n_sites,
+                    const uint8_t* weights, int32_t dmax, int32_t conj,
+                    const void* psi, int32_t psi_dtype, int64_t psi_stride,
+                    void* out, cudaStream_t stream);
+
 /* Two-body correlators, TwoBodyTerm.get_expval / lattice_twobody_exp_val
  * (edlgt/modeling/twobody_term.py:160-264): corr[i * n_sites + j] =
  * corr[j * n_sites + i] = Re <psi| A_i B_j |psi> for each listed pair i < j
