@@ -5,12 +5,28 @@
 //
 // One step: v_0 = psi/|psi|; m Lanczos steps w = H v_j, orthogonalised against
 // the basis (one classical Gram-Schmidt pass over all previous vectors, or
-// two), alpha_j = Re<v_j, w>, beta_{j+1} = |w|; then c = |psi| exp(-i T dt) e_1
-// for the m x m tridiagonal T (scaling and squaring of a Taylor series on the
-// device, exact to double precision) and psi = V c.  A breakdown (beta = 0)
-// leaves zero vectors whose block of T decouples from e_1, so the step needs
-// no host synchronisation.  Replaces scipy's expm_multiply as called by
-// QMB_hamiltonian.time_evolution (edlgt/modeling/qmb_hamiltonian.py:334-426).
+// two; or against v_{j-1}, v_j only), alpha_j = Re<v_j, w>, beta_{j+1} = |w|;
+// then c = |psi| exp(-i T dt) e_1 for the m x m tridiagonal T (Taylor series
+// over substeps on the device, exact to double precision) and psi = V c.  A
+// breakdown (beta = 0) leaves zero vectors whose block of T decouples from
+// e_1, so the step needs no host synchronisation.  Replaces scipy's
+// expm_multiply as called by QMB_hamiltonian.time_evolution
+// (edlgt/modeling/qmb_hamiltonian.py:334-426).
+//
+// The basis is stored unnormalised, u_i = beta_i v_i: the update pass writes
+// u_{j+1} in the vectors' type while it sums |u_{j+1}|^2, and the factors
+// 1 / beta_i go into the coefficients of later passes.  A normalised basis
+// needs the updated w written in f64 and a further pass that reads it back
+// (40 B a row of a complex64 basis).
+//
+// Two forms, chosen by the number of rows (coop_fits):
+//   * large sectors: matvec, dots, coefficients, update as launches over all
+//     rows; for the local recurrence on the packed layout the dots are summed
+//     in the matvec's epilogue (packed.cu) and a step is two launches;
+//   * small sectors (krylov_coop_k): the whole time step is one cooperative
+//     launch.  There the rows are a few hundred per SM, every launch costs
+//     more than its work, and what is left is two grid-wide waits a step.
+#include "gridbar.cuh"
 #include "spmv.cuh"
 
 #include <type_traits>
@@ -20,8 +36,8 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItile = 8;
 constexpr int kMaxM = 64;
+constexpr int64_t kCoopMaxRows = 1024 * edg::kSmCount;  // see krylov_coop_k
 
 template <typename T>
 __device__ __forceinline__ edg::cd ldc(const T* p, int64_t i);
@@ -46,224 +62,293 @@ __device__ __forceinline__ void stc<double2>(double2* p, int64_t i, double re, d
   p[i] = make_double2(re, im);
 }
 
-__device__ __forceinline__ double block_sum1(double a, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-  if (lane == 0) red[warp] = a;
+constexpr int kWarps = kThreads / 32;
+
+// Totals of NV doubles per thread over the block, in every thread of warp 0.
+template <int NV>
+__device__ __forceinline__ void block_totals(double (&v)[NV], double* red /*[kWarps][NV]*/) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if (lane == 0) red[warp * NV + q] = v[q];
+  }
   __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
+  if (warp == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double a = lane < nw ? red[lane * NV + q] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      v[q] = a;
+    }
+  }
   __syncthreads();
-  return t;  // valid in thread 0
 }
 
-// |x|^2 block partials of a complex vector (T storage or double2 working)
-template <typename T>
-__global__ void __launch_bounds__(kThreads) norm_k(const T* __restrict__ x, int64_t n, double* __restrict__ part) {
-  __shared__ double red[kThreads / 32];
+// Thread 0 of the last CTA to arrive gets true, with part[0 .. gridDim.x)
+// summed in a fixed order in *total; `mine` is this CTA's partial (thread 0).
+__device__ __forceinline__ bool last_cta_sum(double mine, double* part, unsigned* ticket, double* total) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = mine;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return false;
+  __threadfence();
   double a = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) a += __ldcg(part + b);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if (threadIdx.x == 0) *ticket = 0u;
+  *total = a;
+  return threadIdx.x == 0;
+}
+
+// |psi|
+template <typename T>
+__global__ void __launch_bounds__(kThreads) norm_k(const T* __restrict__ x, int64_t n, double* __restrict__ part,
+                                                   unsigned* __restrict__ ticket, double* __restrict__ out) {
+  __shared__ double red[kWarps];
+  double a[1] = {0.0};
   for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
     edg::cd v = ldc<T>(x, r);
-    a = fma(v.re, v.re, fma(v.im, v.im, a));
+    a[0] = fma(v.re, v.re, fma(v.im, v.im, a[0]));
   }
-  double t = block_sum1(a, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  block_totals<1>(a, red);
+  double t;
+  if (last_cta_sum(a[0], part, ticket, &t)) out[0] = sqrt(t);
 }
 
-// out[0] = sqrt(sum partials)
-__global__ void __launch_bounds__(kThreads) sqrt_sum_k(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  __shared__ double red[kThreads / 32];
-  double a = 0.0;
-  for (int b = threadIdx.x; b < nb; b += kThreads) a += part[b];
-  double t = block_sum1(a, red);
-  if (threadIdx.x == 0) out[0] = sqrt(t);
-}
-
-// dst = src / s[0] (s = 0 gives zeros)
-template <typename TS, typename TD>
-__global__ void scale_k(const TS* __restrict__ src, int64_t n, const double* __restrict__ s, TD* __restrict__ dst) {
-  const double inv = s[0] > 0.0 ? 1.0 / s[0] : 0.0;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    edg::cd v = ldc<TS>(src, r);
-    stc<TD>(dst, r, v.re * inv, v.im * inv);
-  }
-}
-
-// partial[b][i] = sum_{r in block b} conj(V[i][r]) w[r] for i <= j (complex double)
+// u_0 = psi / |psi| (a zero psi gives zeros); beta[0] = |u_0|
 template <typename T>
-__global__ void __launch_bounds__(kThreads) dots_k(const T* __restrict__ V, int64_t n, int ilo, int j,
+__global__ void scale_k(const T* __restrict__ src, int64_t n, const double* __restrict__ s, T* __restrict__ dst,
+                        double* __restrict__ beta) {
+  const double inv = s[0] > 0.0 ? 1.0 / s[0] : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) beta[0] = s[0] > 0.0 ? 1.0 : 0.0;
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    edg::cd v = ldc<T>(src, r);
+    stc<T>(dst, r, v.re * inv, v.im * inv);
+  }
+}
+
+// Resident CTAs per SM of the two passes over the basis, and their grids: a
+// grid of more CTAs than are resident ends in a part-filled wave.  Rows are
+// taken grid-stride, so that at any time the grid reads one window of each
+// vector: with a contiguous chunk of rows per CTA the dots of 26 complex64
+// vectors (848,614 rows) took 151 us, here 56 (update pass 45).
+template <typename T>
+constexpr int dot_ctas() { return sizeof(T) == 8 ? 3 : 2; }
+constexpr int kUpdateCtas = 3;
+constexpr int kTile = 8;  // vectors per dots tile (w is read once per tile)
+
+// partial[b][i] = sum over the CTA's rows of conj(u_i[r]) w[r], ilo <= i <= j
+template <typename T>
+__global__ void __launch_bounds__(kThreads, dot_ctas<T>()) dots_k(const T* __restrict__ V, int64_t n, int64_t ldv, int ilo, int j,
                                                    const double2* __restrict__ w, double2* __restrict__ partial,
                                                    int ld_i) {
-  __shared__ double red[(kThreads / 32) * kItile * 2];
-  __shared__ double out[kItile * 2];
-  const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-  const int64_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
+  __shared__ double red[kWarps * kTile * 2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i0 = ilo; i0 <= j; i0 += kItile) {
-    double re[kItile], im[kItile];
+  for (int i0 = ilo; i0 <= j; i0 += kTile) {
+    double re[kTile], im[kTile];
 #pragma unroll
-    for (int t = 0; t < kItile; ++t) re[t] = im[t] = 0.0;
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += kThreads) {
-      double2 wr = w[r];
+    for (int t = 0; t < kTile; ++t) re[t] = im[t] = 0.0;
+    const T* Vi = V + (int64_t)i0 * ldv;
+    const int nt = min(kTile, j + 1 - i0);
+    for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
+      const double2 wr = w[r];
+      T x[kTile];
 #pragma unroll
-      for (int t = 0; t < kItile; ++t)
-        if (i0 + t <= j) {
-          edg::cd v = ldc<T>(V, (int64_t)(i0 + t) * n + r);
-          re[t] = fma(v.re, wr.x, fma(v.im, wr.y, re[t]));
-          im[t] = fma(v.re, wr.y, fma(-v.im, wr.x, im[t]));
+      for (int t = 0; t < kTile; ++t)
+        if (t < nt) x[t] = Vi[(int64_t)t * ldv + r];
+#pragma unroll
+      for (int t = 0; t < kTile; ++t)
+        if (t < nt) {
+          re[t] = fma((double)x[t].x, wr.x, fma((double)x[t].y, wr.y, re[t]));
+          im[t] = fma((double)x[t].x, wr.y, fma(-(double)x[t].y, wr.x, im[t]));
         }
     }
 #pragma unroll
-    for (int t = 0; t < kItile; ++t) {
+    for (int t = 0; t < kTile; ++t) {
       double a = re[t], b = im[t];
       for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_down_sync(0xffffffffu, a, o);
         b += __shfl_down_sync(0xffffffffu, b, o);
       }
       if (lane == 0) {
-        red[(warp * kItile + t) * 2] = a;
-        red[(warp * kItile + t) * 2 + 1] = b;
+        red[(warp * kTile + t) * 2] = a;
+        red[(warp * kTile + t) * 2 + 1] = b;
       }
     }
     __syncthreads();
-    if (threadIdx.x < kItile * 2) {
-      double a = 0.0;
-      for (int wi = 0; wi < kThreads / 32; ++wi) a += red[wi * kItile * 2 + threadIdx.x];
-      out[threadIdx.x] = a;
-    }
-    __syncthreads();
-    if (threadIdx.x < kItile) {
-      int t = threadIdx.x;
-      if (i0 + t <= j) partial[(int64_t)blockIdx.x * ld_i + i0 + t] = make_double2(out[2 * t], out[2 * t + 1]);
+    if (threadIdx.x < nt) {
+      double a = 0.0, b = 0.0;
+      for (int wi = 0; wi < kWarps; ++wi) {
+        a += red[(wi * kTile + threadIdx.x) * 2];
+        b += red[(wi * kTile + threadIdx.x) * 2 + 1];
+      }
+      partial[(int64_t)blockIdx.x * ld_i + i0 + threadIdx.x] = make_double2(a, b);
     }
     __syncthreads();
   }
 }
 
-// h[i] = sum_b partial[b][i]; alpha[j] += Re h[j]
-__global__ void __launch_bounds__(kThreads) reduce_h_k(const double2* __restrict__ partial, int nb, int ld_i, int ilo,
-                                                       int j, double2* __restrict__ h, double* __restrict__ alpha_j) {
-  __shared__ double red[kThreads / 32];
+// Coefficients of the update from the dots: coef[i - ilo] = <v_i, w> / beta_i
+// with w = ws * (the vector the dots were taken of), coef[j + 1 - ilo] = ws;
+// ws = 1 / beta_j for the product itself (pass 0), 1 for a vector already
+// updated.  alpha_j = Re <v_j, w>, added to in a second pass.
+__global__ void __launch_bounds__(kThreads) coef_k(const double2* __restrict__ partial, int nb, int ld_i, int ilo,
+                                                   int j, int pass, const double* __restrict__ beta,
+                                                   double2* __restrict__ coef, double* __restrict__ alpha) {
+  __shared__ double red[kWarps * 2];
   const int i = ilo + blockIdx.x;
-  double a = 0.0, b = 0.0;
+  double a[2] = {0.0, 0.0};
   for (int q = threadIdx.x; q < nb; q += kThreads) {
-    double2 p = partial[(int64_t)q * ld_i + i];
-    a += p.x;
-    b += p.y;
+    const double2 p = partial[(int64_t)q * ld_i + i];
+    a[0] += p.x;
+    a[1] += p.y;
   }
-  double ta = block_sum1(a, red);
-  double tb = block_sum1(b, red);
+  block_totals<2>(a, red);
   if (threadIdx.x == 0) {
-    h[i] = make_double2(ta, tb);
-    if (i == j) alpha_j[0] += ta;
+    const double bj = beta[j], bi = beta[i];
+    const double si = bi > 0.0 ? 1.0 / bi : 0.0;
+    const double ws = pass > 0 ? 1.0 : (bj > 0.0 ? 1.0 / bj : 0.0);
+    const double hr = si * (ws * a[0]), hi = si * (ws * a[1]);
+    coef[i - ilo] = make_double2(si * hr, si * hi);
+    if (i == j) {
+      coef[j + 1 - ilo] = make_double2(ws, 0.0);
+      alpha[j] = pass > 0 ? alpha[j] + hr : hr;
+    }
   }
 }
 
-// w[r] -= sum_{i<=j} V[i][r] h[i]; |w|^2 block partials
+// x = ws w - sum_{i} coef_i u_i over ilo <= i <= j; written to out (the next
+// Krylov vector, in T) with beta_{j+1} = |x|, or back to w (a pass that
+// another one follows).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) update_k(const T* __restrict__ V, int64_t n, int ilo, int j,
-                                                     const double2* __restrict__ h, double2* __restrict__ w,
-                                                     double* __restrict__ part) {
+__global__ void __launch_bounds__(kThreads, kUpdateCtas) update_k(const T* __restrict__ V, int64_t n, int64_t ldv, int ilo, int j,
+                                                     const double2* __restrict__ coef, double2* __restrict__ w,
+                                                     T* __restrict__ out, double* __restrict__ part,
+                                                     unsigned* __restrict__ ticket, double* __restrict__ beta) {
+  constexpr int kGroup = 8;  // vectors loaded together
   __shared__ double2 hs[kMaxM + 1];
-  __shared__ double red[kThreads / 32];
-  for (int t = ilo + threadIdx.x; t <= j; t += kThreads) hs[t] = h[t];
+  __shared__ double red[kWarps];
+  const int nv = j + 1 - ilo;
+  for (int t = threadIdx.x; t <= nv; t += kThreads) hs[t] = coef[t];
   __syncthreads();
-  double a = 0.0;
+  const double ws = hs[nv].x;
+  const T* Vi = V + (int64_t)ilo * ldv;
+  double a[1] = {0.0};
   for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
+    const double2 x = w[r];
     double sr = 0.0, si = 0.0;
-    for (int i = ilo; i <= j; ++i) {
-      edg::cd v = ldc<T>(V, (int64_t)i * n + r);
-      sr = fma(v.re, hs[i].x, fma(-v.im, hs[i].y, sr));
-      si = fma(v.re, hs[i].y, fma(v.im, hs[i].x, si));
+    for (int i0 = 0; i0 < nv; i0 += kGroup) {
+      T v[kGroup];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t)
+        if (i0 + t < nv) v[t] = Vi[(int64_t)(i0 + t) * ldv + r];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t)
+        if (i0 + t < nv) {
+          const double2 h = hs[i0 + t];
+          sr = fma((double)v[t].x, h.x, fma(-(double)v[t].y, h.y, sr));
+          si = fma((double)v[t].x, h.y, fma((double)v[t].y, h.x, si));
+        }
     }
-    double2 x = w[r];
-    x.x -= sr;
-    x.y -= si;
-    w[r] = x;
-    a = fma(x.x, x.x, fma(x.y, x.y, a));
+    const double2 y = make_double2(fma(ws, x.x, -sr), fma(ws, x.y, -si));
+    if (out != nullptr)
+      stc<T>(out, r, y.x, y.y);
+    else
+      w[r] = y;
+    a[0] = fma(y.x, y.x, fma(y.y, y.y, a[0]));
   }
-  double t = block_sum1(a, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  if (out == nullptr) return;
+  block_totals<1>(a, red);
+  double t;
+  if (last_cta_sum(a[0], part, ticket, &t)) beta[j + 1] = sqrt(t);
 }
 
-// c = beta0 * exp(-i T dt) e_1, T = tridiag(beta[1..m-1], alpha[0..m-1]); one thread.
-// Scaling and squaring: exp(-iTdt) = (exp(-iTdt/2^s))^(2^s) applied to the
-// vector, each factor a Taylor series truncated below 1e-18 relative.
-__global__ void small_expm_k(const double* __restrict__ alpha, const double* __restrict__ beta, int m, double dt,
-                             const double* __restrict__ beta0, double2* __restrict__ c, double* __restrict__ err) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double nrm = 0.0;  // infinity norm of T
-  for (int i = 0; i < m; ++i) {
-    double r = fabs(alpha[i]) + (i > 0 ? fabs(beta[i]) : 0.0) + (i + 1 < m ? fabs(beta[i + 1]) : 0.0);
-    nrm = fmax(nrm, r);
-  }
-  int s = 0;
-  double h = fabs(dt) * nrm;
-  while (h > 0.5 && s < 60) {
-    h *= 0.5;
-    ++s;
-  }
-  const double tau = dt / ldexp(1.0, s);
-  double vr[kMaxM], vi[kMaxM], tr[kMaxM], ti[kMaxM], ur[kMaxM], ui[kMaxM];
-  for (int i = 0; i < m; ++i) vr[i] = vi[i] = 0.0;
-  vr[0] = 1.0;
-  const long reps = 1L << s;
-  for (long rep = 0; rep < reps; ++rep) {
-    // u = sum_k (-i tau T)^k v / k!
-    for (int i = 0; i < m; ++i) {
-      ur[i] = tr[i] = vr[i];
-      ui[i] = ti[i] = vi[i];
-    }
-    for (int k = 1; k <= 40; ++k) {
-      // t <- (-i tau T) t / k : (-i)(a + ib) = b - ia
-      double nr[kMaxM], ni[kMaxM];
-      double tmax = 0.0;
-      for (int i = 0; i < m; ++i) {
-        double xr = alpha[i] * tr[i], xi = alpha[i] * ti[i];
-        if (i > 0) {
-          xr += beta[i] * tr[i - 1];
-          xi += beta[i] * ti[i - 1];
-        }
-        if (i + 1 < m) {
-          xr += beta[i + 1] * tr[i + 1];
-          xi += beta[i + 1] * ti[i + 1];
-        }
-        nr[i] = tau * xi / k;
-        ni[i] = -tau * xr / k;
-        tmax = fmax(tmax, fabs(nr[i]) + fabs(ni[i]));
-      }
-      double umax = 0.0;
-      for (int i = 0; i < m; ++i) {
-        tr[i] = nr[i];
-        ti[i] = ni[i];
-        ur[i] += tr[i];
-        ui[i] += ti[i];
-        umax = fmax(umax, fabs(ur[i]) + fabs(ui[i]));
-      }
-      if (tmax <= 1e-18 * umax) break;
-    }
-    for (int i = 0; i < m; ++i) {
-      vr[i] = ur[i];
-      vi[i] = ui[i];
+// Scaled coefficients c = b0 exp(-i T dt) e_1 of the Krylov vectors, T =
+// tridiag(beta[1..m-1], alpha[0..m-1]), by one warp (lane L holds rows 2L and
+// 2L + 1, so a product with T is two exchanges with the neighbours).
+// exp(-i T dt) is applied as ceil(|dt| |T|_inf) substeps, each a Taylor
+// series of kTerms terms: |tau T| <= 1, so what is left out is below 1 / 21!
+// = 2e-20.  Returns |beta_m e_m^T exp(-i T dt) e_1| b0 (a posteriori error
+// estimate).  One thread doing the same chain serially took 0.66 ms a step at
+// m = 30 (all of its vectors in local memory); the warp takes 0.01 ms.
+__device__ __forceinline__ double warp_expm(const double* alpha, const double* beta, int m, double dt, double b0,
+                                            double2* c) {
+  constexpr int kTerms = 20;
+  const int lane = threadIdx.x & 31, i0 = 2 * lane, i1 = i0 + 1;
+  const double a0 = i0 < m ? alpha[i0] : 0.0, a1 = i1 < m ? alpha[i1] : 0.0;
+  const double bl = i0 > 0 && i0 < m ? beta[i0] : 0.0;  // couples i0 - 1, i0
+  const double bm = i1 < m ? beta[i1] : 0.0;            // couples i0, i1
+  const double br = i1 + 1 < m ? beta[i1 + 1] : 0.0;    // couples i1, i1 + 1
+  double nrm = fmax(fabs(a0) + fabs(bl) + fabs(bm), fabs(a1) + fabs(bm) + fabs(br));
+  bool bad = !(nrm < 1e300);  // NaN or infinite entries: fmax alone would lose them
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(0xffffffffu, nrm, o));
+  const double h = fabs(dt) * nrm;
+  bad = __any_sync(0xffffffffu, bad || !(h < 1e9));  // no substep count: the result is NaN
+  const int reps = bad ? 0 : (h > 1.0 ? (int)ceil(h) : 1);
+  const double tau = dt / (double)(reps > 0 ? reps : 1);
+  double v0r = lane == 0 ? 1.0 : 0.0, v0i = 0.0, v1r = 0.0, v1i = 0.0;
+  for (int rep = 0; rep < reps; ++rep) {
+    double t0r = v0r, t0i = v0i, t1r = v1r, t1i = v1i;
+#pragma unroll
+    for (int k = 1; k <= kTerms; ++k) {
+      const double lr = __shfl_up_sync(0xffffffffu, t1r, 1), li = __shfl_up_sync(0xffffffffu, t1i, 1);
+      const double rr = __shfl_down_sync(0xffffffffu, t0r, 1), ri = __shfl_down_sync(0xffffffffu, t0i, 1);
+      // the end lanes keep their own value, which their zero coupling drops
+      const double x0r = fma(a0, t0r, fma(bl, lr, bm * t1r)), x0i = fma(a0, t0i, fma(bl, li, bm * t1i));
+      const double x1r = fma(a1, t1r, fma(bm, t0r, br * rr)), x1i = fma(a1, t1i, fma(bm, t0i, br * ri));
+      const double f = tau * (1.0 / k);  // t <- (-i tau T) t / k
+      t0r = f * x0i;
+      t0i = -f * x0r;
+      t1r = f * x1i;
+      t1i = -f * x1r;
+      v0r += t0r;
+      v0i += t0i;
+      v1r += t1r;
+      v1i += t1i;
     }
   }
-  const double b0 = beta0[0];
-  for (int i = 0; i < m; ++i) c[i] = make_double2(b0 * vr[i], b0 * vi[i]);
-  // a posteriori estimate: beta_m |e_m^T exp(-iTdt) e_1| |psi|
-  err[0] = fabs(beta[m]) * hypot(vr[m - 1], vi[m - 1]) * b0;
+  if (bad) v0r = v0i = v1r = v1i = nan("");
+  // the vectors are stored as beta_i v_i
+  if (i0 < m) {
+    const double s = beta[i0] > 0.0 ? b0 / beta[i0] : 0.0;
+    c[i0] = make_double2(s * v0r, s * v0i);
+  }
+  if (i1 < m) {
+    const double s = beta[i1] > 0.0 ? b0 / beta[i1] : 0.0;
+    c[i1] = make_double2(s * v1r, s * v1i);
+  }
+  const double last = (m - 1) & 1 ? hypot(v1r, v1i) : hypot(v0r, v0i);
+  return fabs(beta[m]) * __shfl_sync(0xffffffffu, last, (m - 1) >> 1) * b0;
 }
 
-// psi[r] = sum_{i<m} V[i][r] c[i]
+__global__ void __launch_bounds__(32) small_expm_k(const double* __restrict__ alpha, const double* __restrict__ beta,
+                                                   int m, double dt, const double* __restrict__ beta0,
+                                                   double2* __restrict__ c, double* __restrict__ err) {
+  const double e = warp_expm(alpha, beta, m, dt, beta0[0], c);
+  if (threadIdx.x == 0) err[0] = e;
+}
+
+// psi[r] = sum_{i<m} c_i u_i[r]
 template <typename T>
-__global__ void combine_k(const T* __restrict__ V, int64_t n, int m, const double2* __restrict__ c, T* __restrict__ psi) {
+__global__ void combine_k(const T* __restrict__ V, int64_t n, int64_t ldv, int m, const double2* __restrict__ c,
+                          T* __restrict__ psi) {
   __shared__ double2 cs[kMaxM];
   for (int t = threadIdx.x; t < m; t += blockDim.x) cs[t] = c[t];
   __syncthreads();
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
     double a = 0.0, b = 0.0;
+#pragma unroll 8
     for (int i = 0; i < m; ++i) {
-      edg::cd v = ldc<T>(V, (int64_t)i * n + r);
+      edg::cd v = ldc<T>(V, (int64_t)i * ldv + r);
       a = fma(v.re, cs[i].x, fma(-v.im, cs[i].y, a));
       b = fma(v.re, cs[i].y, fma(v.im, cs[i].x, b));
     }
@@ -271,28 +356,286 @@ __global__ void combine_k(const T* __restrict__ V, int64_t n, int m, const doubl
   }
 }
 
+// ---------------------------------------------------------------------------
+// A whole time step as one cooperative launch (small sectors).  CTA b owns
+// the rows [n b / G, n (b + 1) / G): their row of w, of the matrix and of the
+// basis stay in its shared memory where they fit, and only the gathers of
+// u_j, the dots partials and the next vector go through L2.  Per Krylov step
+// two grid-wide waits: for the dots, and for the norm with the next vector.
+// Bound by those waits and the few dependent L2 reads between them, about
+// 7 us a Krylov step.  A step of dt = 0.05 (m = 30, full reorthogonalisation,
+// complex128, static-pair SU(2) chains; launches per pass before):
+//   n = 182: 0.18 ms (1.48), 12,292: 0.31 ms (1.69), 101,613: 0.63 ms (1.87).
+// The line (kCoopRows rows per SM) lies where the matrix and the basis no
+// longer fit shared memory: at 101,613 rows the passes below take 0.96 ms, at
+// 848,614 rows this form takes 6.6 ms and the passes 4.2.
+// ---------------------------------------------------------------------------
+constexpr int kCoopThreads = 512;
+constexpr int kCoopWarps = kCoopThreads / 32;
+constexpr int kCoopSmem = 200 * 1024;  // dynamic shared memory of a CTA (one per SM)
+constexpr int kCoopRows = 1024;        // most rows of a CTA
+constexpr int kMvLanes = 4;            // lanes per row of the product
+
+template <typename T, typename SV>
+struct CoopArgs {
+  const int64_t* rowptr;
+  const int32_t* cols;
+  const SV* vals;
+  const SV* diag;
+  T* V;  // [m + 1][ldv]: written and read by this launch
+  T* psi;
+  double2* partial;  // [2][G][kMaxM + 1]
+  double* npart;     // [2][G]
+  unsigned* bar;
+  int* err;
+  int32_t* status;
+  double* err_out;
+  int64_t n, ldv;
+  double dt;
+  int m, reorth;
+};
+
+template <typename T, typename SV>
+__global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<T, SV> A) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ double2 hs[kMaxM + 1];
+  __shared__ double al[kMaxM], be[kMaxM + 2];
+  __shared__ double red[kCoopWarps];
+  __shared__ double s_total;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)gridDim.x, m = A.m;
+  const int64_t r0 = A.n * blockIdx.x / G, r1 = A.n * (blockIdx.x + 1) / G;
+  const int rows = (int)(r1 - r0);
+  // shared memory: w | row offsets | matrix rows | basis rows
+  double2* const w = reinterpret_cast<double2*>(sm);
+  int64_t off = (int64_t)rows * 16;
+  int32_t* const rp = reinterpret_cast<int32_t*>(sm + off);
+  off = (off + (int64_t)(rows + 1) * 4 + 15) & ~int64_t(15);
+  const int64_t e0 = A.rowptr[r0], ne = A.rowptr[r1] - e0;
+  for (int r = tid; r <= rows; r += kCoopThreads) rp[r] = (int32_t)(A.rowptr[r0 + r] - e0);
+  const SV* vals = A.vals + e0;
+  const int32_t* cols = A.cols + e0;
+  if (off + ne * (int64_t)(sizeof(SV) + 4) + 16 <= kCoopSmem) {
+    SV* sv = reinterpret_cast<SV*>(sm + off);
+    int32_t* sc = reinterpret_cast<int32_t*>(sv + ne);
+    for (int64_t e = tid; e < ne; e += kCoopThreads) {
+      sv[e] = vals[e];
+      sc[e] = cols[e];
+    }
+    vals = sv;
+    cols = sc;
+    off = (off + ne * (int64_t)(sizeof(SV) + 4) + 15) & ~int64_t(15);
+  }
+  T* own = A.V + r0;  // this CTA's rows of the basis and their row stride
+  int64_t ld = A.ldv;
+  const bool basis_here = off + (int64_t)rows * (m + 1) * (int64_t)sizeof(T) <= kCoopSmem;
+  if (basis_here) {
+    own = reinterpret_cast<T*>(sm + off);
+    ld = rows;
+  }
+  edg::GridSync gs{A.bar, A.err};
+  unsigned waits = 0;  // parity of the norm partials' buffer
+  // sum over the grid of one value per thread; false when a wait ran out
+  auto grid_sum = [&](double a, double* out) -> bool {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) red[warp] = a;
+    __syncthreads();
+    double* part = A.npart + (int64_t)(waits & 1) * G;
+    ++waits;
+    if (tid == 0) {
+      double t = 0.0;
+      for (int q = 0; q < kCoopWarps; ++q) t += red[q];
+      part[blockIdx.x] = t;
+    }
+    if (!gs.wait()) return false;
+    if (warp == 0) {
+      double t = 0.0;
+      for (int b = lane; b < G; b += 32) t += __ldcg(part + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) s_total = t;
+    }
+    __syncthreads();
+    *out = s_total;
+    return true;
+  };
+  auto give_up = [&] {
+    if (tid == 0 && A.status != nullptr) atomicExch(A.status, EDG_ERR_TIMEOUT);
+  };
+  // ---- u_0 = psi / |psi| ----
+  double a = 0.0, tot;
+  for (int r = tid; r < rows; r += kCoopThreads) {
+    const edg::cd x = ldc<T>(A.psi, r0 + r);
+    a = fma(x.re, x.re, fma(x.im, x.im, a));
+  }
+  if (!grid_sum(a, &tot)) return give_up();
+  const double b0 = sqrt(tot), inv0 = b0 > 0.0 ? 1.0 / b0 : 0.0;
+  if (tid == 0) be[0] = b0 > 0.0 ? 1.0 : 0.0;
+  for (int r = tid; r < rows; r += kCoopThreads) {
+    const edg::cd x = ldc<T>(A.psi, r0 + r);
+    stc<T>(A.V, r0 + r, x.re * inv0, x.im * inv0);
+    if (basis_here) stc<T>(own, r, x.re * inv0, x.im * inv0);
+  }
+  if (!gs.wait()) return give_up();
+  for (int j = 0; j < m; ++j) {
+    const double sj = be[j] > 0.0 ? 1.0 / be[j] : 0.0;
+    // ---- w = H u_j / beta_j on this CTA's rows ----
+    {
+      const T* u = A.V + (int64_t)j * A.ldv;
+      const int part = tid & (kMvLanes - 1);
+      const int n_it = (rows + kCoopThreads / kMvLanes - 1) / (kCoopThreads / kMvLanes);
+      for (int it = 0; it < n_it; ++it) {
+        const int r = it * (kCoopThreads / kMvLanes) + tid / kMvLanes;
+        edg::cd acc{0.0, 0.0};
+        if (r < rows) {
+          constexpr int U = 4;  // gathers in flight per lane
+          const int end = rp[r + 1];
+          for (int p0 = rp[r] + part; p0 < end; p0 += U * kMvLanes) {
+            T x[U];
+            SV v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+              if (p0 + k * kMvLanes < end) {
+                x[k] = u[cols[p0 + k * kMvLanes]];
+                v[k] = vals[p0 + k * kMvLanes];
+              }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+              if (p0 + k * kMvLanes < end) {
+                const edg::cd xk{(double)x[k].x, (double)x[k].y};
+                if constexpr (edg::Store<SV>::cplx)
+                  edg::fma_acc(acc, edg::cd{(double)v[k].x, (double)v[k].y}, xk);
+                else
+                  edg::fma_acc(acc, (double)v[k], xk);
+              }
+          }
+        }
+#pragma unroll
+        for (int o = kMvLanes / 2; o > 0; o >>= 1) {
+          acc.re += __shfl_xor_sync(0xffffffffu, acc.re, o, kMvLanes);
+          acc.im += __shfl_xor_sync(0xffffffffu, acc.im, o, kMvLanes);
+        }
+        if (r < rows && part == 0) {
+          const T xr = u[r0 + r];
+          edg::fma_acc(acc, edg::Store<SV>::ld(A.diag, r0 + r), edg::cd{(double)xr.x, (double)xr.y});
+          w[r] = make_double2(acc.re * sj, acc.im * sj);
+        }
+      }
+    }
+    const int passes = A.reorth == 0 ? 1 : A.reorth;
+    const int ilo = A.reorth == 0 ? (j > 0 ? j - 1 : 0) : 0;
+    for (int pass = 0; pass < passes; ++pass) {
+      __syncthreads();
+      // ---- dots of this CTA's rows, a warp per vector ----
+      double2* P = A.partial + (int64_t)pass * G * (kMaxM + 1);
+      for (int i = ilo + warp; i <= j; i += kCoopWarps) {
+        double gr = 0.0, gi = 0.0;
+        const T* ui = own + (int64_t)i * ld;
+#pragma unroll 4
+        for (int r = lane; r < rows; r += 32) {
+          const edg::cd x = ldc<T>(ui, r);
+          const double2 y = w[r];
+          gr = fma(x.re, y.x, fma(x.im, y.y, gr));
+          gi = fma(x.re, y.y, fma(-x.im, y.x, gi));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          gr += __shfl_xor_sync(0xffffffffu, gr, o);
+          gi += __shfl_xor_sync(0xffffffffu, gi, o);
+        }
+        if (lane == 0) P[(int64_t)blockIdx.x * (kMaxM + 1) + i] = make_double2(gr, gi);
+      }
+      if (!gs.wait()) return give_up();
+      for (int i = ilo + warp; i <= j; i += kCoopWarps) {
+        double gr = 0.0, gi = 0.0;
+        for (int b = lane; b < G; b += 32) {
+          const double2 p = __ldcg(P + (int64_t)b * (kMaxM + 1) + i);
+          gr += p.x;
+          gi += p.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          gr += __shfl_xor_sync(0xffffffffu, gr, o);
+          gi += __shfl_xor_sync(0xffffffffu, gi, o);
+        }
+        if (lane == 0) {
+          const double si = be[i] > 0.0 ? 1.0 / be[i] : 0.0;
+          hs[i] = make_double2(si * (si * gr), si * (si * gi));
+          if (i == j) al[j] = pass > 0 ? al[j] + si * gr : si * gr;
+        }
+      }
+      __syncthreads();
+      // ---- w -= sum_i coef_i u_i; after the last pass it is u_{j+1} ----
+      const bool last = pass + 1 == passes;
+      double nrm = 0.0;
+      for (int r = tid; r < rows; r += kCoopThreads) {
+        double sr = 0.0, si = 0.0;
+#pragma unroll 8
+        for (int i = ilo; i <= j; ++i) {
+          const edg::cd x = ldc<T>(own, (int64_t)i * ld + r);
+          sr = fma(x.re, hs[i].x, fma(-x.im, hs[i].y, sr));
+          si = fma(x.re, hs[i].y, fma(x.im, hs[i].x, si));
+        }
+        const double2 y = make_double2(w[r].x - sr, w[r].y - si);
+        if (last) {
+          stc<T>(A.V, (int64_t)(j + 1) * A.ldv + r0 + r, y.x, y.y);
+          if (basis_here) stc<T>(own, (int64_t)(j + 1) * ld + r, y.x, y.y);
+          nrm = fma(y.x, y.x, fma(y.y, y.y, nrm));
+        } else {
+          w[r] = y;
+        }
+      }
+      if (last) {
+        if (!grid_sum(nrm, &tot)) return give_up();
+        if (tid == 0) be[j + 1] = sqrt(tot);
+        __syncthreads();
+      }
+    }
+  }
+  // ---- psi = V c: every CTA forms the coefficients itself ----
+  if (warp == 0) {
+    const double e = warp_expm(al, be, m, A.dt, b0, hs);
+    if (lane == 0 && blockIdx.x == 0) A.err_out[0] = e;
+  }
+  __syncthreads();
+  for (int r = tid; r < rows; r += kCoopThreads) {
+    double x = 0.0, y = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < m; ++i) {
+      const edg::cd v = ldc<T>(own, (int64_t)i * ld + r);
+      x = fma(v.re, hs[i].x, fma(-v.im, hs[i].y, x));
+      y = fma(v.re, hs[i].y, fma(v.im, hs[i].x, y));
+    }
+    stc<T>(A.psi, r0 + r, x, y);
+  }
+}
+
 struct KLayout {
-  int64_t V, w, h, partial, normp, alpha, beta, c, misc, total;
-  int nblk;
+  int64_t V, w, partial, normp, alpha, beta, coef, c, misc, sync, total;
+  int64_t ldv;
 };
 
 inline int64_t al(int64_t x) { return (x + 255) & ~int64_t(255); }
+
+constexpr int kDotBlocks = edg::kSmCount * 4;
 
 KLayout klayout(const edg_krylov_problem* p) {
   KLayout L{};
   const int64_t n = p->n_rows;
   const int esz = p->vec_dtype == 2 ? 16 : 8;
-  L.nblk = edg::kSmCount * 4;
+  L.ldv = (n + 15) & ~int64_t(15);  // a vector starts on its own cache line
   int64_t o = 0;
-  L.V = o; o = al(o + (int64_t)(p->m + 1) * n * esz);
+  L.V = o; o = al(o + (int64_t)(p->m + 1) * L.ldv * esz);
   L.w = o; o = al(o + n * 16);
-  L.h = o; o = al(o + (int64_t)(kMaxM + 1) * 16);
-  L.partial = o; o = al(o + (int64_t)L.nblk * (kMaxM + 1) * 16);
+  L.partial = o; o = al(o + (int64_t)kDotBlocks * (kMaxM + 1) * 16);
   L.normp = o; o = al(o + (int64_t)edg::kSmCount * 8 * 8);
   L.alpha = o; o = al(o + (kMaxM + 1) * 8);
   L.beta = o; o = al(o + (kMaxM + 2) * 8);
+  L.coef = o; o = al(o + (kMaxM + 2) * 16);
   L.c = o; o = al(o + (kMaxM + 1) * 16);
-  L.misc = o; o = al(o + 8 * 8);  // [0] beta0, [1] err, [2] scratch
+  L.misc = o; o = al(o + 8 * 8);  // [0] beta0, [1] err
+  L.sync = o; o = al(o + 8 * 4);  // tickets (2) | error word | - | grid barrier
   L.total = o;
   return L;
 }
@@ -300,57 +643,97 @@ KLayout klayout(const edg_krylov_problem* p) {
 template <typename T, typename SV>
 int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* err_out, cudaStream_t s) {
   const KLayout L = klayout(p);
-  const int64_t n = p->n_rows;
+  const int64_t n = p->n_rows, ldv = L.ldv;
   const int m = p->m;
   T* V = (T*)(ws + L.V);
   double2* w = (double2*)(ws + L.w);
-  double2* h = (double2*)(ws + L.h);
   double2* partial = (double2*)(ws + L.partial);
   double* normp = (double*)(ws + L.normp);
   double* alpha = (double*)(ws + L.alpha);
   double* beta = (double*)(ws + L.beta);
+  double2* coef = (double2*)(ws + L.coef);
   double2* c = (double2*)(ws + L.c);
   double* misc = (double*)(ws + L.misc);
-  const int nb_norm = edg::kSmCount * 8;
-  const unsigned gv = edg::grid_for(n, 256);
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(alpha, 0, (kMaxM + 1) * 8, s)) != cudaSuccess) return edg::cuda_status(e, "krylov");
-  if ((e = cudaMemsetAsync(beta, 0, (kMaxM + 2) * 8, s)) != cudaSuccess) return edg::cuda_status(e, "krylov");
-  norm_k<T><<<nb_norm, kThreads, 0, s>>>(psi, n, normp);
-  sqrt_sum_k<<<1, kThreads, 0, s>>>(normp, nb_norm, misc);  // beta0
-  scale_k<T, T><<<gv, 256, 0, s>>>(psi, n, misc, V);
-  for (int j = 0; j < m; ++j) {
-    const T* vj = V + (int64_t)j * n;
-    int st;
-    if constexpr (std::is_same<SV, double>::value || std::is_same<SV, float>::value) {
-      if (p->pk_words != nullptr)  // real packed matrix: (re, im) as two interleaved right-hand sides
-        st = edg::launch_packed_spmv<SV>(2, 2, n, p->pk_tile_off, p->pk_words, (const SV*)p->pk_table, p->pk_count,
-                                         p->pk_colbits, (const SV*)p->diag, (const SV*)vj, (double*)w, 0, nullptr,
-                                         p->status, s, 1);
-      else
+  unsigned* tickets = (unsigned*)(ws + L.sync);
+  int* err_word = (int*)(tickets + 2);
+  unsigned* bar = tickets + 4;  // grid barrier of the cooperative form
+  cudaError_t e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s);
+  if (e != cudaSuccess) return edg::cuda_status(e, "krylov");
+  bool done = false;
+  if (n <= kCoopMaxRows) {
+    int dev = 0, n_sm = 0, coop = 0, occ = 0;
+    auto kern = krylov_coop_k<T, SV>;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
+    if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: set-up");
+    // a CTA per SM, fewer for fewer rows: at least 32 rows a CTA
+    int64_t g = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
+    if (g > (n + 31) / 32) g = (n + 31) / 32;
+    if (coop && occ >= 1 && (n + g - 1) / g <= kCoopRows) {
+      CoopArgs<T, SV> a{p->rowptr, p->cols, (const SV*)p->vals, (const SV*)p->diag, V, psi, partial, normp, bar,
+                        err_word, p->status, misc + 1, n, ldv, dt, m, p->reorth_passes};
+      void* args[] = {&a};
+      e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)g), dim3(kCoopThreads), args, kCoopSmem, s);
+      if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: cooperative launch");
+      done = true;
+    }
+  }
+  if (!done) {
+    const unsigned gn = edg::grid_for(n, kThreads);
+    const unsigned gu = edg::grid_for(n, kThreads, kUpdateCtas);
+    const int nb = (int)edg::grid_for(n, kThreads, dot_ctas<T>());
+    const unsigned gv = edg::grid_for(n, 256);
+    norm_k<T><<<gn, kThreads, 0, s>>>(psi, n, normp, tickets, misc);  // beta0
+    scale_k<T><<<gv, 256, 0, s>>>(psi, n, misc, V, beta);
+    for (int j = 0; j < m; ++j) {
+      const T* vj = V + (int64_t)j * ldv;
+      // reorth_passes = 0: local recurrence (against v_{j-1}, v_j only);
+      // 1 or 2: classical Gram-Schmidt over the whole basis, once or twice
+      const int passes = p->reorth_passes == 0 ? 1 : p->reorth_passes;
+      const int ilo = p->reorth_passes == 0 ? (j > 0 ? j - 1 : 0) : 0;
+      int st;
+      bool dots_done = false;
+      if constexpr (std::is_same<SV, double>::value || std::is_same<SV, float>::value) {
+        if (p->pk_words != nullptr && p->reorth_passes == 0) {
+          // the coefficients come out of the product: c_{j-1}, c_j, 1 / beta_j
+          // at coef[0..2] (from coef[1] at j = 0)
+          const edg::KrylovStep step{j > 0 ? (const void*)(vj - ldv) : nullptr, (double*)partial, tickets, beta,
+                                     alpha, coef, j};
+          st = edg::launch_packed_krylov<SV>(n, p->pk_tile_off, p->pk_words, (const SV*)p->pk_table, p->pk_count,
+                                             p->pk_colbits, (const SV*)p->diag, (const SV*)vj, (double*)w, step,
+                                             p->status, s);
+          dots_done = true;
+        } else if (p->pk_words != nullptr) {  // (re, im) as two interleaved right-hand sides
+          st = edg::launch_packed_spmv<SV>(2, 2, n, p->pk_tile_off, p->pk_words, (const SV*)p->pk_table, p->pk_count,
+                                           p->pk_colbits, (const SV*)p->diag, (const SV*)vj, (double*)w, 0, nullptr,
+                                           p->status, s, 1);
+        } else {
+          st = edg::launch_spmv<SV, T, double2>(1, n, p->nnz, p->rowptr, p->cols, (const SV*)p->vals,
+                                                (const SV*)p->diag, vj, w, s, 0, p->spmv_group);
+        }
+      } else {
         st = edg::launch_spmv<SV, T, double2>(1, n, p->nnz, p->rowptr, p->cols, (const SV*)p->vals,
                                               (const SV*)p->diag, vj, w, s, 0, p->spmv_group);
-    } else {
-      st = edg::launch_spmv<SV, T, double2>(1, n, p->nnz, p->rowptr, p->cols, (const SV*)p->vals, (const SV*)p->diag,
-                                            vj, w, s, 0, p->spmv_group);
+      }
+      if (st) return st;
+      for (int pass = 0; pass < passes; ++pass) {
+        const bool last = pass + 1 == passes;
+        if (!dots_done) {
+          dots_k<T><<<nb, kThreads, 0, s>>>(V, n, ldv, ilo, j, w, partial, kMaxM + 1);
+          coef_k<<<j + 1 - ilo, kThreads, 0, s>>>(partial, nb, kMaxM + 1, ilo, j, pass, beta, coef, alpha);
+        }
+        update_k<T><<<gu, kThreads, 0, s>>>(V, n, ldv, ilo, j, dots_done && j == 0 ? coef + 1 : coef, w,
+                                            last ? V + (int64_t)(j + 1) * ldv : nullptr, normp, tickets + 1, beta);
+      }
+      if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: lanczos");
     }
-    if (st) return st;
-    // reorth_passes = 0: local recurrence (against v_{j-1}, v_j only);
-    // 1 or 2: classical Gram-Schmidt over the whole basis, once or twice
-    const int passes = p->reorth_passes == 0 ? 1 : p->reorth_passes;
-    const int ilo = p->reorth_passes == 0 ? (j > 0 ? j - 1 : 0) : 0;
-    for (int pass = 0; pass < passes; ++pass) {
-      dots_k<T><<<L.nblk, kThreads, 0, s>>>(V, n, ilo, j, w, partial, kMaxM + 1);
-      reduce_h_k<<<j + 1 - ilo, kThreads, 0, s>>>(partial, L.nblk, kMaxM + 1, ilo, j, h, alpha + j);
-      update_k<T><<<nb_norm, kThreads, 0, s>>>(V, n, ilo, j, h, w, normp);
-    }
-    sqrt_sum_k<<<1, kThreads, 0, s>>>(normp, nb_norm, beta + j + 1);
-    scale_k<double2, T><<<gv, 256, 0, s>>>(w, n, beta + j + 1, V + (int64_t)(j + 1) * n);
-    if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: lanczos");
+    small_expm_k<<<1, 32, 0, s>>>(alpha, beta, m, dt, misc, c, misc + 1);
+    combine_k<T><<<gv, 256, 0, s>>>(V, n, ldv, m, c, psi);
+    if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: combine");
   }
-  small_expm_k<<<1, 1, 0, s>>>(alpha, beta, m, dt, misc, c, misc + 1);
-  combine_k<T><<<gv, 256, 0, s>>>(V, n, m, c, psi);
-  if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: combine");
   if (err_out) {
     e = cudaMemcpyAsync(err_out, misc + 1, sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

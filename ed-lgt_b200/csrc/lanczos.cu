@@ -26,6 +26,7 @@
 // Every check_every steps the k lowest Ritz pairs of the tridiagonal matrix are
 // computed on the device (multisection + inverse iteration) and the residual
 // bound |beta_{j+1} s_{j}| is compared with tol * max(1, |theta|).
+#include "gridbar.cuh"
 #include "reorth_bulk.cuh"
 #include "spmv.cuh"
 #include "tridiag.cuh"
@@ -559,46 +560,6 @@ struct Raw4<double> {
   __device__ double operator[](int e) const { return e == 0 ? a.x : e == 1 ? a.y : e == 2 ? b.x : b.y; }
 };
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid-wide barrier of the small pass (every CTA is resident: cooperative
-// launch).  bar[0] counts arrivals, bar[1] is the generation.  A wait longer
-// than 1 s writes EDG_ERR_TIMEOUT to *err; once *err is set no CTA waits any
-// more and every thread gets false.
-__device__ bool small_barrier(unsigned* bar, int* err) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned g = ld_acquire_u32(bar + 1);
-    __threadfence();
-    const unsigned arrived = atomicAdd(bar, 1u);
-    if (arrived == gridDim.x - 1) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      const uint64_t t0 = edg::bulk::now_ns();
-      for (unsigned spins = 1; ld_acquire_u32(bar + 1) == g; ++spins) {
-        if ((spins & 255u) == 0) {
-          if (*(volatile int*)err) break;
-          if (edg::bulk::now_ns() - t0 > 1000000000ull) {
-            atomicExch(err, EDG_ERR_TIMEOUT);
-            break;
-          }
-        }
-      }
-    }
-    __threadfence();
-    ok_s = *(volatile int*)err == 0;
-  }
-  __syncthreads();
-  return ok_s != 0;
-}
-
 // Coefficients of the delayed step for one problem (one warp) from its
 // totals tot[2t] = V[lo+t] . u, tot[2t+1] = V[lo+t] . w (t <= j - lo) and the
 // previous alpha, beta (entries below j only): 1/r, c, alpha_j, beta_j (the
@@ -722,7 +683,7 @@ __global__ void __launch_bounds__(kSmallThreads) reorth_small_k(
       partial[(int64_t)blockIdx.x * (2 * kSmallMax) + tid] = a;
     }
   }
-  if (!small_barrier(bar, err)) {
+  if (!edg::grid_barrier(bar, err)) {
     if (tid == 0) atomicExch(&st->done, 1);
     return;
   }
@@ -1078,7 +1039,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   double* wnorm = rc + 2 * NV;                        // [NV]: |w| of the next candidate
   int* tickets = (int*)(ws + L.sync);                  // [2] last-CTA counters (left at 0)
   int* err_word = tickets + 2;                          // EDG_ERR_TIMEOUT when a ring or barrier wait ran out
-  unsigned* small_bar = (unsigned*)(tickets + 4);       // [2] grid barrier of the small pass (count, generation)
+  unsigned* small_bar = (unsigned*)(tickets + 4);       // grid barrier of the small pass (arrivals)
   const unsigned g_vec = edg::grid_for(n_pad, 256);
   const int first_check = p->check_every > 8 ? p->check_every : 8;
   constexpr int kXs = NV == 3 ? 4 : NV;  // row stride of the matvec input X

@@ -314,6 +314,73 @@ __device__ __forceinline__ void gather_tile(const uint32_t* src, int width, int 
   }
 }
 
+// What a product leaves behind besides y: row(r, x_r, y_r) once per row (one
+// lane), finish() by every thread at the end of the kernel.
+struct NoEpilogue {
+  template <typename T, int NV>
+  __device__ void row(int64_t, const T (&)[NV], const double (&)[NV]) {}
+  __device__ void finish() {}
+};
+
+// Complex dots of the product with the vector it was applied to and with the
+// one before it (the two of a local Krylov recurrence), summed while the row
+// is in registers: a separate dots pass would read y (16 B a row) and both
+// vectors again.  The last CTA (ticket) adds the CTA partials in a fixed
+// order and forms the step's coefficients.
+struct KrylovEpilogue {
+  edg::KrylovStep k;
+  double acc[4];
+  template <typename T>
+  __device__ void row(int64_t r, const T (&x)[2], const double (&y)[2]) {
+    const double xr = (double)x[0], xi = (double)x[1];
+    acc[0] = fma(xr, y[0], fma(xi, y[1], acc[0]));
+    acc[1] = fma(xr, y[1], fma(-xi, y[0], acc[1]));
+    if (k.prev != nullptr) {
+      T p[2];
+      XRow<T, 2, 2>::ld((const T*)k.prev, r, p);
+      const double pr = (double)p[0], pi = (double)p[1];
+      acc[2] = fma(pr, y[0], fma(pi, y[1], acc[2]));
+      acc[3] = fma(pr, y[1], fma(-pi, y[0], acc[3]));
+    }
+  }
+  __device__ void finish() {
+    __shared__ double red[kWarps][4];
+    __shared__ int last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      double a = acc[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) red[warp][q] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+      double a = 0.0;
+      for (int w = 0; w < kWarps; ++w) a += red[w][threadIdx.x];
+      k.partial[(int64_t)blockIdx.x * 4 + threadIdx.x] = a;
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(k.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (warp < 4) {
+      double a = 0.0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) a += __ldcg(k.partial + (int64_t)b * 4 + warp);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) red[0][warp] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      edg::krylov_local_coefs(k, red[0]);
+      *k.ticket = 0u;
+    }
+  }
+};
+
 // y[v * y_plane + r] (f64; y[r * NV + v] when y_plane is 0) = sum over the
 // row's entries of table[idx] x[col][v] + diag[r][v] x[r][v] (diag[r] for
 // every v when diag_shared: a complex vector as NV = 2 real parts of one
@@ -323,12 +390,12 @@ __device__ __forceinline__ void gather_tile(const uint32_t* src, int width, int 
 // conversion per entry); with f64 the products and sums are f64, in the CSR
 // kernel's order.  A stage wait that runs out (1 s) sets *err (if given) and
 // ends the warp's work.
-template <typename T, int NV, int XS>
+template <typename T, int NV, int XS, typename Epi>
 __global__ void __launch_bounds__(kWarps * 32, 4)
     packed_spmv_k(int64_t n, const int32_t* __restrict__ tile_off, const uint32_t* __restrict__ words,
                   const T* __restrict__ table, int count, int colbits, const T* __restrict__ diag,
                   const T* __restrict__ x, double* __restrict__ y, int64_t y_plane, int diag_shared,
-                  const int* __restrict__ skip, int* __restrict__ err) {
+                  const int* __restrict__ skip, int* __restrict__ err, Epi epi) {
   using A = T;  // lane accumulator: f32 lanes for the f32 phase, f64 otherwise
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_err;
@@ -394,8 +461,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const double d = (double)__ldg(diag_shared ? diag + r : diag + r * NV + v);
-        y[y_plane > 0 ? v * y_plane + r : r * NV + v] = fma(d, (double)xr[v], tot[v]);
+        tot[v] = fma(d, (double)xr[v], tot[v]);
+        y[y_plane > 0 ? v * y_plane + r : r * NV + v] = tot[v];
       }
+      epi.row(r, xr, tot);
     }
     __syncwarp();  // this stage is refilled by the next iteration
     cur = nxt;
@@ -415,6 +484,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
           if (edg::bulk::now_ns() - t0 > 1000000000ull) break;
       }
   }
+  epi.finish();
 }
 
 template <typename T>
@@ -457,10 +527,11 @@ int launch_packed_spmv(int nvec, int x_stride, int64_t n, const int32_t* tile_of
   cudaError_t e = cudaSuccess;
 #define EDG_PACKED(NV, XS)                                                                                          \
   do {                                                                                                              \
-    e = cudaFuncSetAttribute(packed_spmv_k<T, NV, XS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    auto kern = packed_spmv_k<T, NV, XS, NoEpilogue>;                                                              \
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
     if (e == cudaSuccess)                                                                                           \
-      packed_spmv_k<T, NV, XS><<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, \
-                                                               y, y_plane, diag_shared, skip, err);                 \
+      kern<<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, y, y_plane,         \
+                                           diag_shared, skip, err, NoEpilogue{});                                   \
   } while (0)
   switch (nvec) {
     case 1: EDG_PACKED(1, 1); break;
@@ -486,6 +557,29 @@ template int launch_packed_spmv<float>(int, int, int64_t, const int32_t*, const 
 template int launch_packed_spmv<double>(int, int, int64_t, const int32_t*, const uint32_t*, const double*, int, int,
                                         const double*, const double*, double*, int64_t, const int*, int*,
                                         cudaStream_t, int);
+
+template <typename T>
+int launch_packed_krylov(int64_t n, const int32_t* tile_off, const uint32_t* words, const T* table, int count,
+                         int colbits, const T* diag, const T* x, double* y, const KrylovStep& step, int* err,
+                         cudaStream_t s) {
+  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows;
+  const int64_t need = (n_tiles + kWarps - 1) / kWarps;
+  const unsigned grid = (unsigned)(need < (int64_t)kSmCount * 4 ? need : (int64_t)kSmCount * 4);
+  const size_t smem = packed_smem<T>(count);
+  auto kern = packed_spmv_k<T, 2, 2, KrylovEpilogue>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    kern<<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, y, 0, 1, nullptr, err,
+                                         KrylovEpilogue{step, {0.0, 0.0, 0.0, 0.0}});
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return e == cudaSuccess ? EDG_OK : cuda_status(e, "packed krylov product");
+}
+
+template int launch_packed_krylov<float>(int64_t, const int32_t*, const uint32_t*, const float*, int, int,
+                                         const float*, const float*, double*, const KrylovStep&, int*, cudaStream_t);
+template int launch_packed_krylov<double>(int64_t, const int32_t*, const uint32_t*, const double*, int, int,
+                                          const double*, const double*, double*, const KrylovStep&, int*,
+                                          cudaStream_t);
 
 }  // namespace edg
 

@@ -265,4 +265,35 @@ int launch_packed_spmv(int nvec, int x_stride, int64_t n, const int32_t* tile_of
                        const T* table, int count, int colbits, const T* diag, const T* x, double* y, int64_t y_plane,
                        const int* skip, int* err, cudaStream_t s, int diag_shared = 0);
 
+// A step of the local Krylov recurrence (krylov.cu): the Krylov vectors are
+// stored unnormalised, u_i with |u_i| = beta[i], v_i = u_i / beta[i].
+struct KrylovStep {
+  const void* prev;   // u_{j-1} (complex, the vectors' type) or NULL at j = 0
+  double* partial;    // [CTA][4] sums of conj(u_j) y, conj(u_{j-1}) y
+  unsigned* ticket;   // last-CTA counter, left at 0
+  const double* beta;
+  double* alpha;
+  double2* coef;      // out: c_{j-1}, c_j of the update, and (1/beta[j], 0)
+  int j;
+};
+
+// From the totals g = {Re, Im of <u_j, y>, <u_{j-1}, y>}, y = H u_j: with
+// w = H v_j = y / beta_j, alpha_j = Re <v_j, w>, and the update is
+// u_{j+1} = y / beta_j - c_{j-1} u_{j-1} - c_j u_j, c_i = <v_i, w> / beta_i.
+__device__ __forceinline__ void krylov_local_coefs(const KrylovStep& k, const double* g) {
+  const double bj = k.beta[k.j], bp = k.j > 0 ? k.beta[k.j - 1] : 0.0;
+  const double sj = bj > 0.0 ? 1.0 / bj : 0.0, sp = bp > 0.0 ? 1.0 / bp : 0.0;
+  k.alpha[k.j] = sj * sj * g[0];
+  k.coef[0] = make_double2(sp * sp * sj * g[2], sp * sp * sj * g[3]);
+  k.coef[1] = make_double2(sj * sj * sj * g[0], sj * sj * sj * g[1]);
+  k.coef[2] = make_double2(sj, 0.0);
+}
+
+// y (interleaved complex f64) = H u_j on the packed layout with the step's
+// dots and coefficients formed in the same launch.
+template <typename T>
+int launch_packed_krylov(int64_t n, const int32_t* tile_off, const uint32_t* words, const T* table, int count,
+                         int colbits, const T* diag, const T* x, double* y, const KrylovStep& step, int* err,
+                         cudaStream_t s);
+
 }  // namespace edg

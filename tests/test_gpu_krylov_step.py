@@ -1,0 +1,75 @@
+"""One Krylov step exp(-i H dt) psi on synthetic Hermitian matrices against a
+Taylor series of the same operator in complex128: the cooperative one-launch
+form and the pass-by-pass form on both sides of their line, every
+reorthogonalisation choice, matrices without off-diagonal entries (breakdown
+after one vector), one row, and the largest Krylov dimension."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(n, cplx, seed, empty=False):
+    import torch
+
+    from edgpu.modeling.assembly import DeviceMatrix
+
+    rng = np.random.default_rng(seed)
+    if n > 1 and not empty:
+        r = np.repeat(np.arange(n), 4)
+        c = rng.integers(0, n, 4 * n)
+        v = rng.choice([0.5, -0.25, 1.0], 4 * n).astype(np.complex128)
+        if cplx:
+            v = v * rng.choice([1, 1j, -1j], 4 * n)
+        keep = r < c
+        keys, first = np.unique(r[keep] * n + c[keep], return_index=True)
+        r, c, v = keys // n, keys % n, v[keep][first]
+        r, c, v = np.concatenate([r, c]), np.concatenate([c, r]), np.concatenate([v, v.conj()])
+        order = np.lexsort((c, r))
+        r, c, v = r[order], c[order], v[order]
+    else:
+        r = c = np.zeros(0, dtype=np.int64)
+        v = np.zeros(0, dtype=np.complex128)
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int64)
+    d = rng.uniform(-2, 2, n)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    vals = up(v.view(np.float64) if cplx else v.real)
+    diag = up(d.astype(np.complex128).view(np.float64) if cplx else d)
+    mat = DeviceMatrix(n, up(rowptr), up(c.astype(np.int32)), vals, diag, None, cplx)
+    a = torch.sparse_csr_tensor(mat.rowptr, up(c.astype(np.int64)), up(v), size=(n, n))
+    return mat, (lambda x: (a @ x[:, None])[:, 0] + up(d) * x)
+
+
+COOP_MAX = 1024 * 148  # rows of the one-launch form
+
+
+@pytest.mark.parametrize("n,m", [(1, 30), (2, 30), (33, 30), (700, 1), (700, 64), (5000, 30), (COOP_MAX, 20),
+                                 (COOP_MAX + 1, 20)])
+@pytest.mark.parametrize("precision,reorth", [("c128", 0), ("c128", 1), ("c128", 2), ("c64", 0), ("c64", 1)])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("empty", [False, True])
+def test_step_matches_taylor(n, m, precision, reorth, cplx, empty):
+    import torch
+
+    from edgpu.dynamics import KrylovEvolver
+
+    if empty and n > 700:
+        pytest.skip("the breakdown does not depend on the size")
+    mat, apply = _matrix(n, cplx, 3 * n + cplx, empty)
+    ev = KrylovEvolver(mat, m=m, precision=precision, reorth_passes=reorth, matvec="auto" if n % 2 else "csr")
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    psi = torch.randn(n, dtype=torch.complex128, device="cuda", generator=gen) * 3.0
+    # one vector spans the state only to first order in dt: a short step
+    dt = 1e-7 if m == 1 else 0.1
+    want, term = psi.clone(), psi
+    for k in range(1, 40):
+        term = apply(term) * (-1j * dt / k)
+        want = want + term
+    got = psi.to(ev.vdtype).clone()
+    ev.step(got, dt)
+    ev.check_status()
+    err = float(torch.linalg.vector_norm(got.to(torch.complex128) - want) / torch.linalg.vector_norm(want))
+    # c64: a rounding of 2^-24 per stored entry of each basis vector and of psi
+    tol = 5e-6 if precision == "c64" else (1e-5 if m == 1 else 1e-12)
+    assert err < tol, err
