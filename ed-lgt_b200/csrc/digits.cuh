@@ -1,13 +1,15 @@
 // Local states of a sector key, last site first, without 64-bit divisions.
 //
 // The sites are grouped from the last one backwards into chunks whose
-// dimensions multiply to less than 2^32 (a chunk never crosses the words of a
+// dimensions multiply to at most 2^31 (a chunk never crosses the words of a
 // two-word key).  A chunk's value is split off its word with one quotient by
 // the chunk's space: the f64 estimate word * (1 / space) corrected twice by
-// the exact remainder.  Inside a chunk every value is below 2^32, where
-// floor(x / d) = umulhi(ceil(2^64 / d), x) (Lemire, Kaser, Kurz, "Faster
-// remainder by direct computation", 2019, theorem 1 with N = 32, F = 64).
-// A digit then costs a multiply and a multiply-subtract instead of the two
+// the exact remainder.  Inside a chunk every value is below 2^31, where with
+// l = ceil(log2 d) and m = ceil(2^(31 + l) / d) < 2^32
+//   floor(x / d) = (x m) >> (31 + l)
+// (Granlund, Montgomery, "Division by invariant integers using
+// multiplication", 1994, theorem 4.2: m d - 2^(31 + l) < d <= 2^l).  A digit
+// is then a multiply-high, a shift and a multiply-subtract instead of the two
 // 64-bit divisions of key_digit.
 #pragma once
 #include "keys.cuh"
@@ -24,15 +26,17 @@ struct DigitPlan {
   uint64_t chunk_at;              // bit p: position p starts a new chunk
   uint64_t word_at;               // bit p: position p starts the high word
   uint32_t d[EDG_MAX_SITES];      // dimension at position p
-  uint64_t magic[EDG_MAX_SITES];  // ceil(2^64 / d), 0 for d = 1
+  uint32_t magic[EDG_MAX_SITES];  // ceil(2^(31 + l) / d), l = ceil(log2 d)
+  uint32_t shift[EDG_MAX_SITES];  // l - 1 (unused for d = 1)
   uint32_t space[kMaxChunks];     // product of a chunk's dimensions (0: the word's last chunk, taken whole)
   double inv[kMaxChunks];         // 1 / space
 };
 
-// Host: plan of local dimensions d_s (n_hi: sites of the high word, two-word
-// keys).  False when a dimension is below 1 or a word needs too many chunks.
+// Plan of local dimensions d_s (n_hi: sites of the high word, two-word keys);
+// on the host, or by one thread of a CTA whose caller has the dimensions in
+// device memory only.  False when a dimension is below 1 or a word needs too many chunks.
 template <typename Int>
-inline bool make_digit_plan(DigitPlan* p, const Int* dims, int n_sites, int key_words, int n_hi) {
+__host__ __device__ inline bool make_digit_plan(DigitPlan* p, const Int* dims, int n_sites, int key_words, int n_hi) {
   *p = DigitPlan{};
   p->n_sites = n_sites;
   p->key_words = key_words == 2 ? 2 : 1;
@@ -45,7 +49,7 @@ inline bool make_digit_plan(DigitPlan* p, const Int* dims, int n_sites, int key_
     if (d < 1 || d > 65536) return false;
     const bool new_word = pos == 0 || (p->key_words == 2 && s == split - 1);
     if (new_word && pos > 0) p->word_at |= 1ull << pos;
-    if (new_word || prod * (uint64_t)d > 0xFFFFFFFFull) {
+    if (new_word || prod * (uint64_t)d > (1ull << 31)) {
       if (!new_word) {  // the chunk before this one ends inside the word
         p->space[chunk] = (uint32_t)prod;
         p->inv[chunk] = 1.0 / (double)prod;
@@ -56,12 +60,15 @@ inline bool make_digit_plan(DigitPlan* p, const Int* dims, int n_sites, int key_
     }
     prod *= (uint64_t)d;
     p->d[pos] = (uint32_t)d;
-    p->magic[pos] = d > 1 ? ~0ull / (uint64_t)d + 1 : 0;
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    p->magic[pos] = (uint32_t)((((uint64_t)1 << (31 + l)) + (uint64_t)d - 1) / (uint64_t)d);
+    p->shift[pos] = (uint32_t)(l > 0 ? l - 1 : 0);
   }
   return true;
 }
 
-// floor(x / space) with remainder, space < 2^32, x < 2^63.  The first
+// floor(x / space) with remainder, space <= 2^31, x < 2^63.  The first
 // estimate is off by less than 2^11 (f64 rounding of x and of the product),
 // the second by at most one.
 __device__ __forceinline__ uint64_t split_chunk(uint64_t x, uint32_t space, double inv, uint32_t* rem) {
@@ -101,7 +108,7 @@ __device__ __forceinline__ void for_each_digit(const DigitPlan& P, K key, F use)
           x = (uint32_t)word;
       }
       const uint32_t d = P.d[p];
-      const uint32_t q = d > 1 ? (uint32_t)__umul64hi(P.magic[p], (uint64_t)x) : x;
+      const uint32_t q = d > 1 ? __umulhi(P.magic[p], x) >> P.shift[p] : x;
       use(p, (int)(x - q * d));
       x = q;
     }

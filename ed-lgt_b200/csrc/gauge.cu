@@ -7,8 +7,8 @@
 // by memory for 16-byte states: 8 (key) + s_psi read, 16 written.  Replaces a
 // decode of the whole configuration table to the host, its upload as int64
 // and a gather per site: on the 7,133,222-state sector of the L = 16 static
-// pair 235 ms a call with the table already decoded, against 0.14 ms here
-// (complex128 vector, 285 MB: 2.0 TB/s, bound by the decode's instructions).
+// pair 235 ms a call with the table already decoded, against 0.13 ms here
+// (complex128 vector, 285 MB: 2.2 TB/s, bound by the decode's instructions).
 #include "digits.cuh"
 
 namespace {

@@ -3,7 +3,12 @@
 // (edlgt/modeling/local_term.py:119-237 with exp_val_data,
 // edlgt/modeling/qmb_state.py:631-654): local terms only keep the operator
 // diagonal, so an expectation value is a weighted reduction over the basis.
-#include "internal.cuh"
+//
+// One thread takes rows grid-stride, decodes each key (digits.cuh) and adds
+// |psi_r|^2 diag[s][c] to one f64 register per site, the diagonals in shared
+// memory (lanes read a few neighbouring entries: no bank conflicts).  Bound by
+// the decode's instructions, about ten per site and row.
+#include "digits.cuh"
 
 namespace {
 
@@ -26,45 +31,64 @@ __device__ __forceinline__ double prob(const void* psi, int64_t r, int64_t strid
   }
 }
 
-// W = 1: one-word keys; W = 2: two-word keys (low word first) whose high
-// word holds sites [0, n_hi).
-template <int PT, int W>
-__global__ void __launch_bounds__(kThreads) local_expval_k(const uint64_t* __restrict__ keys, int64_t n, int n_hi, int n_sites,
-                                                           edg_site_dims dims, const void* __restrict__ psi,
-                                                           int64_t psi_stride, const double* __restrict__ diag,
-                                                           int dmax, double* __restrict__ out) {
+constexpr int kTableCap = 40 * 1024;  // diagonals larger than this stay in global memory
+
+// CTAs whose accumulators fit an SM's registers (one wave of them is launched)
+constexpr int ctas_for(int ns) { return ns <= 16 ? 3 : ns <= 32 ? 2 : 1; }
+
+// NS >= n_sites sites accumulated in registers.
+template <int PT, int NS, typename K>
+__global__ void __launch_bounds__(kThreads, ctas_for(NS)) local_expval_k(const __grid_constant__ edg::DigitPlan P,
+                                                           const uint64_t* __restrict__ keys, int64_t n,
+                                                           const void* __restrict__ psi, int64_t psi_stride,
+                                                           const double* __restrict__ diag, int dmax, int in_smem,
+                                                           double* __restrict__ out) {
+  extern __shared__ __align__(16) double tab[];  // [n_sites][dmax]
   __shared__ double acc[EDG_MAX_SITES];
-  for (int s = threadIdx.x; s < n_sites; s += kThreads) acc[s] = 0.0;
+  const int ns = P.n_sites;
+  for (int s = threadIdx.x; s < ns; s += kThreads) acc[s] = 0.0;
+  if (in_smem)
+    for (int k = threadIdx.x; k < ns * dmax; k += kThreads) tab[k] = diag[k];
   __syncthreads();
-  double loc[EDG_MAX_SITES];
-  for (int s = 0; s < n_sites; ++s) loc[s] = 0.0;
+  const double* const d = in_smem ? tab : diag;
+  double loc[NS];
+#pragma unroll
+  for (int p = 0; p < NS; ++p) loc[p] = 0.0;
   for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
     const double p2 = prob<PT>(psi, r, psi_stride);
-    uint64_t k = keys[W * r];
-    const int split = W == 2 ? n_hi : 0;
-    for (int s = n_sites - 1; s >= split; --s) {
-      uint64_t d = (uint64_t)dims.d[s];
-      int c = (int)(k % d);
-      k /= d;
-      loc[s] = fma(p2, diag[s * dmax + c], loc[s]);
-    }
-    if (W == 2) {
-      k = keys[2 * r + 1];
-      for (int s = split - 1; s >= 0; --s) {
-        uint64_t d = (uint64_t)dims.d[s];
-        int c = (int)(k % d);
-        k /= d;
-        loc[s] = fma(p2, diag[s * dmax + c], loc[s]);
-      }
-    }
+    edg::for_each_digit<NS>(P, edg::ld_key<K>(keys, r),
+                            [&](int p, int c) { loc[p] = fma(p2, d[(ns - 1 - p) * dmax + c], loc[p]); });
   }
-  for (int s = 0; s < n_sites; ++s) {
-    double v = loc[s];
+#pragma unroll
+  for (int p = 0; p < NS; ++p) {
+    double v = loc[p];
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&acc[s], v);
+    if (p < ns && (threadIdx.x & 31) == 0) atomicAdd(&acc[ns - 1 - p], v);
   }
   __syncthreads();
-  for (int s = threadIdx.x; s < n_sites; s += kThreads) atomicAdd(out + s, acc[s]);
+  for (int s = threadIdx.x; s < ns; s += kThreads) atomicAdd(out + s, acc[s]);
+}
+
+template <int PT, int NS, typename K>
+void launch(const edg::DigitPlan& P, const uint64_t* keys, int64_t n, const void* psi, int64_t stride,
+            const double* diag, int dmax, double* out, cudaStream_t s) {
+  const size_t table = sizeof(double) * (size_t)P.n_sites * dmax;
+  const int in_smem = table <= (size_t)kTableCap;
+  const unsigned g = edg::grid_for(n, kThreads, ctas_for(NS));
+  local_expval_k<PT, NS, K><<<g, kThreads, in_smem ? table : 0, s>>>(P, keys, n, psi, stride, diag, dmax, in_smem,
+                                                                     out);
+}
+
+template <int NS, typename K>
+void launch_pt(int pt, const edg::DigitPlan& P, const uint64_t* keys, int64_t n, const void* psi, int64_t stride,
+               const double* diag, int dmax, double* out, cudaStream_t s) {
+  switch (pt) {
+    case 0: launch<0, NS, K>(P, keys, n, psi, stride, diag, dmax, out, s); break;
+    case 1: launch<1, NS, K>(P, keys, n, psi, stride, diag, dmax, out, s); break;
+    case 2: launch<2, NS, K>(P, keys, n, psi, stride, diag, dmax, out, s); break;
+    default: launch<3, NS, K>(P, keys, n, psi, stride, diag, dmax, out, s); break;
+  }
 }
 
 template <int W>
@@ -78,13 +102,17 @@ int local_expval(const uint64_t* keys, int64_t n, int32_t n_hi, const edg_site_d
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * n_sites, stream);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_local_expval: reset");
   if (n == 0) return EDG_OK;
-  const unsigned g = edg::grid_for(n, kThreads, 4);
-  switch (psi_dtype) {
-    case 0: local_expval_k<0, W><<<g, kThreads, 0, stream>>>(keys, n, n_hi, n_sites, *dims, psi, psi_stride, diag, dmax, out); break;
-    case 1: local_expval_k<1, W><<<g, kThreads, 0, stream>>>(keys, n, n_hi, n_sites, *dims, psi, psi_stride, diag, dmax, out); break;
-    case 2: local_expval_k<2, W><<<g, kThreads, 0, stream>>>(keys, n, n_hi, n_sites, *dims, psi, psi_stride, diag, dmax, out); break;
-    default: local_expval_k<3, W><<<g, kThreads, 0, stream>>>(keys, n, n_hi, n_sites, *dims, psi, psi_stride, diag, dmax, out); break;
-  }
+  EDG_REQUIRE(W == 1 || (reinterpret_cast<uintptr_t>(keys) & 15) == 0,
+              "edg_local_expval_wide: two-word keys must be 16-byte aligned");
+  edg::DigitPlan P;
+  EDG_REQUIRE(edg::make_digit_plan(&P, dims->d, n_sites, W, n_hi), "edg_local_expval: bad local dimensions");
+  using K = typename edg::KeyOf<W>::type;
+  if (n_sites <= 16)
+    launch_pt<16, K>(psi_dtype, P, keys, n, psi, psi_stride, diag, dmax, out, stream);
+  else if (n_sites <= 32)
+    launch_pt<32, K>(psi_dtype, P, keys, n, psi, psi_stride, diag, dmax, out, stream);
+  else
+    launch_pt<EDG_MAX_SITES, K>(psi_dtype, P, keys, n, psi, psi_stride, diag, dmax, out, stream);
   EDG_CHECK_LAUNCH("edg_local_expval");
   return EDG_OK;
 }

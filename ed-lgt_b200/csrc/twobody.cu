@@ -17,7 +17,12 @@
 // conj(psi_row) * a * b * psi_ket in f64 registers.  Blocks reduce their warps
 // per pair in shared memory; a second kernel sums the block partials in a
 // fixed order, so results do not depend on scheduling.
-#include "internal.cuh"
+//
+// When both operators are diagonal and real (densities, Casimirs: the usual
+// case) corr = sum_r |psi_r|^2 a(r) b(r)^T is a contraction over the rows, and
+// up to 32 sites it runs on the f64 tensor instruction (twobody_mma_k); the
+// transition-table kernel then returns at once, and the other way round.
+#include "digits.cuh"
 #include "lookup.cuh"
 
 namespace {
@@ -53,6 +58,7 @@ struct Args {
   int32_t* err;
   int n_sites, dmax, n_pairs;
   int tables_in_smem, diag_in_smem;
+  int mma;  // twobody_mma_k takes real diagonal operators
 };
 
 // Shared memory, in this order: the transition tables [amp | diagonal values
@@ -154,6 +160,7 @@ __global__ void __launch_bounds__(kThreads, 3) twobody_k(const Args a) {
     }
   }
   const bool fast = __syncthreads_and(real_diag) != 0;
+  if (fast && a.mma) return;
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n = a.sec.n;
@@ -285,6 +292,141 @@ __global__ void __launch_bounds__(kThreads, 3) twobody_k(const Args a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Real diagonal operators on up to 8 NB sites: corr = A^T diag(|psi|^2) B over
+// the rows, as m8n8k4 f64 products (sites x sites, four rows deep).  A warp
+// decodes 32 rows (one per lane) into bytes in shared memory; then lane L of
+// the product on site blocks (bi, bj) supplies |psi_r|^2 a_i(r) and b_j(r)
+// for row L % 4 of the step and sites 8 bi + L / 4, 8 bj + L / 4, read from the
+// diagonal tables.  A table row (local state c) is skewed by four doubles, so
+// that the four rows of a half warp, at the same site in different states,
+// mostly fall into different banks.  Against two table reads and two
+// multiply-adds per pair and row, a site's value is read once per row and
+// used in all its pairs: SU(2) L = 16 (7,133,222 rows, 120 pairs, complex128)
+// from 0.78 to 0.27 ms a matrix; bound by the decode and the table reads.
+// Only the blocks that hold a listed pair are multiplied.
+// ---------------------------------------------------------------------------
+constexpr int kMmaTableCap = 32 * 1024;
+__host__ __device__ inline int mma_pitch(int nb) { return 16 * nb + 4; }
+template <int NB>
+struct MmaSmem {
+  static constexpr int kSites = 8 * NB;
+  uint8_t dig[kWarps][32][kSites];  // by position from the last site
+  double w[kWarps][32];
+  double red[kWarps][kSites * kSites];
+};
+
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+template <int PT, int NB>
+__global__ void __launch_bounds__(kThreads, 2)
+    twobody_mma_k(const __grid_constant__ Args a) {
+  constexpr int S = 8 * NB, kPitch = 16 * NB + 4;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned blocks_s;
+  __shared__ edg::DigitPlan P;
+  MmaSmem<NB>& sm = *reinterpret_cast<MmaSmem<NB>*>(smem);
+  double* const tab = reinterpret_cast<double*>(smem + sizeof(MmaSmem<NB>));  // [dmax][pitch]: A's sites, B's sites
+  const int ns = a.n_sites, dm = a.dmax;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int real_diag = 1;
+  if (tid == 0) {
+    blocks_s = 0u;
+    if (!edg::make_digit_plan(&P, a.loc_dims, ns, 1, 0)) {
+      atomicExch(a.err, 1);
+      real_diag = 0;
+    }
+  }
+  for (int k = tid; k < dm * kPitch; k += kThreads) tab[k] = 0.0;
+  __syncthreads();
+  for (int k = tid; k < 2 * ns * dm; k += kThreads) {
+    const int c = a.count[k], b = k % dm, site = k / dm;  // site: operator * ns + site
+    const double2 v = c > 0 ? a.amp[k * dm] : make_double2(0.0, 0.0);
+    real_diag &= c == 0 || (c == 1 && a.ket[k * dm] == b && v.y == 0.0);
+    tab[b * kPitch + (site < ns ? site : S + site - ns)] = v.x;
+  }
+  unsigned blocks = 0u;
+  for (int p = tid; p < a.n_pairs; p += kThreads) {
+    const int pi = a.pair_i[p], pj = a.pair_j[p];
+    if (pi >= 0 && pj >= 0 && pi < ns && pj < ns && pi != pj)
+      blocks |= 1u << ((pi / 8) * NB + pj / 8);
+    else
+      atomicExch(a.err, 2);
+  }
+  if (blocks) atomicOr(&blocks_s, blocks);
+  if (__syncthreads_and(real_diag) == 0) return;
+  blocks = blocks_s;
+  double c[NB][NB][2];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) c[i][j][0] = c[i][j][1] = 0.0;
+  // positions of this lane's sites (sites past the last have zero columns)
+  int pos[NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i) pos[i] = max(ns - 1 - (8 * i + lane / 4), 0);
+  const int64_t n = a.sec.n, n_groups = (n + 31) / 32;
+  for (int64_t g = (int64_t)blockIdx.x * kWarps + warp; g < n_groups; g += (int64_t)gridDim.x * kWarps) {
+    const int64_t r = g * 32 + lane;
+    double w = 0.0;
+    uint32_t packed[2 * NB];
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) packed[q] = 0u;
+    if (r < n) {
+      const double2 v = load_psi<PT>(a.psi, r, a.psi_stride);
+      w = fma(v.x, v.x, v.y * v.y);
+      bool outside = false;
+      edg::for_each_digit<S>(P, __ldg(a.sec.keys + r), [&](int p, int d) {
+        outside |= d >= dm;
+        packed[p / 4] |= (uint32_t)(d < dm ? d : 0) << (8 * (p % 4));
+      });
+      if (outside) atomicExch(a.err, 1);  // a local state beyond the operators' dimension
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) reinterpret_cast<uint32_t*>(sm.dig[warp][lane])[q] = packed[q];
+    sm.w[warp][lane] = w;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int row = 4 * k + (lane & 3);
+      const double wr = sm.w[warp][row];
+      double va[NB], vb[NB];
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        const double* t = tab + sm.dig[warp][row][pos[i]] * kPitch + 8 * i + lane / 4;
+        va[i] = t[0] * wr;
+        vb[i] = t[S];
+      }
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if ((blocks >> (i * NB + j)) & 1u) mma_f64(c[i][j], va[i], vb[j]);
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        sm.red[warp][(8 * i + lane / 4) * S + 8 * j + 2 * (lane & 3) + h] = c[i][j][h];
+  __syncthreads();
+  for (int p = tid; p < a.n_pairs; p += kThreads) {
+    const int pi = a.pair_i[p], pj = a.pair_j[p];
+    double re = 0.0;
+    if (pi >= 0 && pj >= 0 && pi < ns && pj < ns)
+      for (int q = 0; q < kWarps; ++q) re += sm.red[q][pi * S + pj];
+    a.partial[((int64_t)blockIdx.x * a.n_pairs + p) * 2] = re;
+    a.partial[((int64_t)blockIdx.x * a.n_pairs + p) * 2 + 1] = 0.0;
+  }
+}
+
 // corr[i][j] = corr[j][i] = Re sum_b partial[b][p]; one warp per pair, the
 // lanes' strided sums combined by a fixed butterfly.
 __global__ void twobody_reduce_k(const double* __restrict__ partial, int nblk, int n_pairs,
@@ -301,6 +443,34 @@ __global__ void twobody_reduce_k(const double* __restrict__ partial, int nblk, i
   if (lane == 0 && pi >= 0 && pj >= 0 && pi < n_sites && pj < n_sites) {
     corr[(int64_t)pi * n_sites + pj] = s;
     corr[(int64_t)pj * n_sites + pi] = s;
+  }
+}
+
+template <int NB>
+int64_t mma_smem(int dmax) { return (int64_t)sizeof(MmaSmem<NB>) + 8LL * dmax * mma_pitch(NB); }
+
+// Both operators' tables for up to 8 NB sites fit the tensor kernel's shared
+// memory (the digits are bytes).
+inline bool mma_fits(int n_sites, int dmax) {
+  return n_sites <= 32 && 8LL * dmax * mma_pitch((n_sites + 7) / 8) <= kMmaTableCap;
+}
+
+template <int PT, int NB>
+cudaError_t launch_mma(const Args& a, cudaStream_t stream) {
+  const int64_t smem = mma_smem<NB>(a.dmax);
+  cudaError_t e = cudaFuncSetAttribute(twobody_mma_k<PT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  twobody_mma_k<PT, NB><<<kBlocks, kThreads, (size_t)smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
+template <int PT>
+cudaError_t launch_mma_nb(const Args& a, cudaStream_t stream) {
+  switch ((a.n_sites + 7) / 8) {
+    case 1: return launch_mma<PT, 1>(a, stream);
+    case 2: return launch_mma<PT, 2>(a, stream);
+    case 3: return launch_mma<PT, 3>(a, stream);
+    default: return launch_mma<PT, 4>(a, stream);
   }
 }
 
@@ -346,10 +516,22 @@ extern "C" int edg_twobody_expval(const edg_lookup_table* sector, const uint64_t
   e = cudaMemsetAsync(err, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_twobody_expval: flag");
   Args a{*sector, strides, loc_dims, t_count, t_ket, reinterpret_cast<const double2*>(t_amp), pair_i, pair_j, psi,
-         psi_stride, scratch, err, n_sites, dmax, n_pairs, 0, 0};
+         psi_stride, scratch, err, n_sites, dmax, n_pairs, 0, 0, 0};
   a.tables_in_smem = table_bytes(n_sites, dmax) <= kTableSmemCap;
   a.diag_in_smem = dmax * diag_pitch(n_sites) <= kDiagCap;
   const int64_t smem = layout(n_sites, dmax, a.tables_in_smem, a.diag_in_smem).total;
+  // real diagonal operators: the tensor kernel's limits, and the same limit as
+  // the real diagonal table of the other kernel, which decides it skips them
+  a.mma = a.diag_in_smem && mma_fits(n_sites, dmax);
+  if (a.mma) {
+    switch (psi_dtype) {
+      case 0: e = launch_mma_nb<0>(a, stream); break;
+      case 1: e = launch_mma_nb<1>(a, stream); break;
+      case 2: e = launch_mma_nb<2>(a, stream); break;
+      default: e = launch_mma_nb<3>(a, stream); break;
+    }
+    if (e != cudaSuccess) return edg::cuda_status(e, "edg_twobody_expval");
+  }
   switch (psi_dtype) {
     case 0: e = launch<0>(a, smem, stream); break;
     case 1: e = launch<1>(a, smem, stream); break;
