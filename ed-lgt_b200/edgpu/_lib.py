@@ -300,6 +300,8 @@ _SIGS = {
     "edg_lookup": (I32, [C.POINTER(LookupTable), P, I64, P, P]),
     "edg_assemble_count": (I32, [C.POINTER(Assembly), P, P]),
     "edg_assemble_fill": (I32, [C.POINTER(Assembly), P, P, P, P, P, P, P, P]),
+    "edg_assemble_rows": (I32, [C.POINTER(Assembly), I32, P, P, P, P, P, P, P, P]),
+    "edg_assemble_diag": (I32, [C.POINTER(Assembly), P, P, I32, F64, F64, P, P, P]),
     "edg_assemble_compact": (I32, [I64, I32, P, P, P, P, P, P, P]),
     "edg_spmv": (I32, [I32, I64, I64, P, P, P, P, I32, P, P, P]),
     "edg_convert": (I32, [I32, P, I32, P, I64, P]),

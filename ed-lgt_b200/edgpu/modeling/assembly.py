@@ -296,6 +296,11 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
     if not reused:
         raw_tables, terms, real_ok, tables_real, coefs_real = _offdiag_tables(blocks, phase_weights, force_complex,
                                                                               dmax)
+        # instances in the order of their leading sites (stable): a row's
+        # columns then come out almost sorted (the fill kernel's insertion)
+        order = sorted(range(len(terms)), key=lambda i: min(terms[i][0]))
+        terms = [terms[i] for i in order]
+        coefs_real = [coefs_real[i] for i in order] if coefs_real is not None else None
         use_real = real_ok and dterms_real
         arrays = _table_arrays(raw_tables, terms, dmax, not use_real, tables_real, coefs_real)
         keep = [up(a) for a in arrays]
@@ -305,45 +310,36 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
     is_complex = not off["use_real"]
     w = 2 if is_complex else 1
 
-    # ---- diagonal terms: one pass without off-diagonal instances ----
-    diag = off["diag"].clone()
-    present = off["present"].clone()
+    # ---- diagonal terms: one pass over the rows, on top of the off-diagonal
+    # part's own diagonal ----
     n_d = len(dterms)
-    if n_d > 0 and n > 0:
-        dterm_site = np.zeros(n_d, dtype=np.int32)
-        dterm_diag = np.zeros((n_d, dmax, w), dtype=np.float64)
-        dterm_coef = np.zeros((n_d, w), dtype=np.float64)
-        for k, (s, dvec, coef) in enumerate(dterms):
-            dterm_site[k] = s
-            dterm_diag[k, : len(dvec), 0] = dvec.real
-            dterm_coef[k, 0] = coef.real
-            if is_complex:
-                dterm_diag[k, : len(dvec), 1] = dvec.imag
-                dterm_coef[k, 1] = coef.imag
-        dk = [up(dterm_site), up(dterm_diag), up(dterm_coef)]
-        keep += dk
+    extra = complex(extra_diag) if extra_diag is not None and extra_diag != 0 else None
+    if n == 0 or (n_d == 0 and extra is None):
+        diag, present = off["diag"].clone(), off["present"].clone()
+    else:
+        diag = torch.empty(n * w, dtype=torch.float64, device=dev)
+        present = torch.empty(n, dtype=torch.uint8, device=dev)
         a = _assembly_struct(sector, dmax, is_complex)
         a.n_terms = 0
         a.n_dterms = n_d
-        a.dterm_site, a.dterm_diag, a.dterm_coef = ptr(dk[0]), ptr(dk[1]), ptr(dk[2])
-        zeros = torch.zeros(n + 1, dtype=torch.int64, device=dev)
-        one_i = torch.empty(1, dtype=torch.int32, device=dev)
-        one_d = torch.empty(w, dtype=torch.float64, device=dev)
-        row_nnz = torch.empty(n, dtype=torch.int64, device=dev)
-        d_diag = torch.empty(n * w, dtype=torch.float64, device=dev)
-        d_present = torch.empty(n, dtype=torch.uint8, device=dev)
-        err = torch.zeros(1, dtype=torch.int32, device=dev)
-        check(lib.edg_assemble_fill(ctypes.byref(a), ptr(zeros), ptr(one_i), ptr(one_d), ptr(row_nnz), ptr(d_diag),
-                                    ptr(d_present), ptr(err), st), "edg_assemble_fill")
-        diag += d_diag
-        present |= d_present
-    if extra_diag is not None and extra_diag != 0:
-        if is_complex:
-            diag.view(-1, 2)[:, 0] += float(np.real(extra_diag))
-            diag.view(-1, 2)[:, 1] += float(np.imag(extra_diag))
-        else:
-            diag += float(np.real(extra_diag))
-        present.fill_(1)
+        if n_d:
+            dterm_site = np.zeros(n_d, dtype=np.int32)
+            dterm_diag = np.zeros((n_d, dmax, w), dtype=np.float64)
+            dterm_coef = np.zeros((n_d, w), dtype=np.float64)
+            for k, (s, dvec, coef) in enumerate(dterms):
+                dterm_site[k] = s
+                dterm_diag[k, : len(dvec), 0] = dvec.real
+                dterm_coef[k, 0] = coef.real
+                if is_complex:
+                    dterm_diag[k, : len(dvec), 1] = dvec.imag
+                    dterm_coef[k, 1] = coef.imag
+            dk = [up(dterm_site), up(dterm_diag), up(dterm_coef)]
+            keep += dk
+            a.dterm_site, a.dterm_diag, a.dterm_coef = ptr(dk[0]), ptr(dk[1]), ptr(dk[2])
+        ex = extra if extra is not None else 0j
+        check(lib.edg_assemble_diag(ctypes.byref(a), ptr(off["diag"]), ptr(off["present"]),
+                                    0 if extra is None else 1, ex.real, ex.imag, ptr(diag), ptr(present), st),
+              "edg_assemble_diag")
     mat = DeviceMatrix(n, off["rowptr"], off["cols"], off["vals"], diag, present, is_complex,
                        phase_weights if (not is_complex and phase_weights is not None) else None)
     mat._keep = keep  # device tables uploaded by this build
@@ -381,24 +377,27 @@ def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, tabs):
     scratch = torch.empty(lib.edg_scan_scratch_elems(n), dtype=torch.int64, device=dev)
     check(lib.edg_scan_i64(ptr(bound), ptr(offsets), n, ptr(scratch), st), "edg_scan_i64")
     total = int(offsets[n].item())
-    tmp_cols = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-    tmp_vals = torch.empty(max(total, 1) * w, dtype=torch.float64, device=dev)
+    cols = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+    vals = torch.empty(max(total, 1) * w, dtype=torch.float64, device=dev)
     row_nnz = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
     diag = torch.empty(max(n, 1) * w, dtype=torch.float64, device=dev)
     present = torch.empty(max(n, 1), dtype=torch.uint8, device=dev)
-    err = torch.zeros(1, dtype=torch.int32, device=dev)
-    check(lib.edg_assemble_fill(ctypes.byref(a), ptr(offsets), ptr(tmp_cols), ptr(tmp_vals), ptr(row_nnz),
-                                ptr(diag), ptr(present), ptr(err), st), "edg_assemble_fill")
-    rowptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
-    check(lib.edg_scan_i64(ptr(row_nnz), ptr(rowptr), n, ptr(scratch), st), "edg_scan_i64")
-    nnz = int(rowptr[n].item())
-    e = int(err.item())
+    flags = torch.zeros(2, dtype=torch.int32, device=dev)
+    check(lib.edg_assemble_rows(ctypes.byref(a), int(tabs[0].shape[0]), ptr(offsets), ptr(cols), ptr(vals),
+                                ptr(row_nnz), ptr(diag), ptr(present), ptr(flags), st), "edg_assemble_rows")
+    e, merged = flags.tolist()
     if e != 0:
         raise _lib.EdgError(e, "an operator maps a sector configuration outside the sector")
-    cols = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
-    vals = torch.empty(max(nnz, 1) * w, dtype=torch.float64, device=dev)
-    check(lib.edg_assemble_compact(n, 1 if is_complex else 0, ptr(offsets), ptr(tmp_cols), ptr(tmp_vals),
-                                   ptr(rowptr), ptr(cols), ptr(vals), st), "edg_assemble_compact")
-    del tmp_cols, tmp_vals
+    rowptr, nnz = offsets, total
+    if merged:  # some rows are shorter than their bound: close the gaps
+        tmp_cols, tmp_vals = cols, vals
+        rowptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
+        check(lib.edg_scan_i64(ptr(row_nnz), ptr(rowptr), n, ptr(scratch), st), "edg_scan_i64")
+        nnz = int(rowptr[n].item())
+        cols = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
+        vals = torch.empty(max(nnz, 1) * w, dtype=torch.float64, device=dev)
+        check(lib.edg_assemble_compact(n, 1 if is_complex else 0, ptr(offsets), ptr(tmp_cols), ptr(tmp_vals),
+                                       ptr(rowptr), ptr(cols), ptr(vals), st), "edg_assemble_compact")
+        del tmp_cols, tmp_vals
     return {"rowptr": rowptr, "cols": cols[:nnz], "vals": vals[: nnz * w], "diag": diag[: n * w],
             "present": present[:n], "raw_entries": total, "keep": tabs}

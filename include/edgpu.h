@@ -266,6 +266,21 @@ int edg_assemble_fill(const edg_assembly* a, const int64_t* offsets,
                       int32_t* tmp_cols, double* tmp_vals, int64_t* row_nnz,
                       double* diag, uint8_t* diag_present, int32_t* error_flag,
                       cudaStream_t stream);
+/* The same with flags (two int32, zero-initialised): flags[0] as error_flag,
+ * flags[1] set when some row has fewer entries than its window.  While it is
+ * zero, offsets and cols / vals are the final CSR as they are.  n_tables:
+ * number of transition tables (0: unknown; they are then not staged). */
+int edg_assemble_rows(const edg_assembly* a, int32_t n_tables,
+                      const int64_t* offsets, int32_t* cols, double* vals,
+                      int64_t* row_nnz, double* diag, uint8_t* diag_present,
+                      int32_t* flags, cudaStream_t stream);
+/* Diagonal terms alone: diag = (base + their sum) + extra, where base (may be
+ * NULL with base_present) is an earlier diagonal and extra a constant added
+ * to every row when has_extra is not 0 (every row is then present). */
+int edg_assemble_diag(const edg_assembly* a, const double* base,
+                      const uint8_t* base_present, int32_t has_extra,
+                      double extra_re, double extra_im, double* diag,
+                      uint8_t* diag_present, cudaStream_t stream);
 /* Copies the merged windows into the final CSR (rowptr from a scan of
  * row_nnz). */
 int edg_assemble_compact(int64_t n_rows, int32_t complex_values,
