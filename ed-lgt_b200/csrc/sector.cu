@@ -13,6 +13,13 @@
 // Digits of earlier sites are decoded from the parent key.  Kernels are
 // templated on the key type (keys.cuh): uint64_t, or a 128-bit pair of words
 // when the key space exceeds 63 bits.
+//
+// Two forms.  While a level has at most `cap` prefixes, all levels run inside
+// one cooperative launch (levels_coop_k): the sizes stay on the device, so
+// there is no host round trip per level.  A level that would not fit is left
+// to the per-level pair of launches (level_count, level_fill), whose caller
+// reads its size and allocates it.
+#include "gridbar.cuh"
 #include "internal.cuh"
 #include "keys.cuh"
 
@@ -159,6 +166,246 @@ __global__ void __launch_bounds__(kThreads) level_fill(edg_sector_tables t, Leve
   }
 }
 
+// ---------------------------------------------------------------------------
+// All levels in one cooperative launch.  Per level every CTA owns an equal run
+// of parents.  A thread decides all children of a parent at once: the digits
+// its constraints need are decoded once per parent instead of once per child,
+// by multiplications with reciprocals (64-bit divisions were most of a level's
+// time), and the surviving children are bits of a mask kept in shared memory.
+// After one grid-wide wait the CTAs know their output offsets and write the
+// children from the masks (each level is evaluated once); a second wait
+// publishes the level.  Bound by the two waits and the latency of a few
+// dependent loads, about 4 us a level, until levels have 10^5 prefixes.
+// ---------------------------------------------------------------------------
+constexpr int kCoopThreads = 512;
+constexpr int kCoopSmem = 200 * 1024;
+constexpr int kHead = 72;  // int64 words: level sizes [64] | levels done | prefixes | buffer | error | barrier
+
+struct Coop {
+  uint64_t* keys[2];
+  int32_t* sums[2];
+  int64_t* head;
+  int64_t* counts;  // [2][grid]
+  int64_t cap;
+};
+
+// floor(x / y) for x < 2^63, y < 2^62, inv = 1 / y: the f64 estimate, then its
+// remainder divided the same way, then a correction by one.
+__device__ __forceinline__ uint64_t fast_div(uint64_t x, uint64_t y, double inv) {
+  uint64_t q = (uint64_t)((double)x * inv);
+  int64_t r = (int64_t)(x - q * y);
+  const int64_t c = (int64_t)floor((double)r * inv);
+  q += (uint64_t)c;
+  r -= c * (int64_t)y;
+  if (r < 0) --q;
+  if (r >= (int64_t)y) ++q;
+  return q;
+}
+
+template <typename K, typename M>
+__global__ void __launch_bounds__(kCoopThreads, 1) levels_coop_k(const __grid_constant__ edg_sector_tables t,
+                                                                 const Coop C) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  M* const masks = reinterpret_cast<M*>(sm_raw);
+  __shared__ double inv_stride[EDG_MAX_SITES], inv_dim[EDG_MAX_SITES];
+  __shared__ int64_t red[2][kCoopThreads / 32];
+  __shared__ int64_t tot[2];
+  __shared__ int wsum[kCoopThreads / 32];
+  __shared__ uint32_t allowed_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)gridDim.x, n = t.n_sites, dm = t.dmax, ng = t.n_glob;
+  int* const err = reinterpret_cast<int*>(C.head + 67);
+  edg::GridSync gs{reinterpret_cast<unsigned*>(C.head + 68), err};
+  for (int s = tid; s < n; s += kCoopThreads) {
+    inv_stride[s] = 1.0 / (double)t.strides[s];
+    inv_dim[s] = 1.0 / (double)t.loc_dims[s];
+  }
+  auto digit = [&](K key, int s) -> int {
+    const uint64_t d = (uint64_t)t.loc_dims[s];
+    const uint64_t q = fast_div(edg::key_word(key, s, t.n_hi), t.strides[s], inv_stride[s]);
+    return (int)(q - fast_div(q, d, inv_dim[s]) * d);
+  };
+  int64_t n_prev = 1;
+  int cur = 0, depth = 0;
+  for (; depth < n; ++depth) {
+    const int d = t.loc_dims[depth];
+    if (d > (int)sizeof(M) * 8) break;
+    const bool last = depth == n - 1;
+    if (tid == 0) {
+      uint32_t m = 0u;
+      for (int c = 0; c < d; ++c) m |= t.site_allowed[depth * dm + c] ? 1u << c : 0u;
+      allowed_s = m;
+    }
+    __syncthreads();
+    const int64_t p0 = n_prev * blockIdx.x / G, p1 = n_prev * (blockIdx.x + 1) / G;
+    const uint64_t* const pk = C.keys[cur];
+    const int32_t* const ps = C.sums[cur];
+    // ---- which children of each parent survive ----
+    int64_t mine = 0;
+    for (int64_t p = p0 + tid; p < p1; p += kCoopThreads) {
+      K key = K(0);
+      if (depth > 0) {
+        if constexpr (sizeof(K) == 8)
+          key = pk[p];
+        else
+          key = ((K)pk[2 * p + 1] << 64) | (K)pk[2 * p];
+      }
+      uint32_t m = allowed_s;
+      for (int g = 0; g < ng; ++g) {
+        const int32_t prev = depth > 0 ? ps[p * ng + g] : 0;
+        const int32_t* val = t.glob_val + ((int64_t)g * n + depth) * dm;
+        const int32_t target = t.glob_target[g];
+        if (t.glob_type == 0) {
+          const int32_t lo = last ? 0 : t.glob_rem_min[g * (n + 1) + depth + 1];
+          const int32_t hi = last ? 0 : t.glob_rem_max[g * (n + 1) + depth + 1];
+          for (uint32_t b = m; b; b &= b - 1u) {
+            const int c = __ffs(b) - 1;
+            const int32_t s = prev + __ldg(val + c);
+            if (target < s + lo || target > s + hi) m &= ~(1u << c);
+          }
+        } else if (last) {
+          for (uint32_t b = m; b; b &= b - 1u) {
+            const int c = __ffs(b) - 1;
+            if ((prev ^ __ldg(val + c)) != target) m &= ~(1u << c);
+          }
+        }
+      }
+      for (int q = t.pair_start[depth]; q < t.pair_start[depth + 1] && m; ++q) {
+        const int s0 = t.pair_s0[q], s1 = t.pair_s1[q], dir = t.pair_dir[q];
+        const int32_t* v0 = t.link_val + (((int64_t)dir * 2 + 0) * n + s0) * dm;
+        const int32_t* v1 = t.link_val + (((int64_t)dir * 2 + 1) * n + s1) * dm;
+        const int32_t target = t.link_target[dir];
+        const int32_t f0 = s0 == depth ? 0 : __ldg(v0 + digit(key, s0));
+        const int32_t f1 = s1 == depth ? 0 : __ldg(v1 + digit(key, s1));
+        for (uint32_t b = m; b; b &= b - 1u) {
+          const int c = __ffs(b) - 1;
+          const int32_t v = (s0 == depth ? __ldg(v0 + c) : f0) + (s1 == depth ? __ldg(v1 + c) : f1);
+          if (v != target) m &= ~(1u << c);
+        }
+      }
+      if (t.nb_start != nullptr) {
+        for (int q = t.nb_start[depth]; q < t.nb_start[depth + 1] && m; ++q) {
+          const int id = t.nb_id[q];
+          const int32_t* val = t.nb_val + (int64_t)id * n * dm;
+          int32_t acc = 0;
+          int here = 0;  // factors on this level's site
+          for (int e = t.nb_site_start[id]; e < t.nb_site_start[id + 1]; ++e) {
+            const int s = t.nb_sites[e];
+            if (s == depth) {
+              ++here;
+              continue;
+            }
+            const int32_t v = __ldg(val + (int64_t)s * dm + digit(key, s));
+            acc = t.nbody_type == 0 ? acc + v : (acc ^ v);
+          }
+          for (uint32_t b = m; b; b &= b - 1u) {
+            const int c = __ffs(b) - 1;
+            const int32_t v = __ldg(val + (int64_t)depth * dm + c);
+            const int32_t x = t.nbody_type == 0 ? acc + here * v : ((here & 1) ? acc ^ v : acc);
+            if (x != t.nb_target[id]) m &= ~(1u << c);
+          }
+        }
+      }
+      masks[p - p0] = (M)m;
+      mine += __popc(m);
+    }
+    // ---- offsets of the CTAs ----
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (lane == 0) red[0][warp] = mine;
+    __syncthreads();
+    int64_t* const cnt = C.counts + (int64_t)(depth & 1) * G;
+    if (tid == 0) {
+      int64_t a = 0;
+      for (int w = 0; w < kCoopThreads / 32; ++w) a += red[0][w];
+      cnt[blockIdx.x] = a;
+    }
+    if (!gs.wait()) return;
+    int64_t below = 0, all = 0;
+    for (int b = tid; b < G; b += kCoopThreads) {
+      const int64_t v = __ldcg(cnt + b);
+      all += v;
+      below += b < (int)blockIdx.x ? v : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+      below += __shfl_xor_sync(0xffffffffu, below, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = all;
+      red[1][warp] = below;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      int64_t a = 0;
+      for (int w = 0; w < kCoopThreads / 32; ++w) a += red[tid][w];
+      tot[tid] = a;
+    }
+    __syncthreads();
+    const int64_t total = tot[0];
+    int64_t base = tot[1];
+    if (total > C.cap) break;  // too many prefixes: the caller goes on from this level
+    // ---- children in order ----
+    uint64_t* const nk = C.keys[cur ^ 1];
+    int32_t* const nsum = C.sums[cur ^ 1];
+    const int64_t stride = (int64_t)t.strides[depth];
+    for (int64_t q0 = p0; q0 < p1; q0 += kCoopThreads) {
+      const int64_t p = q0 + tid;
+      const uint32_t m = p < p1 ? (uint32_t)masks[p - p0] : 0u;
+      const int c0 = __popc(m);
+      int inc = c0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (lane == 31) wsum[warp] = inc;
+      __syncthreads();
+      int before = 0, here = 0;
+      for (int w = 0; w < kCoopThreads / 32; ++w) {
+        before += w < warp ? wsum[w] : 0;
+        here += wsum[w];
+      }
+      if (m) {
+        K key = K(0);
+        if (depth > 0) {
+          if constexpr (sizeof(K) == 8)
+            key = pk[p];
+          else
+            key = ((K)pk[2 * p + 1] << 64) | (K)pk[2 * p];
+        }
+        int64_t at = base + before + inc - c0;
+        for (uint32_t b = m; b; b &= b - 1u, ++at) {
+          const int c = __ffs(b) - 1;
+          const K kk = key + edg::key_step<K>((int64_t)c * stride, depth, t.n_hi);
+          edg::st_key(nk, at, kk);
+          for (int g = 0; g < ng; ++g) {
+            const int32_t prev = depth > 0 ? ps[p * ng + g] : 0;
+            const int32_t v = __ldg(t.glob_val + ((int64_t)g * n + depth) * dm + c);
+            nsum[at * ng + g] = t.glob_type == 0 ? prev + v : (prev ^ v);
+          }
+        }
+      }
+      base += here;
+      __syncthreads();
+    }
+    if (blockIdx.x == 0 && tid == 0) C.head[depth] = total;
+    cur ^= 1;
+    n_prev = total;
+    if (!gs.wait()) return;
+    if (total == 0) {
+      ++depth;
+      break;
+    }
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    C.head[64] = depth;
+    C.head[65] = n_prev;
+    C.head[66] = cur;
+  }
+}
+
 int check_tables(const edg_sector_tables* t, int32_t depth, int64_t n_prev, const char* who) {
   EDG_REQUIRE(t != nullptr, "%s: null tables", who);
   EDG_REQUIRE(t->n_sites > 0 && t->n_sites <= EDG_MAX_SITES, "%s: n_sites out of range", who);
@@ -172,6 +419,60 @@ int check_tables(const edg_sector_tables* t, int32_t depth, int64_t n_prev, cons
 }
 
 }  // namespace
+
+extern "C" int64_t edg_sector_levels_work_elems(void) { return kHead + 2 * edg::kSmCount; }
+
+extern "C" int64_t edg_sector_levels_cap(const edg_sector_tables* t) {
+  if (t == nullptr || t->n_sites < 1 || t->n_sites > EDG_MAX_SITES) return -1;
+  int d = 1;
+  for (int s = 0; s < t->n_sites; ++s) d = t->loc_dims[s] > d ? t->loc_dims[s] : d;
+  const int bytes = d <= 8 ? 1 : d <= 16 ? 2 : 4;
+  return (int64_t)edg::kSmCount * (kCoopSmem / bytes - 1);
+}
+
+extern "C" int edg_sector_levels(const edg_sector_tables* t, uint64_t* keys0, uint64_t* keys1, int32_t* sums0,
+                                 int32_t* sums1, int64_t cap, int64_t* work, cudaStream_t stream) {
+  int st = check_tables(t, 0, 1, "edg_sector_levels");
+  if (st) return st;
+  EDG_REQUIRE(keys0 && keys1 && sums0 && sums1 && work, "edg_sector_levels: null pointer");
+  EDG_REQUIRE(cap >= 1 && cap <= edg_sector_levels_cap(t), "edg_sector_levels: cap out of range");
+  EDG_REQUIRE(t->key_words != 2 || ((reinterpret_cast<uintptr_t>(keys0) | reinterpret_cast<uintptr_t>(keys1)) & 15) == 0,
+              "edg_sector_levels: two-word keys must be 16-byte aligned");
+  int dmx = 1;
+  for (int s = 0; s < t->n_sites; ++s) {
+    EDG_REQUIRE(t->loc_dims[s] > 0 && t->loc_dims[s] <= t->dmax, "edg_sector_levels: bad local dimension");
+    dmx = t->loc_dims[s] > dmx ? t->loc_dims[s] : dmx;
+  }
+  const bool wide = t->key_words == 2;
+  const int bytes = dmx <= 8 ? 1 : dmx <= 16 ? 2 : 4;
+  const void* kern =
+      wide ? (bytes == 1 ? (const void*)levels_coop_k<edg::u128, uint8_t>
+                         : bytes == 2 ? (const void*)levels_coop_k<edg::u128, uint16_t>
+                                      : (const void*)levels_coop_k<edg::u128, uint32_t>)
+           : (bytes == 1 ? (const void*)levels_coop_k<uint64_t, uint8_t>
+                         : bytes == 2 ? (const void*)levels_coop_k<uint64_t, uint16_t>
+                                      : (const void*)levels_coop_k<uint64_t, uint32_t>);
+  int dev = 0, n_sm = 0, coop = 0, occ = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  const int64_t grid = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
+  const int64_t smem = ((cap + grid - 1) / grid + 1) * bytes;  // masks of a CTA's parents
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, (size_t)smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, kHead * sizeof(int64_t), stream);
+  if (e != cudaSuccess) return edg::cuda_status(e, "edg_sector_levels");
+  if (!coop || occ < 1) {  // nothing done: the caller runs every level itself
+    const int64_t none[3] = {0, 1, 0};
+    e = cudaMemcpyAsync(work + 64, none, sizeof(none), cudaMemcpyHostToDevice, stream);
+    return e == cudaSuccess ? EDG_OK : edg::cuda_status(e, "edg_sector_levels");
+  }
+  Coop c{{keys0, keys1}, {sums0, sums1}, work, work + kHead, cap};
+  edg_sector_tables tab = *t;
+  void* args[] = {&tab, &c};
+  e = cudaLaunchCooperativeKernel(kern, dim3((unsigned)grid), dim3(kCoopThreads), args, (size_t)smem, stream);
+  return e == cudaSuccess ? EDG_OK : edg::cuda_status(e, "edg_sector_levels");
+}
 
 extern "C" int64_t edg_sector_level_blocks(int64_t n_candidates) {
   return edg::ceil_div(n_candidates > 0 ? n_candidates : 1, kTile);

@@ -288,6 +288,9 @@ _SIGS = {
     "edg_version": (I32, []),
     "edg_scan_scratch_elems": (I64, [I64]),
     "edg_scan_i64": (I32, [P, P, I64, P, P]),
+    "edg_sector_levels_cap": (I64, [C.POINTER(SectorTables)]),
+    "edg_sector_levels_work_elems": (I64, []),
+    "edg_sector_levels": (I32, [C.POINTER(SectorTables), P, P, P, P, I64, P, P]),
     "edg_sector_level_blocks": (I64, [I64]),
     "edg_sector_level_count": (I32, [C.POINTER(SectorTables), I32, P, P, I64, P, P, P]),
     "edg_sector_level_fill": (I32, [C.POINTER(SectorTables), I32, P, P, I64, P, P, P, P]),

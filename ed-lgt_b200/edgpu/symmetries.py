@@ -451,18 +451,45 @@ class Sector:
         return self.keys.cpu().numpy().view(np.uint64)
 
 
+# Prefixes a level may have inside the one-launch enumeration (two buffers of
+# keys and sums: 100 MB for one-word keys and one global symmetry).  Larger
+# levels go through one pair of launches each, with a host read of their size.
+LEVELS_CAP = 1 << 22
+
+
 def enumerate_sector(spec: SectorSpec, device=None) -> Sector:
-    """Level-by-level enumeration on the device; returns the sorted sector."""
+    """Level-by-level enumeration on the device; returns the sorted sector.
+
+    All levels of at most ``LEVELS_CAP`` prefixes run inside one launch
+    (``edg_sector_levels``); the levels from the first larger one on are
+    counted, allocated and filled one by one."""
     device = torch.device("cuda") if device is None else torch.device(device)
     tables = _DeviceTables(spec, device)
     st = stream_handle()
     ng = spec.glob_val.shape[0]
     kshape = (lambda m: (m, 2)) if spec.key_words == 2 else (lambda m: (m,))
-    prev_keys = torch.zeros(kshape(1), dtype=torch.int64, device=device)
-    prev_sums = torch.zeros(max(ng, 1), dtype=torch.int32, device=device)
-    n_prev = 1
-    level_sizes = []
-    for depth in range(spec.n_sites):
+    space = int(np.prod(np.asarray(spec.loc_dims).astype(object)))
+    cap = max(1, min(LEVELS_CAP, space, int(lib.edg_sector_levels_cap(C_ref(tables.struct)))))
+    keys = [torch.empty(kshape(cap), dtype=torch.int64, device=device) for _ in range(2)]
+    sums = [torch.empty(max(cap * ng, 1), dtype=torch.int32, device=device) for _ in range(2)]
+    work = torch.empty(int(lib.edg_sector_levels_work_elems()), dtype=torch.int64, device=device)
+    check(lib.edg_sector_levels(C_ref(tables.struct), ptr(keys[0]), ptr(keys[1]), ptr(sums[0]), ptr(sums[1]), cap,
+                                ptr(work), st), "edg_sector_levels")
+    head = work[:68].tolist()
+    done, n_prev, cur, status = head[64:68]
+    if status != 0:
+        raise _lib.EdgError(status - 2**32 if status >= 2**31 else status,
+                            "edg_sector_levels: a grid-wide wait ran out")
+    level_sizes = head[:done]
+    if done:
+        prev_keys, prev_sums = keys[cur], sums[cur]
+    else:  # not even the first level ran: start from the empty prefix
+        n_prev = 1
+        prev_keys = torch.zeros(kshape(1), dtype=torch.int64, device=device)
+        prev_sums = torch.zeros(max(ng, 1), dtype=torch.int32, device=device)
+    for depth in range(done, spec.n_sites):
+        if n_prev == 0:
+            break
         n_cand = n_prev * int(spec.loc_dims[depth])
         nb = lib.edg_sector_level_blocks(n_cand)
         offsets = torch.empty(nb + 1, dtype=torch.int64, device=device)
@@ -477,10 +504,7 @@ def enumerate_sector(spec: SectorSpec, device=None) -> Sector:
                                             ptr(offsets), ptr(next_keys), ptr(next_sums), st), "edg_sector_level_fill")
         prev_keys, prev_sums, n_prev = next_keys, next_sums, total
         level_sizes.append(total)
-        if total == 0:
-            break
-    keys = prev_keys[:n_prev].clone()
-    sector = Sector(keys, spec.loc_dims, device)
+    sector = Sector(prev_keys[:n_prev].clone(), spec.loc_dims, device)
     sector.level_sizes = level_sizes  # surviving prefixes per depth
     sector.n_glob = ng
     return sector

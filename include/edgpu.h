@@ -148,6 +148,21 @@ typedef struct {
  * elements plus edg_scan_scratch_elems of it. */
 int64_t edg_sector_level_blocks(int64_t n_candidates);
 
+/* All levels of the prefix expansion in one cooperative launch, as far as a
+ * level has at most cap prefixes (cap <= edg_sector_levels_cap) and its site
+ * at most 32 states.  keys0, keys1: cap keys each (of key_words words), sums0,
+ * sums1: cap * n_glob int32 each, work: edg_sector_levels_work_elems int64.
+ * work[s] is then the number of prefixes after level s, work[64] the levels
+ * done, work[65] the prefixes of the last of them, work[66] the buffer (0 or
+ * 1) that holds them, and work[67] a status (EDG_ERR_TIMEOUT when a grid-wide
+ * wait ran out).  The remaining levels, if any, are edg_sector_level_count /
+ * edg_sector_level_fill on that buffer. */
+int64_t edg_sector_levels_cap(const edg_sector_tables* t);
+int64_t edg_sector_levels_work_elems(void);
+int edg_sector_levels(const edg_sector_tables* t, uint64_t* keys0,
+                      uint64_t* keys1, int32_t* sums0, int32_t* sums1,
+                      int64_t cap, int64_t* work, cudaStream_t stream);
+
 /* Level `depth` of the prefix expansion: every parent prefix (depth-1 sites,
  * n_prev of them; n_prev = 1 with an empty parent at depth 0) is extended by
  * each state of site `depth`; survivors keep the parent order and the state
