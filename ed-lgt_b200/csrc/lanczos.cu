@@ -7,7 +7,8 @@
 // eigen-solve are double precision.  The reorthogonalisation of a step reads
 // V[lo..j] (lo = 0, or j - window): through the bulk-copy ring passes, or,
 // when at most kSmallMax vectors are read, in one cooperative launch
-// (reorth_small_k).
+// (reorth_small_k).  A single problem of a small sector is solved in one
+// cooperative launch instead (lanczos_coop_k).
 //
 // Step j, delayed classical Gram-Schmidt with reorthogonalisation (DCGS2,
 // Swirydowicz, Langou, Ananthan, Yang, Thomas, Numer. Linear Algebra Appl.
@@ -818,84 +819,13 @@ __global__ void __launch_bounds__(kSmallThreads) reorth_small_k(
   }
 }
 
-// Convergence check after a step, launched after every step (one CTA per
-// problem).  It works only when the state's schedule says a check is due:
-// then each CTA of an unconverged problem finds the invariant-subspace
-// dimension, solves its tridiagonal matrix and tests the residual bounds;
-// the last CTA sets the done flag, schedules the next check from the
-// contraction of the worst residual (never sooner than check_every steps,
-// never later than 4 * check_every) and writes the progress words to the
-// host.  Otherwise block 0 only publishes the step count.
-template <int NV>
-__global__ void __launch_bounds__(kThreads) check_k(DevState* __restrict__ st, const double* __restrict__ alpha,
-                                                    int lda, const double* __restrict__ beta, int ldb, int m_max,
-                                                    int64_t n, int k, double tol, int check_every,
-                                                    double* __restrict__ tri_eval, double* __restrict__ tri_vec,
-                                                    int ld_s, double* __restrict__ tri_work,
-                                                    int32_t* __restrict__ host_progress) {
-  __shared__ int mv_s, exact_s, last_s;
-  volatile DevState* vst = st;
-  if (vst->done) return;
-  const int m = vst->j;
-  const bool due = m >= vst->next_check || m >= m_max || (int64_t)m >= n;
-  if (!due) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && host_progress) {
-      volatile int32_t* hp = host_progress;
-      hp[0] = m;
-    }
-    return;
-  }
-  const int v = blockIdx.x;
-  if (vst->m_conv[v] == 0) {
-    const double* al = alpha + (int64_t)v * lda;
-    const double* be = beta + (int64_t)v * ldb;
-    if (threadIdx.x == 0) {
-      double scale = 0.0;
-      for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(al[i]) + fabs(be[i]));
-      const double thr = 1e-12 * fmax(scale, 1e-300);
-      int mv = m;
-      for (int i = 1; i <= m; ++i)
-        if (fabs(be[i]) <= thr) {
-          mv = i;
-          break;
-        }
-      mv_s = mv;
-      exact_s = mv < m || (mv == m && fabs(be[m]) <= thr) || (int64_t)m == n;
-    }
-    __syncthreads();
-    const int mv = mv_s, kk = k < mv ? k : mv;
-    double* S = tri_vec + (int64_t)v * kMaxK * ld_s;
-    for (int e = threadIdx.x; e < kMaxK * ld_s; e += kThreads) S[e] = 0.0;
-    __syncthreads();
-    tridiag_body(al, be, mv, kk, tri_eval + (int64_t)v * kMaxK, S, ld_s, tri_work + (int64_t)v * 6 * ld_s);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const bool exact = exact_s != 0;
-      bool ok = kk == k || exact;
-      double worst = 0.0;
-      for (int q = 0; q < kk; ++q) {
-        const double theta = tri_eval[(int64_t)v * kMaxK + q];
-        const double last = S[(int64_t)q * ld_s + (mv - 1)];
-        const double r = exact ? 0.0 : fabs(be[mv] * last);
-        vst->resid[v][q] = r;
-        if (r > tol * fmax(1.0, fabs(theta))) ok = false;
-        worst = fmax(worst, r / fmax(1.0, fabs(theta)));
-      }
-      vst->m_use[v] = mv;
-      vst->worst[v] = ok ? 0.0 : worst;
-      if (ok) vst->m_conv[v] = mv;
-      __threadfence();
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) last_s = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!last_s || threadIdx.x != 0) return;
-  __threadfence();
-  vst->ticket = 0;
+// Bookkeeping of a check at dimension m (one thread): whether the solve ends,
+// and otherwise the dimension of the next check.
+__device__ __forceinline__ int after_check(volatile DevState* vst, int nv, int m, int m_max, int64_t n, double tol,
+                                           int check_every) {
   bool all = true;
   double worst = 0.0;
-  for (int vv = 0; vv < NV; ++vv)
+  for (int vv = 0; vv < nv; ++vv)
     if (vst->m_conv[vv] == 0) {
       all = false;
       worst = fmax(worst, vst->worst[vv]);
@@ -918,6 +848,79 @@ __global__ void __launch_bounds__(kThreads) check_k(DevState* __restrict__ st, c
     vst->prev_m = m;
     vst->next_check = m + step;
   }
+  return done;
+}
+
+// Result of one problem's tridiagonal solve (one thread): residual bounds and
+// convergence.
+__device__ __forceinline__ void judge(volatile DevState* vst, int v, int mv, int kk, int k, bool exact, double tol,
+                                      const double* theta_v, double beta_mv, const double* S, int ld_s) {
+  bool ok = kk == k || exact;
+  double worst = 0.0;
+  for (int q = 0; q < kk; ++q) {
+    const double theta = theta_v[q];
+    const double last = S[(int64_t)q * ld_s + (mv - 1)];
+    const double r = exact ? 0.0 : fabs(beta_mv * last);
+    vst->resid[v][q] = r;
+    if (r > tol * fmax(1.0, fabs(theta))) ok = false;
+    worst = fmax(worst, r / fmax(1.0, fabs(theta)));
+  }
+  vst->m_use[v] = mv;
+  vst->worst[v] = ok ? 0.0 : worst;
+  if (ok) vst->m_conv[v] = mv;
+}
+
+// Convergence check after a step, launched after every step (one CTA per
+// problem).  It works only when the state's schedule says a check is due:
+// then each CTA of an unconverged problem finds the invariant-subspace
+// dimension, solves its tridiagonal matrix and tests the residual bounds;
+// the last CTA sets the done flag, schedules the next check from the
+// contraction of the worst residual (never sooner than check_every steps,
+// never later than 4 * check_every) and writes the progress words to the
+// host.  Otherwise block 0 only publishes the step count.
+template <int NV>
+__global__ void __launch_bounds__(kThreads) check_k(DevState* __restrict__ st, const double* __restrict__ alpha,
+                                                    int lda, const double* __restrict__ beta, int ldb, int m_max,
+                                                    int64_t n, int k, double tol, int check_every,
+                                                    double* __restrict__ tri_eval, double* __restrict__ tri_vec,
+                                                    int ld_s, double* __restrict__ tri_work,
+                                                    int32_t* __restrict__ host_progress) {
+  __shared__ int last_s;
+  volatile DevState* vst = st;
+  if (vst->done) return;
+  const int m = vst->j;
+  const bool due = m >= vst->next_check || m >= m_max || (int64_t)m >= n;
+  if (!due) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && host_progress) {
+      volatile int32_t* hp = host_progress;
+      hp[0] = m;
+    }
+    return;
+  }
+  const int v = blockIdx.x;
+  if (vst->m_conv[v] == 0) {
+    const double* al = alpha + (int64_t)v * lda;
+    const double* be = beta + (int64_t)v * ldb;
+    bool ends;
+    const int mv = edg::ritz_dimension(al, be, m, &ends), kk = k < mv ? k : mv;
+    const bool exact = ends || (int64_t)m == n;
+    double* S = tri_vec + (int64_t)v * kMaxK * ld_s;
+    for (int e = threadIdx.x; e < kMaxK * ld_s; e += kThreads) S[e] = 0.0;
+    __syncthreads();
+    tridiag_body(al, be, mv, kk, tri_eval + (int64_t)v * kMaxK, S, ld_s, tri_work + (int64_t)v * 6 * ld_s);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      judge(vst, v, mv, kk, k, exact, tol, tri_eval + (int64_t)v * kMaxK, be[mv], S, ld_s);
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last_s = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last_s || threadIdx.x != 0) return;
+  __threadfence();
+  vst->ticket = 0;
+  const int done = after_check(vst, NV, m, m_max, n, tol, check_every);
   vst->checks = vst->checks + 1;
   vst->done = done;
   __threadfence();
@@ -960,6 +963,335 @@ __global__ void ritz_k(const T* __restrict__ V, int64_t n_pad, int m, const doub
     double acc = 0.0;
     for (int i = 0; i < m; ++i) acc = fma(ldv(V, (int64_t)i * stride_i + g), s[i], acc);
     w[g] = acc;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// A whole solve as one cooperative launch (small sectors).  CTA b owns a run of
+// rows: its part of the matrix, of u and w and, where it fits, of the basis
+// stay in its shared memory.  A step is the product on its rows, the dots of
+// its rows with every vector of the window, a grid-wide wait, the totals and
+// coefficients (formed by every CTA from the same partials in the same
+// order), the update of its rows, and a second wait that publishes the next
+// candidate and |w|.  When a check is due CTA 0 solves the tridiagonal
+// matrices while the others wait.  The arithmetic of a row is that of the
+// passes above; only the order of the sums over rows differs.  Bound by the
+// two waits and the dependent L2 reads between them.  f64, one eigenpair (a
+// graph of five launches a step before): 61 rows 0.37 ms (1.32), 8,953 rows
+// 1.47 (2.81), 73,789 rows 2.08 (3.32), 147,578 rows 3.11 (3.80); mixed
+// precision 0.43 (1.31), 0.73 (1.72), 0.86 (1.87), 1.26 (2.11).  Past kCoopRows
+// rows per SM the basis leaves L2 and the streaming passes take over.  512
+// threads with four loads in flight measured best (1024 threads 2.50 ms at
+// 73,789 rows, eight loads 2.20).
+// ---------------------------------------------------------------------------
+constexpr int kCoopThreads = 512;
+constexpr int kCoopWarps = kCoopThreads / 32;
+constexpr int kCoopRows = 1024;             // most rows of a CTA
+constexpr int kCoopSmem = 190 * 1024;       // dynamic shared memory of a CTA (one per SM)
+constexpr int kCoopLanes = 4;               // lanes per row of the product
+
+template <typename T>
+struct CoopArgs {
+  const int64_t* rowptr;
+  const int32_t* cols;
+  const T* vals;
+  const T* diag;  // [n][NV]
+  const T* v0;    // [n][NV] or NULL
+  T* V;           // [m_max + 1][NV][n_pad], written and read by this launch
+  double* partial;  // [2 (m_max + 1) NV][G]
+  double* npart;    // [2][NV][G]
+  double *tri_eval, *tri_vec, *tri_work;
+  DevState* st;
+  unsigned* bar;
+  int* err;
+  int64_t n, n_pad;
+  uint64_t seed;
+  double tol;
+  int m_max, k, check_every, first_check, win, ld_s;
+};
+
+// Bytes of the fixed part of a CTA's shared memory: u, w | row offsets | alpha,
+// beta | totals.
+__host__ __device__ inline int64_t coop_fixed(int rows, int nv, int m_max) {
+  return (int64_t)rows * nv * 16 + (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)) +
+         (int64_t)nv * (m_max + 2) * 16 + (int64_t)nv * 2 * (m_max + 2) * 8;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs<T> A) {
+  constexpr int NV = 1;  // problems (batches of small ones have their own solver)
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ double red[NV][kCoopWarps];
+  __shared__ double total_s[NV], coef[NV][4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)gridDim.x, m_max = A.m_max;
+  const int64_t r0 = A.n_pad * blockIdx.x / G, r1 = A.n_pad * (blockIdx.x + 1) / G;
+  const int rows = (int)(r1 - r0);
+  double* const u = reinterpret_cast<double*>(sm);  // [NV][rows]
+  double* const w = u + (int64_t)rows * NV;
+  int32_t* const rp = reinterpret_cast<int32_t*>(w + (int64_t)rows * NV);
+  double* const al = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(rp) +
+                                               (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)));  // [NV][m_max + 2]
+  double* const be = al + (int64_t)NV * (m_max + 2);
+  double* const tot = be + (int64_t)NV * (m_max + 2);  // [NV][2 (m_max + 2)]
+  int64_t off = coop_fixed(rows, NV, m_max);
+  // the matrix rows (rows past n are empty)
+  const int64_t e0 = A.rowptr[r0 < A.n ? r0 : A.n], ne = A.rowptr[r1 < A.n ? r1 : A.n] - e0;
+  for (int r = tid; r <= rows; r += kCoopThreads) rp[r] = (int32_t)(A.rowptr[r0 + r < A.n ? r0 + r : A.n] - e0);
+  const T* vals = A.vals + e0;
+  const int32_t* cols = A.cols + e0;
+  if (off + ne * (int64_t)(sizeof(T) + 4) + 16 <= kCoopSmem) {
+    T* sv = reinterpret_cast<T*>(sm + off);
+    int32_t* sc = reinterpret_cast<int32_t*>(sv + ne);
+    for (int64_t e = tid; e < ne; e += kCoopThreads) {
+      sv[e] = vals[e];
+      sc[e] = cols[e];
+    }
+    vals = sv;
+    cols = sc;
+    off = (off + ne * (int64_t)(sizeof(T) + 4) + 15) & ~int64_t(15);
+  }
+  T* own = A.V + r0;  // this CTA's rows of the basis: vector stride ld_i, problem stride ld_v
+  int64_t ld_v = A.n_pad;
+  const bool basis_here = off + (int64_t)rows * NV * (m_max + 1) * (int64_t)sizeof(T) <= kCoopSmem;
+  if (basis_here) {
+    own = reinterpret_cast<T*>(sm + off);
+    ld_v = rows;
+  }
+  const int64_t ld_i = ld_v * NV;
+  edg::GridSync gs{A.bar, A.err};
+  unsigned waits = 0;
+  // totals over the grid of NV values per thread (in total_s); false when a
+  // wait ran out
+  auto grid_sum = [&](double (&a)[NV]) -> bool {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a[v] += __shfl_xor_sync(0xffffffffu, a[v], o);
+      if (lane == 0) red[v][warp] = a[v];
+    }
+    __syncthreads();
+    double* part = A.npart + (int64_t)(waits & 1) * NV * G;
+    ++waits;
+    if (tid < NV) {
+      double t = 0.0;
+      for (int q = 0; q < kCoopWarps; ++q) t += red[tid][q];
+      part[(int64_t)tid * G + blockIdx.x] = t;
+    }
+    if (!gs.wait()) return false;
+    if (warp < NV) {
+      double t = 0.0;
+      for (int b = lane; b < G; b += 32) t += __ldcg(part + (int64_t)warp * G + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) total_s[warp] = t;
+    }
+    __syncthreads();
+    return true;
+  };
+  // writes the candidate u_j (already rounded to T) to the basis
+  auto put = [&](int64_t i, int v, int r, double x) {
+    A.V[(i * NV + v) * A.n_pad + r0 + r] = (T)x;
+    if (basis_here) own[i * ld_i + v * ld_v + r] = (T)x;
+  };
+  // ---- start vector ----
+  double nrm[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    nrm[v] = 0.0;
+    for (int r = tid; r < rows; r += kCoopThreads) {
+      double x = 0.0;
+      if (r0 + r < A.n) {
+        if (A.v0) {
+          x = (double)A.v0[(r0 + r) * NV + v];
+        } else {
+          const uint64_t z = splitmix64(A.seed ^ splitmix64((uint64_t)((r0 + r) * NV + v)));
+          x = ((double)(z >> 11) * (1.0 / 9007199254740992.0)) * 2.0 - 1.0;
+        }
+      }
+      w[v * rows + r] = x;
+      nrm[v] = fma(x, x, nrm[v]);
+    }
+  }
+  for (int i = tid; i < NV * (m_max + 2); i += kCoopThreads) al[i] = be[i] = 0.0;
+  if (!grid_sum(nrm)) return;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const double nb = sqrt(total_s[v]), inv = nb > 0.0 ? 1.0 / nb : 0.0;
+    for (int r = tid; r < rows; r += kCoopThreads) {
+      const double x = (double)(T)(w[v * rows + r] * inv);
+      u[v * rows + r] = x;
+      put(0, v, r, x);
+    }
+  }
+  if (!gs.wait()) return;
+  int next_check = A.first_check;
+  for (int j = 0; j < m_max; ++j) {
+    const int lo = A.win > 0 && j > A.win ? j - A.win : 0;
+    const int n_vec = j + 1 - lo;
+    // ---- w = H u on this CTA's rows ----
+    {
+      const T* x = A.V + (int64_t)j * NV * A.n_pad;
+      const int part = tid & (kCoopLanes - 1);
+      const int n_it = (rows + kCoopThreads / kCoopLanes - 1) / (kCoopThreads / kCoopLanes);
+      for (int it = 0; it < n_it; ++it) {
+        const int r = it * (kCoopThreads / kCoopLanes) + tid / kCoopLanes;
+        double acc[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+        if (r < rows) {
+          constexpr int U = 4;  // gathers in flight per lane
+          const int end = rp[r + 1];
+          for (int p0 = rp[r] + part; p0 < end; p0 += U * kCoopLanes) {
+            T xv[U][NV], a[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+              if (p0 + q * kCoopLanes < end) {
+                const int c = cols[p0 + q * kCoopLanes];
+                a[q] = vals[p0 + q * kCoopLanes];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) xv[q][v] = x[(int64_t)v * A.n_pad + c];
+              }
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+              if (p0 + q * kCoopLanes < end)
+#pragma unroll
+                for (int v = 0; v < NV; ++v) acc[v] = fma((double)a[q], (double)xv[q][v], acc[v]);
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+#pragma unroll
+          for (int o = kCoopLanes / 2; o > 0; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o, kCoopLanes);
+          if (r < rows && part == 0) {
+            const int64_t gr = r0 + r;
+            const double d = gr < A.n ? (double)__ldg(A.diag + gr * NV + v) : 0.0;
+            w[v * rows + r] = fma(d, u[v * rows + r], acc[v]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // ---- dots of this CTA's rows: a warp per vector and problem ----
+    for (int e = warp; e < n_vec * NV; e += kCoopWarps) {
+      const int t = e / NV, v = e - t * NV;
+      const T* b = own + (int64_t)(lo + t) * ld_i + v * ld_v;
+      const double *uv = u + v * rows, *wv = w + v * rows;
+      double s = 0.0, z = 0.0;
+#pragma unroll 4
+      for (int r = lane; r < rows; r += 32) {
+        const double x = (double)b[r];
+        s = fma(x, uv[r], s);
+        z = fma(x, wv[r], z);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        z += __shfl_xor_sync(0xffffffffu, z, o);
+      }
+      if (lane == 0) {
+        A.partial[(int64_t)(2 * e) * G + blockIdx.x] = s;
+        A.partial[(int64_t)(2 * e + 1) * G + blockIdx.x] = z;
+      }
+    }
+    if (!gs.wait()) return;
+    // ---- totals and coefficients ----
+    for (int e = warp; e < 2 * n_vec * NV; e += kCoopWarps) {
+      double a = 0.0;
+      for (int b = lane; b < G; b += 32) a += __ldcg(A.partial + (int64_t)e * G + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) {
+        const int t = (e >> 1) / NV, v = (e >> 1) - t * NV;
+        tot[(int64_t)v * 2 * (m_max + 2) + 2 * t + (e & 1)] = a;
+      }
+    }
+    __syncthreads();
+    if (warp < NV) {
+      double out[4];
+      double* alv = al + (int64_t)warp * (m_max + 2);
+      double* bev = be + (int64_t)warp * (m_max + 2);
+      coef_small(lo, j, tot + (int64_t)warp * 2 * (m_max + 2), alv, bev, out);
+      __syncwarp();
+      if (lane == 0) {
+        for (int q = 0; q < 4; ++q) coef[warp][q] = out[q];
+        alv[j] = out[2];
+        if (j > lo) bev[j] = out[3];
+      }
+    }
+    __syncthreads();
+    // ---- V[j] = q, the next candidate w / r ----
+    const int lpr = rows * 2 <= kCoopThreads ? 2 : 1;  // lanes per row
+    const int part = tid & (lpr - 1);
+    const int n_it = (rows * lpr + kCoopThreads - 1) / kCoopThreads;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const double ri = coef[v][0], c = coef[v][1];
+      const double* tv = tot + (int64_t)v * 2 * (m_max + 2);
+      nrm[v] = 0.0;
+      for (int it = 0; it < n_it; ++it) {
+        const int r = (it * kCoopThreads + tid) / lpr;
+        double su = 0.0, sw = 0.0;
+        if (r < rows) {
+          const T* b = own + (int64_t)lo * ld_i + v * ld_v + r;
+#pragma unroll 8
+          for (int t = part; t < n_vec - 1; t += lpr) {
+            const double x = (double)b[(int64_t)t * ld_i];
+            su = fma(x, tv[2 * t], su);
+            sw = fma(x, tv[2 * t + 1], sw);
+          }
+        }
+        if (lpr == 2) {
+          su += __shfl_xor_sync(0xffffffffu, su, 1);
+          sw += __shfl_xor_sync(0xffffffffu, sw, 1);
+        }
+        if (r < rows && part == 0) {
+          const double q = (double)(T)((u[v * rows + r] - su) * ri);
+          double y = (w[v * rows + r] - sw) - q * c;
+          nrm[v] = fma(y, y, nrm[v]);
+          y = (double)(T)(y * ri);
+          u[v * rows + r] = y;
+          put(j, v, r, q);
+          put(j + 1, v, r, y);
+        }
+      }
+    }
+    if (!grid_sum(nrm)) return;
+    if (tid < NV) be[(int64_t)tid * (m_max + 2) + j + 1] = sqrt(total_s[tid]) * coef[tid][0];
+    __syncthreads();
+    // ---- convergence ----
+    const int m = j + 1;
+    if (m >= next_check || m >= m_max || (int64_t)m >= A.n) {
+      volatile DevState* vst = A.st;
+      if (blockIdx.x == 0) {
+        for (int v = 0; v < NV; ++v) {
+          if (vst->m_conv[v] != 0) continue;
+          const double* alv = al + (int64_t)v * (m_max + 2);
+          const double* bev = be + (int64_t)v * (m_max + 2);
+          double* S = A.tri_vec + (int64_t)v * kMaxK * A.ld_s;
+          bool ends;
+          const int mv = edg::ritz_dimension<kCoopThreads>(alv, bev, m, &ends), kk = A.k < mv ? A.k : mv;
+          const bool exact = ends || (int64_t)m == A.n;
+          for (int e = tid; e < kMaxK * A.ld_s; e += kCoopThreads) S[e] = 0.0;
+          __syncthreads();
+          tridiag_body<kCoopThreads>(alv, bev, mv, kk, A.tri_eval + (int64_t)v * kMaxK, S, A.ld_s,
+                                     A.tri_work + (int64_t)v * 6 * A.ld_s);
+          __syncthreads();
+          if (tid == 0)
+            judge(vst, v, mv, kk, A.k, exact, A.tol, A.tri_eval + (int64_t)v * kMaxK, bev[mv], S, A.ld_s);
+          __syncthreads();
+        }
+        if (tid == 0) {
+          const int done = after_check(vst, NV, m, m_max, A.n, A.tol, A.check_every);
+          vst->checks = vst->checks + 1;
+          vst->j = m;
+          vst->done = done;
+        }
+      }
+      if (!gs.wait()) return;
+      if (vst->done) return;
+      next_check = vst->next_check;
+    }
   }
 }
 
@@ -1057,8 +1389,37 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
       progress[1] = 0;
     }
   }
+  // small sectors: the whole solve in one cooperative launch (the instrumented
+  // path times the passes one by one)
+  bool coop_done = false;
+  if (NV == 1 && p->stats == nullptr && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
+    int dev = 0, n_sm = 0, coop = 0, occ = 0;
+    auto kern = lanczos_coop_k<T>;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
+    if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: set-up");
+    int64_t g = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
+    if (g > (n_pad + 255) / 256) g = (n_pad + 255) / 256;  // fewer CTAs than rows to keep them busy
+    const int rows = (int)((n_pad + g - 1) / g);
+    if (coop && occ >= 1 && rows <= kCoopRows && coop_fixed(rows, NV, L.m_max) <= kCoopSmem) {
+      state_init_k<<<1, 32, 0, s>>>(st, first_check, p->reorth_window);
+      if ((e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s)) != cudaSuccess)
+        return edg::cuda_status(e, "edg_lanczos: tickets");
+      CoopArgs<T> a{p->rowptr, p->cols, (const T*)p->vals, (const T*)p->diag, (const T*)p->v0, V, partial, normp,
+                    tri_eval, tri_vec, tri_work, st, small_bar, err_word, n, n_pad, p->seed, p->tol, L.m_max, k,
+                    p->check_every, first_check, p->reorth_window, ld_s};
+      void* args[] = {&a};
+      e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)g), dim3(kCoopThreads), args, kCoopSmem, s);
+      if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: cooperative launch");
+      coop_done = true;
+    }
+  }
   // padding rows (r >= n) of w are zero from start_k on, so every Krylov plane
   // written from w has zero padding and no reset of V is needed
+  if (!coop_done) {
   start_k<T, NV><<<edg::grid_for(n_pad * NV, 256), 256, 0, s>>>(n, n_pad, p->seed, (const T*)p->v0, w);
   norm_k<NV><<<L.nblk_upd, kThreads, 0, s>>>(w, n_pad, normp);
   beta_k<NV><<<1, kThreads, 0, s>>>(normp, L.nblk_upd, h);
@@ -1069,6 +1430,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   if ((e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s)) != cudaSuccess)
     return edg::cuda_status(e, "edg_lanczos: tickets");
   if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: start");
+  }
   // the reorthogonalisation passes: persistent grids of the bulk-copy kernels
   const size_t dot_smem = sizeof(edg::bulk::Smem<T>);
   const size_t upd_smem = sizeof(edg::bulk::Smem<T>);
@@ -1207,7 +1569,9 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   int64_t launches = 9;
   DevState hs{};
   int rc_ = EDG_OK;
-  if (timing) {
+  if (coop_done) {
+    // everything is in the one launch
+  } else if (timing) {
     // instrumented: steps launched one by one with events around each phase
     cudaEvent_t ev[4];
     for (auto& x : ev) cudaEventCreate(&x);

@@ -516,34 +516,25 @@ __global__ void __launch_bounds__(kThreads) tiled_lanczos_k(Params p) {
         if (m > I.m_cap) continue;
         const double* al = I.f + I.L.alpha;
         const double* be = I.f + I.L.beta;
-        __shared__ int mv_s, exact_s, done_s;
-        if (threadIdx.x == 0) {
-          double scale = 0.0;
-          for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(__ldcg(al + i)) + fabs(__ldcg(be + i)));
-          const double thr = 1e-12 * fmax(scale, 1e-300);
-          int mv = m;
-          for (int i = 1; i <= m; ++i)
-            if (fabs(__ldcg(be + i)) <= thr) { mv = i; break; }
-          mv_s = mv;
-          exact_s = mv < m || (mv == m && fabs(__ldcg(be + m)) <= thr) || (int64_t)m == I.dim;
-        }
-        __syncthreads();
-        const int mv = mv_s, kk = p.k < mv ? p.k : mv;
-        const int64_t ld = I.m_cap + 1;
-        for (int64_t e = threadIdx.x; e < (int64_t)p.k * ld; e += kThreads) I.f[I.L.S + e] = 0.0;
+        __shared__ int done_s;
         // the coefficients were written by other CTAs: stage them through L2
         double* a_s = sz;
         double* b_s = sz + (kMaxIter + 1);
-        for (int i = threadIdx.x; i <= mv; i += kThreads) {
-          if (i < mv) a_s[i] = __ldcg(al + i);
+        for (int i = threadIdx.x; i <= m; i += kThreads) {
+          if (i < m) a_s[i] = __ldcg(al + i);
           b_s[i] = __ldcg(be + i);
         }
+        __syncthreads();
+        bool ends;
+        const int mv = edg::ritz_dimension(a_s, b_s, m, &ends), kk = p.k < mv ? p.k : mv;
+        const bool exact = ends || (int64_t)m == I.dim;
+        const int64_t ld = I.m_cap + 1;
+        for (int64_t e = threadIdx.x; e < (int64_t)p.k * ld; e += kThreads) I.f[I.L.S + e] = 0.0;
         __syncthreads();
         double* ev = I.f + I.L.misc + 8 + kMaxK;
         edg::tridiag_body(a_s, b_s, mv, kk, ev, I.f + I.L.S, (int)ld, I.f + I.L.tri);
         __syncthreads();
         if (threadIdx.x == 0) {
-          const bool exact = exact_s != 0;
           bool ok = kk == p.k || exact;
           double* rs = I.f + I.L.misc + 8;
           for (int q = 0; q < kk; ++q) {
