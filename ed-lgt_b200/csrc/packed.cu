@@ -19,20 +19,29 @@
 //   edg_pack_encode       writes the tile offsets and the packed words (binary
 //                         search of each value in the sorted table).
 //
-// Matvec (packed_spmv_k): one warp takes tiles of 16 consecutive rows.  A
-// tile is a contiguous, 64-byte-aligned range of the stream, which lane 0
-// copies into one of the warp's two shared-memory stages with a bulk
-// asynchronous copy (completion on the stage's mbarrier) one tile ahead,
-// while the tile offsets are loaded two tiles ahead; two lanes per row then
-// walk their row from shared memory (lane j takes entries j, j + 2, j + 4,
-// ...; the two lanes of all 16 rows read 32 consecutive words), gathering x
-// rows.  The stream is read with whole-range copies that bypass the load
-// pipeline (the CSR kernel's loads touch one segment per row of the warp on
-// every load), which leaves the L1 data pipe to the gathers.  f32 matrices
-// (the f32 Krylov phase) sum each lane's products in f32 and add the lane
-// sums and the diagonal term in f64, so no conversion happens per entry; f64
+// Matvec (packed_spmv_k): one warp takes a tile, or two neighbouring tiles, at
+// a time.  Their words are one contiguous, 64-byte-aligned range of the stream,
+// which lane 0 copies into one of the warp's two shared-memory stages with a
+// bulk asynchronous copy (completion on the stage's mbarrier) one step ahead,
+// while the tile offsets are loaded two steps ahead; two lanes per row then
+// walk the rows of each tile from shared memory (lane j takes entries j, j + 2,
+// j + 4, ...; the two lanes of all 16 rows read 32 consecutive words),
+// gathering x rows.  The stream is read with whole-range copies that bypass the
+// load pipeline (the CSR kernel's loads touch one segment per row of the warp
+// on every load), which leaves the L1 data pipe to the gathers.  f32 matrices
+// (the f32 Krylov phase) sum each lane's products in f32 and add the lane sums
+// and the diagonal term in f64, so no conversion happens per entry; f64
 // matrices sum in f64 in the CSR kernel's order (bit-identical to the CSR
 // kernel with two threads a row).
+//
+// Two tiles a step when an x row has at most 8 bytes: the two lanes of a row
+// exchange halves, lane 0 finishes the first tile's row and lane 1 the
+// second's, so that the diagonal, y and the epilogue run with all lanes at
+// work (one tile at a time they were more than half of the instructions).
+// complex64 on SU(2) L = 16 (7,133,222 rows, 124M words, with the Krylov
+// epilogue): 283 -> 221 us; one f32 vector on the L = 14 ring 37.0 -> 33.0 us.
+// Wider x rows live off L1, which the larger stages shrink (three f64 vectors
+// on the ring: 76 us one tile at a time, 95 with two).
 #include <algorithm>
 
 #include "reorth_bulk.cuh"
@@ -41,8 +50,11 @@
 namespace {
 
 constexpr int kTileRows = 16;   // rows of a warp tile (two lanes a row)
-constexpr int kTileWords = 512;  // staged entries of a tile; longer tiles read the stream directly
-constexpr int kStageWords = kTileWords + 4;
+// Tiles a warp takes at a time, and the words of a stage (24 a row of a pair,
+// 32 a row of a single tile; longer ones read the stream directly).
+template <typename T, int XS>
+constexpr int tiles_of() { return sizeof(T) * XS <= 8 ? 2 : 1; }
+constexpr int stage_words(int tiles) { return tiles == 2 ? 768 : 516; }
 constexpr int kWarps = 8;  // warps of a CTA
 
 template <typename T>
@@ -197,36 +209,30 @@ __global__ void pack_encode_k(int64_t n, int64_t total, const int64_t* __restric
   if (t0 < 4) words[total + t0] = 0xFFFFFFFFu;
 }
 
-struct Tile {
-  int64_t r0;
-  int nr;  // rows of the tile (0: past the end)
-};
-__device__ __forceinline__ Tile tile_of(int64_t t, int64_t n) {
-  const int64_t r0 = t * kTileRows;
-  const int64_t left = n - r0;
-  return {r0, left <= 0 ? 0 : (int)(left < kTileRows ? left : kTileRows)};
+// Lanes 0..NT hold tile_off[NT t + lane] of step t (clamped to the last offset:
+// a step past the end, or the missing second tile of the last pair, is empty).
+template <int NT>
+__device__ __forceinline__ int32_t load_head(const int32_t* __restrict__ tile_off, int64_t t, int64_t n_tiles,
+                                             int lane) {
+  const int64_t i = NT * t + lane;
+  return lane <= NT ? __ldg(tile_off + (i < n_tiles ? i : n_tiles)) : 0;
 }
 
-// Lanes 0 and 1 hold tile_off[t], tile_off[t + 1].
-__device__ __forceinline__ int32_t load_head(const int32_t* __restrict__ tile_off, int64_t t, Tile tl, int lane) {
-  return tl.nr > 0 && lane < 2 ? __ldg(tile_off + t + lane) : 0;
-}
-
-// A tile's words [e0, e0 + 16 width) (e0 a multiple of 16: 64-byte aligned);
-// `fits` when they fit the stage.
+// A step's words [e0, e0 + 16 (wa + wb)) (e0 a multiple of 16: 64-byte
+// aligned), wa and wb the widths of its tiles; `fits` when they fit the stage.
 struct Range {
-  int32_t e0, width, quads;
+  int32_t e0, wa, wb, quads;
   bool fits;
 };
-__device__ __forceinline__ Range range_of(Tile tl, int32_t head) {
+template <int NT>
+__device__ __forceinline__ Range range_of(int32_t head) {
   const int32_t e0 = __shfl_sync(0xffffffffu, head, 0);
-  const int32_t e1 = __shfl_sync(0xffffffffu, head, 1);
-  const int32_t width = tl.nr > 0 ? (e1 - e0) / kTileRows : 0;
-  const int32_t quads = width * (kTileRows / 4);
-  return {e0, width, quads, width * kTileRows <= kTileWords};
+  const int32_t em = __shfl_sync(0xffffffffu, head, 1);
+  const int32_t e1 = NT == 2 ? __shfl_sync(0xffffffffu, head, 2) : em;
+  return {e0, (em - e0) / kTileRows, (e1 - em) / kTileRows, (e1 - e0) / 4, e1 - e0 <= stage_words(NT) / 16 * 16};
 }
 
-// Lane 0 copies the tile's range into a stage with one bulk asynchronous copy
+// Lane 0 copies the step's range into a stage with one bulk asynchronous copy
 // (this GPU's memory, no multicast) completing on the stage's mbarrier;
 // returns whether a copy was issued (warp-uniform).
 __device__ __forceinline__ bool stage_tile(const uint32_t* __restrict__ words, Range rg, uint32_t* stage,
@@ -397,6 +403,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
                   const T* __restrict__ x, double* __restrict__ y, int64_t y_plane, int diag_shared,
                   const int* __restrict__ skip, int* __restrict__ err, Epi epi) {
   using A = T;  // lane accumulator: f32 lanes for the f32 phase, f64 otherwise
+  constexpr int NT = tiles_of<T, XS>(), kStageWords = stage_words(NT);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_err;
   if (skip != nullptr && *skip) return;
@@ -415,47 +422,54 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   __syncthreads();
   uint32_t* const stage0 = stage_all + warp * 2 * kStageWords;  // two stages of kStageWords
   const uint32_t cmask = (1u << colbits) - 1u;
-  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows;
+  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows, n_steps = (n_tiles + NT - 1) / NT;
   const int64_t step = (int64_t)gridDim.x * kWarps;
   const int s = lane >> 1, j = lane & 1;
   int64_t t = (int64_t)blockIdx.x * kWarps + warp;
-  // pipeline: the words of tile t are staged one tile ahead, the tile
-  // offsets loaded two tiles ahead
-  Tile cur = tile_of(t, n), nxt = tile_of(t + step, n);
-  int32_t h_cur = load_head(tile_off, t, cur, lane);
-  int32_t h_nxt = load_head(tile_off, t + step, nxt, lane);
-  Range rg_cur = range_of(cur, h_cur);
+  // pipeline: the words of step t are staged one step ahead, the tile offsets
+  // loaded two steps ahead
+  int32_t h_nxt = load_head<NT>(tile_off, t + step, n_tiles, lane);
+  Range rg_cur = range_of<NT>(load_head<NT>(tile_off, t, n_tiles, lane));
   // bit s of pend: a copy into stage s is in flight; bit s of phase: the
   // parity of that stage's mbarrier for its next completion
   unsigned pend = stage_tile(words, rg_cur, stage0, &bar[0], lane) ? 1u : 0u;
   unsigned phase = 0u;
   int b = 0;
-  for (; t < n_tiles; t += step) {
-    const Tile nn = tile_of(t + 2 * step, n);
-    const Range rg_nxt = range_of(nxt, h_nxt);
+  for (; t < n_steps; t += step) {
+    const Range rg_nxt = range_of<NT>(h_nxt);
     if (stage_tile(words, rg_nxt, stage0 + (b ^ 1) * kStageWords, &bar[b ^ 1], lane)) pend |= 2u >> b;
-    const int32_t h_nn = load_head(tile_off, t + 2 * step, nn, lane);
+    h_nxt = load_head<NT>(tile_off, t + 2 * step, n_tiles, lane);
     if (pend & (1u << b)) {
       const bool ok = edg::bulk::wait_bounded(&bar[b], (phase >> b) & 1u, &s_err);
       if (!__all_sync(0xffffffffu, ok)) break;  // warp-uniform
       pend &= ~(1u << b);
       phase ^= 1u << b;
     }
-    A acc[NV];
+    A acc[NT][NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) acc[v] = (A)0;
+    for (int h = 0; h < NT; ++h)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[h][v] = (A)0;
+    const uint32_t* const src = rg_cur.fits ? stage0 + b * kStageWords : words + rg_cur.e0;
     if (rg_cur.fits)
-      gather_tile<T, A, NV, XS>(stage0 + b * kStageWords, rg_cur.width, s, j, tab, colbits, cmask, x, acc, true);
+      gather_tile<T, A, NV, XS>(src, rg_cur.wa, s, j, tab, colbits, cmask, x, acc[0], true);
     else
-      gather_tile<T, A, NV, XS>(words + rg_cur.e0, rg_cur.width, s, j, tab, colbits, cmask, x, acc, false);
+      gather_tile<T, A, NV, XS>(src, rg_cur.wa, s, j, tab, colbits, cmask, x, acc[0], false);
+    if constexpr (NT == 2) {
+      if (rg_cur.fits)
+        gather_tile<T, A, NV, XS>(src + kTileRows * rg_cur.wa, rg_cur.wb, s, j, tab, colbits, cmask, x, acc[1], true);
+      else
+        gather_tile<T, A, NV, XS>(src + kTileRows * rg_cur.wa, rg_cur.wb, s, j, tab, colbits, cmask, x, acc[1], false);
+    }
+    // lane j of a row's two lanes finishes the row of tile j
     double tot[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      tot[v] = (double)acc[v];
-      tot[v] += __shfl_xor_sync(0xffffffffu, tot[v], 1, 2);
+      const A other = __shfl_xor_sync(0xffffffffu, j == 0 ? acc[NT - 1][v] : acc[0][v], 1);
+      tot[v] = (double)(j == 0 ? acc[0][v] : acc[NT - 1][v]) + (double)other;
     }
-    if (s < cur.nr && j == 0) {
-      const int64_t r = cur.r0 + s;
+    const int64_t r = (int64_t)NT * kTileRows * t + kTileRows * j + s;
+    if (r < n && j < NT) {
       T xr[NV];
       XRow<T, NV, XS>::ld(x, r, xr);
 #pragma unroll
@@ -467,10 +481,6 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
       epi.row(r, xr, tot);
     }
     __syncwarp();  // this stage is refilled by the next iteration
-    cur = nxt;
-    nxt = nn;
-    h_cur = h_nxt;
-    h_nxt = h_nn;
     rg_cur = rg_nxt;
     b ^= 1;
   }
@@ -487,9 +497,16 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   epi.finish();
 }
 
-template <typename T>
+template <typename T, int XS>
 size_t packed_smem(int count) {
-  return sizeof(uint32_t) * kWarps * 2 * kStageWords + sizeof(uint64_t) * kWarps * 2 + sizeof(T) * (size_t)count;
+  return sizeof(uint32_t) * kWarps * 2 * stage_words(tiles_of<T, XS>()) + sizeof(uint64_t) * kWarps * 2 + sizeof(T) * (size_t)count;
+}
+
+// One wave: four resident CTAs an SM, each warp a step at a time.
+unsigned packed_grid(int64_t n, int tiles) {
+  const int64_t steps = (n + (int64_t)tiles * kTileRows - 1) / ((int64_t)tiles * kTileRows);
+  const int64_t need = (steps + kWarps - 1) / kWarps;
+  return (unsigned)(need < (int64_t)edg::kSmCount * 4 ? need : (int64_t)edg::kSmCount * 4);
 }
 
 template <typename T>
@@ -520,18 +537,16 @@ template <typename T>
 int launch_packed_spmv(int nvec, int x_stride, int64_t n, const int32_t* tile_off, const uint32_t* words,
                        const T* table, int count, int colbits, const T* diag, const T* x, double* y, int64_t y_plane,
                        const int* skip, int* err, cudaStream_t s, int diag_shared) {
-  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows;
-  const int64_t need = (n_tiles + kWarps - 1) / kWarps;
-  const unsigned grid = (unsigned)(need < (int64_t)kSmCount * 4 ? need : (int64_t)kSmCount * 4);
-  const size_t smem = packed_smem<T>(count);
   cudaError_t e = cudaSuccess;
 #define EDG_PACKED(NV, XS)                                                                                          \
   do {                                                                                                              \
     auto kern = packed_spmv_k<T, NV, XS, NoEpilogue>;                                                              \
+    const size_t smem = packed_smem<T, XS>(count);                                                                 \
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
     if (e == cudaSuccess)                                                                                           \
-      kern<<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, y, y_plane,         \
-                                           diag_shared, skip, err, NoEpilogue{});                                   \
+      kern<<<packed_grid(n, tiles_of<T, XS>()), kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, \
+                                                                        diag, x, y, y_plane, diag_shared, skip,    \
+                                                                        err, NoEpilogue{});                         \
   } while (0)
   switch (nvec) {
     case 1: EDG_PACKED(1, 1); break;
@@ -562,10 +577,8 @@ template <typename T>
 int launch_packed_krylov(int64_t n, const int32_t* tile_off, const uint32_t* words, const T* table, int count,
                          int colbits, const T* diag, const T* x, double* y, const KrylovStep& step, int* err,
                          cudaStream_t s) {
-  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows;
-  const int64_t need = (n_tiles + kWarps - 1) / kWarps;
-  const unsigned grid = (unsigned)(need < (int64_t)kSmCount * 4 ? need : (int64_t)kSmCount * 4);
-  const size_t smem = packed_smem<T>(count);
+  const unsigned grid = packed_grid(n, tiles_of<T, 2>());
+  const size_t smem = packed_smem<T, 2>(count);
   auto kern = packed_spmv_k<T, 2, 2, KrylovEpilogue>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
