@@ -1392,7 +1392,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   // small sectors: the whole solve in one cooperative launch (the instrumented
   // path times the passes one by one)
   bool coop_done = false;
-  if (NV == 1 && p->stats == nullptr && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
+  if (NV == 1 && p->stats == nullptr && (p->vals != nullptr || p->nnz == 0) && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
     int dev = 0, n_sm = 0, coop = 0, occ = 0;
     auto kern = lanczos_coop_k<T>;
     e = cudaGetDevice(&dev);
@@ -1729,6 +1729,8 @@ int check_problem(const edg_lanczos_problem* p) {
 }
 
 }  // namespace
+
+extern "C" int64_t edg_lanczos_small_rows(void) { return (int64_t)kCoopRows * edg::kSmCount / 4 * 4; }
 
 extern "C" int64_t edg_lanczos_workspace_bytes(const edg_lanczos_problem* p) {
   if (check_problem(p)) return -1;

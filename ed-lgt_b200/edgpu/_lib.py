@@ -14,7 +14,7 @@ from ._build import LIB_PATH
 
 __all__ = ["lib", "check", "EdgError", "MAX_SITES", "MAX_OPS", "SectorTables", "LookupTable", "Assembly",
            "LanczosProblem", "SiteDims", "KrylovProblem", "SmallBatch", "ZnTranslation", "ZnLattice", "ZnBasis",
-           "ZN_MAX_SITES", "ZN_MAX_GROUP", "EXPORTED_SYMBOLS", "ptr", "stream_handle"]
+           "ZN_MAX_SITES", "ZN_MAX_GROUP", "EXPORTED_SYMBOLS", "ptr", "stream_handle", "upload_arrays"]
 
 MAX_SITES = 64
 MAX_OPS = 4
@@ -319,6 +319,7 @@ _SIGS = {
     "edg_pack_encode": (I32, [I32, I64, I64, P, P, P, P, I32, I32, P, P, P, P, P]),
     "edg_spmv_packed": (I32, [I32, I64, I32, P, P, P, I32, I32, P, P, I32, P, I64, P, P]),
     "edg_spmv_group": (I32, [I32, I64, I64, P, P, P, P, I32, P, P, I32, P]),
+    "edg_lanczos_small_rows": (I64, []),
     "edg_lanczos_workspace_bytes": (I64, [C.POINTER(LanczosProblem)]),
     "edg_lanczos": (I32, [C.POINTER(LanczosProblem), P, I64, P, P, P, P, P]),
     "edg_tridiag_lowest": (I32, [P, P, I32, I32, P, P, P, P]),
@@ -406,6 +407,29 @@ def ptr(t) -> int | None:
     if t is None:
         return None
     return t.data_ptr()
+
+
+def upload_arrays(device, arrays):
+    """Device copies of several host arrays by one transfer: ``arrays`` maps
+    names to (array, dtype); each becomes a flat tensor view, 16-byte aligned,
+    of one buffer (an empty array gets one zero element)."""
+    import numpy as np
+    import torch
+
+    flat, spans, at = [], [], 0
+    for a, dtype in arrays.values():
+        a = np.ascontiguousarray(a, dtype=dtype).reshape(-1)
+        if a.size == 0:
+            a = np.zeros(1, dtype=dtype)
+        flat.append(a)
+        spans.append((at, at + a.nbytes))
+        at = (at + a.nbytes + 15) // 16 * 16
+    host = np.zeros(at, dtype=np.uint8)
+    for a, (lo, hi) in zip(flat, spans):
+        host[lo:hi] = a.view(np.uint8)
+    buf = torch.from_numpy(host).to(device)
+    kinds = {"uint8": torch.uint8, "int32": torch.int32, "float64": torch.float64}
+    return {name: buf[lo:hi].view(kinds[a.dtype.name]) for name, a, (lo, hi) in zip(arrays, flat, spans)}
 
 
 def stream_handle(stream=None) -> int | None:

@@ -17,7 +17,6 @@ ordering agree with the reference:
 
 from __future__ import annotations
 
-from itertools import product
 from math import prod
 
 import numpy as np
@@ -33,6 +32,9 @@ __all__ = [
     "staggered_mask",
     "site_is_even",
     "link_site_pairs",
+    "neighbor_pairs",
+    "plaquette_quads",
+    "site_coords",
     "origin_surfaces",
     "border_labels",
 ]
@@ -121,27 +123,55 @@ def lattice_labels(lvals, has_obc, staggered_basis):
     ]
 
 
+def site_coords(lvals):
+    """(n_sites, dim) coordinates in linear site order (x fastest)."""
+    grid = np.indices(tuple(int(l) for l in reversed(lvals))).reshape(len(lvals), -1)
+    return grid[::-1].T
+
+
+def _shifted(coords, lvals, axis, has_obc):
+    """Linear index of every site moved one step along ``axis`` (an index into
+    coords' columns), and whether that step stays on the lattice."""
+    strides = np.array(_strides(lvals), dtype=np.int64)
+    moved = coords.copy()
+    moved[:, axis] = (moved[:, axis] + 1) % int(lvals[axis])
+    inside = np.ones(len(coords), dtype=bool) if not has_obc[axis] else coords[:, axis] < int(lvals[axis]) - 1
+    return moved, moved @ strides, inside
+
+
+def neighbor_pairs(lvals, axis, has_obc):
+    """neighbor_sites of every site at once: (n_sites, 2) links leaving the
+    sites along ``axis`` and which of them exist."""
+    coords = site_coords(lvals)
+    _, to, inside = _shifted(coords, lvals, AXES.index(axis), has_obc)
+    return np.stack([np.arange(len(coords)), to], axis=1), inside
+
+
+def plaquette_quads(lvals, axes, has_obc):
+    """plaquette_sites of every site at once: (n_sites, 4) corners and which of
+    the plaquettes exist."""
+    coords = site_coords(lvals)
+    ia, ib = AXES.index(axes[0]), AXES.index(axes[1])
+    ma, a, in_a = _shifted(coords, lvals, ia, has_obc)
+    _, b, in_b = _shifted(coords, lvals, ib, has_obc)
+    _, ab, _ = _shifted(ma, lvals, ib, has_obc)
+    return np.stack([np.arange(len(coords)), a, b, ab], axis=1), in_a & in_b
+
+
 def staggered_mask(lvals, stag_label):
     """Boolean lattice-shaped mask of even or odd sites."""
     if stag_label not in ("even", "odd"):
         raise ValueError(f"stag_label must be 'even' or 'odd', got {stag_label}")
-    mask = np.zeros(tuple(lvals), dtype=bool)
-    for coords in product(*[range(l) for l in lvals]):
-        even = site_is_even(coords)
-        mask[coords] = even if stag_label == "even" else not even
-    return mask
+    even = np.indices(tuple(lvals)).sum(axis=0) % 2 == 0
+    return even if stag_label == "even" else ~even
 
 
 def link_site_pairs(lvals, has_obc):
     """Per-axis arrays of linked site pairs, in linear site order."""
     out = []
     for axis in AXES[: len(lvals)]:
-        pairs = []
-        for ii in range(prod(lvals)):
-            s = neighbor_sites(zig_zag(lvals, ii), lvals, axis, has_obc)
-            if s is not None:
-                pairs.append(s)
-        out.append(np.array(pairs, dtype=np.int32).reshape(-1, 2))
+        pairs, inside = neighbor_pairs(lvals, axis, has_obc)
+        out.append(np.ascontiguousarray(pairs[inside], dtype=np.int32).reshape(-1, 2))
     return out
 
 

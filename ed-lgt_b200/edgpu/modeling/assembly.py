@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from .. import _lib
-from .._lib import check, lib, ptr, stream_handle
+from .._lib import check, lib, ptr, stream_handle, upload_arrays
 from .terms import TermBlock
 
 __all__ = ["DeviceMatrix", "assemble_blocks", "OP_TOL"]
@@ -122,6 +122,12 @@ def _phase_vec(weights_row):
     return np.power(1j, np.asarray(weights_row, dtype=np.int64) % 4)
 
 
+def _nonzero(m):
+    """np.nonzero of a complex array (several times faster than testing the
+    complex values)."""
+    return np.nonzero((m.real != 0) | (m.imag != 0))
+
+
 def _offdiag_signature(blocks, phase_weights, force_complex, dmax):
     """Content hash of everything the off-diagonal part of the matrix depends
     on: the off-diagonal blocks' operators, instances, strengths and h.c.
@@ -145,51 +151,65 @@ def _offdiag_tables(blocks, phase_weights, force_complex, dmax):
     """Local transition tables and instance records of the off-diagonal
     blocks, and whether they admit the real form (every gauge-transformed
     table has one common phase and every instance's total phase is real)."""
-    raw_tables = []  # list of (d x d) complex matrices
-    table_site = []
-    table_index = {}
+    keys = []  # (block, factor, site, conjugated) of every table
+    index = {}
     terms = []  # (sites tuple, tables tuple, coef)
     for bi, b in enumerate(blocks):
         if b.diagonal:
             continue
+        sites = b.sites.tolist()
         for dag in ([False, True] if b.add_dagger else [False]):
-            for inst in b.sites:
+            coef = complex(np.conj(b.strength) if dag else b.strength)
+            for inst in sites:
                 tabs = []
                 for j, s in enumerate(inst):
-                    key = (bi, j, int(s), dag)
-                    if key not in table_index:
-                        m = np.asarray(b.ops[j][int(s)], dtype=np.complex128)
-                        if dag:
-                            m = m.conj().T
-                        table_index[key] = len(raw_tables)
-                        raw_tables.append(m)
-                        table_site.append(int(s))
-                    tabs.append(table_index[key])
-                if len(set(int(s) for s in inst)) != len(inst):
+                    key = (bi, j, s, dag)
+                    t = index.get(key)
+                    if t is None:
+                        t = index[key] = len(keys)
+                        keys.append(key)
+                    tabs.append(t)
+                if len(set(inst)) != len(inst):
                     raise ValueError("a term instance acts twice on the same site")
-                coef = np.conj(b.strength) if dag else b.strength
-                terms.append((tuple(int(s) for s in inst), tuple(tabs), complex(coef)))
+                terms.append((tuple(inst), tuple(tabs), coef))
+    table_site = [k[2] for k in keys]
+    raw_tables = np.zeros((len(keys),) + (() if not keys else blocks[keys[0][0]].ops[0].shape[-2:]),
+                          dtype=np.complex128)
+    same = {}  # tables that come from one operator: one gather
+    for t, (bi, j, s, dag) in enumerate(keys):
+        same.setdefault((bi, j, dag), ([], []))
+        same[bi, j, dag][0].append(t)
+        same[bi, j, dag][1].append(s)
+    for (bi, j, dag), (ts, ss) in same.items():
+        m = np.asarray(blocks[bi].ops[j])[ss]
+        raw_tables[ts] = m.conj().transpose(0, 2, 1) if dag else m
     real_ok, tables_real, coefs_real = False, None, None
-    if not force_complex and raw_tables:
-        # every table at once: gauge-transform, then its common phase (the
-        # phase of its largest entry above OP_TOL, the first in row-major
-        # order), as _uniform_phase does table by table
-        M = np.stack(raw_tables)
+    if not force_complex and len(raw_tables):
+        # every table at once, on its nonzero entries: gauge-transform, then the
+        # table's common phase (the phase of its largest entry above OP_TOL,
+        # the first in row-major order), as _uniform_phase does table by table
+        nt, d = raw_tables.shape[:2]
+        ti, bi, ki = _nonzero(raw_tables)
+        v = raw_tables[ti, bi, ki]
         if phase_weights is not None:
             phi = _phase_vec(np.asarray(phase_weights)[np.asarray(table_site)])  # (nt, d)
-            M = np.conj(phi)[:, :, None] * M * phi[:, None, :]
-        mag = np.abs(M)
+            v = np.conj(phi)[ti, bi] * v * phi[ti, ki]
+        mag = np.abs(v)
         keep = mag > OP_TOL
-        flat = np.where(keep, mag, -1.0).reshape(len(raw_tables), -1)
-        big = np.take_along_axis(M.reshape(len(raw_tables), -1), flat.argmax(axis=1)[:, None], axis=1)[:, 0]
-        ph = np.where(keep.reshape(len(raw_tables), -1).any(axis=1), big / np.where(big == 0, 1.0, np.abs(big)),
-                      1.0 + 0.0j)
-        rot = M / ph[:, None, None]
-        bad = keep & (np.abs(rot.imag) > 1e-12 * np.maximum(1.0, np.abs(rot)))
+        big_at = np.zeros((nt, d * d))
+        big_at[ti, bi * d + ki] = np.where(keep, mag, 0.0)
+        first = big_at.argmax(axis=1)
+        full = np.zeros((nt, d * d), dtype=np.complex128)
+        full[ti, bi * d + ki] = v
+        big = np.where(big_at[np.arange(nt), first] > 0.0, full[np.arange(nt), first], 0.0)
+        ph = np.where(big == 0, 1.0 + 0.0j, big / np.where(big == 0, 1.0, np.abs(big)))
+        v = v / ph[ti]
+        bad = keep & (np.abs(v.imag) > 1e-12 * np.maximum(1.0, np.abs(v)))
         ok = not bad.any()
         if ok:
-            tabs_t = list(rot.real)
-            phases = list(ph)
+            tabs_t = np.zeros((nt, d, d))
+            tabs_t[ti, bi, ki] = v.real
+            phases = ph.tolist()
         if ok:
             cr = []
             for sites, tabs, coef in terms:
@@ -214,33 +234,36 @@ def _table_arrays(raw_tables, terms, dmax, is_complex, tables_real, coefs_real):
     t_count = np.zeros((nt, dmax), dtype=np.int32)
     t_ket = np.zeros((nt, dmax, dmax), dtype=np.uint8)
     t_amp = np.zeros((nt, dmax, dmax, 2 if is_complex else 1), dtype=np.float64)
-    if raw_tables:
-        mags = np.abs(np.stack([np.asarray(m, dtype=np.complex128) for m in raw_tables]))[:, :dmax, :dmax]
-        vals = np.stack(raw_tables if is_complex else [np.asarray(m) for m in tables_real])[:, :dmax, :dmax]
-        keep = mags > OP_TOL
-        k = mags.shape[-1]
-        order = np.argsort(~keep, axis=-1, kind="stable")  # kept kets first, ascending
-        cnt = keep.sum(axis=-1)
-        valid = np.arange(k)[None, None, :] < cnt[..., None]
-        t_count[:, : mags.shape[1]] = cnt
-        t_ket[:, : mags.shape[1], :k] = np.where(valid, order, 0)
-        picked = np.take_along_axis(vals, order, axis=-1)
+    if len(raw_tables):
+        raw = np.asarray(raw_tables)[:, :dmax, :dmax]
+        ti, bi, ki = _nonzero(raw)
+        on = np.abs(raw[ti, bi, ki]) > OP_TOL
+        ti, bi, ki = ti[on], bi[on], ki[on]
+        v = raw[ti, bi, ki] if is_complex else np.asarray(tables_real)[ti, bi, ki]
+        # kets of a bra are neighbours and ascending: their positions count up
+        # from the bra's first one
+        row = ti * dmax + bi
+        cnt = np.bincount(row, minlength=nt * dmax)
+        pos = np.arange(len(row)) - (np.cumsum(cnt) - cnt)[row]
+        t_count[:] = cnt.reshape(nt, dmax)
+        t_ket[ti, bi, pos] = ki
+        t_amp[ti, bi, pos, 0] = v.real
         if is_complex:
-            t_amp[:, : mags.shape[1], :k, 0] = np.where(valid, picked.real, 0.0)
-            t_amp[:, : mags.shape[1], :k, 1] = np.where(valid, picked.imag, 0.0)
-        else:
-            t_amp[:, : mags.shape[1], :k, 0] = np.where(valid, np.real(picked), 0.0)
+            t_amp[ti, bi, pos, 1] = v.imag
     n_terms = len(terms)
     term_nops = np.zeros(max(n_terms, 1), dtype=np.int32)
     term_site = np.zeros((max(n_terms, 1), _lib.MAX_OPS), dtype=np.int32)
     term_table = np.zeros((max(n_terms, 1), _lib.MAX_OPS), dtype=np.int32)
     term_coef = np.zeros((max(n_terms, 1), 2 if is_complex else 1), dtype=np.float64)
-    for k_, (sites, tabs, coef) in enumerate(terms):
-        if len(sites) > _lib.MAX_OPS:
+    by_nops = {}  # instances with the same number of factors: one assignment
+    for k_, (sites, _, _) in enumerate(terms):
+        by_nops.setdefault(len(sites), []).append(k_)
+    for nops, rows in by_nops.items():
+        if nops > _lib.MAX_OPS:
             raise ValueError(f"at most {_lib.MAX_OPS} operator factors per term instance")
-        term_nops[k_] = len(sites)
-        term_site[k_, : len(sites)] = sites
-        term_table[k_, : len(tabs)] = tabs
+        term_nops[rows] = nops
+        term_site[rows, :nops] = [terms[k_][0] for k_ in rows]
+        term_table[rows, :nops] = [terms[k_][1] for k_ in rows]
     if n_terms:
         if is_complex:
             c = np.array([t[2] for t in terms], dtype=np.complex128)
@@ -275,18 +298,12 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
     st = stream_handle()
     n = len(sector)
 
-    # diagonal terms: (site, diag vector, coef)
-    dterms = []
-    for b in blocks:
-        if not b.diagonal:
-            continue
-        for inst in b.sites:
-            s = int(inst[0])
-            dterms.append((s, np.diagonal(np.asarray(b.ops[0][s], dtype=np.complex128)).copy(), complex(b.strength)))
-    dterms_real = all(not np.any(np.abs(dvec.imag) > 1e-12) and abs(coef.imag) <= 1e-12 for _, dvec, coef in dterms)
-
-    def up(a):
-        return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    # diagonal terms: sites, their operators' diagonals, strengths
+    dblocks = [b for b in blocks if b.diagonal and len(b.sites)]
+    dsite = np.concatenate([b.sites[:, 0] for b in dblocks]) if dblocks else np.zeros(0, dtype=np.int64)
+    ddiag = [np.diagonal(np.asarray(b.ops[0]), axis1=-2, axis2=-1)[b.sites[:, 0]] for b in dblocks]
+    dterms_real = all(not np.any(np.abs(v.imag) > 1e-12) and abs(b.strength.imag) <= 1e-12
+                      for v, b in zip(ddiag, dblocks))
 
     # ---- off-diagonal part: reused or built ----
     sig = _offdiag_signature(blocks, phase_weights, force_complex, dmax)
@@ -303,8 +320,9 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
         coefs_real = [coefs_real[i] for i in order] if coefs_real is not None else None
         use_real = real_ok and dterms_real
         arrays = _table_arrays(raw_tables, terms, dmax, not use_real, tables_real, coefs_real)
-        keep = [up(a) for a in arrays]
-        off = _assemble_offdiag(sector, dev, st, n, 1 if use_real else 2, dmax, not use_real, len(terms), keep)
+        keep = list(upload_arrays(dev, {k: (a, a.dtype) for k, a in enumerate(arrays)}).values())
+        n_tables = arrays[0].shape[0]
+        off = _assemble_offdiag(sector, dev, st, n, 1 if use_real else 2, dmax, not use_real, len(terms), n_tables, keep)
         off.update(sig=sig, real_ok=real_ok, use_real=use_real)
         sector._offdiag_cache = off
     is_complex = not off["use_real"]
@@ -312,7 +330,7 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
 
     # ---- diagonal terms: one pass over the rows, on top of the off-diagonal
     # part's own diagonal ----
-    n_d = len(dterms)
+    n_d = len(dsite)
     extra = complex(extra_diag) if extra_diag is not None and extra_diag != 0 else None
     if n == 0 or (n_d == 0 and extra is None):
         diag, present = off["diag"].clone(), off["present"].clone()
@@ -323,19 +341,21 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
         a.n_terms = 0
         a.n_dterms = n_d
         if n_d:
-            dterm_site = np.zeros(n_d, dtype=np.int32)
-            dterm_diag = np.zeros((n_d, dmax, w), dtype=np.float64)
-            dterm_coef = np.zeros((n_d, w), dtype=np.float64)
-            for k, (s, dvec, coef) in enumerate(dterms):
-                dterm_site[k] = s
-                dterm_diag[k, : len(dvec), 0] = dvec.real
-                dterm_coef[k, 0] = coef.real
+            vals = np.zeros((n_d, dmax, w), dtype=np.float64)
+            coef = np.zeros((n_d, w), dtype=np.float64)
+            at = 0
+            for v, b in zip(ddiag, dblocks):
+                rows = slice(at, at + len(v))
+                vals[rows, : v.shape[1], 0] = v.real
+                coef[rows, 0] = b.strength.real
                 if is_complex:
-                    dterm_diag[k, : len(dvec), 1] = dvec.imag
-                    dterm_coef[k, 1] = coef.imag
-            dk = [up(dterm_site), up(dterm_diag), up(dterm_coef)]
-            keep += dk
-            a.dterm_site, a.dterm_diag, a.dterm_coef = ptr(dk[0]), ptr(dk[1]), ptr(dk[2])
+                    vals[rows, : v.shape[1], 1] = v.imag
+                    coef[rows, 1] = b.strength.imag
+                at += len(v)
+            dk = upload_arrays(dev, {"site": (dsite, np.int32), "diag": (vals, np.float64),
+                                     "coef": (coef, np.float64)})
+            keep += dk.values()
+            a.dterm_site, a.dterm_diag, a.dterm_coef = ptr(dk["site"]), ptr(dk["diag"]), ptr(dk["coef"])
         ex = extra if extra is not None else 0j
         check(lib.edg_assemble_diag(ctypes.byref(a), ptr(off["diag"]), ptr(off["present"]),
                                     0 if extra is None else 1, ex.real, ex.imag, ptr(diag), ptr(present), st),
@@ -345,6 +365,7 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
     mat._keep = keep  # device tables uploaded by this build
     mat.raw_entries = off["raw_entries"]  # generated entries before the per-row merge
     mat.offdiag_reused = reused  # off-diagonal part shared with an earlier build
+    mat._shared = off["layouts"]  # layouts of that part, shared by the matrices that share it
     return mat
 
 
@@ -360,7 +381,7 @@ def _assembly_struct(sector, dmax, is_complex):
     return a
 
 
-def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, tabs):
+def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, n_tables, tabs):
     """Off-diagonal instances only: count, scan, fill (with per-row merge)
     and compaction; returns the CSR, the diagonal contributions of
     instances whose ket is the bra, and their presence flags."""
@@ -383,7 +404,7 @@ def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, tabs):
     diag = torch.empty(max(n, 1) * w, dtype=torch.float64, device=dev)
     present = torch.empty(max(n, 1), dtype=torch.uint8, device=dev)
     flags = torch.zeros(2, dtype=torch.int32, device=dev)
-    check(lib.edg_assemble_rows(ctypes.byref(a), int(tabs[0].shape[0]), ptr(offsets), ptr(cols), ptr(vals),
+    check(lib.edg_assemble_rows(ctypes.byref(a), n_tables, ptr(offsets), ptr(cols), ptr(vals),
                                 ptr(row_nnz), ptr(diag), ptr(present), ptr(flags), st), "edg_assemble_rows")
     e, merged = flags.tolist()
     if e != 0:
@@ -400,4 +421,4 @@ def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, tabs):
                                        ptr(rowptr), ptr(cols), ptr(vals), st), "edg_assemble_compact")
         del tmp_cols, tmp_vals
     return {"rowptr": rowptr, "cols": cols[:nnz], "vals": vals[: nnz * w], "diag": diag[: n * w],
-            "present": present[:n], "raw_entries": total, "keep": tabs}
+            "present": present[:n], "raw_entries": total, "keep": tabs, "layouts": {}}

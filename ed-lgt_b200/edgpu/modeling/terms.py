@@ -16,7 +16,7 @@ from math import prod
 
 import numpy as np
 
-from ..lattice import neighbor_sites, plaquette_sites, zig_zag
+from ..lattice import neighbor_pairs, plaquette_quads, site_coords, zig_zag
 
 __all__ = ["TermBlock", "LocalTerm", "TwoBodyTerm", "PlaquetteTerm", "NBodyTerm"]
 
@@ -70,6 +70,12 @@ class QMBTerm:
 
     def _mask_ok(self, coords, mask):
         return mask is None or bool(np.asarray(mask)[tuple(coords)])
+
+    def _selected(self, mask):
+        """Which sites the mask keeps, all at once."""
+        if mask is None:
+            return np.ones(self.n_sites, dtype=bool)
+        return np.asarray(mask)[tuple(site_coords(self.lvals).T)].astype(bool)
 
     def get_staggered_conditions(self, coords, stag_label):
         """even / odd sublattice selection by (-1)^sum(coords) (qmb_term.py:105-127)."""
@@ -126,8 +132,8 @@ class LocalTerm(QMBTerm):
     def get_Hamiltonian(self, strength, mask=None):
         if not np.isscalar(strength):
             raise TypeError(f"strength must be SCALAR not a {type(strength)}")
-        sites = [ii for ii in range(self.n_sites) if self._mask_ok(zig_zag(self.lvals, ii), mask)]
-        return TermBlock([self.op], np.array(sites).reshape(-1, 1), strength, diagonal=True, name=self.op_name)
+        sites = np.flatnonzero(self._selected(mask))
+        return TermBlock([self.op], sites.reshape(-1, 1), strength, diagonal=True, name=self.op_name)
 
     def get_expval(self, psi, stag_label=None, print_values=True, get_variance=False):
         """Per-site <psi| op_s |psi> in ``self.obs`` and their average over the
@@ -159,14 +165,9 @@ class TwoBodyTerm(QMBTerm):
     def get_Hamiltonian(self, strength, add_dagger=False, mask=None):
         if not np.isscalar(strength):
             raise TypeError(f"strength must be SCALAR, not {type(strength)}")
-        inst = []
-        for ii in range(self.n_sites):
-            coords = zig_zag(self.lvals, ii)
-            sl = neighbor_sites(coords, self.lvals, self.axis, self.has_obc)
-            if sl is None or not self._mask_ok(coords, mask):
-                continue
-            inst.append(sl)
-        return TermBlock(self.op_list, np.array(inst).reshape(-1, 2), strength, add_dagger=add_dagger,
+        pairs, inside = neighbor_pairs(self.lvals, self.axis, self.has_obc)
+        inst = pairs[inside & self._selected(mask)]
+        return TermBlock(self.op_list, inst.reshape(-1, 2), strength, add_dagger=add_dagger,
                          name="-".join(self.op_names_list or []))
 
     def get_expval(self, psi):
@@ -189,14 +190,9 @@ class PlaquetteTerm(QMBTerm):
     def get_Hamiltonian(self, strength, add_dagger=False, mask=None):
         if not np.isscalar(strength):
             raise TypeError(f"strength must be scalar, not {type(strength)}")
-        inst = []
-        for ii in range(self.n_sites):
-            coords = zig_zag(self.lvals, ii)
-            sl = plaquette_sites(coords, self.lvals, self.axes, self.has_obc)
-            if sl is None or not self._mask_ok(coords, mask):
-                continue
-            inst.append(sl)
-        return TermBlock(self.op_list, np.array(inst).reshape(-1, 4), strength, add_dagger=add_dagger,
+        quads, inside = plaquette_quads(self.lvals, self.axes, self.has_obc)
+        inst = quads[inside & self._selected(mask)]
+        return TermBlock(self.op_list, inst.reshape(-1, 4), strength, add_dagger=add_dagger,
                          name="-".join(self.op_names_list or []))
 
     def get_expval(self, psi, component="real", stag_label=None):

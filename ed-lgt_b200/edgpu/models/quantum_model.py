@@ -21,7 +21,7 @@ import torch
 
 from .. import _lib
 from .._lib import check, lib, ptr, stream_handle
-from ..lattice import lattice_labels, link_site_pairs, neighbor_sites, staggered_mask, zig_zag
+from ..lattice import lattice_labels, link_site_pairs, neighbor_sites, site_coords, staggered_mask, zig_zag
 from ..modeling import LocalTerm, NBodyTerm, PlaquetteTerm, QMB_hamiltonian, QMB_state, TwoBodyTerm
 from ..modeling.assembly import assemble_blocks
 from ..operators.common import project
@@ -187,27 +187,33 @@ class QuantumModel:
             for ii in range(self.n_sites):
                 self.gauge_states_per_site.append(self.gauge_states[self.lattice_labels[ii]])
         dmax = int(np.max(self.loc_dims))
+        # sites that share a basis (border label and background selection)
+        # share every projected operator
+        groups = {}
+        for jj in range(self.n_sites):
+            if self.gauge_basis is None:
+                groups.setdefault(None, []).append(jj)
+            else:
+                cols = None if cols_per_site is None else tuple(cols_per_site[jj])
+                groups.setdefault((self.lattice_labels[jj], cols), []).append(jj)
+        bases = {}
+        for key in groups:
+            if key is None:
+                continue
+            basis = self.gauge_basis[key[0]]
+            if key[1] is not None:
+                basis = basis[:, list(key[1])]
+            bases[key] = basis.toarray() if hasattr(basis, "toarray") else np.asarray(basis)
         self.ops = {}
-        cache = {}
         for name, op in ops_dict.items():
             arr = np.zeros((self.n_sites, dmax, dmax), dtype=np.complex128)
-            for jj in range(self.n_sites):
-                d = int(self.loc_dims[jj])
-                if self.gauge_basis is not None:
-                    lab = self.lattice_labels[jj]
-                    cols = None if cols_per_site is None else tuple(cols_per_site[jj])
-                    key = (name, lab, cols)
-                    if key not in cache:
-                        basis = self.gauge_basis[lab]
-                        if cols is not None:
-                            basis = basis[:, list(cols)]
-                        cache[key] = project(basis, op)
-                    eff = cache[key]
-                else:
-                    eff = op.toarray() if hasattr(op, "toarray") else np.asarray(op)
+            dense = op.toarray() if hasattr(op, "toarray") else np.asarray(op)
+            for key, members in groups.items():
+                eff = dense if key is None else project(bases[key], dense)
                 if self.basis_projector is not None:
                     eff = project(self.basis_projector, eff)
-                arr[jj, :d, :d] = eff
+                d = int(self.loc_dims[members[0]])
+                arr[members, :d, :d] = eff
             self.ops[name] = arr
 
     def _bg_values(self, states):
@@ -263,8 +269,8 @@ class QuantumModel:
 
     def _matter_phase_weights(self, number_op):
         """Per-site exponents x_s * n(c) of the real form's gauge transform."""
-        n = np.rint(np.real(np.array([np.diagonal(number_op[s]) for s in range(self.n_sites)]))).astype(np.int64)
-        xs = np.array([zig_zag(self.lvals, s)[0] for s in range(self.n_sites)], dtype=np.int64)
+        n = np.rint(np.real(np.diagonal(number_op, axis1=1, axis2=2))).astype(np.int64)
+        xs = site_coords(self.lvals)[:, 0].astype(np.int64)
         return (xs[:, None] * n) % 4
 
     # ---------------------------------------------------------- solve

@@ -222,11 +222,15 @@ class PackedLayout:
 
 
 def packed_layout(mat):
-    """The matrix's dictionary-packed layout (built once, kept on the matrix),
-    or None when the matrix does not pack."""
-    if not hasattr(mat, "_packed"):
-        mat._packed = PackedLayout.build(mat)
-    return mat._packed
+    """The matrix's dictionary-packed layout, or None when the matrix does not
+    pack.  Built once per off-diagonal part: the matrices of a coupling sweep
+    that share their CSR arrays share its layout as well."""
+    home = getattr(mat, "_shared", None)
+    if home is None:
+        home = mat._shared = {}
+    if "packed" not in home:
+        home["packed"] = PackedLayout.build(mat)
+    return home["packed"]
 
 
 def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
@@ -384,10 +388,16 @@ def lanczos(mat, k=1, tol=1e-12, max_iter=400, check_every=5, seed=1234, v0=None
     """f64 Lanczos on a real DeviceMatrix; returns (evals[k], evecs (n, k) device)."""
     if mat.is_complex:
         raise NotImplementedError("complex Hermitian Lanczos: assemble the real form of the model")
-    g = group or (tune_spmv_group(mat, 1, 0, vals=mat.vals) if tune else 0)
+    g = group or (tune_spmv_group(mat, 1, 0, vals=mat.vals) if tune and not _one_launch(mat, 1, stats) else 0)
     r = run_lanczos(0, mat.n, mat.nnz, mat.rowptr, mat.cols, mat.vals, mat.diag, nvec=1, k=k, max_iter=max_iter,
                     tol=tol, check_every=check_every, seed=seed, v0=v0, stats=stats, group=g)
     return r.evals[0], r.evecs[:, :, 0].T.contiguous(), r
+
+
+def _one_launch(mat, nvec, stats):
+    """Whether ``edg_lanczos`` solves this problem in one cooperative launch,
+    which reads the CSR arrays and has no matvec to tune."""
+    return nvec == 1 and stats is None and mat.n <= lib.edg_lanczos_small_rows()
 
 
 def stack_diagonals(diags, dtype):
@@ -419,12 +429,12 @@ def lanczos_mixed(mat, diags=None, k=1, tol32=1e-4, tol=1e-12, max_iter=400, ref
         raise NotImplementedError("mixed Lanczos needs the real form")
     diags = [mat.diag] if diags is None else list(diags)
     nvec = len(diags)
-    if vals32 is None:
-        vals32 = mat.vals.to(torch.float32)
     if diag32 is None:
         diag32 = stack_diagonals(diags, torch.float32)
     if diag64 is None:
         diag64 = stack_diagonals(diags, torch.float64)
+    # (the one-launch solver has no layout to choose)
+    tune = tune and not _one_launch(mat, nvec, stats32 if stats32 is not None else stats64)
     if sell is None and packed is None and tune and not group32:
         fmt, param = tune_matvec32(mat, nvec, vals32)
         if fmt == "sell":
@@ -435,6 +445,10 @@ def lanczos_mixed(mat, diags=None, k=1, tol32=1e-4, tol=1e-12, max_iter=400, ref
             sell, group32 = False, param
     lay = sell_layout(mat, vals32) if sell is True else (sell or None)
     pk = packed_layout(mat) if packed is True else (packed or None)
+    if vals32 is None and (pk is None or nvec == 1):
+        # (a batch on the packed layout has its f32 values there; a single small
+        # problem reads the CSR arrays)
+        vals32 = mat.vals.to(torch.float32)
     g32 = group32 or (tune_spmv_group(mat, nvec, 1, vals=vals32) if tune and pk is None else 0)
     g64 = group64 or (tune_spmv_group(mat, nvec, 0, vals=mat.vals) if tune and pk is None else 0)
     r32 = run_lanczos(1, mat.n, mat.nnz, mat.rowptr, mat.cols, vals32, diag32, nvec=nvec, k=k, max_iter=max_iter,

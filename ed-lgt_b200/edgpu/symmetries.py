@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check, lib, ptr, stream_handle
+from ._lib import check, lib, ptr, stream_handle, upload_arrays
 
 __all__ = [
     "Sector",
@@ -91,21 +91,10 @@ def get_symmetry_sector_generators(op_list, action: str) -> np.ndarray:
     operators) or ``"link"`` (list over directions of pairs of operators).
     """
     if action in ("global", "nbody"):
-        n_sites, dmax = op_list[0].shape[0], op_list[0].shape[1]
-        out = np.zeros((len(op_list), n_sites, dmax))
-        for i, op in enumerate(op_list):
-            for s in range(n_sites):
-                out[i, s] = np.real(np.diagonal(op[s]))
-        return out
+        return np.stack([np.real(np.diagonal(op, axis1=1, axis2=2)) for op in op_list]).astype(float)
     if action == "link":
-        n_dirs = len(op_list)
-        n_sites, dmax = op_list[0][0].shape[0], op_list[0][0].shape[1]
-        out = np.zeros((n_dirs, 2, n_sites, dmax))
-        for d in range(n_dirs):
-            for e in range(2):
-                for s in range(n_sites):
-                    out[d, e, s] = np.real(np.diagonal(op_list[d][e][s]))
-        return out
+        return np.stack([np.stack([np.real(np.diagonal(op, axis1=1, axis2=2)) for op in pair])
+                         for pair in op_list]).astype(float)
     raise ValueError(f"action must be 'global', 'link' or 'nbody', got {action!r}")
 
 
@@ -280,32 +269,26 @@ class _DeviceTables:
     """Device copies of a SectorSpec plus the ctypes struct pointing at them."""
 
     def __init__(self, spec: SectorSpec, device):
-        def dev(a, dtype):
-            a = np.ascontiguousarray(a)
-            if a.size == 0:
-                a = np.zeros(1, dtype=a.dtype)
-            return torch.from_numpy(a.astype(dtype, copy=False)).to(device)
-
-        self._keep = {
-            "allowed": dev(spec.site_allowed, np.uint8),
-            "gv": dev(spec.glob_val, np.int32),
-            "gt": dev(spec.glob_target, np.int32),
-            "gmin": dev(spec.glob_rem_min, np.int32),
-            "gmax": dev(spec.glob_rem_max, np.int32),
-            "lv": dev(spec.link_val, np.int32),
-            "lt": dev(spec.link_target, np.int32),
-            "ps": dev(spec.pair_start, np.int32),
-            "p0": dev(spec.pair_s0, np.int32),
-            "p1": dev(spec.pair_s1, np.int32),
-            "pd": dev(spec.pair_dir, np.int32),
-            "nv": dev(spec.nb_val, np.int32),
-            "nt": dev(spec.nb_target, np.int32),
-            "ns": dev(spec.nb_start, np.int32),
-            "ni": dev(spec.nb_id, np.int32),
-            "nss": dev(spec.nb_site_start, np.int32),
-            "nsi": dev(spec.nb_sites, np.int32),
-        }
-        k = self._keep
+        k = upload_arrays(device, {
+            "allowed": (spec.site_allowed, np.uint8),
+            "gv": (spec.glob_val, np.int32),
+            "gt": (spec.glob_target, np.int32),
+            "gmin": (spec.glob_rem_min, np.int32),
+            "gmax": (spec.glob_rem_max, np.int32),
+            "lv": (spec.link_val, np.int32),
+            "lt": (spec.link_target, np.int32),
+            "ps": (spec.pair_start, np.int32),
+            "p0": (spec.pair_s0, np.int32),
+            "p1": (spec.pair_s1, np.int32),
+            "pd": (spec.pair_dir, np.int32),
+            "nv": (spec.nb_val, np.int32),
+            "nt": (spec.nb_target, np.int32),
+            "ns": (spec.nb_start, np.int32),
+            "ni": (spec.nb_id, np.int32),
+            "nss": (spec.nb_site_start, np.int32),
+            "nsi": (spec.nb_sites, np.int32),
+        })
+        self._keep = k
         t = _lib.SectorTables()
         t.n_sites = spec.n_sites
         t.dmax = spec.dmax

@@ -470,6 +470,10 @@ typedef struct {
 } edg_lanczos_problem;
 
 /* Bytes of device workspace edg_lanczos needs. */
+/* Rows up to which a single problem (nvec 1, no stats, vals given) is solved
+ * in one cooperative launch, which reads the CSR arrays whatever layout is
+ * passed beside them. */
+int64_t edg_lanczos_small_rows(void);
 int64_t edg_lanczos_workspace_bytes(const edg_lanczos_problem* p);
 /* Runs to convergence (synchronizes every check_every steps).  Outputs:
  * evals [nvec][k] (f64), evecs [k][n_rows][nvec] in the problem dtype (may be
