@@ -34,6 +34,7 @@
 
 #include <chrono>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -961,6 +962,7 @@ __global__ void ritz_k(const T* __restrict__ V, int64_t n_pad, int m, const doub
     const int v = (int)(g / n_pad);
     const double* s = S + ((int64_t)v * ldk + e) * lds;
     double acc = 0.0;
+#pragma unroll 8
     for (int i = 0; i < m; ++i) acc = fma(ldv(V, (int64_t)i * stride_i + g), s[i], acc);
     w[g] = acc;
   }
@@ -976,8 +978,8 @@ __global__ void ritz_k(const T* __restrict__ V, int64_t n_pad, int m, const doub
 // candidate and |w|.  When a check is due CTA 0 solves the tridiagonal
 // matrices while the others wait.  The arithmetic of a row is that of the
 // passes above; only the order of the sums over rows differs.  Bound by the
-// two waits and the dependent L2 reads between them.  f64, one eigenpair (a
-// graph of five launches a step before): 61 rows 0.37 ms (1.32), 8,953 rows
+// two waits and the dependent L2 reads between them.  f64, one eigenpair (five
+// launches a step before): 61 rows 0.37 ms (1.32), 8,953 rows
 // 1.47 (2.81), 73,789 rows 2.08 (3.32), 147,578 rows 3.11 (3.80); mixed
 // precision 0.43 (1.31), 0.73 (1.72), 0.86 (1.87), 1.26 (2.11).  Past kCoopRows
 // rows per SM the basis leaves L2 and the streaming passes take over.  512
@@ -1330,9 +1332,10 @@ Layout make_layout(const edg_lanczos_problem* p) {
   L.normp = off; off = align256(off + (int64_t)L.nblk_upd * nv * 8);
   L.alpha = off; off = align256(off + (int64_t)nv * (L.m_max + 1) * 8);   // [nv][m_max+1]
   L.beta = off; off = align256(off + (int64_t)nv * (L.m_max + 2) * 8);    // [nv][m_max+2]
-  L.tri_eval = off; off = align256(off + (int64_t)nv * kMaxK * 8);
   L.tri_vec = off; off = align256(off + (int64_t)nv * kMaxK * (L.m_max + 1) * 8);
   L.tri_work = off; off = align256(off + (int64_t)nv * 6 * (L.m_max + 1) * 8);
+  // read back together at the end of a solve
+  L.tri_eval = off; off = align256(off + (int64_t)nv * kMaxK * 8);
   L.sync = off; off = align256(off + 8 * (int64_t)sizeof(int));  // last-CTA tickets | error word | grid barrier
   L.state = off; off = align256(off + (int64_t)sizeof(DevState));
   L.total = off;
@@ -1598,59 +1601,55 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
     }
     for (auto& x : ev) cudaEventDestroy(x);
   } else {
-    // graph of kStepsPerGraph steps (each with its check), replayed one
-    // replay ahead of the host, which polls the device's progress words
-    constexpr int kStepsPerGraph = 4;
-    cudaStream_t cs = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: capture");
-    for (int q = 0; q < kStepsPerGraph && rc_ == EDG_OK; ++q) {
-      rc_ = enqueue_step(cs);
-      if (rc_ == EDG_OK) enqueue_check(cs);
-    }
-    cudaError_t ec = cudaStreamEndCapture(cs, &graph);
-    if (rc_ == EDG_OK && ec != cudaSuccess) rc_ = edg::cuda_status(ec, "edg_lanczos: capture");
-    if (rc_ == EDG_OK && (ec = cudaGraphInstantiate(&exec, graph, 0)) != cudaSuccess)
-      rc_ = edg::cuda_status(ec, "edg_lanczos: graph instantiate");
+    // groups of kGroup steps (each with its check), one group ahead of the
+    // host, which polls the device's progress words.  Plain launches: a step
+    // of the passes takes longer on the device than its three to five launches
+    // on the host, and a graph of them has to be captured, instantiated and
+    // destroyed on every call (0.45 ms of a 3.5 ms f32 solve of three problems
+    // at 1.2M rows).
+    constexpr int kGroup = 4;
     int enq = 0;
     const int limit = (int)(L.m_max < n ? L.m_max : n);
-    if (rc_ == EDG_OK) {
-      ec = cudaGraphLaunch(exec, s);
-      if (ec != cudaSuccess) rc_ = edg::cuda_status(ec, "edg_lanczos: graph launch");
-      enq += kStepsPerGraph;
-    }
+    auto enqueue_group = [&]() -> int {
+      for (int q = 0; q < kGroup; ++q) {
+        const int st_ = enqueue_step(s);
+        if (st_) return st_;
+        enqueue_check(s);
+      }
+      enq += kGroup;
+      const cudaError_t eg = cudaGetLastError();
+      return eg == cudaSuccess ? EDG_OK : edg::cuda_status(eg, "edg_lanczos: steps");
+    };
+    rc_ = enqueue_group();
     while (rc_ == EDG_OK) {
       const bool more = enq < limit;
-      if (more) {
-        ec = cudaGraphLaunch(exec, s);
-        if (ec != cudaSuccess) {
-          rc_ = edg::cuda_status(ec, "edg_lanczos: graph launch");
-          break;
-        }
-        enq += kStepsPerGraph;
-      }
-      const int target = more ? enq - kStepsPerGraph : limit;
+      if (more && (rc_ = enqueue_group())) break;
+      const int target = more ? enq - kGroup : limit;
       rc_ = wait_progress(target < limit ? target : limit);
       if (rc_) break;
       if (progress ? progress[1] != 0 : (read_state(&hs) == EDG_OK && hs.done)) break;
       if (!more) break;
     }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamSynchronize(s);
-    cudaStreamDestroy(cs);
-    if (rc_) return rc_;
+    if (rc_) {
+      cudaStreamSynchronize(s);
+      return rc_;
+    }
     launches += (int64_t)enq * launches_per_step;
   }
-  if ((rc_ = read_state(&hs))) return rc_;
-  const int j_end = hs.j;
-  std::vector<double> hev((size_t)NV * kMaxK);
-  e = cudaMemcpyAsync(hev.data(), tri_eval, sizeof(double) * NV * kMaxK, cudaMemcpyDeviceToHost, s);
+  // Ritz values, error word and state by one copy
+  std::vector<char> back((size_t)(L.total - L.tri_eval));
+  e = cudaMemcpyAsync(back.data(), ws + L.tri_eval, back.size(), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: ritz values");
+  if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: state");
+  memcpy(&hs, back.data() + (L.state - L.tri_eval), sizeof(DevState));
+  const int j_end = hs.j;
+  int h_err = 0;
+  memcpy(&h_err, back.data() + (L.sync - L.tri_eval) + 2 * sizeof(int), sizeof(int));
+  if (h_err != 0) {
+    edg::set_error("edg_lanczos: a ring, stage or grid-wide wait ran out");
+    return EDG_ERR_TIMEOUT;
+  }
+  const double* hev = reinterpret_cast<const double*>(back.data());
   int m_all = 1;
   for (int v = 0; v < NV; ++v) {
     const int mv = hs.m_conv[v] ? hs.m_conv[v] : (hs.m_use[v] ? hs.m_use[v] : 1);
@@ -1673,14 +1672,8 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: ritz vectors");
   }
-  int h_err = 0;
-  e = cudaMemcpyAsync(&h_err, err_word, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: finish");
-  if (h_err != 0) {
-    edg::set_error("edg_lanczos: a shared-memory ring wait of the reorthogonalisation ran out");
-    return EDG_ERR_TIMEOUT;
-  }
   if (timing) {
     launches += 2 + (evecs ? 4 * k : 0);
     p->stats[0] = t_spmv;

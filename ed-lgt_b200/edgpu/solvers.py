@@ -352,8 +352,9 @@ def run_lanczos(dtype, n, nnz, rowptr, cols, vals, diag, nvec=1, k=1, max_iter=3
     ``stats``: optional float64 numpy array of 6 entries filled with the
     phase timings of the run (see edg_lanczos_problem.stats); the steps are
     then launched one by one with events around each phase.  Without it the
-    steps run as replays of a CUDA graph; ``poll_host=False`` makes the host
-    synchronise once per replay instead of polling pinned progress words.
+    host launches groups of steps, one group ahead (or, for a single small
+    problem, the whole solve at once); ``poll_host=False`` makes it
+    synchronise once per group instead of polling pinned progress words.
     ``sell``: a :class:`SellLayout` of the matrix (f32 path only) for the
     matvec.  ``window``: 0 for full reorthogonalisation, W > 0 to
     orthogonalise each step against the last W Krylov vectors only.

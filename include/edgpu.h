@@ -419,11 +419,12 @@ int edg_convert(int32_t dtype_in, const void* in, int32_t dtype_out, void* out,
 /* eigensolve in f64 on the device.  Stops when the k lowest Ritz values of */
 /* every problem have residual |beta_{j+1} s_j| <= tol * max(1, |theta|),   */
 /* or after max_iter steps.  The step index, the convergence checks and     */
-/* their schedule live on the device: the host records a few steps (and     */
-/* their checks) in a CUDA graph and replays it, one replay ahead, polling  */
-/* the progress words the device writes to host_progress; no stream         */
-/* synchronisation happens inside the step loop.  With stats set, the steps */
-/* are launched one by one with CUDA events around each phase instead.      */
+/* their schedule live on the device: the host launches steps (and their    */
+/* checks) a group at a time, one group ahead, polling the progress words   */
+/* the device writes to host_progress; no stream synchronisation happens    */
+/* inside the step loop.  With stats set, the steps are launched one by one */
+/* with CUDA events around each phase instead.  A single small problem      */
+/* (edg_lanczos_small_rows) is one cooperative launch.                       */
 /* A step that reorthogonalises against at most 8 vectors (reorth_window of  */
 /* 1..7, or max_iter <= 8) does it in one cooperative launch (dots, a grid    */
 /* barrier with a 1 s limit, update); the device must support cooperative   */
