@@ -339,6 +339,8 @@ _SIGS = {
     "edg_lanczos_tiled_batch": (I32, [C.POINTER(TiledBatch), P]),
     "edg_krylov_workspace_bytes": (I64, [C.POINTER(KrylovProblem)]),
     "edg_krylov_step": (I32, [C.POINTER(KrylovProblem), P, F64, P, I64, P, P]),
+    "edg_krylov_orth_bytes": (I64, [I32]),
+    "edg_krylov_orth": (I32, [I64, I64, P, I32, P, I32, P, P, I32, P, I64, P]),
     "edg_twobody_scratch_elems": (I64, [I32]),
     "edg_twobody_expval": (I32, [C.POINTER(LookupTable), P, P, I32, P, P, P, I32, P, P, I32, P, I32, I64, P, P, I64, P]),
     "edg_csr_to_dense": (I32, [I32, I64, P, P, P, P, P, P, P]),
@@ -350,6 +352,7 @@ _SIGS = {
     "edg_momentum_rowmap": (I32, [P, P, P, I64, I64, P, P, P, P]),
     "edg_momentum_expand": (I32, [I64, P, P, P, P, P]),
     "edg_momentum_reduce": (I32, [I64, P, P, P, P, P, P]),
+    "edg_momentum_dense": (I32, [I64, P, P, P, P, P, I32, P, P, P, P, P, P]),
     "edg_part_scratch_elems": (I64, [U64]),
     "edg_part_map": (I32, [P, I64, C.POINTER(PartSpec), P, P, I64, C.POINTER(I64), P, I64, P]),
     "edg_psi_matrix": (I32, [P, I32, I64, P, P, I64, I64, P, I32, P, P]),

@@ -9,7 +9,7 @@ Mirrors ``QuantumModel.set_momentum_sector`` (edlgt/models/quantum_model.py:
 term (``nbody_data_momentum*``, :1394-1969), here H_k = B^dagger H B is
 applied without being formed: ``edg_momentum_expand``, the sector matvec,
 ``edg_momentum_reduce``.  Spectra come from a dense Hermitian solve of H_k
-(columns applied to unit vectors) up to ``DENSE_MAX`` momentum states and from
+(one kernel) up to ``DENSE_MAX`` momentum states and from
 a fully reorthogonalised Lanczos above that.
 """
 
@@ -152,20 +152,20 @@ class MomentumBasis:
     # ------------------------------------------------------------ host view
     def host_arrays(self) -> dict:
         """The reference's momentum_basis dict (CSC and CSR of B, host)."""
-        cp = self.col_ptr.cpu().numpy()
-        ri = self.row_idx[: self.nnz].cpu().numpy().astype(np.int32)
-        dv = self.data[: self.nnz].cpu().numpy()
+        # narrowed on the device: half the bytes to copy, no pass over them here
+        has = self.row_col[: self.n_rows] >= 0
+        r_ptr = torch.zeros(self.n_rows + 1, dtype=torch.int32, device=self.device)
+        torch.cumsum(has, 0, dtype=torch.int32, out=r_ptr[1:])
+        dv, rv, rc = self.data[: self.nnz], self.row_val[: self.n_rows], self.row_col[: self.n_rows]
+        if self.nnz < self.n_rows:
+            rv, rc = rv[has], rc[has]
         if self.zero_k:
-            dv = dv.real.copy()
-        rc = self.row_col[: self.n_rows].cpu().numpy()
-        rv = self.row_val[: self.n_rows].cpu().numpy()
-        has = rc >= 0
-        r_ptr = np.zeros(self.n_rows + 1, dtype=np.int32)
-        r_ptr[1:] = np.cumsum(has)
-        r_val = rv[has].real.copy() if self.zero_k else rv[has]
-        return {"pair_mode": False, "n_rows": self.n_rows, "n_cols": self.n_cols, "L_col_ptr": cp.astype(np.int32),
-                "L_row_idx": ri, "L_data": dv, "R_row_ptr": r_ptr, "R_col_idx": rc[has].astype(np.int32),
-                "R_data": r_val}
+            dv, rv = dv.real, rv.real
+        cp, ri, dv, r_ptr, rc, rv = (x.cpu().numpy() for x in (
+            self.col_ptr.to(torch.int32), self.row_idx[: self.nnz], dv.contiguous(), r_ptr, rc.to(torch.int32),
+            rv.contiguous()))
+        return {"pair_mode": False, "n_rows": self.n_rows, "n_cols": self.n_cols, "L_col_ptr": cp,
+                "L_row_idx": ri, "L_data": dv, "R_row_ptr": r_ptr, "R_col_idx": rc, "R_data": rv}
 
     # ------------------------------------------------------------ operator
     def bind(self, ham):
@@ -186,33 +186,43 @@ class MomentumBasis:
 
     def matvec(self, x: torch.Tensor) -> torch.Tensor:
         """y = B^dagger H B x for a complex128 momentum-space vector."""
-        mat, rv, dv, diag = self._bound
         x = x.to(torch.complex128).contiguous()
+        return self._product()(ptr(x))
+
+    def _product(self):
+        """A function of a vector's address that returns H_k times it, on this
+        stream, in buffers made once: each call overwrites the result of the
+        one before."""
+        mat, rv, dv, diag = self._bound
         v = torch.empty(self.n_rows, dtype=torch.complex128, device=self.device)
-        check(lib.edg_momentum_expand(self.n_rows, ptr(self.row_col), ptr(rv), ptr(x), ptr(v), stream_handle()),
-              "edg_momentum_expand")
         w = torch.empty_like(v)
-        if mat.is_complex:
-            code, nvec = 2, 1
-        else:
-            code, nvec = 0, 2  # a complex vector is two interleaved real ones
-        check(lib.edg_spmv(code, mat.n, mat.nnz, ptr(mat.rowptr), ptr(mat.cols) if mat.nnz else None,
-                           ptr(mat.vals) if mat.nnz else None, ptr(diag), nvec, ptr(v), ptr(w), stream_handle()),
-              "edg_spmv")
         y = torch.empty(self.n_cols, dtype=torch.complex128, device=self.device)
-        check(lib.edg_momentum_reduce(self.n_cols, ptr(self.col_ptr), ptr(self.row_idx), ptr(dv), ptr(w), ptr(y),
-                                      stream_handle()), "edg_momentum_reduce")
-        return y
+        # on a real matrix a complex vector is two interleaved real ones
+        code, nvec = (2, 1) if mat.is_complex else (0, 2)
+        st = stream_handle()
+        expand = (self.n_rows, ptr(self.row_col), ptr(rv))
+        spmv = (code, mat.n, mat.nnz, ptr(mat.rowptr), ptr(mat.cols) if mat.nnz else None,
+                ptr(mat.vals) if mat.nnz else None, ptr(diag), nvec, ptr(v), ptr(w), st)
+        reduce = (self.n_cols, ptr(self.col_ptr), ptr(self.row_idx), ptr(dv), ptr(w), ptr(y), st)
+
+        def apply(x, _alive=(mat, rv, dv, diag, v, w)):  # the tensors behind the addresses
+            check(lib.edg_momentum_expand(*expand, x, spmv[8], st), "edg_momentum_expand")
+            check(lib.edg_spmv(*spmv), "edg_spmv")
+            check(lib.edg_momentum_reduce(*reduce), "edg_momentum_reduce")
+            return y
+
+        return apply
 
     def dense(self) -> torch.Tensor:
-        """H_k as a dense (n_cols, n_cols) complex128 matrix (column by column)."""
+        """H_k as a dense (n_cols, n_cols) complex128 matrix
+        (``edg_momentum_dense``)."""
+        mat, rv, dv, _ = self._bound
         m = self.n_cols
         out = torch.empty((m, m), dtype=torch.complex128, device=self.device)
-        e = torch.zeros(m, dtype=torch.complex128, device=self.device)
-        for c in range(m):
-            e.zero_()
-            e[c] = 1.0
-            out[:, c] = self.matvec(e)
+        check(lib.edg_momentum_dense(m, ptr(self.col_ptr), ptr(self.row_idx), ptr(dv), ptr(self.row_col), ptr(rv),
+                                     1 if mat.is_complex else 0, ptr(mat.rowptr), ptr(mat.cols) if mat.nnz else None,
+                                     ptr(mat.vals) if mat.nnz else None, ptr(mat.diag), ptr(out), stream_handle()),
+              "edg_momentum_dense")
         return out
 
     def lowest(self, k, tol=1e-12, max_iter=None, seed=0):
@@ -228,7 +238,7 @@ class MomentumBasis:
             w, v = torch.linalg.eigh(h)
             self.last_matvecs = m
             return w[:k].cpu().numpy(), v[:, :k]
-        w, v, its = _lanczos(self.matvec, m, k, tol, max_iter or min(m, 400), self.device, seed)
+        w, v, its = _lanczos(self._product(), m, k, tol, max_iter or min(m, 400), self.device, seed)
         self.last_matvecs = its
         return w, v
 
@@ -290,31 +300,40 @@ def krylov_evolve(apply, psi0, time_line, m_krylov=40, tol=1e-12):
 
 def _lanczos(apply, m, k, tol, max_iter, device, seed):
     """Lanczos with two classical Gram-Schmidt passes against the whole basis
-    on complex128 vectors; converged when every wanted Ritz pair has
-    |beta_j s_jk| <= tol max(1, |theta_k|)."""
+    on complex128 vectors (``edg_krylov_orth``); converged when every wanted
+    Ritz pair has |beta_j s_jk| <= tol max(1, |theta_k|).  The host reads the
+    coefficients every fifth step, when it tests for convergence."""
     from scipy.linalg import eigh_tridiagonal
 
+    max_iter = min(max_iter, 14000)  # the most basis vectors edg_krylov_orth takes
     gen = torch.Generator(device=device).manual_seed(seed)
     q = torch.randn(m, dtype=torch.complex128, device=device, generator=gen)
-    Q = torch.empty((max_iter + 1, m), dtype=torch.complex128, device=device)
-    Q[0] = q / torch.linalg.vector_norm(q)
-    alpha, beta = [], []
+    Q = torch.empty((max_iter + 1, m), dtype=torch.complex128, device=device)  # unnormalised: |Q[i]| = beta[i]
+    torch.div(q, torch.linalg.vector_norm(q), out=Q[0])
+    coef = torch.zeros((2, max_iter + 1), dtype=torch.float64, device=device)  # alpha, beta
+    coef[1, 0] = 1.0
+    wb = lib.edg_krylov_orth_bytes(max_iter)
+    work = torch.empty(wb, dtype=torch.uint8, device=device)
+    step = (ptr(coef[0]), ptr(coef[1]), max_iter, ptr(work), wb, stream_handle())
+    q0 = Q.data_ptr()
     theta = s = None
     for j in range(max_iter):
-        w = apply(Q[j])
-        a = float(torch.vdot(Q[j], w).real)
-        alpha.append(a)
-        for _ in range(2):
-            w = w - Q[: j + 1].T @ (Q[: j + 1].conj() @ w)
-        b = float(torch.linalg.vector_norm(w))
-        done = b <= 1e-14 * max(1.0, abs(a)) or j + 1 == max_iter
+        w = apply(q0 + 16 * m * j)
+        check(lib.edg_krylov_orth(m, m, q0, j, ptr(w), 2, *step), "edg_krylov_orth")
+        done = j + 1 == max_iter
         if j + 1 >= k and (done or (j + 1) % 5 == 0):
-            theta, s = eigh_tridiagonal(np.array(alpha), np.array(beta), select="i", select_range=(0, k - 1))
-            res = np.abs(b * s[-1, :])
+            alpha, beta = coef[:, : j + 2].cpu().numpy()
+            n = j + 1
+            # a breakdown, once k steps are taken, ends the recurrence at its step
+            ends = np.nonzero(beta[k: n + 1] <= 1e-14 * np.maximum(1.0, np.abs(alpha[k - 1: n])))[0]
+            if len(ends):
+                n, done = k + int(ends[0]), True
+            if not np.all(beta[:n] > 0):
+                raise ValueError(f"the start vector spans fewer than {k} states of the momentum sector")
+            theta, s = eigh_tridiagonal(alpha[:n], beta[1:n], select="i", select_range=(0, k - 1))
+            res = np.abs(beta[n] * s[-1, :])
             if done or np.all(res <= tol * np.maximum(1.0, np.abs(theta))):
                 break
-        beta.append(b)
-        Q[j + 1] = w / b
-    n_used = len(alpha)
-    vecs = Q[:n_used].T @ torch.from_numpy(s.astype(np.complex128)).to(device)
-    return theta, vecs, n_used
+    n = s.shape[0]
+    vecs = Q[:n].T @ torch.from_numpy((s / beta[:n, None]).astype(np.complex128)).to(device)
+    return theta, vecs, n

@@ -651,6 +651,20 @@ int edg_krylov_step(const edg_krylov_problem* p, void* psi, double dt,
                     void* workspace, int64_t workspace_bytes, double* err_out,
                     cudaStream_t stream);
 
+/* One step of a complex128 Lanczos recurrence on the caller's product: w = H
+ * u_j in, u_{j+1} out.  V: max_vectors + 1 vectors of n complex entries, ldv
+ * apart, stored unnormalised: v_i = u_i / beta[i], with V[0] and beta[0] = |u_0|
+ * set by the caller.  w / beta[j] is orthogonalised against the j + 1 vectors
+ * by `passes` classical Gram-Schmidt passes and written to V[j+1]; alpha[j] =
+ * Re <v_j, H v_j>, beta[j+1] = its norm.  w is overwritten.  Everything stays
+ * on the device (alpha: max_vectors doubles, beta: max_vectors + 1); the steps
+ * of a run are taken in order from j = 0 with the same work buffer. */
+int64_t edg_krylov_orth_bytes(int32_t max_vectors);
+int edg_krylov_orth(int64_t n, int64_t ldv, double* V, int32_t j, double* w,
+                    int32_t passes, double* alpha, double* beta,
+                    int32_t max_vectors, void* work, int64_t work_bytes,
+                    cudaStream_t stream);
+
 /* ------------------------------------------------------------------------ */
 /* Local (diagonal) observables                                              */
 /* Replaces LocalTerm.get_expval in a symmetry sector (edlgt/modeling/       */
@@ -780,6 +794,15 @@ int edg_momentum_expand(int64_t n_rows, const int64_t* row_col, const double* ro
 /* y = B^dagger w (complex128, w [n_rows], y [n_cols]), fixed summation order. */
 int edg_momentum_reduce(int64_t n_cols, const int64_t* col_ptr, const int32_t* row_idx, const double* data,
                         const double* w, double* y, cudaStream_t stream);
+/* H_k = B^dagger H B as a dense matrix, out [n_cols][n_cols] complex (row
+ * major), from the sector matrix (CSR and diagonal; interleaved complex when
+ * complex_values) and B's columns and row map. */
+int edg_momentum_dense(int64_t n_cols, const int64_t* col_ptr,
+                       const int32_t* row_idx, const double* data,
+                       const int64_t* row_col, const double* row_val,
+                       int32_t complex_values, const int64_t* rowptr, const int32_t* cols,
+                       const double* vals, const double* diag, double* out,
+                       cudaStream_t stream);
 
 /* ------------------------------------------------------------------------
  * Bipartitions.  Replaces QuantumModel._get_partition with
