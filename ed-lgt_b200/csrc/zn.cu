@@ -15,13 +15,15 @@
 // found by binary search and its projector B
 // (edlgt/symmetries/translational_sym.py:567-819).
 //
-// Matvec.  One thread per representative row (persistent grid, lookup
-// tables in shared memory): the diagonal from the key, then each hopping and
-// plaquette image is encoded, looked up in the orbit table (one 4-byte
-// load) and its x row gathered (nvec interleaved instances, one 32-byte
-// sector for 8 f32 instances).  Element: amplitude * sign *
+// Matvec.  One thread per representative row (persistent grid): the diagonal
+// from the key; the Gauss index of each hopping and plaquette image from the
+// row's own, its entry in the orbit table (4 bytes), and the x row that the
+// entry names (nvec interleaved instances, one 32-byte sector for 8 f32
+// instances).  Element: amplitude * sign *
 // sqrt(|Stab r'| / |Stab r|), the zero-momentum projection of
 // nbody_data_momentum (translational_sym.py:1394-1969) done on the fly.
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace {
@@ -31,12 +33,6 @@ struct Zn {
   static constexpr int kBits = ZN == 2 ? 1 : 2;
   static constexpr uint64_t kMask = (1ull << kBits) - 1;
   __device__ static __forceinline__ int field(uint64_t key, int l) { return (int)((key >> (kBits * l)) & kMask); }
-  __device__ static __forceinline__ uint64_t set(uint64_t key, int l, int v) {
-    const int sh = kBits * l;
-    return (key & ~(kMask << sh)) | ((uint64_t)v << sh);
-  }
-  __device__ static __forceinline__ int inc(int v) { return v + 1 == ZN ? 0 : v + 1; }
-  __device__ static __forceinline__ int dec(int v) { return v == 0 ? ZN - 1 : v - 1; }
   __device__ static __forceinline__ int mod(int v) {
     v %= ZN;
     return v < 0 ? v + ZN : v;
@@ -183,50 +179,216 @@ __global__ void __launch_bounds__(256) zn_orbit_k(const __grid_constant__ edg_zn
 }
 
 // ---------------------------------------------------------------- matvec
-// One x row (the nvec interleaved instances of a column) in 16-byte loads.
-template <typename T, int NV>
-__device__ __forceinline__ void load_row(const T* __restrict__ p, T (&v)[NV]) {
-  if constexpr (NV * sizeof(T) >= 16) {
-    constexpr int kVec = 16 / sizeof(T);
+// Policy of data that is read once in a long while: first to leave L2, not
+// kept in L1.
+__device__ __forceinline__ uint64_t once_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
+// One x row (the nvec interleaved instances of a column) in 16-byte loads, or
+// in 32-byte ones (WIDE), which fetch a whole sector a lane.
+template <typename T, int NV, bool WIDE, bool ONCE>
+__device__ __forceinline__ void load_row(const T* __restrict__ p, T (&v)[NV], uint64_t policy) {
+  constexpr int kBytes = WIDE ? 32 : (NV * sizeof(T) >= 16 ? 16 : sizeof(T));
+  constexpr int kVec = kBytes / sizeof(T);
+  static_assert(NV % kVec == 0);
 #pragma unroll
-    for (int i = 0; i < NV / kVec; ++i) {
-      if constexpr (sizeof(T) == 4) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p) + i);
-        v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
-      } else {
-        const double2 a = __ldg(reinterpret_cast<const double2*>(p) + i);
-        v[2 * i] = a.x; v[2 * i + 1] = a.y;
-      }
+  for (int i = 0; i < NV; i += kVec) {
+    if constexpr (sizeof(T) == 4 && kVec == 8) {
+      if constexpr (ONCE)
+        asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;"
+            : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3]), "=f"(v[i + 4]), "=f"(v[i + 5]),
+              "=f"(v[i + 6]), "=f"(v[i + 7])
+            : "l"(p + i), "l"(policy));
+      else
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3]), "=f"(v[i + 4]), "=f"(v[i + 5]),
+              "=f"(v[i + 6]), "=f"(v[i + 7])
+            : "l"(p + i));
+    } else if constexpr (sizeof(T) == 4 && kVec == 4) {
+      if constexpr (ONCE)
+        asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+            : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
+            : "l"(p + i), "l"(policy));
+      else
+        asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+            : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
+            : "l"(p + i));
+    } else if constexpr (sizeof(T) == 8 && kVec == 4) {
+      if constexpr (ONCE)
+        asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+            : "=d"(v[i]), "=d"(v[i + 1]), "=d"(v[i + 2]), "=d"(v[i + 3])
+            : "l"(p + i), "l"(policy));
+      else
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(v[i]), "=d"(v[i + 1]), "=d"(v[i + 2]), "=d"(v[i + 3])
+            : "l"(p + i));
+    } else if constexpr (sizeof(T) == 8 && kVec == 2) {
+      if constexpr (ONCE)
+        asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+            : "=d"(v[i]), "=d"(v[i + 1])
+            : "l"(p + i), "l"(policy));
+      else
+        asm("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v[i]), "=d"(v[i + 1]) : "l"(p + i));
+    } else {
+      v[i] = __ldg(p + i);
     }
-  } else {
+  }
+}
+
+template <typename T, int NV, bool WIDE>
+__device__ __forceinline__ void store_row(T* __restrict__ p, const T (&v)[NV]) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = __ldg(p + i);
+  for (int i = 0; i < NV; i += WIDE ? 32 / (int)sizeof(T) : 1) {
+    if constexpr (WIDE && sizeof(T) == 4)
+      asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + i), "f"(v[i]), "f"(v[i + 1]),
+                   "f"(v[i + 2]), "f"(v[i + 3]), "f"(v[i + 4]), "f"(v[i + 5]), "f"(v[i + 6]), "f"(v[i + 7])
+                   : "memory");
+    else if constexpr (WIDE)
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p + i), "d"(v[i]), "d"(v[i + 1]), "d"(v[i + 2]),
+                   "d"(v[i + 3])
+                   : "memory");
+    else
+      p[i] = v[i];
+  }
+}
+
+// Asynchronous copy of one orbit entry to shared memory.
+__device__ __forceinline__ void copy_entry(uint32_t* to, const uint32_t* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+
+// Sum of E^2 over the links of a key.
+template <int ZN>
+__device__ __forceinline__ double field_energy(const edg_zn_lattice& L, uint64_t key) {
+  const uint64_t f = key & (~0ull >> (64 - L.field_bits));
+  if constexpr (ZN == 2) {
+    const int n1 = __popcll(f);
+    return (double)(L.n_links - n1) * L.esq[0] + (double)n1 * L.esq[1];
+  } else {
+    const uint64_t low = 0x5555555555555555ull;
+    const int n3 = ZN == 4 ? __popcll(f & (f >> 1) & low) : 0;
+    const int n1 = __popcll(f & low) - n3, n2 = __popcll((f >> 1) & low) - n3;
+    return (double)(L.n_links - n1 - n2 - n3) * L.esq[0] + (double)n1 * L.esq[1] + (double)n2 * L.esq[2] +
+           (double)n3 * L.esq[3];
   }
 }
 
 constexpr int kMvThreads = 256;
 
-// Images whose loads are in flight together: four for f32 rows, two for f64
-// rows (register budget).
-template <typename T>
-constexpr int group_of() { return sizeof(T) == 4 ? 4 : 2; }
+// What a row's images need of the lattice, a link or a plaquette at a time.
+// Raising the field of link l adds step[l] to a configuration's cotree index
+// (its Gauss index within one occupation), less zn step[l] from the top value;
+// lowering is the opposite; step is zero for a tree link, whose field is no
+// digit.  The index of an image is so the row's own plus a constant and one
+// term for each field that wraps (mod 2^32; pow_cot is below), not a fresh
+// encoding from the tables.  Masks are over links, one bit each.
+struct alignas(16) ZnLink {
+  uint32_t pair, tail;     // occupation bits of both sites, of the tail
+  uint32_t between, sign;  // Jordan-Wigner mask, 1 for eta < 0
+  uint32_t mask, step, turn, unused;  // turn = zn step
+};
+struct alignas(16) ZnPlaq {
+  uint32_t m0, m1, m2, m3;  // links raised, raised, lowered, lowered by U_p
+  uint32_t t0, t1, t2, t3;  // their turns
+  uint32_t step, unused[3]; // steps of the raised less those of the lowered
+};
+struct ZnTables {
+  ZnLink link[2 * EDG_ZN_MAX_SITES];
+  ZnPlaq plaq[EDG_ZN_MAX_SITES];
+};
 
-// Images are handled a group at a time (G links, or G/2 plaquettes in both
-// directions): the G orbit-table loads are issued together, then the G x-row
-// loads, then the arithmetic, so that each thread keeps several independent
-// gathers in flight instead of one dependent pair per image.
-template <int ZN, typename T, int NV>
-__global__ void __launch_bounds__(kMvThreads, 2) zn_matvec_k(const __grid_constant__ edg_zn_lattice L, const edg_zn_basis B,
+ZnTables make_tables(const edg_zn_lattice* L) {
+  ZnTables t{};
+  uint32_t w = 1;
+  for (int c = 0; c < L->n_cot; ++c, w *= (uint32_t)L->zn) t.link[L->cot_link[c]].step = w;
+  for (int l = 0; l < L->n_links; ++l) {
+    ZnLink& k = t.link[l];
+    k.tail = 1u << L->link_tail[l];
+    k.pair = k.tail | (1u << L->link_head[l]);
+    k.between = L->link_between[l];
+    k.sign = L->link_eta[l] < 0 ? 1u : 0u;
+    k.mask = 1u << l;
+    k.turn = (uint32_t)L->zn * k.step;
+  }
+  for (int p = 0; p < L->n_sites; ++p) {
+    ZnPlaq& k = t.plaq[p];
+    const ZnLink* l[4];
+    for (int i = 0; i < 4; ++i) l[i] = &t.link[L->plaq[p][i]];
+    k.m0 = l[0]->mask, k.m1 = l[1]->mask, k.m2 = l[2]->mask, k.m3 = l[3]->mask;
+    k.t0 = l[0]->turn, k.t1 = l[1]->turn, k.t2 = l[2]->turn, k.t3 = l[3]->turn;
+    k.step = l[0]->step + l[1]->step - l[2]->step - l[3]->step;
+  }
+  return t;
+}
+
+// The even bits of a word, closed up.
+__device__ __forceinline__ uint32_t even_bits(uint64_t v) {
+  v &= 0x5555555555555555ull;
+  v = (v | v >> 1) & 0x3333333333333333ull;
+  v = (v | v >> 2) & 0x0F0F0F0F0F0F0F0Full;
+  v = (v | v >> 4) & 0x00FF00FF00FF00FFull;
+  v = (v | v >> 8) & 0x0000FFFF0000FFFFull;
+  return (uint32_t)(v | v >> 16);
+}
+
+// Links of a key at the top value and at zero, one bit a link.
+template <int ZN>
+__device__ __forceinline__ uint32_t top_links(uint64_t key) {
+  if constexpr (ZN == 2) return (uint32_t)key;
+  if constexpr (ZN == 3) return even_bits(key >> 1);
+  return even_bits(key & (key >> 1));
+}
+template <int ZN>
+__device__ __forceinline__ uint32_t zero_links(uint64_t key) {
+  if constexpr (ZN == 2) return ~(uint32_t)key;
+  return even_bits(~(key | (key >> 1)));
+}
+
+// CTAs an SM and bytes of x rows a thread has in flight together.  Rows of a
+// whole sector or more: 128 bytes at two CTAs; at three the 245,518,920-row
+// product gets slower (8 f32: 67.9 ms against 55.3, 4 f64: 61.6 against 51.3),
+// since the plaquette rows that more threads read leave L2 sooner, where
+// 4,592,128 rows gain less (0.645 ms against 0.655, 0.493 against 0.568).
+// Narrower rows: three CTAs (4 f32: 48.5 ms against 50.5, 0.423 against 0.525).
+template <typename T, int NV>
+constexpr int ctas_of() { return NV * sizeof(T) >= 32 ? 2 : 3; }
+template <typename T, int NV>
+constexpr int group_of() {
+  constexpr int g = (NV * sizeof(T) >= 32 ? 128 : 64) / (NV * (int)sizeof(T));
+  return g > 8 ? 8 : g;
+}
+
+// A thread owns row r.  First the orbit entries of all its images are copied to
+// its slots of shared memory (asynchronously: no registers, and no image waits
+// for another); then the x rows they name are gathered group by group, hops
+// before plaquettes.  slots: [n_links + 2 n_sites][kMvThreads].
+// What bounds it, over the rows of one occupation in turn: plaquettes stay
+// within that occupation's rows (51 MB of 8 f32 instances on 4 x 3 Z_3), which
+// L2 holds; the rows a hop names are spread over another occupation's and come
+// from DRAM, half of each 64-byte access unused (225 GB read for 17.7 GB of x,
+// y and keys).  Their loads pass L1 by and leave L2 first: 68.6 ms without
+// that, 55.3 with it (8 f32, 245,518,920 rows).  Below one sector a row the
+// instructions of the index arithmetic bound it (1 f32: 33 ms).  Encoding every
+// image from the tables and one orbit load before each group of four x rows:
+// 105 ms and 60.
+// WIDE: x and y rows in 32-byte accesses (both 32-byte aligned): a 16-byte load
+// asks for every sector twice.
+template <int ZN, typename T, int NV, bool WIDE>
+__global__ void __launch_bounds__(kMvThreads, ctas_of<T, NV>()) zn_matvec_k(const __grid_constant__ edg_zn_lattice L,
+                                                          const __grid_constant__ ZnTables tab, const edg_zn_basis B,
                                                           const double* __restrict__ coup, const T* __restrict__ x,
                                                           T* __restrict__ y) {
-  using Z = Zn<ZN>;
-  constexpr int kGroup = group_of<T>();
-  extern __shared__ uint64_t zsm[];
+  constexpr int kGroup = group_of<T, NV>();
+  extern __shared__ uint32_t slots[];
   __shared__ double c_t[NV], c_m[NV], c_e[NV], c_b[NV];
   __shared__ double sq_div[8], isq_div[8];
-  const int n_chunks = (L.field_bits + 7) / 8;
-  uint64_t* lut = zsm;
-  uint32_t* rank = (uint32_t*)(zsm + n_chunks * 256);
+  __shared__ ZnTables S;
+  for (int i = threadIdx.x; i < (int)(sizeof(ZnTables) / 16); i += kMvThreads)
+    reinterpret_cast<uint4*>(&S)[i] = reinterpret_cast<const uint4*>(&tab)[i];
   if (threadIdx.x < NV) {
     c_t[threadIdx.x] = -coup[4 * threadIdx.x + 0];
     c_m[threadIdx.x] = coup[4 * threadIdx.x + 1];
@@ -238,86 +400,98 @@ __global__ void __launch_bounds__(kMvThreads, 2) zn_matvec_k(const __grid_consta
     sq_div[threadIdx.x] = sqrt(d);
     isq_div[threadIdx.x] = 1.0 / sqrt(d);
   }
-  load_tables(L, lut, rank);
-  const int F = L.field_bits;
+  __syncthreads();
+  const int F = L.field_bits, n_chunks = (F + 7) / 8;
   const uint64_t pc = (uint64_t)L.pow_cot;
+  uint32_t* const mine = slots + threadIdx.x;
+  const uint64_t policy = once_policy();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < B.n_rows; r += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t key = B.keys[r];
+    const uint64_t key = __ldcs((const unsigned long long*)B.keys + r);
     const uint32_t occ = (uint32_t)(key >> F);
-    const uint32_t self = B.orbit[gauss_index(lut, rank, key, F, n_chunks, pc)];
+    int n_hop = 0;
+    uint32_t neg = 0;  // signs of the hops, by slot
+    uint32_t self;
+    {
+      uint32_t dig = 0;
+      for (int k = 0; k < n_chunks; ++k) dig += (uint32_t)__ldg(L.chunk_lut + k * 256 + (int)((key >> (8 * k)) & 255u));
+      const uint32_t* const own = B.orbit + (uint64_t)__ldg(L.occ_rank + occ) * pc;
+      self = own[dig];
+      const uint32_t top = top_links<ZN>(key), zero = zero_links<ZN>(key);
+      // hopping: c^dag_tail U c_head (tail empty, head full) and its conjugate
+#pragma unroll 4
+      for (int l = 0; l < L.n_links; ++l) {
+        const ZnLink k = S.link[l];
+        const uint32_t at = occ & k.pair;
+        if (at != 0 && at != k.pair) {
+          const bool up = (at & k.tail) == 0;
+          const uint32_t d = ((up ? top : zero) & k.mask) ? k.step - k.turn : k.step;
+          neg |= ((__popc(occ & k.between) ^ k.sign) & 1u) << n_hop;
+          copy_entry(mine + n_hop * kMvThreads,
+                     B.orbit + (uint64_t)__ldg(L.occ_rank + (occ ^ k.pair)) * pc + (uint32_t)(up ? dig + d : dig - d));
+          ++n_hop;
+        }
+      }
+      // plaquettes U_p and U_p^dag
+#pragma unroll 2
+      for (int p = 0; p < L.n_sites; ++p) {
+        const ZnPlaq k = S.plaq[p];
+        uint32_t a = dig + k.step, b = dig - k.step;
+        if (top & k.m0) a -= k.t0;
+        if (top & k.m1) a -= k.t1;
+        if (zero & k.m2) a += k.t2;
+        if (zero & k.m3) a += k.t3;
+        if (zero & k.m0) b += k.t0;
+        if (zero & k.m1) b += k.t1;
+        if (top & k.m2) b -= k.t2;
+        if (top & k.m3) b -= k.t3;
+        uint32_t* const to = mine + (L.n_links + 2 * p) * kMvThreads;
+        copy_entry(to, own + a);
+        copy_entry(to + kMvThreads, own + b);
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    double sum[NV], out[NV];
+    auto gather = [&](auto hops, const uint32_t* list, int n) {
+      // a multiple of four images for the plaquettes: no partial group up to there
+      constexpr bool kFull = !decltype(hops)::value && kGroup <= 4;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) sum[v] = 0.0;
+      for (int i0 = 0; i0 < n; i0 += kGroup, list += kGroup * kMvThreads) {
+        uint32_t e[kGroup];
+        T xv[kGroup][NV];
+#pragma unroll
+        for (int c = 0; c < kGroup; ++c) {
+          e[c] = kFull || i0 + c < n ? list[c * kMvThreads] : 0xFFFFFFFFu;
+          if (e[c] != 0xFFFFFFFFu) load_row<T, NV, WIDE, decltype(hops)::value>(x + (int64_t)(e[c] & 0x0FFFFFFFu) * NV, xv[c], policy);
+        }
+#pragma unroll
+        for (int c = 0; c < kGroup; ++c)
+          if (e[c] != 0xFFFFFFFFu) {
+            uint32_t sg = e[c];
+            if constexpr (decltype(hops)::value) sg ^= neg << (31 - c);
+            const double s = sq_div[(e[c] >> 28) & 7u];
+            const double a = __hiloint2double(__double2hiint(s) ^ (int)(sg & 0x80000000u), __double2loint(s));
+#pragma unroll
+            for (int v = 0; v < NV; ++v) sum[v] = fma(a, (double)xv[c][v], sum[v]);
+          }
+        if constexpr (decltype(hops)::value) neg >>= kGroup;
+      }
+    };
     const double inv_s = isq_div[(self >> 28) & 7u];
-    double ah[NV], ap[NV];
+    gather(std::true_type{}, mine, n_hop);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) ah[v] = ap[v] = 0.0;
-    // hopping: c^dag_tail U c_head (tail empty, head full) and its conjugate;
-    // links in groups (n_links = 2 * n_sites is a multiple of four)
-    for (int l0 = 0; l0 < L.n_links; l0 += kGroup) {
-      uint32_t e[kGroup];
-      int neg[kGroup];
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c) {
-        const int l = l0 + c;
-        const int ta = L.link_tail[l], he = L.link_head[l];
-        const uint32_t nt = (occ >> ta) & 1u, nh = (occ >> he) & 1u;
-        e[c] = 0xFFFFFFFFu;
-        neg[c] = (int)(__popc(occ & L.link_between[l]) & 1) ^ (L.link_eta[l] < 0);
-        if (nt != nh) {
-          const int f = Z::field(key, l);
-          uint64_t k2 = Z::set(key, l, nt == 0 ? Z::inc(f) : Z::dec(f));
-          k2 ^= ((1ull << ta) | (1ull << he)) << F;
-          e[c] = B.orbit[gauss_index(lut, rank, k2, F, n_chunks, pc)];
-        }
-      }
-      T xv[kGroup][NV];
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c)
-        if (e[c] != 0xFFFFFFFFu) load_row<T, NV>(x + (int64_t)(e[c] & 0x0FFFFFFFu) * NV, xv[c]);
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c)
-        if (e[c] != 0xFFFFFFFFu) {
-          const double s = sq_div[(e[c] >> 28) & 7u] * inv_s;
-          const double a = (neg[c] ^ (int)(e[c] >> 31)) ? -s : s;
-#pragma unroll
-          for (int v = 0; v < NV; ++v) ah[v] = fma(a, (double)xv[c][v], ah[v]);
-        }
-    }
-    // plaquettes U_p and U_p^dag, kGroup / 2 plaquettes per group
-    for (int p0 = 0; p0 < L.n_sites; p0 += kGroup / 2) {
-      uint32_t e[kGroup];
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c) {
-        const int p = p0 + c / 2, dir = c & 1;
-        const int l0 = L.plaq[p][0], l1 = L.plaq[p][1], l2 = L.plaq[p][2], l3 = L.plaq[p][3];
-        uint64_t k2 = key;
-        k2 = Z::set(k2, l0, dir == 0 ? Z::inc(Z::field(key, l0)) : Z::dec(Z::field(key, l0)));
-        k2 = Z::set(k2, l1, dir == 0 ? Z::inc(Z::field(key, l1)) : Z::dec(Z::field(key, l1)));
-        k2 = Z::set(k2, l2, dir == 0 ? Z::dec(Z::field(key, l2)) : Z::inc(Z::field(key, l2)));
-        k2 = Z::set(k2, l3, dir == 0 ? Z::dec(Z::field(key, l3)) : Z::inc(Z::field(key, l3)));
-        e[c] = B.orbit[gauss_index(lut, rank, k2, F, n_chunks, pc)];
-      }
-      T xv[kGroup][NV];
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c)
-        if (e[c] != 0xFFFFFFFFu) load_row<T, NV>(x + (int64_t)(e[c] & 0x0FFFFFFFu) * NV, xv[c]);
-#pragma unroll
-      for (int c = 0; c < kGroup; ++c)
-        if (e[c] != 0xFFFFFFFFu) {
-          const double s = sq_div[(e[c] >> 28) & 7u] * inv_s;
-          const double a = (e[c] >> 31) ? -s : s;
-#pragma unroll
-          for (int v = 0; v < NV; ++v) ap[v] = fma(a, (double)xv[c][v], ap[v]);
-        }
-    }
-    double esq = 0.0;
-    for (int l = 0; l < L.n_links; ++l) esq += L.esq[Z::field(key, l)];
+    for (int v = 0; v < NV; ++v) out[v] = c_t[v] * (inv_s * sum[v]);
+    gather(std::false_type{}, mine + L.n_links * kMvThreads, 2 * L.n_sites);
+    const double esq = field_energy<ZN>(L, key);
     const double mass = (double)(__popc(occ & L.even_mask) - __popc(occ & ~L.even_mask));
     T xr[NV];
-    load_row<T, NV>(x + r * NV, xr);
+    load_row<T, NV, WIDE, false>(x + r * NV, xr, policy);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       const double d = c_e[v] * esq + c_m[v] * mass;
-      y[r * NV + v] = (T)(fma(d, (double)xr[v], fma(c_t[v], ah[v], c_b[v] * ap[v])));
+      xr[v] = (T)(fma(d, (double)xr[v], fma(c_b[v], inv_s * sum[v], out[v])));
     }
+    store_row<T, NV, WIDE>(y + r * NV, xr);
   }
 }
 
@@ -348,7 +522,7 @@ size_t table_smem(const edg_zn_lattice* L) {
 
 template <typename K>
 int set_smem(K kernel, size_t smem, const char* where) {
-  if (smem > 48 * 1024) {
+  if (smem > 40 * 1024) {  // 48 KB less the kernels' own static arrays
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return edg::cuda_status(e, where);
   }
@@ -364,15 +538,18 @@ unsigned persistent_grid(K kernel, int threads, size_t smem, int64_t n_items) {
   return edg::grid_for(n_items, threads, per_sm);
 }
 
-template <int ZN, typename T, int NV>
+template <int ZN, typename T, int NV, bool WIDE>
 int launch_matvec(const edg_zn_lattice* L, const edg_zn_basis* B, const double* coup, const void* x, void* y,
                   cudaStream_t stream) {
-  const size_t smem = table_smem(L);
-  auto kern = zn_matvec_k<ZN, T, NV>;
+  if constexpr (!WIDE && NV * sizeof(T) % 32 == 0) {
+    if ((((uintptr_t)x | (uintptr_t)y) & 31u) == 0) return launch_matvec<ZN, T, NV, true>(L, B, coup, x, y, stream);
+  }
+  const size_t smem = sizeof(uint32_t) * kMvThreads * (size_t)(L->n_links + 2 * L->n_sites);
+  auto kern = zn_matvec_k<ZN, T, NV, WIDE>;
   int st = set_smem(kern, smem, "edg_zn_matvec");
   if (st != EDG_OK) return st;
   const unsigned grid = persistent_grid(kern, kMvThreads, smem, B->n_rows);
-  kern<<<grid, kMvThreads, smem, stream>>>(*L, *B, coup, (const T*)x, (T*)y);
+  kern<<<grid, kMvThreads, smem, stream>>>(*L, make_tables(L), *B, coup, (const T*)x, (T*)y);
   EDG_CHECK_LAUNCH("edg_zn_matvec");
   return EDG_OK;
 }
@@ -382,8 +559,8 @@ int dispatch_matvec(const edg_zn_lattice* L, const edg_zn_basis* B, const double
                     const void* x, void* y, cudaStream_t s) {
 #define EDG_ZN_MV(NV)                                                           \
   case NV:                                                                      \
-    return dtype == 0 ? launch_matvec<ZN, double, NV>(L, B, coup, x, y, s)      \
-                      : launch_matvec<ZN, float, NV>(L, B, coup, x, y, s);
+    return dtype == 0 ? launch_matvec<ZN, double, NV, false>(L, B, coup, x, y, s)      \
+                      : launch_matvec<ZN, float, NV, false>(L, B, coup, x, y, s);
   switch (nvec) {
     EDG_ZN_MV(1)
     EDG_ZN_MV(2)

@@ -248,3 +248,29 @@ def test_matvec_rejects_bad_arguments():
     x = torch.zeros((eng.n_rows, 3), dtype=torch.float64, device="cuda")
     with pytest.raises(EdgError):
         eng.matvec(x, torch.zeros_like(x), coup, 3)
+
+
+@pytest.mark.parametrize("nvec,dtype", [(8, "float32"), (4, "float64"), (8, "float64"), (4, "float32"), (1, "float64")])
+@pytest.mark.parametrize("shift", [0, 16])
+def test_matvec_row_alignment(nvec, dtype, shift):
+    """The same product from x and to y at any 16-byte boundary (32-byte
+    accesses need more), with nothing written past y."""
+    import torch
+
+    from edgpu.models.zn_model import ZnModel
+
+    e = ZnModel((4, 2), 3, device="cuda").engine
+    dt = getattr(torch, dtype)
+    n, off = e.n_rows * nvec, shift // torch.empty(0, dtype=dt).element_size()
+    coup = torch.tensor([[1.0, 0.3 + v, 0.7, -0.6] for v in range(nvec)], dtype=torch.float64, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(n, dtype=dt, device="cuda", generator=gen)
+    ref = torch.empty_like(x)
+    e.matvec(x, ref, coup, nvec)
+    for ox, oy in ((off, 0), (0, off), (off, off)):
+        xs = torch.zeros(n + 16, dtype=dt, device="cuda")
+        ys = torch.full((n + 16,), 7.0, dtype=dt, device="cuda")
+        xs[ox: ox + n] = x
+        e.matvec(xs[ox: ox + n], ys[oy: oy + n], coup, nvec)
+        assert torch.equal(ys[oy: oy + n], ref)
+        assert bool((ys[:oy] == 7).all()) and bool((ys[oy + n:] == 7).all())
