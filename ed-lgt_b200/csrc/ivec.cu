@@ -25,6 +25,10 @@ struct Slot<float> {
     const float4 a = *reinterpret_cast<const float4*>(p);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   }
+  __device__ static __forceinline__ void raw(const float* p, float (&v)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  }
   __device__ static __forceinline__ void store(float* p, const double (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
   }
@@ -36,6 +40,7 @@ struct Slot<double> {
     const double2 b = reinterpret_cast<const double2*>(p)[1];
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
   }
+  __device__ static __forceinline__ void raw(const double* p, double (&v)[4]) { load(p, v); }
   __device__ static __forceinline__ void store(double* p, const double (&v)[4]) {
     reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
     reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
@@ -192,56 +197,62 @@ __global__ void __launch_bounds__(kThreads) combine_k(T* __restrict__ V, int64_t
   }
 }
 
-// Dots of a tile of KT basis vectors against two vectors at once (the
+// Dots of a tile of four basis vectors against two vectors at once (the
 // lagged candidate u and the new matvec result w of a delayed Gram-Schmidt
 // step): partial[block][i][r][class][4], r = 0 for x1, 1 for x2.
-template <typename T, int NV, int KT>
-__global__ void __launch_bounds__(kThreads) dots2_k(const T* __restrict__ V, int64_t stride, int m,
-                                                    const T* __restrict__ x1, const T* __restrict__ x2,
-                                                    int64_t n_slots, double* __restrict__ partial) {
+// The 32 sums of a thread end in one lane each by halving (31 exchanges, 5 a
+// sum before), and the grid is one resident wave, so that the sums' way out of
+// the registers is paid once a CTA: 345,546 rows of 4 f32 instances, 0 to 24
+// basis vectors, 44 us a step before and 20 here (the basis alone takes 13 at
+// the copy rate).
+constexpr int kTile2 = 4;
+template <typename T, int NV>
+__global__ void __launch_bounds__(kThreads, 2) dots2_k(const T* __restrict__ V, int64_t stride, int m,
+                                                       const T* __restrict__ x1, const T* __restrict__ x2,
+                                                       int64_t n_slots, double* __restrict__ partial) {
   constexpr int P = classes<NV>();
-  __shared__ double red[kWarps][KT][2][P][4];
-  const int i0 = blockIdx.y * KT;
-  const int ni = min(KT, m - i0);
-  double acc[KT][2][4];
+  constexpr int kSums = kTile2 * 8;  // index 8 i + 4 r + j
+  static_assert(kSums == 32 && P <= 2);
+  __shared__ double red[kWarps][kSums][P];
+  const int i0 = blockIdx.y * kTile2;
+  const int ni = min(kTile2, m - i0);
+  double acc[kSums];
 #pragma unroll
-  for (int i = 0; i < KT; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][0][j] = acc[i][1][j] = 0.0;
+  for (int q = 0; q < kSums; ++q) acc[q] = 0.0;
   for (int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x; s < n_slots; s += (int64_t)gridDim.x * kThreads) {
     double a[4], b[4], vv[4];
     Slot<T>::load(x1 + 4 * s, a);
     Slot<T>::load(x2 + 4 * s, b);
 #pragma unroll
-    for (int i = 0; i < KT; ++i) {
+    for (int i = 0; i < kTile2; ++i) {
       if (i < ni) {
         Slot<T>::load(V + (int64_t)(i0 + i) * stride + 4 * s, vv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          acc[i][0][j] = fma(vv[j], a[j], acc[i][0][j]);
-          acc[i][1][j] = fma(vv[j], b[j], acc[i][1][j]);
+          acc[8 * i + j] = fma(vv[j], a[j], acc[8 * i + j]);
+          acc[8 * i + 4 + j] = fma(vv[j], b[j], acc[8 * i + 4 + j]);
         }
       }
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < KT; ++i)
+  for (int o = 16; o >= P; o >>= 1) {
+    const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int q = 0; q < o; ++q) {
+      const double send = up ? acc[q] : acc[q + o];
+      acc[q] = (up ? acc[q + o] : acc[q]) + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        double x = acc[i][r][j];
-#pragma unroll
-        for (int o = 16; o >= P; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane < P) red[warp][i][r][lane][j] = x;
-      }
+  for (int q = 0; q < P; ++q) red[warp][(lane & ~(P - 1)) + q][lane & (P - 1)] = acc[q];
   __syncthreads();
-  for (int t = threadIdx.x; t < KT * 2 * P * 4; t += kThreads) {
-    const int i = t / (2 * P * 4), r = (t / (P * 4)) % 2, q = t % (P * 4);
+  for (int t = threadIdx.x; t < kSums * P; t += kThreads) {
+    const int i = t / (8 * P), r = (t / (4 * P)) % 2, c = (t / 4) % P, j = t % 4;
     double x = 0.0;
-    for (int k = 0; k < kWarps; ++k) x += red[k][i][r][q / 4][q % 4];
-    if (i < ni) partial[(((int64_t)blockIdx.x * m + i0 + i) * 2 + r) * (P * 4) + q] = x;
+    for (int k = 0; k < kWarps; ++k) x += red[k][8 * i + 4 * r + j][c];
+    if (i < ni) partial[(((int64_t)blockIdx.x * m + i0 + i) * 2 + r) * (P * 4) + 4 * c + j] = x;
   }
 }
 
@@ -283,47 +294,60 @@ __global__ void __launch_bounds__(kThreads) dots2_reduce_k(const double* __restr
 // w <- w - sum_i V_i z_i - q c (one pass of w against V_0..V_j), with the
 // squared norm of the stored w per CTA and slot class (reduced by
 // dots_reduce_k).
+// A thread keeps kAhead basis rows in flight, and the scalars of the step are a
+// warp's sums, an instance each: 22 us a step, where one row at a time and a
+// thread's loop over the coefficients took 31 (sizes as for dots2_k).
 template <typename T, int NV>
-__global__ void __launch_bounds__(kThreads) dcgs_update_k(T* __restrict__ V, int64_t stride, int j,
+__global__ void __launch_bounds__(kThreads, 3) dcgs_update_k(T* __restrict__ V, int64_t stride, int j,
                                                           const double* __restrict__ hu,
                                                           const double* __restrict__ hw, T* __restrict__ w,
                                                           int64_t n_slots, double* __restrict__ partial) {
   constexpr int P = classes<NV>();
-  __shared__ double ss[kMaxM * 8], zs[kMaxM * 8];
+  constexpr int kAhead = sizeof(T) == 4 ? 6 : 3;
+  __shared__ double2 sz[kMaxM * 8];  // (s, z) of a vector and instance
   __shared__ double rinv[8], cq[8];
   __shared__ double red[kWarps][P][4];
-  for (int t = threadIdx.x; t < j * NV; t += kThreads) {
-    ss[t] = hu[t];
-    zs[t] = hw[t];
-  }
-  if (threadIdx.x < NV) {
-    const int v = threadIdx.x;
-    double s2 = 0.0, sz = 0.0;
-    for (int i = 0; i < j; ++i) {
-      s2 = fma(hu[i * NV + v], hu[i * NV + v], s2);
-      sz = fma(hu[i * NV + v], hw[i * NV + v], sz);
+  for (int t = threadIdx.x; t < j * NV; t += kThreads) sz[t] = make_double2(hu[t], hw[t]);
+  static_assert(kMaxM <= 32 && NV <= kWarps);
+  if (threadIdx.x < 32 * NV) {
+    const int v = threadIdx.x >> 5, i = threadIdx.x & 31;
+    const double si = i < j ? hu[i * NV + v] : 0.0;
+    double s2 = si * si, sw = i < j ? si * hw[i * NV + v] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      sw += __shfl_xor_sync(0xffffffffu, sw, o);
     }
-    const double r2 = hu[j * NV + v] - s2;
-    const double ri = r2 > 0.0 ? 1.0 / sqrt(r2) : 0.0;
-    rinv[v] = ri;
-    cq[v] = (hw[j * NV + v] - sz) * ri;
+    if (i == 0) {
+      const double r2 = hu[j * NV + v] - s2;
+      const double ri = r2 > 0.0 ? 1.0 / sqrt(r2) : 0.0;
+      rinv[v] = ri;
+      cq[v] = (hw[j * NV + v] - sw) * ri;
+    }
   }
   __syncthreads();
   T* U = V + (int64_t)j * stride;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x; s < n_slots; s += (int64_t)gridDim.x * kThreads) {
-    double uv[4], wv[4], vv[4];
+    double uv[4], wv[4];
     Slot<T>::load(U + 4 * s, uv);
     Slot<T>::load(w + 4 * s, wv);
     const int base = (int)((4 * s) % NV);
-    for (int i = 0; i < j; ++i) {
-      Slot<T>::load(V + (int64_t)i * stride + 4 * s, vv);
+    for (int i0 = 0; i0 < j; i0 += kAhead) {
+      T raw[kAhead][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int v = (base + k) % NV;
-        uv[k] = fma(-vv[k], ss[i * NV + v], uv[k]);
-        wv[k] = fma(-vv[k], zs[i * NV + v], wv[k]);
-      }
+      for (int t = 0; t < kAhead; ++t)
+        if (i0 + t < j) Slot<T>::raw(V + (int64_t)(i0 + t) * stride + 4 * s, raw[t]);
+#pragma unroll
+      for (int t = 0; t < kAhead; ++t)
+        if (i0 + t < j) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const double2 c = sz[(i0 + t) * NV + (base + k) % NV];
+            uv[k] = fma(-(double)raw[t][k], c.x, uv[k]);
+            wv[k] = fma(-(double)raw[t][k], c.y, wv[k]);
+          }
+        }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -476,22 +500,17 @@ int run_dots(int64_t n_elems, const void* V, int64_t stride, int m, const void* 
   return run_dots_kt<T, NV, 4>(n_elems, V, stride, m, w, h, scratch, stream);
 }
 
-template <typename T, int NV, int KT>
+template <typename T, int NV>
 int run_dots2(int64_t n_elems, const void* V, int64_t stride, int m, const void* x1, const void* x2, double* h1,
               double* h2, double* scratch, cudaStream_t stream) {
   const int64_t n_slots = n_elems / 4;
-  const int tiles = (m + KT - 1) / KT;
-  int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dots2_k<T, NV, KT>, kThreads, 0) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
+  const int tiles = (m + kTile2 - 1) / kTile2;
   int64_t nbx = edg::ceil_div(n_slots, kThreads);
-  const int64_t cap = (int64_t)edg::kSmCount * (per_sm < 8 ? per_sm : 8);
-  const int64_t cap_t = cap / tiles > edg::kSmCount ? cap / tiles : edg::kSmCount;
-  if (nbx > cap_t) nbx = cap_t;
+  const int64_t cap = edg::kSmCount * 2 / tiles;  // one wave of resident CTAs
+  if (nbx > cap) nbx = cap;
   if (nbx < 1) nbx = 1;
-  dots2_k<T, NV, KT><<<dim3((unsigned)nbx, tiles), kThreads, 0, stream>>>((const T*)V, stride, m, (const T*)x1,
-                                                                         (const T*)x2, n_slots, scratch);
+  dots2_k<T, NV><<<dim3((unsigned)nbx, tiles), kThreads, 0, stream>>>((const T*)V, stride, m, (const T*)x1,
+                                                                      (const T*)x2, n_slots, scratch);
   dots2_reduce_k<NV><<<2 * m, kThreads, 0, stream>>>(scratch, (int)nbx, m, h1, h2);
   return EDG_OK;
 }
@@ -662,7 +681,7 @@ extern "C" int edg_iv_dots2(int32_t dtype, int64_t n_elems, int32_t nvec, const 
     if (e == cudaSuccess) e = cudaMemsetAsync(h2, 0, sizeof(double) * (size_t)m * nvec, stream);
     return e == cudaSuccess ? EDG_OK : edg::cuda_status(e, "edg_iv_dots2");
   }
-#define CALL(T, NV) run_dots2<T, NV, 4>(n_elems, V, stride, m, x1, x2, h1, h2, scratch, stream)
+#define CALL(T, NV) run_dots2<T, NV>(n_elems, V, stride, m, x1, x2, h1, h2, scratch, stream)
   EDG_IV_DISPATCH(CALL)
 #undef CALL
   if (st != EDG_OK) return st;

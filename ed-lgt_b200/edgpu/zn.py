@@ -294,9 +294,12 @@ def trlan_batched(apply, n_rows, nvec, dtype, m, k_keep, k_want, tol, max_cycles
 def _auto_m(vec_bytes, cap, reserve_vectors=3):
     """Basis length that fits the free device memory (w, a copy and a margin
     besides the basis), at most cap."""
-    torch.cuda.empty_cache()  # blocks cached by torch count as free here
-    free, _ = torch.cuda.mem_get_info()
-    fit = int((free - (1 << 30)) // max(vec_bytes, 1)) - reserve_vectors
+    for _ in range(2):
+        free, _ = torch.cuda.mem_get_info()
+        fit = int((free - (1 << 30)) // max(vec_bytes, 1)) - reserve_vectors
+        if fit >= cap:
+            break
+        torch.cuda.empty_cache()  # blocks cached by torch count as free here
     return max(4, min(cap, fit))
 
 
