@@ -155,3 +155,38 @@ def test_tiled_single_row_and_tiny_instances(dev):
     tb.check_status()
     for i, w in enumerate(dense):
         assert abs(e[i] - w[0]) < 1e-10 * max(1.0, abs(w[0])), (i, e[i], w[0])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("tile_rows,dims", [(4, (4, 251, 256, 257, 520)), (256, (255, 1100)), (260, (260, 1100)),
+                                            (512, (513, 1100)), (516, (515, 1100)), (1024, (1100,))])
+def test_tiles_per_instance_and_rows_per_tile(precision, tile_rows, dims, dev):
+    """Instances on both sides of the tile count whose partial sums every item
+    takes for itself (64), alone and together, and tiles around the lengths at
+    which lanes share a quad of rows: the well's eigenpair to the solver's
+    tolerance."""
+    import torch
+    from scipy.sparse import diags
+
+    from edgpu.batch import TiledBatch
+    from edgpu.modeling.assembly import DeviceMatrix
+
+    rng = np.random.default_rng(sum(dims) + tile_rows)
+    t = lambda a, dt: torch.from_numpy(np.array(a, dtype=dt)).to(dev)  # noqa: E731
+    mats, ref = [], []
+    for n in dims:
+        d = rng.uniform(0, 1, n)
+        d[n // 3] = -9.0  # an isolated lowest state
+        bands = [rng.uniform(-1, 1, n - o) for o in (1, 2, 3)]
+        off = diags(bands + bands, [1, 2, 3, -1, -2, -3], shape=(n, n)).tocsr()
+        mats.append(DeviceMatrix(n, t(off.indptr, np.int64), t(off.indices, np.int32), t(off.data, np.float64),
+                                 t(d, np.float64), t(np.ones(n), np.uint8), False))
+        ref.append(off.toarray() + np.diag(d))
+    tb = TiledBatch(mats, precision=precision, tile_rows=tile_rows, lanes=2, want_vectors=True)
+    e = tb.solve(use_graph=False).cpu().numpy()[:, 0]
+    tb.check_status()
+    vecs = np.split(tb.evecs.cpu().numpy(), np.cumsum(dims)[:-1])
+    for h, ei, v in zip(ref, e, vecs):
+        w = np.linalg.eigvalsh(h)[0]
+        assert abs(ei - w) <= (1e-10 if precision == "fp64" else 1e-9) * abs(w)
+        assert np.linalg.norm(h @ v - w * v) <= 1e-4 * abs(w) and abs(np.linalg.norm(v) - 1) <= 1e-10
