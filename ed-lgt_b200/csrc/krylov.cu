@@ -417,10 +417,11 @@ __global__ void combine_k(const T* __restrict__ V, int64_t n, int64_t ldv, int m
 // basis stay in its shared memory where they fit, and only the gathers of
 // u_j, the dots partials and the next vector go through L2.  Per Krylov step
 // two grid-wide waits: for the dots, and for the norm with the next vector.
-// Bound by those waits and the few dependent L2 reads between them, about
-// 7 us a Krylov step.  A step of dt = 0.05 (m = 30, full reorthogonalisation,
+// Bound by those waits and the dependent L2 reads between them: the partials of
+// a sum are asked for together, and those of the norm while the product runs
+// (12,292 rows: 0.31 ms without, 0.29 with).  A step of dt = 0.05 (m = 30, full reorthogonalisation,
 // complex128, static-pair SU(2) chains; launches per pass before):
-//   n = 182: 0.18 ms (1.48), 12,292: 0.31 ms (1.69), 101,613: 0.63 ms (1.87).
+//   n = 12,292: 0.29 ms (1.69), 101,613: 0.61 ms (1.87).
 // The line (kCoopRows rows per SM) lies where the matrix and the basis no
 // longer fit shared memory: at 101,613 rows the passes below take 0.96 ms, at
 // 848,614 rows this form takes 6.6 ms and the passes 4.2.
@@ -450,13 +451,20 @@ struct CoopArgs {
   int m, reorth;
 };
 
+template <typename SV>
+__device__ __forceinline__ void load_diag(const SV* __restrict__ d, int64_t r, edg::cd& o) {
+  if constexpr (edg::Store<SV>::cplx)
+    o = edg::cd{(double)d[r].x, (double)d[r].y};
+  else
+    o.re = (double)d[r];
+}
+
 template <typename T, typename SV>
 __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<T, SV> A) {
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ double2 hs[kMaxM + 1];
   __shared__ double al[kMaxM], be[kMaxM + 2];
   __shared__ double red[kCoopWarps];
-  __shared__ double s_total;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = (int)gridDim.x, m = A.m;
   const int64_t r0 = A.n * blockIdx.x / G, r1 = A.n * (blockIdx.x + 1) / G;
@@ -489,43 +497,50 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
     ld = rows;
   }
   edg::GridSync gs{A.bar, A.err};
+  // one value per thread to this CTA's partial, and a grid-wide wait
   unsigned waits = 0;  // parity of the norm partials' buffer
-  // sum over the grid of one value per thread; false when a wait ran out
-  auto grid_sum = [&](double a, double* out) -> bool {
+  auto post_sum = [&](double a) -> bool {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (lane == 0) red[warp] = a;
     __syncthreads();
-    double* part = A.npart + (int64_t)(waits & 1) * G;
     ++waits;
     if (tid == 0) {
       double t = 0.0;
       for (int q = 0; q < kCoopWarps; ++q) t += red[q];
-      part[blockIdx.x] = t;
+      A.npart[(int64_t)(waits & 1) * G + blockIdx.x] = t;
     }
-    if (!gs.wait()) return false;
-    if (warp == 0) {
-      double t = 0.0;
-      for (int b = lane; b < G; b += 32) t += __ldcg(part + b);
+    return gs.wait();
+  };
+  // the partials of the last post_sum (a warp's loads, all in flight), and
+  // their sum
+  constexpr int kPer = (edg::kSmCount + 31) / 32;
+  double np[kPer];
+  auto load_sum = [&] {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) s_total = t;
-    }
-    __syncthreads();
-    *out = s_total;
-    return true;
+    for (int k = 0; k < kPer; ++k)
+      np[k] = lane + 32 * k < G ? __ldcg(A.npart + (int64_t)(waits & 1) * G + lane + 32 * k) : 0.0;
+  };
+  auto take_sum = [&] {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) t += np[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
   };
   auto give_up = [&] {
     if (tid == 0 && A.status != nullptr) atomicExch(A.status, EDG_ERR_TIMEOUT);
   };
   // ---- u_0 = psi / |psi| ----
-  double a = 0.0, tot;
+  double a = 0.0;
   for (int r = tid; r < rows; r += kCoopThreads) {
     const edg::cd x = ldc<T>(A.psi, r0 + r);
     a = fma(x.re, x.re, fma(x.im, x.im, a));
   }
-  if (!grid_sum(a, &tot)) return give_up();
-  const double b0 = sqrt(tot), inv0 = b0 > 0.0 ? 1.0 / b0 : 0.0;
+  if (!post_sum(a)) return give_up();
+  load_sum();
+  const double b0 = sqrt(take_sum()), inv0 = b0 > 0.0 ? 1.0 / b0 : 0.0;
   if (tid == 0) be[0] = b0 > 0.0 ? 1.0 : 0.0;
   for (int r = tid; r < rows; r += kCoopThreads) {
     const edg::cd x = ldc<T>(A.psi, r0 + r);
@@ -534,8 +549,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
   }
   if (!gs.wait()) return give_up();
   for (int j = 0; j < m; ++j) {
-    const double sj = be[j] > 0.0 ? 1.0 / be[j] : 0.0;
-    // ---- w = H u_j / beta_j on this CTA's rows ----
+    // ---- w = H u_j on this CTA's rows; |u_j| meanwhile ----
+    if (j > 0 && warp == 0) load_sum();
     {
       const T* u = A.V + (int64_t)j * A.ldv;
       const int part = tid & (kMvLanes - 1);
@@ -543,6 +558,12 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
       for (int it = 0; it < n_it; ++it) {
         const int r = it * (kCoopThreads / kMvLanes) + tid / kMvLanes;
         edg::cd acc{0.0, 0.0};
+        T xr{};
+        edg::cd dr{0.0, 0.0};
+        if (r < rows && part == 0) {
+          xr = u[r0 + r];
+          load_diag(A.diag, r0 + r, dr);
+        }
         if (r < rows) {
           constexpr int U = 4;  // gathers in flight per lane
           const int end = rp[r + 1];
@@ -572,11 +593,17 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
           acc.im += __shfl_xor_sync(0xffffffffu, acc.im, o, kMvLanes);
         }
         if (r < rows && part == 0) {
-          const T xr = u[r0 + r];
-          edg::fma_acc(acc, edg::Store<SV>::ld(A.diag, r0 + r), edg::cd{(double)xr.x, (double)xr.y});
-          w[r] = make_double2(acc.re * sj, acc.im * sj);
+          if constexpr (edg::Store<SV>::cplx)
+            edg::fma_acc(acc, dr, edg::cd{(double)xr.x, (double)xr.y});
+          else
+            edg::fma_acc(acc, dr.re, edg::cd{(double)xr.x, (double)xr.y});
+          w[r] = make_double2(acc.re, acc.im);
         }
       }
+    }
+    if (j > 0 && warp == 0) {
+      const double t = take_sum();
+      if (lane == 0) be[j] = sqrt(t);
     }
     const int passes = A.reorth == 0 ? 1 : A.reorth;
     const int ilo = A.reorth == 0 ? (j > 0 ? j - 1 : 0) : 0;
@@ -602,22 +629,37 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
         if (lane == 0) P[(int64_t)blockIdx.x * (kMaxM + 1) + i] = make_double2(gr, gi);
       }
       if (!gs.wait()) return give_up();
-      for (int i = ilo + warp; i <= j; i += kCoopWarps) {
-        double gr = 0.0, gi = 0.0;
-        for (int b = lane; b < G; b += 32) {
-          const double2 p = __ldcg(P + (int64_t)b * (kMaxM + 1) + i);
-          gr += p.x;
-          gi += p.y;
-        }
+      // the product was not divided by beta_j: the first pass does
+      const double ws = pass > 0 ? 1.0 : (be[j] > 0.0 ? 1.0 / be[j] : 0.0);
+      for (int i0 = ilo + warp; i0 <= j; i0 += 2 * kCoopWarps) {
+        double2 p[2][kPer];  // two vectors' partials in flight
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          gr += __shfl_xor_sync(0xffffffffu, gr, o);
-          gi += __shfl_xor_sync(0xffffffffu, gi, o);
-        }
-        if (lane == 0) {
-          const double si = be[i] > 0.0 ? 1.0 / be[i] : 0.0;
-          hs[i] = make_double2(si * (si * gr), si * (si * gi));
-          if (i == j) al[j] = pass > 0 ? al[j] + si * gr : si * gr;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int k = 0; k < kPer; ++k)
+            p[h][k] = i0 + h * kCoopWarps <= j && lane + 32 * k < G
+                          ? __ldcg(P + (int64_t)(lane + 32 * k) * (kMaxM + 1) + i0 + h * kCoopWarps)
+                          : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          double gr = 0.0, gi = 0.0;
+#pragma unroll
+          for (int k = 0; k < kPer; ++k) {
+            gr += p[h][k].x;
+            gi += p[h][k].y;
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            gr += __shfl_xor_sync(0xffffffffu, gr, o);
+            gi += __shfl_xor_sync(0xffffffffu, gi, o);
+          }
+          const int i = i0 + h * kCoopWarps;
+          if (lane == 0 && i <= j) {
+            const double si = be[i] > 0.0 ? 1.0 / be[i] : 0.0;
+            gr *= ws, gi *= ws;
+            hs[i] = make_double2(si * (si * gr), si * (si * gi));
+            if (i == j) al[j] = pass > 0 ? al[j] + si * gr : si * gr;
+          }
         }
       }
       __syncthreads();
@@ -632,7 +674,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
           sr = fma(x.re, hs[i].x, fma(-x.im, hs[i].y, sr));
           si = fma(x.re, hs[i].y, fma(x.im, hs[i].x, si));
         }
-        const double2 y = make_double2(w[r].x - sr, w[r].y - si);
+        const double2 y = make_double2(fma(ws, w[r].x, -sr), fma(ws, w[r].y, -si));
         if (last) {
           stc<T>(A.V, (int64_t)(j + 1) * A.ldv + r0 + r, y.x, y.y);
           if (basis_here) stc<T>(own, (int64_t)(j + 1) * ld + r, y.x, y.y);
@@ -641,15 +683,15 @@ __global__ void __launch_bounds__(kCoopThreads, 1) krylov_coop_k(const CoopArgs<
           w[r] = y;
         }
       }
-      if (last) {
-        if (!grid_sum(nrm, &tot)) return give_up();
-        if (tid == 0) be[j + 1] = sqrt(tot);
-        __syncthreads();
-      }
+      if (last && !post_sum(nrm)) return give_up();
     }
   }
   // ---- psi = V c: every CTA forms the coefficients itself ----
   if (warp == 0) {
+    load_sum();
+    const double t = take_sum();
+    if (lane == 0) be[m] = sqrt(t);
+    __syncwarp();
     const double e = warp_expm(al, be, m, A.dt, b0, hs);
     if (lane == 0 && blockIdx.x == 0) A.err_out[0] = e;
   }
