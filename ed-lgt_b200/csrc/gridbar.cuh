@@ -68,4 +68,26 @@ struct GridSync {
   }
 };
 
+// A lane's share of the sum of n values, stride apart, that other CTAs wrote:
+// every 32nd, N of them in flight.  A plain loop asks for a few at a time and
+// for its remainder one by one, an L2 round trip each.
+template <int N>
+__device__ __forceinline__ double lane_share(const double* p, int64_t stride, int n) {
+  double a = 0.0;
+  for (int b = threadIdx.x & 31; b < n; b += 32 * N) {
+    double v[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = b + 32 * k < n ? __ldcg(p + (b + 32 * k) * stride) : 0.0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) a += v[k];
+  }
+  return a;
+}
+
+__device__ __forceinline__ double warp_sum(double a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
 }  // namespace edg

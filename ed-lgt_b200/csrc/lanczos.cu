@@ -692,10 +692,8 @@ __global__ void __launch_bounds__(kSmallThreads) reorth_small_k(
   // ---- totals and coefficients (every CTA, the same order everywhere) -----
   for (int e = warp; e < NV * 2 * n_vec; e += kSmallThreads / 32) {
     const int vv = e / (2 * n_vec), rem = e - vv * 2 * n_vec;
-    double a = 0.0;
-    for (int bb = lane; bb < G; bb += 32) a += __ldcg(partial + (int64_t)(vv * G + bb) * (2 * kSmallMax) + rem);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    const double a =
+        edg::warp_sum(edg::lane_share<8>(partial + (int64_t)vv * G * (2 * kSmallMax) + rem, 2 * kSmallMax, G));
     if (lane == 0) tot[vv][rem] = a;
   }
   __syncthreads();
@@ -804,10 +802,7 @@ __global__ void __launch_bounds__(kSmallThreads) reorth_small_k(
   if (!last) return;
   __threadfence();
   if (warp < NV) {  // warp v: lanes stride over the CTAs, fixed-order butterfly
-    double a = 0.0;
-    for (int bb = lane; bb < (int)gridDim.x; bb += 32) a += __ldcg(norm_partial + (int64_t)bb * NV + warp);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    const double a = edg::warp_sum(edg::lane_share<10>(norm_partial + warp, NV, (int)gridDim.x));
     if (lane == 0) {
       const double nv = sqrt(a);
       wnorm[warp] = nv;
@@ -978,19 +973,21 @@ __global__ void ritz_k(const T* __restrict__ V, int64_t n_pad, int m, const doub
 // candidate and |w|.  When a check is due CTA 0 solves the tridiagonal
 // matrices while the others wait.  The arithmetic of a row is that of the
 // passes above; only the order of the sums over rows differs.  Bound by the
-// two waits and the dependent L2 reads between them.  f64, one eigenpair (five
-// launches a step before): 61 rows 0.37 ms (1.32), 8,953 rows
-// 1.47 (2.81), 73,789 rows 2.08 (3.32), 147,578 rows 3.11 (3.80); mixed
-// precision 0.43 (1.31), 0.73 (1.72), 0.86 (1.87), 1.26 (2.11).  Past kCoopRows
-// rows per SM the basis leaves L2 and the streaming passes take over.  512
-// threads with four loads in flight measured best (1024 threads 2.50 ms at
-// 73,789 rows, eight loads 2.20).
+// two waits and the dependent L2 reads between them: loads go out in predicated
+// batches, since a plain unrolled loop fetches its remainder one by one (73,789
+// rows 2.05 ms so).  f64, one eigenpair (five launches a step before): 61 rows
+// 0.35 ms (1.32), 8,953 rows 1.22 (2.81), 73,789 rows 1.78 (3.32), 147,578 rows
+// 2.89 (3.80); mixed precision 0.37 (1.31), 0.68 (1.72), 0.85 (1.87), 1.16
+// (2.11).  Past kCoopRows rows per SM the basis leaves L2 and the streaming
+// passes take over.  512 threads measured best (1024: 2.50 ms at 73,789 rows
+// when 512 took 2.08).
 // ---------------------------------------------------------------------------
 constexpr int kCoopThreads = 512;
 constexpr int kCoopWarps = kCoopThreads / 32;
 constexpr int kCoopRows = 1024;             // most rows of a CTA
 constexpr int kCoopSmem = 190 * 1024;       // dynamic shared memory of a CTA (one per SM)
 constexpr int kCoopLanes = 4;               // lanes per row of the product
+constexpr int kAhead = 12;                  // vectors of a row in flight (update)
 
 template <typename T>
 struct CoopArgs {
@@ -1022,6 +1019,10 @@ __host__ __device__ inline int64_t coop_fixed(int rows, int nv, int m_max) {
 template <typename T>
 __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs<T> A) {
   constexpr int NV = 1;  // problems (batches of small ones have their own solver)
+  // vectors and rows of a lane in flight in the dots (an f32 basis is mostly in
+  // shared memory, where a second vector only costs: 73,789 rows mixed 0.85 ms
+  // a solve against 1.34; f64 1.78 against 1.83 with one)
+  constexpr int kVecs = sizeof(T) == 8 ? 2 : 1, kRowsAhead = sizeof(T) == 8 ? 8 : 12;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ double red[NV][kCoopWarps];
   __shared__ double total_s[NV], coef[NV][4];
@@ -1062,6 +1063,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
   }
   const int64_t ld_i = ld_v * NV;
   edg::GridSync gs{A.bar, A.err};
+  constexpr int kPer = (edg::kSmCount + 31) / 32;  // partials of a lane (one CTA an SM)
   unsigned waits = 0;
   // totals over the grid of NV values per thread (in total_s); false when a
   // wait ran out
@@ -1082,10 +1084,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     }
     if (!gs.wait()) return false;
     if (warp < NV) {
-      double t = 0.0;
-      for (int b = lane; b < G; b += 32) t += __ldcg(part + (int64_t)warp * G + b);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      const double t = edg::warp_sum(edg::lane_share<kPer>(part + (int64_t)warp * G, 1, G));
       if (lane == 0) total_s[warp] = t;
     }
     __syncthreads();
@@ -1175,37 +1174,67 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     }
     __syncthreads();
     // ---- dots of this CTA's rows: a warp per vector and problem ----
-    for (int e = warp; e < n_vec * NV; e += kCoopWarps) {
-      const int t = e / NV, v = e - t * NV;
-      const T* b = own + (int64_t)(lo + t) * ld_i + v * ld_v;
-      const double *uv = u + v * rows, *wv = w + v * rows;
-      double s = 0.0, z = 0.0;
-#pragma unroll 4
-      for (int r = lane; r < rows; r += 32) {
-        const double x = (double)b[r];
-        s = fma(x, uv[r], s);
-        z = fma(x, wv[r], z);
+    for (int e0 = warp; e0 < n_vec * NV; e0 += kVecs * kCoopWarps) {
+      double s[kVecs], z[kVecs];
+      const T* b[kVecs];
+#pragma unroll
+      for (int h = 0; h < kVecs; ++h) {
+        const int e = e0 + h * kCoopWarps, t = e / NV, v = e - t * NV;
+        b[h] = own + (int64_t)(lo + t) * ld_i + v * ld_v;
+        s[h] = z[h] = 0.0;
+      }
+      static_assert(NV == 1, "u and w are one problem's");
+      for (int r = lane; r < rows; r += 32 * kRowsAhead) {
+        T x[kVecs][kRowsAhead];
+#pragma unroll
+        for (int h = 0; h < kVecs; ++h)
+#pragma unroll
+          for (int q = 0; q < kRowsAhead; ++q)
+            x[h][q] = e0 + h * kCoopWarps < n_vec && r + 32 * q < rows ? b[h][r + 32 * q] : T(0);
+#pragma unroll
+        for (int q = 0; q < kRowsAhead; ++q)
+          if (r + 32 * q < rows) {
+            const double uq = u[r + 32 * q], wq = w[r + 32 * q];
+#pragma unroll
+            for (int h = 0; h < kVecs; ++h) {
+              s[h] = fma((double)x[h][q], uq, s[h]);
+              z[h] = fma((double)x[h][q], wq, z[h]);
+            }
+          }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        z += __shfl_xor_sync(0xffffffffu, z, o);
-      }
-      if (lane == 0) {
-        A.partial[(int64_t)(2 * e) * G + blockIdx.x] = s;
-        A.partial[(int64_t)(2 * e + 1) * G + blockIdx.x] = z;
+      for (int h = 0; h < kVecs; ++h) {
+        const int e = e0 + h * kCoopWarps;
+        s[h] = edg::warp_sum(s[h]);
+        z[h] = edg::warp_sum(z[h]);
+        if (lane == 0 && e < n_vec) {
+          A.partial[(int64_t)(2 * e) * G + blockIdx.x] = s[h];
+          A.partial[(int64_t)(2 * e + 1) * G + blockIdx.x] = z[h];
+        }
       }
     }
     if (!gs.wait()) return;
     // ---- totals and coefficients ----
-    for (int e = warp; e < 2 * n_vec * NV; e += kCoopWarps) {
-      double a = 0.0;
-      for (int b = lane; b < G; b += 32) a += __ldcg(A.partial + (int64_t)e * G + b);
+    for (int e0 = warp; e0 < 2 * n_vec * NV; e0 += 4 * kCoopWarps) {
+      double p[4][kPer];  // four sums' partials in flight
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0) {
-        const int t = (e >> 1) / NV, v = (e >> 1) - t * NV;
-        tot[(int64_t)v * 2 * (m_max + 2) + 2 * t + (e & 1)] = a;
+      for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+          const int e = e0 + h * kCoopWarps, b = lane + 32 * k;
+          p[h][k] = e < 2 * n_vec * NV && b < G ? __ldcg(A.partial + (int64_t)e * G + b) : 0.0;
+        }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        double a = 0.0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) a += p[h][k];
+        a = edg::warp_sum(a);
+        const int e = e0 + h * kCoopWarps;
+        if (lane == 0 && e < 2 * n_vec * NV) {
+          const int t = (e >> 1) / NV, v = (e >> 1) - t * NV;
+          tot[(int64_t)v * 2 * (m_max + 2) + 2 * t + (e & 1)] = a;
+        }
       }
     }
     __syncthreads();
@@ -1236,11 +1265,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
         double su = 0.0, sw = 0.0;
         if (r < rows) {
           const T* b = own + (int64_t)lo * ld_i + v * ld_v + r;
-#pragma unroll 8
-          for (int t = part; t < n_vec - 1; t += lpr) {
-            const double x = (double)b[(int64_t)t * ld_i];
-            su = fma(x, tv[2 * t], su);
-            sw = fma(x, tv[2 * t + 1], sw);
+          for (int t = part; t < n_vec - 1; t += kAhead * lpr) {
+            T x[kAhead];
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q) x[q] = t + q * lpr < n_vec - 1 ? b[(int64_t)(t + q * lpr) * ld_i] : T(0);
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q)
+              if (t + q * lpr < n_vec - 1) {
+                su = fma((double)x[q], tv[2 * (t + q * lpr)], su);
+                sw = fma((double)x[q], tv[2 * (t + q * lpr) + 1], sw);
+              }
           }
         }
         if (lpr == 2) {
