@@ -2,6 +2,7 @@
 #pragma once
 #include "reorth_bulk.cuh"
 #include "edgpu.h"
+#include "internal.cuh"
 
 namespace edg {
 
@@ -88,6 +89,19 @@ __device__ __forceinline__ double warp_sum(double a) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
   return a;
+}
+
+// CTAs of a small cooperative solve of n rows: one up to 256 rows, where no CTA
+// waits for another (a Krylov step at 182 rows 145 us, with three CTAs 198; an
+// f64 ground state at 141 rows 0.54 ms, 0.62); past that at least 128 rows a
+// CTA, at most one an SM.  Fewer rows a CTA mean more partials in every sum
+// (Krylov step at 12,292 rows: 291 us with 83 rows a CTA, 267 with 128, 274
+// with 256; f64 ground state at 8,953 rows: 1.13 ms with 64, 1.11 with 128,
+// 1.22 with 256).
+inline int64_t coop_ctas(int64_t n, int n_sm) {
+  if (n <= 256) return 1;
+  const int64_t g = (n + 127) / 128, most = n_sm < kSmCount ? n_sm : kSmCount;
+  return g < most ? g : most;
 }
 
 }  // namespace edg

@@ -419,9 +419,9 @@ __global__ void combine_k(const T* __restrict__ V, int64_t n, int64_t ldv, int m
 // two grid-wide waits: for the dots, and for the norm with the next vector.
 // Bound by those waits and the dependent L2 reads between them: the partials of
 // a sum are asked for together, and those of the norm while the product runs
-// (12,292 rows: 0.31 ms without, 0.29 with).  A step of dt = 0.05 (m = 30, full reorthogonalisation,
+// (12,292 rows: 0.31 ms without, 0.29 with, 0.27 on fewer CTAs).  A step of dt = 0.05 (m = 30, full reorthogonalisation,
 // complex128, static-pair SU(2) chains; launches per pass before):
-//   n = 12,292: 0.29 ms (1.69), 101,613: 0.61 ms (1.87).
+//   n = 182: 0.14 ms (1.48), 12,292: 0.27 ms (1.69), 101,613: 0.61 ms (1.87).
 // The line (kCoopRows rows per SM) lies where the matrix and the basis no
 // longer fit shared memory: at 101,613 rows the passes below take 0.96 ms, at
 // 848,614 rows this form takes 6.6 ms and the passes 4.2.
@@ -766,9 +766,7 @@ int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* e
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: set-up");
-    // a CTA per SM, fewer for fewer rows: at least 32 rows a CTA
-    int64_t g = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
-    if (g > (n + 31) / 32) g = (n + 31) / 32;
+    const int64_t g = edg::coop_ctas(n, n_sm);
     if (coop && occ >= 1 && (n + g - 1) / g <= kCoopRows) {
       CoopArgs<T, SV> a{p->rowptr, p->cols, (const SV*)p->vals, (const SV*)p->diag, V, psi, partial, normp, bar,
                         err_word, p->status, misc + 1, n, ldv, dt, m, p->reorth_passes};

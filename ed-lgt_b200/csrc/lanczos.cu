@@ -976,8 +976,8 @@ __global__ void ritz_k(const T* __restrict__ V, int64_t n_pad, int m, const doub
 // two waits and the dependent L2 reads between them: loads go out in predicated
 // batches, since a plain unrolled loop fetches its remainder one by one (73,789
 // rows 2.05 ms so).  f64, one eigenpair (five launches a step before): 61 rows
-// 0.35 ms (1.32), 8,953 rows 1.22 (2.81), 73,789 rows 1.78 (3.32), 147,578 rows
-// 2.89 (3.80); mixed precision 0.37 (1.31), 0.68 (1.72), 0.85 (1.87), 1.16
+// 0.35 ms (1.32), 8,953 rows 1.11 (2.81), 73,789 rows 1.78 (3.32), 147,578 rows
+// 2.89 (3.80); mixed precision 0.37 (1.31), 0.63 (1.72), 0.82 (1.87), 1.16
 // (2.11).  Past kCoopRows rows per SM the basis leaves L2 and the streaming
 // passes take over.  512 threads measured best (1024: 2.50 ms at 73,789 rows
 // when 512 took 2.08).
@@ -1438,8 +1438,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: set-up");
-    int64_t g = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
-    if (g > (n_pad + 255) / 256) g = (n_pad + 255) / 256;  // fewer CTAs than rows to keep them busy
+    const int64_t g = edg::coop_ctas(n_pad, n_sm);
     const int rows = (int)((n_pad + g - 1) / g);
     if (coop && occ >= 1 && rows <= kCoopRows && coop_fixed(rows, NV, L.m_max) <= kCoopSmem) {
       state_init_k<<<1, 32, 0, s>>>(st, first_check, p->reorth_window);
