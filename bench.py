@@ -77,6 +77,13 @@ def model_kwargs():
     return dict(spin=0.5, pure_theory=False, lvals=[L], has_obc=[not PBC], sectors=[L])
 
 
+def reference_missing():
+    """Why the reference arm cannot run (None when it can): its package is an
+    untracked install beside the sources."""
+    path = os.path.join(os.environ.get("EDLGT_PATH", os.path.join(ROOT, "baseline", "_ref")), "edlgt")
+    return None if os.path.isdir(path) else "ed-lgt is not installed under baseline/_ref"
+
+
 def stock_reference(steps, warmup, fmt="auto", couplings=SWEEP, timeout=3000):
     """Run the unmodified ed-lgt through its model API in a child process
     (oracle/stock_ref.py, which never loads this engine); returns its JSON."""
@@ -198,6 +205,9 @@ def run_reference(args):
     """The reference arm: stock ed-lgt on the host cores, rank 0 only (no
     process group is created, so other ranks exit at once)."""
     if int(os.environ.get("RANK", "0")) != 0:
+        return
+    if reference_missing():
+        print(json.dumps({"impl": "reference", "unavailable": reference_missing()}), flush=True)
         return
     # a reference pipeline takes about 12 s on 16 host cores: at most
     # REF_MAX_PIPELINES of them are timed (the rate is their mean), so the arm
@@ -492,7 +502,9 @@ def run_edgpu(args, world, rank, local):
 
     # ---------------- CPU baseline (rank 0, bounded sample) ------------------
     cpu = None
-    if rank == 0 and not args.no_cpu:
+    if rank == 0 and not args.no_cpu and reference_missing():
+        print(f"no CPU baseline: {reference_missing()}", file=sys.stderr)
+    elif rank == 0 and not args.no_cpu:
         # the format trial of the stock runner: one full pipeline per matvec
         # format; the faster one is the sample
         res = stock_reference(0, 1, fmt="auto", couplings=(1.0,))
