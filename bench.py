@@ -280,12 +280,12 @@ def setup_phases(dev, reps=3):
     return {
         "sector_enumeration": {"ms": sec_ms, "levels": len(sec.level_sizes), "algorithmic_bytes": int(enum_bytes),
                                "GBps": enum_bytes / (sec_ms * 1e-3) / 1e9,
-                               "includes": "model construction (operator tables) + level-by-level enumeration, "
-                                           "one host read of each level's size"},
+                               "includes": "model construction (operator tables) + enumeration of all levels in one "
+                                           "launch, one host read of the result's size"},
         "assembly": {"ms": asm_ms, "raw_entries": int(getattr(mat, "raw_entries", 0)), "nnz": nnz,
                      "algorithmic_bytes": int(asm_bytes), "GBps": asm_bytes / (asm_ms * 1e-3) / 1e9,
                      "includes": "build_Hamiltonian(g^2=1): term tables, count, scan, fill (key search per "
-                                 "transition), per-row merge, compaction"},
+                                 "transition), entries in place, duplicates merged"},
     }
 
 
