@@ -863,7 +863,7 @@ int check_k(const edg_krylov_problem* p) {
 // matvec of a momentum sector): the same three kernels a pass as the steps
 // above, with everything the host would read kept on the device.  What bounds
 // a short step is the host: 12,329 momentum states (147,578 sector rows), 55
-// steps with library products and two reads a step took 12.9 ms, here 5.0, of
+// steps with library products and two reads a step took 12.9 ms, here 4.6, of
 // which the nine kernels a step take 3.0.
 extern "C" int64_t edg_krylov_orth_bytes(int32_t max_vectors) {
   if (max_vectors < 1 || max_vectors > kMaxOrth) return -1;

@@ -302,7 +302,7 @@ def _lanczos(apply, m, k, tol, max_iter, device, seed):
     """Lanczos with two classical Gram-Schmidt passes against the whole basis
     on complex128 vectors (``edg_krylov_orth``); converged when every wanted
     Ritz pair has |beta_j s_jk| <= tol max(1, |theta_k|).  The host reads the
-    coefficients every fifth step, when it tests for convergence."""
+    coefficients when it tests for convergence, every fifth to twentieth step."""
     from scipy.linalg import eigh_tridiagonal
 
     max_iter = min(max_iter, 14000)  # the most basis vectors edg_krylov_orth takes
@@ -317,11 +317,12 @@ def _lanczos(apply, m, k, tol, max_iter, device, seed):
     step = (ptr(coef[0]), ptr(coef[1]), max_iter, ptr(work), wb, stream_handle())
     q0 = Q.data_ptr()
     theta = s = None
+    next_check, last = 5 * ((k + 4) // 5), None
     for j in range(max_iter):
         w = apply(q0 + 16 * m * j)
         check(lib.edg_krylov_orth(m, m, q0, j, ptr(w), 2, *step), "edg_krylov_orth")
         done = j + 1 == max_iter
-        if j + 1 >= k and (done or (j + 1) % 5 == 0):
+        if j + 1 >= k and (done or j + 1 >= next_check):
             alpha, beta = coef[:, : j + 2].cpu().numpy()
             n = j + 1
             # a breakdown, once k steps are taken, ends the recurrence at its step
@@ -334,6 +335,13 @@ def _lanczos(apply, m, k, tol, max_iter, device, seed):
             res = np.abs(beta[n] * s[-1, :])
             if done or np.all(res <= tol * np.maximum(1.0, np.abs(theta))):
                 break
+            # the next check where the contraction so far reaches the tolerance,
+            # less a fifth: a read stops the device for about 0.1 ms
+            worst, wait = float(np.max(res / np.maximum(1.0, np.abs(theta)))), 5
+            if last is not None and 0.0 < worst < last[1] and tol > 0.0:
+                need = np.log(tol / worst) * (n - last[0]) / np.log(worst / last[1])
+                wait = 5 * int(min(4, max(1, 0.8 * need // 5)))
+            next_check, last = n + wait, (n, worst)
     n = s.shape[0]
     vecs = Q[:n].T @ torch.from_numpy((s / beta[:n, None]).astype(np.complex128)).to(device)
     return theta, vecs, n
