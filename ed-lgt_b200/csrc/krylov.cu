@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, dot_ctas<T>()) dots_k(const T* __res
                                                    int ld_i) {
   __shared__ double red[kWarps * kTile * 2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i0 = ilo; i0 <= j; i0 += kTile) {
+  for (int i0 = ilo + (int)blockIdx.y * kTile; i0 <= j; i0 += (int)gridDim.y * kTile) {
     double re[kTile], im[kTile];
 #pragma unroll
     for (int t = 0; t < kTile; ++t) re[t] = im[t] = 0.0;
@@ -863,8 +863,8 @@ int check_k(const edg_krylov_problem* p) {
 // matvec of a momentum sector): the same three kernels a pass as the steps
 // above, with everything the host would read kept on the device.  What bounds
 // a short step is the host: 12,329 momentum states (147,578 sector rows), 55
-// steps with library products and two reads a step took 12.9 ms, here 4.6, of
-// which the nine kernels a step take 3.0.
+// steps with library products and two reads a step took 12.9 ms, here 4.2, of
+// which the nine kernels a step take 2.6.
 extern "C" int64_t edg_krylov_orth_bytes(int32_t max_vectors) {
   if (max_vectors < 1 || max_vectors > kMaxOrth) return -1;
   return al((int64_t)edg::kSmCount * 2 * (max_vectors + 1) * 16) + al((int64_t)edg::kSmCount * 8 * 8) +
@@ -893,6 +893,10 @@ extern "C" int edg_krylov_orth(int64_t n, int64_t ldv, double* V, int32_t j, dou
   unsigned* ticket = (unsigned*)ws;
   const double2* basis = (const double2*)V;
   const int nb = (int)edg::grid_for(n, kThreads, dot_ctas<double2>());
+  // few rows: tiles of vectors side by side, up to two CTAs an SM (12,329 rows,
+  // 49 CTAs a tile: 7.3 us a pass one after the other, here 3.7)
+  const int tiles = j / kTile + 1, room = 2 * edg::kSmCount / nb;
+  const unsigned ny = (unsigned)(room < 1 ? 1 : (room < tiles ? room : tiles));
   const unsigned gu = edg::grid_for(n, kThreads, kUpdateCtas);
   if (j == 0) {
     cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(unsigned), stream);
@@ -904,7 +908,7 @@ extern "C" int edg_krylov_orth(int64_t n, int64_t ldv, double* V, int32_t j, dou
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_orth");
   }
   for (int pass = 0; pass < passes; ++pass) {
-    dots_k<double2><<<nb, kThreads, 0, stream>>>(basis, n, ldv, 0, j, (const double2*)w, partial, ld_i);
+    dots_k<double2><<<dim3(nb, ny), kThreads, 0, stream>>>(basis, n, ldv, 0, j, (const double2*)w, partial, ld_i);
     coef_k<<<j + 1, kThreads, 0, stream>>>(partial, nb, ld_i, 0, j, pass, beta, coef, alpha);
     update_k<double2><<<gu, kThreads, (j + 2) * sizeof(double2), stream>>>(
         basis, n, ldv, 0, j, coef, (double2*)w, pass + 1 == passes ? (double2*)V + (int64_t)(j + 1) * ldv : nullptr,
