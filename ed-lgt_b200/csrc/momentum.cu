@@ -224,16 +224,40 @@ __global__ void expand_k(int64_t n_rows, const int64_t* __restrict__ row_col, co
   }
 }
 
-__global__ void reduce_k(int64_t n_cols, const int64_t* __restrict__ col_ptr, const int32_t* __restrict__ row_idx,
+// y = B^dagger w: kColLanes lanes a column, up to four entries of each in
+// flight, summed in a fixed order.  With one thread a column the chain of a
+// column's gathers bounds it (12,329 columns of 12 entries: 6.5 us, here 3.7).
+constexpr int kColLanes = 4;
+__global__ void __launch_bounds__(kThreads) reduce_k(int64_t n_cols, const int64_t* __restrict__ col_ptr, const int32_t* __restrict__ row_idx,
                          const double2* __restrict__ data, const double2* __restrict__ w, double2* __restrict__ y) {
-  for (int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x; c < n_cols; c += (int64_t)gridDim.x * kThreads) {
+  const int lane = threadIdx.x & (kColLanes - 1);
+  const int64_t step = (int64_t)gridDim.x * (kThreads / kColLanes);
+  for (int64_t c0 = (int64_t)blockIdx.x * (kThreads / kColLanes); c0 < n_cols; c0 += step) {
+    const int64_t c = c0 + threadIdx.x / kColLanes;
+    const int64_t end = c < n_cols ? col_ptr[c + 1] : 0;
     double re = 0.0, im = 0.0;
-    for (int64_t p = col_ptr[c]; p < col_ptr[c + 1]; ++p) {
-      const double2 b = data[p], wv = w[row_idx[p]];
-      re = fma(b.x, wv.x, fma(b.y, wv.y, re));  // conj(b) * w
-      im = fma(b.x, wv.y, fma(-b.y, wv.x, im));
+    for (int64_t p = c < n_cols ? col_ptr[c] + lane : 0; p < end; p += 4 * kColLanes) {
+      double2 b[4], wv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (p + q * kColLanes < end) {
+          b[q] = data[p + q * kColLanes];
+          wv[q] = w[row_idx[p + q * kColLanes]];
+        }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (p + q * kColLanes < end) {
+          re = fma(b[q].x, wv[q].x, fma(b[q].y, wv[q].y, re));  // conj(b) * w
+          im = fma(b[q].x, wv[q].y, fma(-b[q].y, wv[q].x, im));
+        }
     }
-    y[c] = make_double2(re, im);
+    __syncwarp();
+#pragma unroll
+    for (int o = kColLanes / 2; o > 0; o >>= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (c < n_cols && lane == 0) y[c] = make_double2(re, im);
   }
 }
 
@@ -435,7 +459,7 @@ extern "C" int edg_momentum_reduce(int64_t n_cols, const int64_t* col_ptr, const
                                    const double* w, double* y, cudaStream_t stream) {
   EDG_REQUIRE(n_cols >= 0 && (n_cols == 0 || (col_ptr && y && w)), "edg_momentum_reduce: null argument");
   if (n_cols == 0) return EDG_OK;
-  reduce_k<<<edg::grid_for(n_cols, kThreads), kThreads, 0, stream>>>(n_cols, col_ptr, row_idx, (const double2*)data,
+  reduce_k<<<edg::grid_for(n_cols * kColLanes, kThreads), kThreads, 0, stream>>>(n_cols, col_ptr, row_idx, (const double2*)data,
                                                                      (const double2*)w, (double2*)y);
   EDG_CHECK_LAUNCH("edg_momentum_reduce");
   return EDG_OK;

@@ -55,3 +55,26 @@ def test_dense_matrix_is_the_matvec(ucs, k, real_form):
     eye = torch.eye(mom.n_cols, dtype=torch.complex128, device="cuda")
     ref = torch.stack([mom.matvec(eye[c]) for c in range(mom.n_cols)], dim=1)
     assert float((h - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("n_cols", [1, 63, 64, 65, 3000])
+def test_reduce_column_lengths(n_cols):
+    """B^dagger w for columns of 0 to 33 entries: sums of at most 33 products
+    of order one in another order (1e-13 each)."""
+    from edgpu._lib import check, lib, ptr, stream_handle
+
+    rng = np.random.default_rng(n_cols)
+    lengths = rng.choice([0, 1, 3, 4, 5, 15, 16, 17, 33], n_cols)
+    col_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    nnz, n_rows = int(col_ptr[-1]), 500
+    rows = rng.integers(0, n_rows, nnz).astype(np.int32)
+    data = rng.uniform(-1, 1, nnz) + 1j * rng.uniform(-1, 1, nnz)
+    w = rng.uniform(-1, 1, n_rows) + 1j * rng.uniform(-1, 1, n_rows)
+    up = lambda a: torch.from_numpy(np.concatenate([a, np.zeros(1, a.dtype)])).cuda()  # noqa: E731
+    cp, ri, dv, wv = torch.from_numpy(col_ptr).cuda(), up(rows), up(data), up(w)
+    y = torch.full((n_cols + 1,), 7.0, dtype=torch.complex128, device="cuda")
+    check(lib.edg_momentum_reduce(n_cols, ptr(cp), ptr(ri), ptr(dv), ptr(wv), ptr(y), stream_handle()),
+          "edg_momentum_reduce")
+    ref = np.array([np.sum(data[a:b].conj() * w[rows[a:b]]) for a, b in zip(col_ptr[:-1], col_ptr[1:])])
+    out = y.cpu().numpy()
+    assert np.max(np.abs(out[:n_cols] - ref)) <= 1e-13 * 33 and out[n_cols] == 7.0
