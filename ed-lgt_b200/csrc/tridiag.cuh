@@ -49,17 +49,18 @@ __device__ inline int sturm_count(const double* d, const double* e2, int m, doub
   return cnt;
 }
 
-// What a convergence check needs of the coefficients al[0..m-1], be[0..m]:
-// the dimension mv at which the recurrence ends (the first i >= 1 with |be[i]|
-// <= 1e-12 max(|al| + |be|), else m) and whether it ends there.  For the
-// calling CTA (NT threads); every thread gets both.
+// What a convergence check needs of the coefficients al[0..m-1], be[1..m]
+// (be[0] couples nothing and is not read: callers need not set it): the
+// dimension mv at which the recurrence ends (the first i >= 1 with |be[i]| <=
+// 1e-12 max(|al| + |be|), else m) and whether it ends there.  For the calling
+// CTA (NT threads); every thread gets both.
 template <int NT = kTriThreads>
 __device__ inline int ritz_dimension(const double* al, const double* be, int m, bool* ends) {
   __shared__ double mx[NT / 32];
   __shared__ int first_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double scale = 0.0;
-  for (int i = tid; i < m; i += NT) scale = fmax(scale, fabs(al[i]) + fabs(be[i]));
+  for (int i = tid; i < m; i += NT) scale = fmax(scale, fabs(al[i]) + (i > 0 ? fabs(be[i]) : 0.0));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
   if (lane == 0) mx[warp] = scale;

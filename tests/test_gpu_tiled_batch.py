@@ -190,3 +190,44 @@ def test_tiles_per_instance_and_rows_per_tile(precision, tile_rows, dims, dev):
         w = np.linalg.eigvalsh(h)[0]
         assert abs(ei - w) <= (1e-10 if precision == "fp64" else 1e-9) * abs(w)
         assert np.linalg.norm(h @ v - w * v) <= 1e-4 * abs(w) and abs(np.linalg.norm(v) - 1) <= 1e-10
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("fill", [1e200, float("nan")])
+@pytest.mark.parametrize("tile_rows", [4, 512])
+def test_workspace_contents_do_not_matter(tile_rows, fill, precision, dev):
+    """A solve on a workspace that holds large values (recycled memory) takes
+    the same steps to the same energies as on a cleared one, on both sides of
+    the tile count that has a phase of its own; the fp64 energies to the
+    solver's tolerance against dense algebra."""
+    import torch
+    from scipy.sparse import diags
+
+    from edgpu.batch import TiledBatch
+    from edgpu.modeling.assembly import DeviceMatrix
+
+    rng = np.random.default_rng(11)
+    t = lambda a, dt: torch.from_numpy(np.array(a, dtype=dt)).to(dev)  # noqa: E731
+    mats, ref = [], []
+    for n in (40, 300):
+        A = diags([rng.uniform(-1, 1, n - 1)], [1])
+        A = (A + A.T).tocsr()
+        d = rng.uniform(0, 1, n)
+        d[n // 3] = -9.0  # an isolated lowest state
+        mats.append(DeviceMatrix(n, t(A.indptr, np.int64), t(A.indices, np.int32), t(A.data, np.float64),
+                                 t(d, np.float64), t(np.ones(n), np.uint8), False))
+        ref.append(np.linalg.eigvalsh(A.toarray() + np.diag(d))[0])
+    tb = TiledBatch(mats, precision=precision, tile_rows=tile_rows, lanes=2)
+    got = []
+    for value in (0.0, fill):
+        for plan in (tb.plan32, tb.plan64):
+            if plan is not None:
+                plan.workspace[: plan.workspace.numel() // 8 * 8].view(torch.float64).fill_(value)
+        e = tb.solve(use_graph=False).cpu().numpy()[:, 0].copy()
+        tb.check_status()
+        got.append((e, tb.iters.cpu().numpy().copy(), tb.iters32.cpu().numpy().copy() if tb.plan32 else None))
+    (e0, it0, it32), (e1, it1, jt32) = got
+    assert np.array_equal(e0, e1) and np.array_equal(it0, it1)
+    assert it32 is None or np.array_equal(it32, jt32)
+    for e, w in zip(e1, ref):
+        assert abs(e - w) <= (1e-10 if precision == "fp64" else 1e-9) * max(1.0, abs(w))
