@@ -737,6 +737,14 @@ KLayout klayout(const edg_krylov_problem* p) {
   return L;
 }
 
+// Whether a step may run as krylov_coop_k: few enough rows, and the CSR arrays
+// at hand, which that kernel reads whatever layout is passed beside them (a
+// problem may come with its packed layout alone).
+bool one_launch(const edg_krylov_problem* p) {
+  const bool csr = p->cols != nullptr && p->vals != nullptr, diagonal = p->nnz == 0 && p->pk_words == nullptr;
+  return p->n_rows <= kCoopMaxRows && (csr || diagonal);
+}
+
 template <typename T, typename SV>
 int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* err_out, cudaStream_t s) {
   const KLayout L = klayout(p);
@@ -757,7 +765,7 @@ int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* e
   cudaError_t e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s);
   if (e != cudaSuccess) return edg::cuda_status(e, "krylov");
   bool done = false;
-  if (n <= kCoopMaxRows) {
+  if (one_launch(p)) {
     int dev = 0, n_sm = 0, coop = 0, occ = 0;
     auto kern = krylov_coop_k<T, SV>;
     e = cudaGetDevice(&dev);
@@ -854,6 +862,8 @@ int check_k(const edg_krylov_problem* p) {
                    p->pk_count <= EDG_PACK_MAX_VALUES && p->pk_colbits >= 1 && p->pk_colbits <= 31 &&
                    p->n_rows < ((int64_t)1 << p->pk_colbits)),
               "edg_krylov: a packed layout needs a real matrix (mat_dtype 0 or 1) and a complete layout");
+  EDG_REQUIRE(p->nnz == 0 || (p->cols && p->vals) || p->pk_words,
+              "edg_krylov: off-diagonal entries without CSR arrays or a packed layout");
   return EDG_OK;
 }
 
@@ -921,6 +931,11 @@ extern "C" int edg_krylov_orth(int64_t n, int64_t ldv, double* V, int32_t j, dou
 extern "C" int64_t edg_krylov_workspace_bytes(const edg_krylov_problem* p) {
   if (check_k(p)) return -1;
   return klayout(p).total;
+}
+
+extern "C" int edg_krylov_one_launch(const edg_krylov_problem* p) {
+  if (check_k(p)) return -1;
+  return one_launch(p) ? 1 : 0;
 }
 
 extern "C" int edg_krylov_step(const edg_krylov_problem* p, void* psi, double dt, void* workspace,

@@ -1429,7 +1429,10 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   // small sectors: the whole solve in one cooperative launch (the instrumented
   // path times the passes one by one)
   bool coop_done = false;
-  if (NV == 1 && p->stats == nullptr && (p->vals != nullptr || p->nnz == 0) && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
+  // (the kernel reads the CSR arrays: a problem may come with another layout alone)
+  const bool csr = (p->cols != nullptr && p->vals != nullptr) ||
+                   (p->nnz == 0 && p->pk_words == nullptr && p->sell_entries == nullptr);
+  if (NV == 1 && p->stats == nullptr && csr && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
     int dev = 0, n_sm = 0, coop = 0, occ = 0;
     auto kern = lanczos_coop_k<T>;
     e = cudaGetDevice(&dev);
@@ -1751,6 +1754,8 @@ int check_problem(const edg_lanczos_problem* p) {
                   (p->pk_tile_off && p->pk_table && p->pk_count >= 1 && p->pk_count <= EDG_PACK_MAX_VALUES &&
                    p->pk_colbits >= 1 && p->pk_colbits <= 31 && p->n_rows < ((int64_t)1 << p->pk_colbits)),
               "edg_lanczos: incomplete or inconsistent packed layout");
+  EDG_REQUIRE(p->nnz == 0 || (p->cols && p->vals) || p->pk_words || (p->sell_entries && p->dtype == 1),
+              "edg_lanczos: off-diagonal entries without CSR arrays or another layout");
   return EDG_OK;
 }
 

@@ -338,6 +338,7 @@ _SIGS = {
     "edg_tiled_batch_header_bytes": (I32, [I32]),
     "edg_lanczos_tiled_batch": (I32, [C.POINTER(TiledBatch), P]),
     "edg_krylov_workspace_bytes": (I64, [C.POINTER(KrylovProblem)]),
+    "edg_krylov_one_launch": (I32, [C.POINTER(KrylovProblem)]),
     "edg_krylov_step": (I32, [C.POINTER(KrylovProblem), P, F64, P, I64, P, P]),
     "edg_krylov_orth_bytes": (I64, [I32]),
     "edg_krylov_orth": (I32, [I64, I64, P, I32, P, I32, P, P, I32, P, I64, P]),

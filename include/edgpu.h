@@ -471,7 +471,7 @@ typedef struct {
 } edg_lanczos_problem;
 
 /* Bytes of device workspace edg_lanczos needs. */
-/* Rows up to which a single problem (nvec 1, no stats, vals given) is solved
+/* Rows up to which a single problem (nvec 1, no stats, CSR arrays given) is solved
  * in one cooperative launch, which reads the CSR arrays whatever layout is
  * passed beside them. */
 int64_t edg_lanczos_small_rows(void);
@@ -645,6 +645,11 @@ typedef struct {
 } edg_krylov_problem;
 
 int64_t edg_krylov_workspace_bytes(const edg_krylov_problem* p);
+/* 1 when a step of this problem is one cooperative launch (few rows, CSR
+ * arrays given; it reads those and the diagonal, not the packed layout), on a
+ * device that has such launches; 0 when it is a launch per pass; -1 for a bad
+ * problem. */
+int edg_krylov_one_launch(const edg_krylov_problem* p);
 /* One step of length dt in place on psi [n_rows] (complex, vec_dtype).
  * err_out (host, may be NULL): a posteriori error estimate of the step. */
 int edg_krylov_step(const edg_krylov_problem* p, void* psi, double dt,

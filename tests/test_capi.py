@@ -198,3 +198,60 @@ def test_lanczos_problem_rejects_an_incomplete_packed_layout():
     assert _lib.lib.edg_lanczos_workspace_bytes(ctypes.byref(p)) > 0
     p.pk_colbits = 9  # 2^9 rows: fewer than the 1000 rows
     assert _lib.lib.edg_lanczos_workspace_bytes(ctypes.byref(p)) == -1
+
+
+def test_krylov_problem_with_a_packed_layout_alone():
+    """A problem that comes with its packed layout and no CSR arrays is
+    accepted and is not one for the one-launch form, which reads the CSR
+    arrays; entries without either are refused."""
+    from edgpu import _lib
+
+    L = _lib.lib
+    p = _lib.KrylovProblem()
+    p.vec_dtype, p.mat_dtype, p.n_rows, p.nnz, p.m = 2, 0, 1000, 5000, 30
+    p.rowptr = p.diag = p.cols = p.vals = p.status = 16
+    one = lambda: L.edg_krylov_one_launch(ctypes.byref(p))  # noqa: E731
+    assert one() == 1
+    p.pk_tile_off = p.pk_words = p.pk_table = 16
+    p.pk_count, p.pk_colbits = 4, 11
+    assert one() == 1  # both are there: the CSR arrays are read
+    for cols, vals in ((None, 16), (16, None), (None, None)):
+        p.cols, p.vals = cols, vals
+        assert one() == 0 and L.edg_krylov_workspace_bytes(ctypes.byref(p)) > 0
+    p.nnz = 0  # not counted by a caller that only has the layout
+    assert one() == 0
+    p.pk_words = None
+    assert one() == 1  # a diagonal matrix
+    p.nnz = 5000
+    assert one() == -1 and "without CSR arrays" in _lib.last_error()
+    assert L.edg_krylov_workspace_bytes(ctypes.byref(p)) == -1
+    p.cols = p.vals = 16
+    p.n_rows = 1024 * 148
+    assert one() == 1
+    p.n_rows += 1
+    assert one() == 0
+
+
+def test_lanczos_problem_without_matrix_entries_is_refused():
+    """Off-diagonal entries need the CSR arrays, a packed layout or (f32) a
+    SELL layout."""
+    from edgpu import _lib
+
+    size = lambda: _lib.lib.edg_lanczos_workspace_bytes(ctypes.byref(p))  # noqa: E731
+    p = _lib.LanczosProblem()
+    p.dtype, p.n_rows, p.nnz, p.nvec, p.k, p.max_iter, p.tol, p.check_every = 1, 1000, 5000, 1, 1, 50, 1e-8, 5
+    p.rowptr = p.diag = 16
+    for cols, vals in ((None, None), (None, 16), (16, None)):
+        p.cols, p.vals = cols, vals
+        assert size() == -1 and "without CSR arrays" in _lib.last_error()
+    p.cols = p.vals = 16
+    assert size() > 0
+    p.cols = p.vals = None
+    p.pk_words = p.pk_table = p.pk_tile_off = 16
+    p.pk_count, p.pk_colbits = 4, 11
+    assert size() > 0
+    p.pk_words = None
+    p.sell_entries = p.sell_perm = p.sell_width = p.sell_off = 16
+    assert size() > 0
+    p.dtype = 0  # the f64 path does not read it
+    assert size() == -1

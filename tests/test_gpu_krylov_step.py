@@ -73,3 +73,34 @@ def test_step_matches_taylor(n, m, precision, reorth, cplx, empty):
     # c64: a rounding of 2^-24 per stored entry of each basis vector and of psi
     tol = 5e-6 if precision == "c64" else (1e-5 if m == 1 else 1e-12)
     assert err < tol, err
+
+
+@pytest.mark.parametrize("n", [33, 700, 5000, COOP_MAX, COOP_MAX + 1])
+@pytest.mark.parametrize("precision,reorth", [("c128", 0), ("c128", 1), ("c64", 0), ("c64", 2)])
+def test_step_on_a_packed_layout_alone(n, precision, reorth):
+    """A problem without CSR arrays takes the packed product at every size."""
+    import torch
+
+    from edgpu._lib import ptr
+    from edgpu.dynamics import KrylovEvolver
+    from edgpu.solvers import PackedLayout
+
+    mat, apply = _matrix(n, False, n)
+    pk = PackedLayout.build(mat)
+    ev = KrylovEvolver(mat, m=30, precision=precision, reorth_passes=reorth, matvec="csr")
+    p = ev.p
+    p.pk_tile_off, p.pk_words, p.pk_count, p.pk_colbits = ptr(pk.tile_off), ptr(pk.words), pk.count, pk.colbits
+    p.pk_table = ptr(pk.table(0 if precision == "c128" else 1))
+    p.cols = p.vals = None
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    psi = torch.randn(n, dtype=torch.complex128, device="cuda", generator=gen)
+    dt = 0.1
+    want, term = psi.clone(), psi
+    for k in range(1, 40):
+        term = apply(term) * (-1j * dt / k)
+        want = want + term
+    got = psi.to(ev.vdtype).clone()
+    ev.step(got, dt)
+    ev.check_status()
+    err = float(torch.linalg.vector_norm(got.to(torch.complex128) - want) / torch.linalg.vector_norm(want))
+    assert err < (5e-6 if precision == "c64" else 1e-12), err

@@ -93,3 +93,28 @@ def test_residuals_on_both_sides_of_the_line(n, dtype, window):
     # f32: the vector's own rounding (2^-24) times |H| beside the tolerance
     assert float(torch.linalg.vector_norm(res)) < (1e-4 if dtype else 1e-9)
     assert abs(float(torch.linalg.vector_norm(x)) - 1) < (1e-6 if dtype else 1e-13)
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("kept", ["none", "vals", "cols"])
+def test_packed_layout_alone(dtype, kept):
+    """A single problem whose CSR arrays are not all given takes the packed
+    product below the one-launch form's line too."""
+    import torch
+
+    from edgpu.modeling.assembly import DeviceMatrix
+    from edgpu.solvers import PackedLayout, run_lanczos
+
+    n = 3000
+    rowptr, cols, vals, diag, (r, c, v, d) = _matrix(n, n)
+    pk = PackedLayout.build(DeviceMatrix(n, rowptr, cols, vals, diag, None, False))
+    t = torch.float32 if dtype else torch.float64
+    got = run_lanczos(dtype, n, int(cols.numel()), rowptr, cols if kept == "cols" else None,
+                      vals.to(t) if kept == "vals" else None, diag.to(t)[:, None].contiguous(), packed=pk,
+                      max_iter=300, tol=1e-5 if dtype else 1e-12)
+    h = np.diag(d)
+    h[r, c] += v
+    e = np.linalg.eigvalsh(h)
+    # f32: the error is quadratic in the residual bound, beside the rounding
+    # (2^-24) of the vectors times |H|
+    assert abs(got.evals[0, 0] - e[0]) < (2e-6 if dtype else 1e-12) * np.abs(e).max()
