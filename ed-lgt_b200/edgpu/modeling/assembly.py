@@ -323,7 +323,8 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
         keep = list(upload_arrays(dev, {k: (a, a.dtype) for k, a in enumerate(arrays)}).values())
         n_tables = arrays[0].shape[0]
         off = _assemble_offdiag(sector, dev, st, n, 1 if use_real else 2, dmax, not use_real, len(terms), n_tables, keep)
-        off.update(sig=sig, real_ok=real_ok, use_real=use_real)
+        off.update(sig=sig, real_ok=real_ok, use_real=use_real,
+                   layouts={"arrays": (off["rowptr"], off["cols"], off["vals"])})
         sector._offdiag_cache = off
     is_complex = not off["use_real"]
     w = 2 if is_complex else 1
@@ -365,7 +366,8 @@ def assemble_blocks(sector, blocks, phase_weights=None, force_complex=False, ext
     mat._keep = keep  # device tables uploaded by this build
     mat.raw_entries = off["raw_entries"]  # generated entries before the per-row merge
     mat.offdiag_reused = reused  # off-diagonal part shared with an earlier build
-    mat._shared = off["layouts"]  # layouts of that part, shared by the matrices that share it
+    # that part's arrays and their layout, for the matrices that share them
+    mat._shared = off["layouts"]
     return mat
 
 
@@ -421,4 +423,4 @@ def _assemble_offdiag(sector, dev, st, n, w, dmax, is_complex, n_terms, n_tables
                                        ptr(rowptr), ptr(cols), ptr(vals), st), "edg_assemble_compact")
         del tmp_cols, tmp_vals
     return {"rowptr": rowptr, "cols": cols[:nnz], "vals": vals[: nnz * w], "diag": diag[: n * w],
-            "present": present[:n], "raw_entries": total, "keep": tabs, "layouts": {}}
+            "present": present[:n], "raw_entries": total, "keep": tabs}

@@ -221,16 +221,59 @@ class PackedLayout:
                                   ptr(err) if err is not None else None, stream_handle()), "edg_spmv_packed")
 
 
+class _KeptLayout:
+    """A packed layout (or None: the matrix does not pack) beside the tensors it
+    was made of, which it keeps alive, and their modification counts."""
+
+    def __init__(self, mat, layout):
+        self.layout = layout
+        self.arrays = _csr_arrays(mat)
+        self.versions = _versions(self.arrays)
+
+    def fits(self, mat):
+        """Whether the matrix still holds these tensors, unmodified."""
+        now = _csr_arrays(mat)
+        return all(a is b for a, b in zip(self.arrays, now)) and self.versions == _versions(now)
+
+
+def _csr_arrays(mat):
+    return mat.rowptr, mat.cols, mat.vals
+
+
+def _versions(tensors):
+    """In-place modifications of the tensors so far (inference tensors do not
+    count theirs)."""
+    return [None if t.is_inference() else t._version for t in tensors]
+
+
+def _layout_home(mat):
+    """Where the matrices of one off-diagonal part share its layout (None for a
+    matrix that holds other arrays than that part)."""
+    home = getattr(mat, "_shared", None)
+    return home if home is not None and all(a is b for a, b in zip(home["arrays"], _csr_arrays(mat))) else None
+
+
+def _kept_layout(mat):
+    home = _layout_home(mat)
+    for kept in (getattr(mat, "_packed", None), home.get("packed") if home else None):
+        if kept is not None and kept.fits(mat):
+            return kept
+    return None
+
+
 def packed_layout(mat):
     """The matrix's dictionary-packed layout, or None when the matrix does not
     pack.  Built once per off-diagonal part: the matrices of a coupling sweep
-    that share their CSR arrays share its layout as well."""
-    home = getattr(mat, "_shared", None)
-    if home is None:
-        home = mat._shared = {}
-    if "packed" not in home:
-        home["packed"] = PackedLayout.build(mat)
-    return home["packed"]
+    that share their CSR arrays share its layout as well, as long as those
+    arrays are the ones it was built from."""
+    kept = _kept_layout(mat)
+    if kept is None:
+        kept = _KeptLayout(mat, PackedLayout.build(mat))
+        home = _layout_home(mat)
+        if home is not None:
+            home["packed"] = kept
+    mat._packed = kept
+    return kept.layout
 
 
 def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
@@ -288,7 +331,7 @@ def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
         t = t_of(lambda: pk.launch(1, nvec, diag, x, xs, y, mat.n))
         if t < best_t:
             best, best_t = ("packed", 2), t
-    # layouts that lost are not kept on the matrix
+    # layouts that lost are not kept
     keep = best[1] if best[0] == "sell" else None
     mat._sell32 = {w: l for w, l in getattr(mat, "_sell32", {}).items() if w == keep}
     ctx.put(key, ({"csr": 0, "sell": 1, "packed": 2}[best[0]], best[1]))

@@ -274,3 +274,25 @@ def test_krylov_evolution_on_packed_matches_csr(precision, tol):
     a, b = states["auto"], states["csr"]
     assert abs(float(torch.linalg.vector_norm(a)) - 1.0) < tol
     assert float(torch.max(torch.abs(a - b))) < tol
+
+
+def test_layout_is_shared_by_a_coupling_sweep_and_not_past_other_values():
+    """Matrices of one off-diagonal part share the layout; one that was given
+    other values packs its own, and both products are their own matrix's."""
+    import torch
+
+    from edgpu.solvers import packed_layout
+
+    model, g0, m0 = build("su2_1d_L8_obc", device="cuda")
+    mats = []
+    for g in (g0, 2 * g0, 3 * g0):
+        model.build_Hamiltonian(g, m0)
+        mats.append(model.H.mat)
+    mats[2].vals = 3.0 * mats[2].vals
+    lays = [packed_layout(mt) for mt in mats]
+    assert lays[0] is lays[1] and lays[2] is not lays[0]
+    x = torch.randn((mats[0].n, 1), dtype=torch.float64, device="cuda")
+    for mt, lay in zip(mats, lays):
+        y = _packed(lay, 0, mt.diag[:, None].contiguous(), x, 1, 1)
+        want = torch.from_numpy(mt.to_scipy() @ x[:, 0].cpu().numpy()).to("cuda")
+        assert float((y.reshape(-1)[: mt.n] - want).abs().max()) < 1e-12 * float(want.abs().max())
