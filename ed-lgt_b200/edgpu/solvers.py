@@ -276,6 +276,13 @@ def packed_layout(mat):
     return kept.layout
 
 
+def _forget_layout(mat):
+    mat._packed = None
+    home = _layout_home(mat)
+    if home is not None:
+        home.pop("packed", None)
+
+
 def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
     """Autotuner of the f32 Krylov path's matvec: times, in that path's
     configuration (f32 values and x with padded rows, f64 planar output),
@@ -326,6 +333,7 @@ def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
                                                  stream_handle()), "edg_spmv_sell"))
         if t < best_t:
             best, best_t = ("sell", wdw), t
+    was_packed = _kept_layout(mat) is not None
     pk = packed_layout(mat) if vals32_is_rounded else None
     if pk is not None:
         t = t_of(lambda: pk.launch(1, nvec, diag, x, xs, y, mat.n))
@@ -334,6 +342,8 @@ def tune_matvec32(mat, nvec, vals32=None, reps=5, ctx=None):
     # layouts that lost are not kept
     keep = best[1] if best[0] == "sell" else None
     mat._sell32 = {w: l for w, l in getattr(mat, "_sell32", {}).items() if w == keep}
+    if pk is not None and best[0] != "packed" and not was_packed:
+        _forget_layout(mat)
     ctx.put(key, ({"csr": 0, "sell": 1, "packed": 2}[best[0]], best[1]))
     return best
 

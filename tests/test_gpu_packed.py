@@ -296,3 +296,37 @@ def test_layout_is_shared_by_a_coupling_sweep_and_not_past_other_values():
         y = _packed(lay, 0, mt.diag[:, None].contiguous(), x, 1, 1)
         want = torch.from_numpy(mt.to_scipy() @ x[:, 0].cpu().numpy()).to("cuda")
         assert float((y.reshape(-1)[: mt.n] - want).abs().max()) < 1e-12 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("used", [False, True])
+def test_a_layout_the_tuner_rejects_is_released(used, monkeypatch):
+    """A packed layout that was built for the tuner's trial alone and lost is
+    kept by nobody; one that was in use before the trial stays."""
+    import gc
+    import weakref
+
+    import torch
+
+    from edgpu.context import Context
+    from edgpu.solvers import PackedLayout, packed_layout, tune_matvec32
+
+    made = []
+    build_layout, launch = PackedLayout.build.__func__, PackedLayout.launch
+
+    def building(cls, mat):
+        lay = build_layout(cls, mat)
+        made.append(weakref.ref(lay))
+        return lay
+
+    def slow(self, *args, **kw):
+        torch.cuda._sleep(10_000_000)  # about 5 ms beside a product of a few us
+        launch(self, *args, **kw)
+
+    monkeypatch.setattr(PackedLayout, "build", classmethod(building))
+    monkeypatch.setattr(PackedLayout, "launch", slow)
+    mat = _model("su2_1d_L10_pbc", "cuda").H.mat
+    if used:
+        packed_layout(mat)
+    assert tune_matvec32(mat, 3, ctx=Context())[0] != "packed"
+    gc.collect()
+    assert len(made) == 1 and (made[0]() is not None) == used
