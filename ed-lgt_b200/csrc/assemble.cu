@@ -526,6 +526,9 @@ struct Setup {
   bool wide, many;  // two-word keys; more than 16 sites
 };
 
+constexpr int kDiagCap = 64 * 1024;                     // diagonals kept in shared memory
+constexpr int kMostDigits = kThreads * EDG_MAX_SITES;  // digits of a CTA's rows
+
 inline int round16(int64_t b) { return (int)((b + 15) & ~int64_t(15)); }
 
 int make_setup(const edg_assembly* a, const char* who, Setup* s) {
@@ -556,7 +559,7 @@ int launch_fill(const edg_assembly* a, const Setup& s, int n_tables, int from_di
     p.ket = round16(e);
   }
   auto kern = fill_k<V, K, NS>;
-  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.total());
+  cudaError_t ce = edg::allow_smem(kern, p.windows + kMostDigits + 3 * kTableCap + 32);
   int occ = 1;
   if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, p.total());
   if (ce != cudaSuccess) return edg::cuda_status(ce, "edg_assemble_fill");
@@ -569,10 +572,10 @@ template <typename V, typename K, int NS>
 int launch_diag(const edg_assembly* a, const Setup& s, const double* base, const uint8_t* base_present, int has_extra,
                 double re, double im, double* diag, uint8_t* present, cudaStream_t stream) {
   const size_t table = (size_t)a->n_dterms * a->dmax * sizeof(V);
-  const int in_smem = table <= 64 * 1024;
+  const int in_smem = table <= (size_t)kDiagCap;
   const size_t smem = s.parts.digits + (in_smem ? table : 0);
   auto kern = diag_k<V, K, NS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = edg::allow_smem(kern, kMostDigits + kDiagCap);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_assemble_diag");
   kern<<<edg::grid_for(a->sector.n, kThreads, 16), kThreads, smem, stream>>>(
       *a, s.P, in_smem, base, base_present, has_extra, re, im, diag, present);
@@ -621,7 +624,7 @@ extern "C" int edg_assemble_count(const edg_assembly* a, int64_t* row_bound, cud
   if ((st = make_setup(a, "edg_assemble_count", &s))) return st;
   auto kern = s.wide ? count_k<edg::u128, EDG_MAX_SITES> : s.many ? count_k<uint64_t, EDG_MAX_SITES>
                                                                   : count_k<uint64_t, 16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.parts.total());
+  cudaError_t e = edg::allow_smem(kern, kMostDigits + 2 * kTableCap);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_assemble_count");
   kern<<<edg::grid_for(a->sector.n, kThreads, 8), kThreads, s.parts.total(), stream>>>(*a, s.P, s.parts, row_bound);
   EDG_CHECK_LAUNCH("edg_assemble_count");

@@ -178,9 +178,10 @@ extern "C" int edg_lanczos_small_batched(const edg_small_batch* b, int32_t* queu
               "edg_lanczos_small_batched: need 1 <= k <= 16, max_iter >= 1, check_every >= 1");
   if (b->n_inst == 0) return EDG_OK;
   const size_t smem = sizeof(double) * ((size_t)b->max_dim + 2 * (size_t)(b->max_iter + 1) + (size_t)b->max_iter + 2);
-  EDG_REQUIRE(smem <= 200 * 1024, "edg_lanczos_small_batched: max_dim + max_iter too large for shared memory");
+  constexpr size_t kMost = 200 * 1024;
+  EDG_REQUIRE(smem <= kMost, "edg_lanczos_small_batched: max_dim + max_iter too large for shared memory");
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(batched_lanczos_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = edg::allow_smem(batched_lanczos_k, kMost);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos_small_batched: smem attribute");
   }
   const int grid = b->n_inst < edg::kSmCount * 2 ? b->n_inst : edg::kSmCount * 2;

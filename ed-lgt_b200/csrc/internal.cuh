@@ -29,6 +29,15 @@ inline unsigned grid_for(int64_t n, int threads, int ctas_per_sm = 8) {
   return (unsigned)(need < cap ? need : cap);
 }
 
+// Allows a kernel `most` bytes of dynamic shared memory, the most that any of
+// its launches asks for.  The limit belongs to the kernel and not to a launch:
+// were it set to what one call needs, another host thread with a smaller
+// problem could lower it between this call and the launch after it.
+template <typename K>
+inline cudaError_t allow_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 }  // namespace edg
 
 #define EDG_CHECK_LAUNCH(where)                                         \

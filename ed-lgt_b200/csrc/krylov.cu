@@ -771,7 +771,7 @@ int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* e
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
+    if (e == cudaSuccess) e = edg::allow_smem(kern, kCoopSmem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: set-up");
     const int64_t g = edg::coop_ctas(n, n_sm);
@@ -913,8 +913,7 @@ extern "C" int edg_krylov_orth(int64_t n, int64_t ldv, double* V, int32_t j, dou
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_orth");
   }
   if ((j + 2) * sizeof(double2) > 40 * 1024) {  // above the limit a kernel has without asking
-    cudaError_t e = cudaFuncSetAttribute(update_k<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)((j + 2) * sizeof(double2)));
+    cudaError_t e = edg::allow_smem(update_k<double2>, (kMaxOrth + 1) * sizeof(double2));
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_orth");
   }
   for (int pass = 0; pass < passes; ++pass) {

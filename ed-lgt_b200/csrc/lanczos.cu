@@ -1438,7 +1438,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopSmem);
+    if (e == cudaSuccess) e = edg::allow_smem(kern, kCoopSmem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, kCoopSmem);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: set-up");
     const int64_t g = edg::coop_ctas(n_pad, n_sm);
@@ -1475,9 +1475,8 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   const size_t upd_smem = sizeof(edg::bulk::Smem<T>);
   const int64_t n_seg = (n_pad / 4 + edg::bulk::kSegQuads - 1) / edg::bulk::kSegQuads;
   int occ_dot = 0, occ_upd = 0, n_sm = 0, dev = 0;
-  e = cudaFuncSetAttribute(dots_bulk_k<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dot_smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(update_bulk_k<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)upd_smem);
+  e = edg::allow_smem(dots_bulk_k<T, NV>, dot_smem);
+  if (e == cudaSuccess) e = edg::allow_smem(update_bulk_k<T, NV>, upd_smem);
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)

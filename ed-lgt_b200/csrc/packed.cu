@@ -523,7 +523,7 @@ int pack_encode(int64_t n, int64_t total, const int64_t* rowptr, const int32_t* 
   const int64_t n_tiles = (n + kTileRows - 1) / kTileRows;
   const unsigned grid = edg::grid_for(n_tiles * kTileRows + 4, 256);
   const size_t smem = sizeof(T) * (size_t)count;
-  cudaFuncSetAttribute(pack_encode_k<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static_assert(sizeof(T) * EDG_PACK_MAX_VALUES <= 48 * 1024, "within the limit a kernel has without asking");
   pack_encode_k<T><<<grid, 256, smem, s>>>(n, total, rowptr, cols, vals, table, count, colbits, offsets, tile_off,
                                            words, missing);
   return EDG_OK;
@@ -542,7 +542,7 @@ int launch_packed_spmv(int nvec, int x_stride, int64_t n, const int32_t* tile_of
   do {                                                                                                              \
     auto kern = packed_spmv_k<T, NV, XS, NoEpilogue>;                                                              \
     const size_t smem = packed_smem<T, XS>(count);                                                                 \
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
+    e = edg::allow_smem(kern, packed_smem<T, XS>(EDG_PACK_MAX_VALUES));                                            \
     if (e == cudaSuccess)                                                                                           \
       kern<<<packed_grid(n, tiles_of<T, XS>()), kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, \
                                                                         diag, x, y, y_plane, diag_shared, skip,    \
@@ -580,7 +580,7 @@ int launch_packed_krylov(int64_t n, const int32_t* tile_off, const uint32_t* wor
   const unsigned grid = packed_grid(n, tiles_of<T, 2>());
   const size_t smem = packed_smem<T, 2>(count);
   auto kern = packed_spmv_k<T, 2, 2, KrylovEpilogue>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = edg::allow_smem(kern, packed_smem<T, 2>(EDG_PACK_MAX_VALUES));
   if (e == cudaSuccess)
     kern<<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, y, 0, 1, nullptr, err,
                                          KrylovEpilogue{step, {0.0, 0.0, 0.0, 0.0}});

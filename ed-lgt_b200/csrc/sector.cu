@@ -458,8 +458,9 @@ extern "C" int edg_sector_levels(const edg_sector_tables* t, uint64_t* keys0, ui
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   const int64_t grid = n_sm < edg::kSmCount ? n_sm : edg::kSmCount;
   const int64_t smem = ((cap + grid - 1) / grid + 1) * bytes;  // masks of a CTA's parents
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, (size_t)smem);
+  if (e == cudaSuccess) e = edg::allow_smem(kern, kCoopSmem);
+  if (e == cudaSuccess && smem <= kCoopSmem)  // (more on a device with fewer SMs: a run of parents is longer)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kCoopThreads, (size_t)smem);
   if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, kHead * sizeof(int64_t), stream);
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_sector_levels");
   if (!coop || occ < 1) {  // nothing done: the caller runs every level itself

@@ -458,7 +458,7 @@ inline bool mma_fits(int n_sites, int dmax) {
 template <int PT, int NB>
 cudaError_t launch_mma(const Args& a, cudaStream_t stream) {
   const int64_t smem = mma_smem<NB>(a.dmax);
-  cudaError_t e = cudaFuncSetAttribute(twobody_mma_k<PT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = edg::allow_smem(twobody_mma_k<PT, NB>, sizeof(MmaSmem<NB>) + kMmaTableCap);
   if (e != cudaSuccess) return e;
   twobody_mma_k<PT, NB><<<kBlocks, kThreads, (size_t)smem, stream>>>(a);
   return cudaGetLastError();
@@ -478,7 +478,7 @@ template <int PT>
 cudaError_t launch(const Args& a, int64_t smem, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(twobody_k<PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    cudaError_t e = edg::allow_smem(twobody_k<PT>, 96 * 1024);
     if (e != cudaSuccess) return e;
     configured = true;
   }

@@ -520,10 +520,14 @@ size_t table_smem(const edg_zn_lattice* L) {
   return sizeof(uint64_t) * 256 * (size_t)((L->field_bits + 7) / 8) + sizeof(uint32_t) * ((size_t)1 << L->n_sites);
 }
 
+// most: of any lattice (table_smem and a row's slots grow with its sites).
+constexpr size_t kMostTables = sizeof(uint64_t) * 256 * 8 + (sizeof(uint32_t) << EDG_ZN_MAX_SITES);
+constexpr size_t kMostSlots = sizeof(uint32_t) * kMvThreads * 4 * EDG_ZN_MAX_SITES;
+
 template <typename K>
-int set_smem(K kernel, size_t smem, const char* where) {
+int set_smem(K kernel, size_t smem, size_t most, const char* where) {
   if (smem > 40 * 1024) {  // 48 KB less the kernels' own static arrays
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = edg::allow_smem(kernel, most);
     if (e != cudaSuccess) return edg::cuda_status(e, where);
   }
   return EDG_OK;
@@ -546,7 +550,7 @@ int launch_matvec(const edg_zn_lattice* L, const edg_zn_basis* B, const double* 
   }
   const size_t smem = sizeof(uint32_t) * kMvThreads * (size_t)(L->n_links + 2 * L->n_sites);
   auto kern = zn_matvec_k<ZN, T, NV, WIDE>;
-  int st = set_smem(kern, smem, "edg_zn_matvec");
+  int st = set_smem(kern, smem, kMostSlots, "edg_zn_matvec");
   if (st != EDG_OK) return st;
   const unsigned grid = persistent_grid(kern, kMvThreads, smem, B->n_rows);
   kern<<<grid, kMvThreads, smem, stream>>>(*L, make_tables(L), *B, coup, (const T*)x, (T*)y);
@@ -620,7 +624,7 @@ extern "C" int edg_zn_orbit_table(const edg_zn_lattice* L, const uint64_t* keys,
   if (e != cudaSuccess) return edg::cuda_status(e, "edg_zn_orbit_table: memset");
   if (n_rows == 0) return EDG_OK;
   const size_t smem = table_smem(L);
-  st = set_smem(zn_orbit_k, smem, "edg_zn_orbit_table");
+  st = set_smem(zn_orbit_k, smem, kMostTables, "edg_zn_orbit_table");
   if (st != EDG_OK) return st;
   const unsigned grid = persistent_grid(zn_orbit_k, 256, smem, n_rows);
   zn_orbit_k<<<grid, 256, smem, stream>>>(*L, keys, n_rows, orbit);
