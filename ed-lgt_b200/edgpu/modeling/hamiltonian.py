@@ -26,6 +26,16 @@ __all__ = ["QMB_hamiltonian", "QMB_state"]
 _PSI_CODES = {torch.float64: 0, torch.float32: 1, torch.complex128: 2, torch.complex64: 3}
 
 
+def _is_plain(x):
+    """Whether a tensor is its values in memory and nothing else: a kernel on
+    its address would lose reverse- or forward-mode derivatives, the batch of
+    vmap, the record of a trace, and a lazy conjugation or sign."""
+    return (type(x) is torch.Tensor and not x.requires_grad and not x.is_conj() and not x.is_neg()
+            and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and torch.autograd.forward_ad.unpack_dual(x).tangent is None
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing())
+
+
 class QMB_state:
     """A state vector in the sector basis (host copy made on first access)."""
 
@@ -253,11 +263,10 @@ class QMB_hamiltonian:
         if tab is None:
             return psi
         # one vector over the sector's rows, read in place; anything else (a
-        # stack of states, another dtype or device, autograd) is a product
-        # with the phases
-        if (psi.dim() == 1 and psi.shape[0] == len(self.sector) and psi.stride(0) >= 1 and psi.dtype in _PSI_CODES
-                and psi.device == self.sector.keys.device and not psi.requires_grad and not psi.is_conj()
-                and not psi.is_neg()):
+        # stack of states, another dtype or device, a tensor that a derivative,
+        # vmap or a trace follows) is a product with the phases
+        if (_is_plain(psi) and psi.dim() == 1 and psi.shape[0] == len(self.sector) and psi.stride(0) >= 1
+                and psi.dtype in _PSI_CODES and psi.device == self.sector.keys.device):
             return self._apply_phase(tab, psi, conj)
         ph = self._apply_phase(tab, None, conj)
         return ph * psi.to(torch.complex128)
