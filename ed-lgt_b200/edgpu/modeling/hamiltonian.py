@@ -222,15 +222,17 @@ class QMB_hamiltonian:
     # -------------------------------------------------------------- phases
     def _phase_table(self):
         """Device bytes [n_sites][dmax] of the real form's phase exponents
-        (None if not used); kept on the matrix they belong to."""
+        (None if not used); kept on the matrix they belong to, beside their
+        host values."""
         mat = self.mat
         w = mat.phase_weights if mat is not None else None
         if w is None:
             return None
-        if getattr(mat, "_phase_bytes", None) is None:
-            t = np.ascontiguousarray(np.asarray(w, dtype=np.int64) % 4, dtype=np.uint8)
-            mat._phase_bytes = torch.from_numpy(t).to(self.sector.device)
-        return mat._phase_bytes
+        t = np.ascontiguousarray(np.asarray(w, dtype=np.int64) % 4, dtype=np.uint8)
+        kept = getattr(mat, "_phase_bytes", None)
+        if kept is None or not np.array_equal(kept[0], t):
+            kept = mat._phase_bytes = (t, torch.from_numpy(t.copy()).to(self.sector.device))
+        return kept[1]
 
     def _apply_phase(self, tab, psi, conj):
         """i**(+-e(row)) psi as complex128 (``edg_gauge_apply``); the phases

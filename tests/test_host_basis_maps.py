@@ -92,3 +92,20 @@ def test_lazy_conjugation_and_sign(maps):
         assert torch.equal(f(x.conj()), phase * x.conj())
         y = x.conj().imag  # a lazy sign
         assert y.is_neg() and torch.equal(f(y), phase * y)
+
+
+def test_phase_table_follows_the_matrix():
+    """Exponents that are replaced or changed in place after a first use."""
+    from types import SimpleNamespace
+
+    ham = QMB_hamiltonian([N], N, sector=_Sector())
+    w = np.arange(12).reshape(4, 3)
+    ham.mat = SimpleNamespace(phase_weights=w)
+    assert np.array_equal(ham._phase_table().numpy(), w % 4)
+    assert ham._phase_table() is ham._phase_table()
+    w[2, 1] += 1
+    assert np.array_equal(ham._phase_table().numpy(), w % 4)
+    ham.mat.phase_weights = w[:, ::-1] + 2
+    assert np.array_equal(ham._phase_table().numpy(), (w[:, ::-1] + 2) % 4)
+    ham.mat.phase_weights = None
+    assert ham._phase_table() is None
