@@ -737,12 +737,13 @@ KLayout klayout(const edg_krylov_problem* p) {
   return L;
 }
 
-// Whether a step may run as krylov_coop_k: few enough rows, and the CSR arrays
-// at hand, which that kernel reads whatever layout is passed beside them (a
-// problem may come with its packed layout alone).
-bool one_launch(const edg_krylov_problem* p) {
+// Whether a step may run as krylov_coop_k: few enough rows, the CSR arrays at
+// hand, which that kernel reads whatever layout is passed beside them (a
+// problem may come with its packed layout alone), and a way to report a grid-wide
+// wait that ran out (the problem's status word, or a result the call waits for).
+bool one_launch(const edg_krylov_problem* p, bool reports) {
   const bool csr = p->cols != nullptr && p->vals != nullptr, diagonal = p->nnz == 0 && p->pk_words == nullptr;
-  return p->n_rows <= kCoopMaxRows && (csr || diagonal);
+  return reports && p->n_rows <= kCoopMaxRows && (csr || diagonal);
 }
 
 template <typename T, typename SV>
@@ -765,7 +766,7 @@ int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* e
   cudaError_t e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s);
   if (e != cudaSuccess) return edg::cuda_status(e, "krylov");
   bool done = false;
-  if (one_launch(p)) {
+  if (one_launch(p, p->status != nullptr || err_out != nullptr)) {
     int dev = 0, n_sm = 0, coop = 0, occ = 0;
     auto kern = krylov_coop_k<T, SV>;
     e = cudaGetDevice(&dev);
@@ -841,9 +842,16 @@ int run_step(const edg_krylov_problem* p, T* psi, double dt, char* ws, double* e
     if ((e = cudaGetLastError()) != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: combine");
   }
   if (err_out) {
+    int waits = 0;
     e = cudaMemcpyAsync(err_out, misc + 1, sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&waits, err_word, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_krylov_step: error estimate");
+    if (waits != 0) {
+      *err_out = nan("");
+      edg::set_error("edg_krylov_step: a grid-wide wait ran out");
+      return EDG_ERR_TIMEOUT;
+    }
   }
   return EDG_OK;
 }
@@ -934,7 +942,7 @@ extern "C" int64_t edg_krylov_workspace_bytes(const edg_krylov_problem* p) {
 
 extern "C" int edg_krylov_one_launch(const edg_krylov_problem* p) {
   if (check_k(p)) return -1;
-  return one_launch(p) ? 1 : 0;
+  return one_launch(p, p->status != nullptr) ? 1 : 0;
 }
 
 extern "C" int edg_krylov_step(const edg_krylov_problem* p, void* psi, double dt, void* workspace,

@@ -89,10 +89,11 @@ class KrylovEvolver:
         self.vdtype = torch.complex128 if precision == "c128" else torch.complex64
 
     def check_status(self):
-        """Raise if a stage wait of the packed matvec ran out (one host read)."""
+        """Raise if a bounded wait of a step ran out (one host read)."""
         st = int(self.status.item())
         if st != 0:
-            raise _lib.EdgError(st, "edg_krylov_step: a stage wait of the packed matvec ran out")
+            raise _lib.EdgError(st, "edg_krylov_step: a stage wait of the packed matvec or a grid-wide wait of a "
+                                    "one-launch step ran out")
 
     def step(self, psi: torch.Tensor, dt: float, want_error=False):
         err = np.zeros(1) if want_error else None

@@ -641,17 +641,20 @@ typedef struct {
   int32_t pk_colbits;         /* real right-hand sides; used when pk_words  */
                               /* is not NULL                                */
   int32_t* status;        /* optional device word: EDG_ERR_TIMEOUT when a   */
-                          /* stage wait of the packed matvec ran out        */
+                          /* stage wait of the packed matvec or a grid-wide */
+                          /* wait of a one-launch step ran out              */
 } edg_krylov_problem;
 
 int64_t edg_krylov_workspace_bytes(const edg_krylov_problem* p);
 /* 1 when a step of this problem is one cooperative launch (few rows, CSR
- * arrays given; it reads those and the diagonal, not the packed layout), on a
- * device that has such launches; 0 when it is a launch per pass; -1 for a bad
- * problem. */
+ * arrays and a status word given; it reads those arrays and the diagonal, not
+ * the packed layout), on a device that has such launches; 0 when it is a launch
+ * per pass; -1 for a bad problem. */
 int edg_krylov_one_launch(const edg_krylov_problem* p);
 /* One step of length dt in place on psi [n_rows] (complex, vec_dtype).
- * err_out (host, may be NULL): a posteriori error estimate of the step. */
+ * err_out (host, may be NULL): a posteriori error estimate of the step; the
+ * call then waits for it, and returns EDG_ERR_TIMEOUT with NaN there when a
+ * grid-wide wait ran out. */
 int edg_krylov_step(const edg_krylov_problem* p, void* psi, double dt,
                     void* workspace, int64_t workspace_bytes, double* err_out,
                     cudaStream_t stream);

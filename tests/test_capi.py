@@ -255,3 +255,30 @@ def test_lanczos_problem_without_matrix_entries_is_refused():
     assert size() > 0
     p.dtype = 0  # the f64 path does not read it
     assert size() == -1
+
+
+def test_krylov_one_launch_form_needs_a_way_to_report():
+    """Its grid-wide waits are bounded: without a status word a step that has
+    no result to wait for is not one for that form."""
+    from edgpu import _lib
+
+    p = _lib.KrylovProblem()
+    p.vec_dtype, p.mat_dtype, p.n_rows, p.nnz, p.m = 2, 0, 1000, 5000, 30
+    p.rowptr = p.diag = p.cols = p.vals = 16
+    assert _lib.lib.edg_krylov_one_launch(ctypes.byref(p)) == 0
+    p.status = 16
+    assert _lib.lib.edg_krylov_one_launch(ctypes.byref(p)) == 1
+
+
+def test_krylov_status_names_both_waits():
+    from edgpu import _lib
+    from edgpu.dynamics import KrylovEvolver
+
+    class Status:
+        def item(self):
+            return -7
+
+    ev = KrylovEvolver.__new__(KrylovEvolver)
+    ev.status = Status()
+    with pytest.raises(_lib.EdgError, match="grid-wide wait"):
+        ev.check_status()

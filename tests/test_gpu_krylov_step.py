@@ -104,3 +104,31 @@ def test_step_on_a_packed_layout_alone(n, precision, reorth):
     ev.check_status()
     err = float(torch.linalg.vector_norm(got.to(torch.complex128) - want) / torch.linalg.vector_norm(want))
     assert err < (5e-6 if precision == "c64" else 1e-12), err
+
+
+@pytest.mark.parametrize("n", [33, 5000])
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("status,want_error", [(True, True), (False, True), (False, False)])
+def test_step_with_and_without_a_status_word(n, precision, status, want_error):
+    """The same step reports to a status word, through the error estimate's
+    return, or has neither and takes the passes."""
+    import torch
+
+    from edgpu.dynamics import KrylovEvolver
+
+    mat, apply = _matrix(n, False, n)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    psi = torch.randn(n, dtype=torch.complex128, device="cuda", generator=gen)
+    want, term = psi.clone(), psi
+    for k in range(1, 40):
+        term = apply(term) * (-0.1j / k)
+        want = want + term
+    ev = KrylovEvolver(mat, m=30, precision=precision, matvec="csr")
+    if not status:
+        ev.p.status = None
+    got = psi.to(ev.vdtype).clone()
+    e = ev.step(got, 0.1, want_error=want_error)
+    ev.check_status()
+    assert e is None or 0.0 <= e < 1e-10
+    err = float(torch.linalg.vector_norm(got.to(torch.complex128) - want) / torch.linalg.vector_norm(want))
+    assert err < (5e-6 if precision == "c64" else 1e-12), err
