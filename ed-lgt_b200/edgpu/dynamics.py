@@ -29,7 +29,8 @@ class KrylovEvolver:
     ``matvec``: "auto" uses the dictionary-packed tiled layout of a real
     matrix when it packs (a complex vector is two real right-hand sides of
     it; f32 lane sums for complex64, f64 for complex128), else CSR;
-    "csr" forces CSR."""
+    "csr" forces CSR.  A sector small enough for a step in one launch
+    (``edg_krylov_one_launch``) has its CSR arrays read by that launch."""
 
     def __init__(self, mat, m=30, precision="c128", reorth_passes=1, spmv_group=None, matvec="auto"):
         if precision not in ("c128", "c64"):
@@ -60,33 +61,49 @@ class KrylovEvolver:
         p.diag = ptr(diag)
         p.m = self.m
         p.reorth_passes = reorth_passes
-        self.packed = None
-        if matvec == "auto" and not mat.is_complex:
-            from .solvers import packed_layout
-
-            self.packed = packed_layout(mat)
-        if spmv_group is None:
-            # a complex vector is two real right-hand sides for a real matrix:
-            # tune the CSR kernel on that shape (real forms only)
-            from .solvers import tune_spmv_group
-
-            spmv_group = 0 if (mat.is_complex or self.packed is not None) else tune_spmv_group(
-                mat, 2, 0 if precision == "c128" else 1, vals=mat.vals if precision == "c128" else vals)
-        p.spmv_group = int(spmv_group)
-        if self.packed is not None:
-            pk = self.packed
-            p.pk_tile_off, p.pk_words = ptr(pk.tile_off), ptr(pk.words)
-            p.pk_table = ptr(pk.table(0 if precision == "c128" else 1))
-            p.pk_count, p.pk_colbits = pk.count, pk.colbits
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         p.status = ptr(self.status)
         self.p = p
+        self._may_pack, self._layout = matvec == "auto" and not mat.is_complex, None
+        if lib.edg_krylov_one_launch(ctypes.byref(p)) == 1:
+            # the step reads the CSR arrays in one launch: no layout, no kernel
+            # variant to choose
+            p.spmv_group = int(spmv_group or 0)
+        else:
+            self._choose_matvec(spmv_group)
         wb = lib.edg_krylov_workspace_bytes(ctypes.byref(p))
         if wb < 0:
             raise _lib.EdgError(-1, _lib.last_error())
         self.ws = torch.empty(wb, dtype=torch.uint8, device=dev)
         self.wb = wb
         self.vdtype = torch.complex128 if precision == "c128" else torch.complex64
+
+    @property
+    def packed(self):
+        """The matrix's packed layout with matvec "auto", where it packs (a
+        one-launch step does not read it: it is then built when asked for)."""
+        if self._may_pack and self._layout is None:
+            from .solvers import packed_layout
+
+            self._layout = packed_layout(self.mat)
+        return self._layout
+
+    def _choose_matvec(self, spmv_group):
+        """The packed layout or the threads a CSR row of the matvec."""
+        mat, p, c128 = self.mat, self.p, self.precision == "c128"
+        pk = self.packed
+        if pk is not None:
+            p.pk_tile_off, p.pk_words = ptr(pk.tile_off), ptr(pk.words)
+            p.pk_table = ptr(pk.table(0 if c128 else 1))
+            p.pk_count, p.pk_colbits = pk.count, pk.colbits
+        if spmv_group is None:
+            # a complex vector is two real right-hand sides for a real matrix:
+            # tune the CSR kernel on that shape (real forms only)
+            from .solvers import tune_spmv_group
+
+            spmv_group = 0 if (mat.is_complex or pk is not None) else tune_spmv_group(
+                mat, 2, 0 if c128 else 1, vals=mat.vals if c128 else self.vals)
+        p.spmv_group = int(spmv_group)
 
     def check_status(self):
         """Raise if a bounded wait of a step ran out (one host read)."""
