@@ -11,11 +11,14 @@ diagonal, e.g. identity shifts); the matrix lives on the device.
 
 from __future__ import annotations
 
+import ctypes
 import logging
 
 import numpy as np
 import torch
 
+from .. import _lib
+from .._lib import check, lib, ptr, stream_handle
 from .assembly import assemble_blocks
 from .terms import TermBlock
 
@@ -30,10 +33,11 @@ def _is_plain(x):
     """Whether a tensor is its values in memory and nothing else: a kernel on
     its address would lose reverse- or forward-mode derivatives, the batch of
     vmap, the record of a trace, and a lazy conjugation or sign."""
+    fw = torch.autograd.forward_ad
     return (type(x) is torch.Tensor and not x.requires_grad and not x.is_conj() and not x.is_neg()
             and not torch._C._functorch.is_functorch_wrapped_tensor(x)
-            and torch.autograd.forward_ad.unpack_dual(x).tangent is None
-            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing())
+            and (fw._current_level < 0 or fw.unpack_dual(x).tangent is None)
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._is_tracing())
 
 
 class QMB_state:
@@ -228,20 +232,17 @@ class QMB_hamiltonian:
         w = mat.phase_weights if mat is not None else None
         if w is None:
             return None
-        t = np.ascontiguousarray(np.asarray(w, dtype=np.int64) % 4, dtype=np.uint8)
+        w = np.asarray(w)
+        now = (w.dtype, w.shape, w.tobytes())
         kept = getattr(mat, "_phase_bytes", None)
-        if kept is None or not np.array_equal(kept[0], t):
-            kept = mat._phase_bytes = (t, torch.from_numpy(t.copy()).to(self.sector.device))
+        if kept is None or kept[0] != now:
+            t = np.ascontiguousarray(w.astype(np.int64) % 4, dtype=np.uint8)
+            kept = mat._phase_bytes = (now, torch.from_numpy(t).to(self.sector.device))
         return kept[1]
 
     def _apply_phase(self, tab, psi, conj):
         """i**(+-e(row)) psi as complex128 (``edg_gauge_apply``); the phases
         themselves for psi = None."""
-        import ctypes
-
-        from .. import _lib
-        from .._lib import check, lib, ptr, stream_handle
-
         sec = self.sector
         n = len(sec)
         dims = _lib.SiteDims()
@@ -376,7 +377,6 @@ class QMB_hamiltonian:
         """The sector matrix as a dense device array (``edg_csr_to_dense``), in
         the assembled (possibly real) form, or with the real form's phases put
         back: H = D H' D^dagger, the reference's basis."""
-        from .._lib import check, lib, ptr, stream_handle
 
         n = self.shape[0]
         if n > self.DENSE_MAX:
