@@ -26,22 +26,27 @@
 // while the tile offsets are loaded two steps ahead; two lanes per row then
 // walk the rows of each tile from shared memory (lane j takes entries j, j + 2,
 // j + 4, ...; the two lanes of all 16 rows read 32 consecutive words),
-// gathering x rows.  The stream is read with whole-range copies that bypass the
-// load pipeline (the CSR kernel's loads touch one segment per row of the warp
-// on every load), which leaves the L1 data pipe to the gathers.  f32 matrices
-// (the f32 Krylov phase) sum each lane's products in f32 and add the lane sums
-// and the diagonal term in f64, so no conversion happens per entry; f64
-// matrices sum in f64 in the CSR kernel's order (bit-identical to the CSR
-// kernel with two threads a row).
+// gathering x rows.  What a stage does not hold is read from the stream.  The
+// stream is read with whole-range copies that bypass the load pipeline (the CSR
+// kernel's loads touch one segment per row of the warp on every load), which
+// leaves the L1 data pipe to the gathers.  f32 matrices (the f32 Krylov phase)
+// sum each lane's products in f32 and add the lane sums and the diagonal term in
+// f64, so no conversion happens per entry; f64 matrices sum in f64 in the CSR
+// kernel's order (bit-identical to the CSR kernel with two threads a row).
 //
 // Two tiles a step when an x row has at most 8 bytes: the two lanes of a row
 // exchange halves, lane 0 finishes the first tile's row and lane 1 the
 // second's, so that the diagonal, y and the epilogue run with all lanes at
 // work (one tile at a time they were more than half of the instructions).
 // complex64 on SU(2) L = 16 (7,133,222 rows, 124M words, with the Krylov
-// epilogue): 283 -> 221 us; one f32 vector on the L = 14 ring 37.0 -> 33.0 us.
-// Wider x rows live off L1, which the larger stages shrink (three f64 vectors
-// on the ring: 76 us one tile at a time, 95 with two).
+// epilogue): 283 us one tile at a time, 222 with two; one f32 vector on the
+// L = 14 ring 36.3 and 31.1 us.  Wider x rows live off L1 and take one tile
+// (three f64 vectors on the ring: 76 us, 95 with two).
+//
+// A pair is worth it while its tiles fit the stage: the mean width of the
+// matrix's pairs decides (kPairMax of the epilogues).  Rows of 32 neighbouring
+// entries, 1.2M rows, one f32 vector: 47 us one tile at a time, 63 in pairs of
+// which 38 entries of 64 are staged, 70 in pairs read from the stream.
 #include <algorithm>
 
 #include "reorth_bulk.cuh"
@@ -50,11 +55,15 @@
 namespace {
 
 constexpr int kTileRows = 16;   // rows of a warp tile (two lanes a row)
-// Tiles a warp takes at a time, and the words of a stage (24 a row of a pair,
-// 32 a row of a single tile; longer ones read the stream directly).
+// Tiles a warp takes at a time, at most, and the words of a stage: 38 entries of
+// a row where pairs of tiles are the rule (of both tiles together), else 32.
+// Four CTAs an SM then leave the gathers 92 KB of L1, whose lines are what
+// misses wait in: with 768 words (28 KB left) rows of 16 entries in random
+// columns, 1.2M rows, took 148 us for one f32 vector instead of 80.  (The
+// kernels' registers keep the SM at four CTAs; a fifth would take that L1 too.)
 template <typename T, int XS>
 constexpr int tiles_of() { return sizeof(T) * XS <= 8 ? 2 : 1; }
-constexpr int stage_words(int tiles) { return tiles == 2 ? 768 : 516; }
+constexpr int stage_words(int tiles) { return tiles == 2 ? 608 : 516; }
 constexpr int kWarps = 8;  // warps of a CTA
 
 template <typename T>
@@ -219,32 +228,33 @@ __device__ __forceinline__ int32_t load_head(const int32_t* __restrict__ tile_of
 }
 
 // A step's words [e0, e0 + 16 (wa + wb)) (e0 a multiple of 16: 64-byte
-// aligned), wa and wb the widths of its tiles; `fits` when they fit the stage.
+// aligned), wa and wb the widths of its tiles.
 struct Range {
-  int32_t e0, wa, wb, quads;
-  bool fits;
+  int32_t e0, wa, wb;
 };
 template <int NT>
 __device__ __forceinline__ Range range_of(int32_t head) {
   const int32_t e0 = __shfl_sync(0xffffffffu, head, 0);
   const int32_t em = __shfl_sync(0xffffffffu, head, 1);
   const int32_t e1 = NT == 2 ? __shfl_sync(0xffffffffu, head, 2) : em;
-  return {e0, (em - e0) / kTileRows, (e1 - em) / kTileRows, (e1 - e0) / 4, e1 - e0 <= stage_words(NT) / 16 * 16};
+  return {e0, (em - e0) / kTileRows, (e1 - em) / kTileRows};
 }
 
-// Lane 0 copies the step's range into a stage with one bulk asynchronous copy
-// (this GPU's memory, no multicast) completing on the stage's mbarrier;
-// returns whether a copy was issued (warp-uniform).
+// Lane 0 copies the step's words, or as many as the stage holds, into a stage
+// with one bulk asynchronous copy (this GPU's memory, no multicast) completing on
+// the stage's mbarrier; returns whether a copy was issued (warp-uniform).
+template <int CAP>
 __device__ __forceinline__ bool stage_tile(const uint32_t* __restrict__ words, Range rg, uint32_t* stage,
                                            uint64_t* bar, int lane) {
-  const bool issue = rg.fits && rg.quads > 0;
-  if (issue && lane == 0) {
+  const int width = rg.wa + rg.wb;
+  if (width > 0 && lane == 0) {
+    const unsigned bytes = (unsigned)(width < CAP ? width : CAP) * (kTileRows * 4u);
     // the stage was last read through the generic proxy (ordered by __syncwarp)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    edg::bulk::mbar_expect_tx(bar, (unsigned)rg.quads * 16u);
-    edg::bulk::bulk_g2s(stage, words + rg.e0, (unsigned)rg.quads * 16u, bar);
+    edg::bulk::mbar_expect_tx(bar, bytes);
+    edg::bulk::bulk_g2s(stage, words + rg.e0, bytes, bar);
   }
-  return issue;
+  return width > 0;
 }
 
 // x row (NV entries at stride XS) as stored
@@ -291,22 +301,24 @@ struct XRow<double, NV, 4> {
   }
 };
 
-// The tile's rows, two lanes a row (lane j of row s takes entries k = j,
-// j + 2, ... of it), from the stage (shared) or the stream: acc[v] +=
-// table[idx] x[col][v] in the accumulator type A (f32 lane sums for an f32
-// matrix, f64 for f64), four gathers in flight.  Entry k of the tile's rows
-// is the run of words [16 k, 16 k + 16), so lanes j = 0, 1 read 32
-// consecutive words (no bank conflicts); padding words are skipped.
-template <typename T, typename A, int NV, int XS>
-__device__ __forceinline__ void gather_tile(const uint32_t* src, int width, int s, int j, const T* tab, int colbits,
-                                            uint32_t cmask, const T* __restrict__ x, A (&acc)[NV], bool shared) {
+// The rows of a tile, two lanes a row (lane j of row s takes entries k = j,
+// j + 2, ... of it), acc[v] += table[idx] x[col][v] in the accumulator type A
+// (f32 lane sums for an f32 matrix, f64 for f64), four gathers in flight.  Entry
+// k of the tile's rows is the run of words [16 k, 16 k + 16), so lanes j = 0, 1
+// read 32 consecutive words (no bank conflicts); padding words are skipped.
+// ALL: the tile is in the stage; else its entries from k = staged on are read
+// from the stream.
+template <typename T, typename A, int NV, int XS, bool ALL>
+__device__ __forceinline__ void gather_tile(const uint32_t* stage, const uint32_t* __restrict__ stream, int staged,
+                                            int width, int s, int j, const T* tab, int colbits, uint32_t cmask,
+                                            const T* __restrict__ x, A (&acc)[NV]) {
   for (int k0 = j; k0 < width; k0 += 8) {
     uint32_t w[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int k = k0 + 2 * q;
       const int off = kTileRows * k + s;
-      w[q] = k < width ? (shared ? src[off] : __ldg(src + off)) : 0xFFFFFFFFu;
+      w[q] = k < width ? (ALL || k < staged ? stage[off] : __ldg(stream + off)) : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -321,8 +333,13 @@ __device__ __forceinline__ void gather_tile(const uint32_t* src, int width, int 
 }
 
 // What a product leaves behind besides y: row(r, x_r, y_r) once per row (one
-// lane), finish() by every thread at the end of the kernel.
+// lane), finish() by every thread at the end of the kernel.  kPairMax: the mean
+// width of a pair of tiles up to which they are taken together: what a stage
+// holds, and some more where the epilogue is paid per row (rows of 20 entries,
+// 1.2M rows: f64 39.4 us one by one, 45.1 in pairs; eight complex64 Krylov steps
+// with rows of 24: 608 us one by one, 617 in pairs; of 20: 590 in pairs).
 struct NoEpilogue {
+  static constexpr int kPairMax = 38;
   template <typename T, int NV>
   __device__ void row(int64_t, const T (&)[NV], const double (&)[NV]) {}
   __device__ void finish() {}
@@ -334,6 +351,7 @@ struct NoEpilogue {
 // vectors again.  The last CTA (ticket) adds the CTA partials in a fixed
 // order and forms the step's coefficients.
 struct KrylovEpilogue {
+  static constexpr int kPairMax = 44;
   edg::KrylovStep k;
   double acc[4];
   template <typename T>
@@ -387,6 +405,104 @@ struct KrylovEpilogue {
   }
 };
 
+// What the steps of a product need (see packed_spmv_k).
+template <typename T>
+struct Product {
+  int64_t n;
+  const int32_t* tile_off;
+  const uint32_t* words;
+  const T *table, *diag, *x;
+  double* y;
+  int64_t y_plane;
+  int count, colbits, diag_shared;
+  const int* skip;
+  int* err;
+};
+
+// A warp's steps of NT tiles each.  stage0: its two stages of STAGE words.
+template <typename T, int NV, int XS, int NT, int STAGE, typename Epi>
+__device__ __forceinline__ void warp_steps(const Product<T>& p, const T* tab, uint32_t* stage0, uint64_t* bar,
+                                           int* s_err, Epi& epi) {
+  using A = T;  // lane accumulator: f32 lanes for the f32 phase, f64 otherwise
+  constexpr int kCap = STAGE / kTileRows;  // entries of a row that a stage holds
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t cmask = (1u << p.colbits) - 1u;
+  const int64_t n_tiles = (p.n + kTileRows - 1) / kTileRows, n_steps = (n_tiles + NT - 1) / NT;
+  const int64_t step = (int64_t)gridDim.x * kWarps;
+  const int s = lane >> 1, j = lane & 1;
+  int64_t t = (int64_t)blockIdx.x * kWarps + warp;
+  // pipeline: the words of step t are staged one step ahead, the tile offsets
+  // loaded two steps ahead
+  int32_t h_nxt = load_head<NT>(p.tile_off, t + step, n_tiles, lane);
+  Range rg_cur = range_of<NT>(load_head<NT>(p.tile_off, t, n_tiles, lane));
+  // bit s of pend: a copy into stage s is in flight; bit s of phase: the
+  // parity of that stage's mbarrier for its next completion
+  unsigned pend = stage_tile<kCap>(p.words, rg_cur, stage0, &bar[0], lane) ? 1u : 0u;
+  unsigned phase = 0u;
+  int b = 0;
+  for (; t < n_steps; t += step) {
+    const Range rg_nxt = range_of<NT>(h_nxt);
+    if (stage_tile<kCap>(p.words, rg_nxt, stage0 + (b ^ 1) * STAGE, &bar[b ^ 1], lane)) pend |= 2u >> b;
+    h_nxt = load_head<NT>(p.tile_off, t + 2 * step, n_tiles, lane);
+    if (pend & (1u << b)) {
+      const bool ok = edg::bulk::wait_bounded(&bar[b], (phase >> b) & 1u, s_err);
+      if (!__all_sync(0xffffffffu, ok)) break;  // warp-uniform
+      pend &= ~(1u << b);
+      phase ^= 1u << b;
+    }
+    A acc[NT][NV];
+#pragma unroll
+    for (int h = 0; h < NT; ++h)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[h][v] = (A)0;
+    const uint32_t* const st = stage0 + b * STAGE;
+    const int wa = rg_cur.wa, wb = rg_cur.wb;
+    if (wa + wb <= kCap) {
+      gather_tile<T, A, NV, XS, true>(st, nullptr, 0, wa, s, j, tab, p.colbits, cmask, p.x, acc[0]);
+      if constexpr (NT == 2)
+        gather_tile<T, A, NV, XS, true>(st + kTileRows * wa, nullptr, 0, wb, s, j, tab, p.colbits, cmask, p.x, acc[1]);
+    } else {
+      const uint32_t* const src = p.words + rg_cur.e0;
+      gather_tile<T, A, NV, XS, false>(st, src, kCap, wa, s, j, tab, p.colbits, cmask, p.x, acc[0]);
+      if constexpr (NT == 2)
+        gather_tile<T, A, NV, XS, false>(st + kTileRows * wa, src + kTileRows * wa, kCap - wa, wb, s, j, tab,
+                                         p.colbits, cmask, p.x, acc[1]);
+    }
+    // lane j of a row's two lanes finishes the row of tile j
+    double tot[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const A other = __shfl_xor_sync(0xffffffffu, j == 0 ? acc[NT - 1][v] : acc[0][v], 1);
+      tot[v] = (double)(j == 0 ? acc[0][v] : acc[NT - 1][v]) + (double)other;
+    }
+    const int64_t r = (int64_t)NT * kTileRows * t + kTileRows * j + s;
+    if (r < p.n && j < NT) {
+      T xr[NV];
+      XRow<T, NV, XS>::ld(p.x, r, xr);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double d = (double)__ldg(p.diag_shared ? p.diag + r : p.diag + r * NV + v);
+        tot[v] = fma(d, (double)xr[v], tot[v]);
+        p.y[p.y_plane > 0 ? v * p.y_plane + r : r * NV + v] = tot[v];
+      }
+      epi.row(r, xr, tot);
+    }
+    __syncwarp();  // this stage is refilled by the next iteration
+    rg_cur = rg_nxt;
+    b ^= 1;
+  }
+  if (pend != 0u) {  // only after a wait ran out
+    if (lane == 0 && p.err != nullptr) atomicExch(p.err, EDG_ERR_TIMEOUT);
+    // copies still in flight land before the CTA leaves (bounded again)
+    for (int s2 = 0; s2 < 2; ++s2)
+      if (pend & (1u << s2)) {
+        const uint64_t t0 = edg::bulk::now_ns();
+        while (!edg::bulk::mbar_try_wait(&bar[s2], (phase >> s2) & 1u))
+          if (edg::bulk::now_ns() - t0 > 1000000000ull) break;
+      }
+  }
+}
+
 // y[v * y_plane + r] (f64; y[r * NV + v] when y_plane is 0) = sum over the
 // row's entries of table[idx] x[col][v] + diag[r][v] x[r][v] (diag[r] for
 // every v when diag_shared: a complex vector as NV = 2 real parts of one
@@ -397,103 +513,31 @@ struct KrylovEpilogue {
 // kernel's order.  A stage wait that runs out (1 s) sets *err (if given) and
 // ends the warp's work.
 template <typename T, int NV, int XS, typename Epi>
-__global__ void __launch_bounds__(kWarps * 32, 4)
-    packed_spmv_k(int64_t n, const int32_t* __restrict__ tile_off, const uint32_t* __restrict__ words,
-                  const T* __restrict__ table, int count, int colbits, const T* __restrict__ diag,
-                  const T* __restrict__ x, double* __restrict__ y, int64_t y_plane, int diag_shared,
-                  const int* __restrict__ skip, int* __restrict__ err, Epi epi) {
-  using A = T;  // lane accumulator: f32 lanes for the f32 phase, f64 otherwise
+__global__ void __launch_bounds__(kWarps * 32, 4) packed_spmv_k(const __grid_constant__ Product<T> p, Epi epi) {
   constexpr int NT = tiles_of<T, XS>(), kStageWords = stage_words(NT);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_err;
-  if (skip != nullptr && *skip) return;
+  if (p.skip != nullptr && *p.skip) return;
   uint32_t* stage_all = reinterpret_cast<uint32_t*>(smem_raw);  // [kWarps][2][kStageWords]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + sizeof(uint32_t) * kWarps * 2 * kStageWords);
   T* tab = reinterpret_cast<T*>(smem_raw + sizeof(uint32_t) * kWarps * 2 * kStageWords + sizeof(uint64_t) * kWarps * 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint64_t* const bar = bars + 2 * warp;
+  const int64_t n_tiles = (p.n + kTileRows - 1) / kTileRows;
+  const int64_t total = NT == 2 ? (int64_t)__ldg(p.tile_off + n_tiles) : 0;
   if (threadIdx.x == 0) s_err = 0;
   if (lane == 0) {
     edg::bulk::mbar_init(&bar[0], 1);
     edg::bulk::mbar_init(&bar[1], 1);
     edg::bulk::fence_mbar_init();
   }
-  for (int i = threadIdx.x; i < count; i += blockDim.x) tab[i] = table[i];
+  for (int i = threadIdx.x; i < p.count; i += blockDim.x) tab[i] = p.table[i];
   __syncthreads();
-  uint32_t* const stage0 = stage_all + warp * 2 * kStageWords;  // two stages of kStageWords
-  const uint32_t cmask = (1u << colbits) - 1u;
-  const int64_t n_tiles = (n + kTileRows - 1) / kTileRows, n_steps = (n_tiles + NT - 1) / NT;
-  const int64_t step = (int64_t)gridDim.x * kWarps;
-  const int s = lane >> 1, j = lane & 1;
-  int64_t t = (int64_t)blockIdx.x * kWarps + warp;
-  // pipeline: the words of step t are staged one step ahead, the tile offsets
-  // loaded two steps ahead
-  int32_t h_nxt = load_head<NT>(tile_off, t + step, n_tiles, lane);
-  Range rg_cur = range_of<NT>(load_head<NT>(tile_off, t, n_tiles, lane));
-  // bit s of pend: a copy into stage s is in flight; bit s of phase: the
-  // parity of that stage's mbarrier for its next completion
-  unsigned pend = stage_tile(words, rg_cur, stage0, &bar[0], lane) ? 1u : 0u;
-  unsigned phase = 0u;
-  int b = 0;
-  for (; t < n_steps; t += step) {
-    const Range rg_nxt = range_of<NT>(h_nxt);
-    if (stage_tile(words, rg_nxt, stage0 + (b ^ 1) * kStageWords, &bar[b ^ 1], lane)) pend |= 2u >> b;
-    h_nxt = load_head<NT>(tile_off, t + 2 * step, n_tiles, lane);
-    if (pend & (1u << b)) {
-      const bool ok = edg::bulk::wait_bounded(&bar[b], (phase >> b) & 1u, &s_err);
-      if (!__all_sync(0xffffffffu, ok)) break;  // warp-uniform
-      pend &= ~(1u << b);
-      phase ^= 1u << b;
-    }
-    A acc[NT][NV];
-#pragma unroll
-    for (int h = 0; h < NT; ++h)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[h][v] = (A)0;
-    const uint32_t* const src = rg_cur.fits ? stage0 + b * kStageWords : words + rg_cur.e0;
-    if (rg_cur.fits)
-      gather_tile<T, A, NV, XS>(src, rg_cur.wa, s, j, tab, colbits, cmask, x, acc[0], true);
-    else
-      gather_tile<T, A, NV, XS>(src, rg_cur.wa, s, j, tab, colbits, cmask, x, acc[0], false);
-    if constexpr (NT == 2) {
-      if (rg_cur.fits)
-        gather_tile<T, A, NV, XS>(src + kTileRows * rg_cur.wa, rg_cur.wb, s, j, tab, colbits, cmask, x, acc[1], true);
-      else
-        gather_tile<T, A, NV, XS>(src + kTileRows * rg_cur.wa, rg_cur.wb, s, j, tab, colbits, cmask, x, acc[1], false);
-    }
-    // lane j of a row's two lanes finishes the row of tile j
-    double tot[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const A other = __shfl_xor_sync(0xffffffffu, j == 0 ? acc[NT - 1][v] : acc[0][v], 1);
-      tot[v] = (double)(j == 0 ? acc[0][v] : acc[NT - 1][v]) + (double)other;
-    }
-    const int64_t r = (int64_t)NT * kTileRows * t + kTileRows * j + s;
-    if (r < n && j < NT) {
-      T xr[NV];
-      XRow<T, NV, XS>::ld(x, r, xr);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const double d = (double)__ldg(diag_shared ? diag + r : diag + r * NV + v);
-        tot[v] = fma(d, (double)xr[v], tot[v]);
-        y[y_plane > 0 ? v * y_plane + r : r * NV + v] = tot[v];
-      }
-      epi.row(r, xr, tot);
-    }
-    __syncwarp();  // this stage is refilled by the next iteration
-    rg_cur = rg_nxt;
-    b ^= 1;
-  }
-  if (pend != 0u) {  // only after a wait ran out
-    if (lane == 0 && err != nullptr) atomicExch(err, EDG_ERR_TIMEOUT);
-    // copies still in flight land before the CTA leaves (bounded again)
-    for (int s2 = 0; s2 < 2; ++s2)
-      if (pend & (1u << s2)) {
-        const uint64_t t0 = edg::bulk::now_ns();
-        while (!edg::bulk::mbar_try_wait(&bar[s2], (phase >> s2) & 1u))
-          if (edg::bulk::now_ns() - t0 > 1000000000ull) break;
-      }
-  }
+  uint32_t* const stage0 = stage_all + warp * 2 * kStageWords;
+  if (NT == 2 && 2 * total <= n_tiles * (kTileRows * Epi::kPairMax))
+    warp_steps<T, NV, XS, NT, kStageWords>(p, tab, stage0, bar, &s_err, epi);
+  else
+    warp_steps<T, NV, XS, 1, kStageWords>(p, tab, stage0, bar, &s_err, epi);
   epi.finish();
 }
 
@@ -502,10 +546,10 @@ size_t packed_smem(int count) {
   return sizeof(uint32_t) * kWarps * 2 * stage_words(tiles_of<T, XS>()) + sizeof(uint64_t) * kWarps * 2 + sizeof(T) * (size_t)count;
 }
 
-// One wave: four resident CTAs an SM, each warp a step at a time.
-unsigned packed_grid(int64_t n, int tiles) {
-  const int64_t steps = (n + (int64_t)tiles * kTileRows - 1) / ((int64_t)tiles * kTileRows);
-  const int64_t need = (steps + kWarps - 1) / kWarps;
+// One wave: four resident CTAs an SM, each warp a step (of one tile or a pair)
+// at a time.
+unsigned packed_grid(int64_t n) {
+  const int64_t tiles = (n + kTileRows - 1) / kTileRows, need = (tiles + kWarps - 1) / kWarps;
   return (unsigned)(need < (int64_t)edg::kSmCount * 4 ? need : (int64_t)edg::kSmCount * 4);
 }
 
@@ -538,15 +582,14 @@ int launch_packed_spmv(int nvec, int x_stride, int64_t n, const int32_t* tile_of
                        const T* table, int count, int colbits, const T* diag, const T* x, double* y, int64_t y_plane,
                        const int* skip, int* err, cudaStream_t s, int diag_shared) {
   cudaError_t e = cudaSuccess;
+  const Product<T> p{n, tile_off, words, table, diag, x, y, y_plane, count, colbits, diag_shared, skip, err};
 #define EDG_PACKED(NV, XS)                                                                                          \
   do {                                                                                                              \
     auto kern = packed_spmv_k<T, NV, XS, NoEpilogue>;                                                              \
     const size_t smem = packed_smem<T, XS>(count);                                                                 \
     e = edg::allow_smem(kern, packed_smem<T, XS>(EDG_PACK_MAX_VALUES));                                            \
     if (e == cudaSuccess)                                                                                           \
-      kern<<<packed_grid(n, tiles_of<T, XS>()), kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, \
-                                                                        diag, x, y, y_plane, diag_shared, skip,    \
-                                                                        err, NoEpilogue{});                         \
+      kern<<<packed_grid(n), kWarps * 32, smem, s>>>(p, NoEpilogue{});                                              \
   } while (0)
   switch (nvec) {
     case 1: EDG_PACKED(1, 1); break;
@@ -577,13 +620,14 @@ template <typename T>
 int launch_packed_krylov(int64_t n, const int32_t* tile_off, const uint32_t* words, const T* table, int count,
                          int colbits, const T* diag, const T* x, double* y, const KrylovStep& step, int* err,
                          cudaStream_t s) {
-  const unsigned grid = packed_grid(n, tiles_of<T, 2>());
+  const unsigned grid = packed_grid(n);
   const size_t smem = packed_smem<T, 2>(count);
   auto kern = packed_spmv_k<T, 2, 2, KrylovEpilogue>;
   cudaError_t e = edg::allow_smem(kern, packed_smem<T, 2>(EDG_PACK_MAX_VALUES));
   if (e == cudaSuccess)
-    kern<<<grid, kWarps * 32, smem, s>>>(n, tile_off, words, table, count, colbits, diag, x, y, 0, 1, nullptr, err,
-                                         KrylovEpilogue{step, {0.0, 0.0, 0.0, 0.0}});
+    kern<<<grid, kWarps * 32, smem, s>>>(
+        Product<T>{n, tile_off, words, table, diag, x, y, 0, count, colbits, 1, nullptr, err},
+        KrylovEpilogue{step, {0.0, 0.0, 0.0, 0.0}});
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? EDG_OK : cuda_status(e, "packed krylov product");
 }

@@ -377,7 +377,6 @@ class QMB_hamiltonian:
         """The sector matrix as a dense device array (``edg_csr_to_dense``), in
         the assembled (possibly real) form, or with the real form's phases put
         back: H = D H' D^dagger, the reference's basis."""
-
         n = self.shape[0]
         if n > self.DENSE_MAX:
             raise ValueError(f"dense matrices limited to {self.DENSE_MAX} states, the sector has {n}")

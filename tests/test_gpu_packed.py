@@ -330,3 +330,92 @@ def test_a_layout_the_tuner_rejects_is_released(used, monkeypatch):
     assert tune_matvec32(mat, 3, ctx=Context())[0] != "packed"
     gc.collect()
     assert len(made) == 1 and (made[0]() is not None) == used
+
+
+# widths of a pair of tiles around what a stage holds (38 entries a row of a
+# pair together or of one tile; 32 where single tiles are the rule)
+_PAIRS = [(38, 0), (19, 19), (19, 20), (20, 19), (38, 38), (38, 39), (39, 1), (32, 33), (1, 38), (0, 38), (0, 0),
+          (25, 30), (13, 14), (48, 2), (2, 48), (37, 2), (40, 44)]
+
+
+def _paired(dev, wide):
+    """Several steps a warp on one wave of CTAs (4,736 warps), an odd number of
+    tiles and a last tile of five rows; pairs of a mean width that is taken one
+    tile at a time (wide: 44 and more) or together."""
+    import torch
+
+    from edgpu.modeling.assembly import DeviceMatrix
+
+    n_tiles = 2 * 4736 * 3 + 1
+    n = 16 * (n_tiles - 1) + 5
+    rng = np.random.default_rng(17)
+    order = rng.integers(0, len(_PAIRS), n_tiles // 2 + 1)
+    pairs = np.array(_PAIRS)[order]
+    if not wide:
+        pairs[rng.random(len(pairs)) < 0.4] = 0
+    assert (pairs.sum(axis=1).mean() > 44) == wide and (wide or pairs.sum(axis=1).mean() < 38)
+    width = pairs.reshape(-1)[:n_tiles]
+    lens = np.floor(rng.random((n_tiles, 16)) * (width[:, None] + 1)).astype(np.int64)
+    lens[np.arange(n_tiles), rng.integers(0, 5, n_tiles)] = width  # the widest row (of the last tile's five too)
+    lens = lens.reshape(-1)[:n]
+    rowptr = np.concatenate([[0], np.cumsum(lens)])
+    rows = np.repeat(np.arange(n), lens)
+    k = np.arange(len(rows)) - rowptr[rows]
+    # distinct columns of a row, ascending from a start that leaves room
+    cols = (rows * 7919) % (n - 48 * 61) + 61 * k
+    pool = rng.standard_normal(7)
+    vals = pool[rng.integers(0, 7, len(rows))]
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)  # noqa: E731
+    mat = DeviceMatrix(n, t(rowptr), t(cols.astype(np.int32)), t(vals), t(rng.standard_normal(n)), None, False)
+    csr = torch.sparse_csr_tensor(mat.rowptr, t(cols), mat.vals, size=(n, n))
+    return mat, csr
+
+
+@pytest.mark.parametrize("wide", [False, True])
+def test_tiles_around_the_stage(wide):
+    import torch
+
+    from edgpu.solvers import PackedLayout
+
+    mat, csr = _paired("cuda", wide)
+    lay, n = PackedLayout.build(mat), mat.n
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for nvec in (1, 2, 3):
+        for dtype, tdt in ((0, torch.float64), (1, torch.float32)):
+            x = torch.randn((n, nvec), dtype=tdt, device="cuda", generator=g)
+            diag = torch.randn((n, nvec), dtype=tdt, device="cuda", generator=g)
+            y = _packed(lay, dtype, diag, x, nvec, nvec)
+            if dtype == 0:
+                assert torch.equal(y, _csr_planar(mat, 0, mat.vals, diag, x, nvec, nvec))
+                continue
+            a = torch.sparse_csr_tensor(csr.crow_indices(), csr.col_indices(), mat.vals.to(tdt).double(), size=(n, n))
+            xd, dd = x.double(), diag.double()
+            ref = a @ xd + dd * xd
+            mag = torch.sparse_csr_tensor(csr.crow_indices(), csr.col_indices(), a.values().abs(), size=(n, n))
+            scale = mag @ xd.abs() + (dd * xd).abs()
+            # a lane's 24 products in f32, one rounding each; the rest in f64
+            assert bool(((y.T - ref).abs() <= 25 * 2.0**-24 * scale + 1e-300).all())
+
+
+@pytest.mark.parametrize("precision,tol", [("c128", 1e-12), ("c64", 5e-6)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_krylov_dots_on_tiles_around_the_stage(wide, precision, tol):
+    """The dots of the packed product's epilogue over the same tiles: a step of
+    two products against the CSR passes."""
+    import torch
+
+    from edgpu.dynamics import KrylovEvolver
+
+    mat, _ = _paired("cuda", wide)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    psi = torch.randn(mat.n, dtype=torch.complex128, device="cuda", generator=g)
+    out = []
+    for matvec in ("auto", "csr"):
+        ev = KrylovEvolver(mat, m=2, precision=precision, reorth_passes=0, matvec=matvec)
+        assert bool(ev.p.pk_words) == (matvec == "auto")
+        x = psi.to(ev.vdtype).clone()
+        err = ev.step(x, 0.02, want_error=True)
+        ev.check_status()
+        out.append((x.to(torch.complex128), err))
+    assert float(torch.linalg.vector_norm(out[0][0] - out[1][0]) / torch.linalg.vector_norm(psi)) < tol
+    assert abs(out[0][1] - out[1][1]) < tol * max(1.0, out[1][1])
