@@ -104,4 +104,11 @@ inline int64_t coop_ctas(int64_t n, int n_sm) {
   return g < most ? g : most;
 }
 
+// Whether a small cooperative solve's product suits its few threads (512 an SM
+// against 1,024 to 2,048 of the passes): at most `total` entries, and `per_cta`
+// a CTA.  See the callers' figures.
+inline bool coop_entries(int64_t nnz, int64_t n, int64_t total, int64_t per_cta) {
+  return nnz <= total && nnz <= per_cta * coop_ctas(n, kSmCount);
+}
+
 }  // namespace edg

@@ -737,13 +737,21 @@ KLayout klayout(const edg_krylov_problem* p) {
   return L;
 }
 
-// Whether a step may run as krylov_coop_k: few enough rows, the CSR arrays at
-// hand, which that kernel reads whatever layout is passed beside them (a
-// problem may come with its packed layout alone), and a way to report a grid-wide
-// wait that ran out (the problem's status word, or a result the call waits for).
+// Whether a step may run as krylov_coop_k: few enough rows and entries, the CSR
+// arrays at hand, which that kernel reads whatever layout is passed beside them
+// (a problem may come with its packed layout alone), and a way to report a
+// grid-wide wait that ran out (the problem's status word, or a result the call
+// waits for).  The lines on the entries lie where columns are random, the worst
+// case for its gathers (m = 30, passes / one launch): complex128 100,000 rows
+// 0.763 / 0.743 ms at 2.0M entries and 0.887 / 1.264 at 3.0M, complex64 60,000
+// rows 0.982 / 0.903 at 3.0M and 1.063 / 1.404 at 4.0M; on a few CTAs (complex
+// matrix, 1,000 rows) 0.744 / 0.654 at 27,000 a CTA and 0.819 / 0.945 at 49,000.
+// With neighbouring columns the one launch still gains there (150,000 rows, 3.0M
+// entries: 1.13 times) and loses past 4M.
 bool one_launch(const edg_krylov_problem* p, bool reports) {
   const bool csr = p->cols != nullptr && p->vals != nullptr, diagonal = p->nnz == 0 && p->pk_words == nullptr;
-  return reports && p->n_rows <= kCoopMaxRows && (csr || diagonal);
+  return reports && p->n_rows <= kCoopMaxRows && (csr || diagonal) &&
+         edg::coop_entries(p->nnz, p->n_rows, p->vec_dtype == 2 ? 2000000 : 3000000, 27000);
 }
 
 template <typename T, typename SV>

@@ -1382,6 +1382,24 @@ __global__ void zero_k(double* p, int n) {
   if (t < n) p[t] = 0.0;
 }
 
+// Whether a problem may be solved by lanczos_coop_k: a single one that is not
+// instrumented, few enough rows and entries, and the CSR arrays at hand, which
+// that kernel reads (a problem may come with another layout alone).  The lines
+// on the entries lie where columns are random, the worst case for its gathers
+// (passes / one launch): f64 100,000 rows 1.08 / 1.08 ms at 6.0M entries, 20,000
+// rows 0.755 / 0.728 at 4.0M and 0.832 / 0.916 at 6.0M, 2,000 rows 0.441 / 0.422
+// at 98,000 a CTA; mixed precision 150,000 rows 0.819 / 0.765 at 3.0M and 0.937 /
+// 0.948 at 3.9M, 2,000 rows 0.625 / 0.573 at 55,000 a CTA and 0.665 / 0.731 at
+// 98,000.
+bool one_launch(const edg_lanczos_problem* p) {
+  const bool csr = (p->cols != nullptr && p->vals != nullptr) ||
+                   (p->nnz == 0 && p->pk_words == nullptr && p->sell_entries == nullptr);
+  const bool f64 = p->dtype == 0;
+  return p->nvec == 1 && p->stats == nullptr && csr &&
+         ((p->n_rows + 3) & ~int64_t(3)) <= (int64_t)kCoopRows * edg::kSmCount &&
+         edg::coop_entries(p->nnz, p->n_rows, f64 ? 4500000 : 3500000, f64 ? 100000 : 60000);
+}
+
 template <typename T, int NV>
 int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* evecs, int32_t* iters_out,
                 double* resid_out, cudaStream_t s) {
@@ -1429,10 +1447,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
   // small sectors: the whole solve in one cooperative launch (the instrumented
   // path times the passes one by one)
   bool coop_done = false;
-  // (the kernel reads the CSR arrays: a problem may come with another layout alone)
-  const bool csr = (p->cols != nullptr && p->vals != nullptr) ||
-                   (p->nnz == 0 && p->pk_words == nullptr && p->sell_entries == nullptr);
-  if (NV == 1 && p->stats == nullptr && csr && n_pad <= (int64_t)kCoopRows * edg::kSmCount) {
+  if (NV == 1 && one_launch(p)) {
     int dev = 0, n_sm = 0, coop = 0, occ = 0;
     auto kern = lanczos_coop_k<T>;
     e = cudaGetDevice(&dev);
@@ -1761,6 +1776,11 @@ int check_problem(const edg_lanczos_problem* p) {
 }  // namespace
 
 extern "C" int64_t edg_lanczos_small_rows(void) { return (int64_t)kCoopRows * edg::kSmCount / 4 * 4; }
+
+extern "C" int edg_lanczos_one_launch(const edg_lanczos_problem* p) {
+  if (check_problem(p)) return -1;
+  return one_launch(p) ? 1 : 0;
+}
 
 extern "C" int64_t edg_lanczos_workspace_bytes(const edg_lanczos_problem* p) {
   if (check_problem(p)) return -1;

@@ -320,6 +320,7 @@ _SIGS = {
     "edg_spmv_packed": (I32, [I32, I64, I32, P, P, P, I32, I32, P, P, I32, P, I64, P, P]),
     "edg_spmv_group": (I32, [I32, I64, I64, P, P, P, P, I32, P, P, I32, P]),
     "edg_lanczos_small_rows": (I64, []),
+    "edg_lanczos_one_launch": (I32, [C.POINTER(LanczosProblem)]),
     "edg_lanczos_workspace_bytes": (I64, [C.POINTER(LanczosProblem)]),
     "edg_lanczos": (I32, [C.POINTER(LanczosProblem), P, I64, P, P, P, P, P]),
     "edg_tridiag_lowest": (I32, [P, P, I32, I32, P, P, P, P]),

@@ -442,16 +442,19 @@ def lanczos(mat, k=1, tol=1e-12, max_iter=400, check_every=5, seed=1234, v0=None
     """f64 Lanczos on a real DeviceMatrix; returns (evals[k], evecs (n, k) device)."""
     if mat.is_complex:
         raise NotImplementedError("complex Hermitian Lanczos: assemble the real form of the model")
-    g = group or (tune_spmv_group(mat, 1, 0, vals=mat.vals) if tune and not _one_launch(mat, 1, stats) else 0)
+    g = group or (tune_spmv_group(mat, 1, 0, vals=mat.vals) if tune and not _one_launch(mat, 1, stats, 0) else 0)
     r = run_lanczos(0, mat.n, mat.nnz, mat.rowptr, mat.cols, mat.vals, mat.diag, nvec=1, k=k, max_iter=max_iter,
                     tol=tol, check_every=check_every, seed=seed, v0=v0, stats=stats, group=g)
     return r.evals[0], r.evecs[:, :, 0].T.contiguous(), r
 
 
-def _one_launch(mat, nvec, stats):
+def _one_launch(mat, nvec, stats, dtype):
     """Whether ``edg_lanczos`` solves this problem in one cooperative launch,
     which reads the CSR arrays and has no matvec to tune."""
-    return nvec == 1 and stats is None and mat.n <= lib.edg_lanczos_small_rows()
+    if nvec != 1 or stats is not None:
+        return False
+    p = _problem(dtype, mat.n, mat.nnz, mat.rowptr, mat.cols, mat.vals, mat.diag, 1, 1, 1, 1.0, 1, 0, None)
+    return lib.edg_lanczos_one_launch(ctypes.byref(p)) == 1
 
 
 def stack_diagonals(diags, dtype):
@@ -488,7 +491,8 @@ def lanczos_mixed(mat, diags=None, k=1, tol32=1e-4, tol=1e-12, max_iter=400, ref
     if diag64 is None:
         diag64 = stack_diagonals(diags, torch.float64)
     # (the one-launch solver has no layout to choose)
-    tune = tune and not _one_launch(mat, nvec, stats32 if stats32 is not None else stats64)
+    tune64 = tune and not _one_launch(mat, nvec, stats64, 0)
+    tune = tune and not _one_launch(mat, nvec, stats32, 1)
     if sell is None and packed is None and tune and not group32:
         fmt, param = tune_matvec32(mat, nvec, vals32)
         if fmt == "sell":
@@ -504,7 +508,7 @@ def lanczos_mixed(mat, diags=None, k=1, tol32=1e-4, tol=1e-12, max_iter=400, ref
         # problem reads the CSR arrays)
         vals32 = mat.vals.to(torch.float32)
     g32 = group32 or (tune_spmv_group(mat, nvec, 1, vals=vals32) if tune and pk is None else 0)
-    g64 = group64 or (tune_spmv_group(mat, nvec, 0, vals=mat.vals) if tune and pk is None else 0)
+    g64 = group64 or (tune_spmv_group(mat, nvec, 0, vals=mat.vals) if tune64 and pk is None else 0)
     r32 = run_lanczos(1, mat.n, mat.nnz, mat.rowptr, mat.cols, vals32, diag32, nvec=nvec, k=k, max_iter=max_iter,
                       tol=tol32, check_every=check_every, seed=seed, stats=stats32, group=g32, sell=lay,
                       window=window32, packed=pk)

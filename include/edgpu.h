@@ -424,7 +424,7 @@ int edg_convert(int32_t dtype_in, const void* in, int32_t dtype_out, void* out,
 /* the device writes to host_progress; no stream synchronisation happens    */
 /* inside the step loop.  With stats set, the steps are launched one by one */
 /* with CUDA events around each phase instead.  A single small problem      */
-/* (edg_lanczos_small_rows) is one cooperative launch.                       */
+/* (edg_lanczos_one_launch) is one cooperative launch.                       */
 /* A step that reorthogonalises against at most 8 vectors (reorth_window of  */
 /* 1..7, or max_iter <= 8) does it in one cooperative launch (dots, a grid    */
 /* barrier with a 1 s limit, update); the device must support cooperative   */
@@ -470,11 +470,13 @@ typedef struct {
   int32_t pk_colbits;          /* pk_words is not NULL                      */
 } edg_lanczos_problem;
 
-/* Bytes of device workspace edg_lanczos needs. */
-/* Rows up to which a single problem (nvec 1, no stats, CSR arrays given) is solved
- * in one cooperative launch, which reads the CSR arrays whatever layout is
- * passed beside them. */
+/* Rows up to which a single problem (nvec 1, no stats, CSR arrays given) with
+ * few entries is solved in one cooperative launch, which reads the CSR arrays
+ * whatever layout is passed beside them; and whether a problem is (1; 0 when it
+ * is a launch per pass, -1 for a bad problem), on a device with such launches. */
 int64_t edg_lanczos_small_rows(void);
+int edg_lanczos_one_launch(const edg_lanczos_problem* p);
+/* Bytes of device workspace edg_lanczos needs. */
 int64_t edg_lanczos_workspace_bytes(const edg_lanczos_problem* p);
 /* Runs to convergence (synchronizes every check_every steps).  Outputs:
  * evals [nvec][k] (f64), evecs [k][n_rows][nvec] in the problem dtype (may be
@@ -646,8 +648,8 @@ typedef struct {
 } edg_krylov_problem;
 
 int64_t edg_krylov_workspace_bytes(const edg_krylov_problem* p);
-/* 1 when a step of this problem is one cooperative launch (few rows, CSR
- * arrays and a status word given; it reads those arrays and the diagonal, not
+/* 1 when a step of this problem is one cooperative launch (few rows and
+ * entries, CSR arrays and a status word given; it reads those arrays and the diagonal, not
  * the packed layout), on a device that has such launches; 0 when it is a launch
  * per pass; -1 for a bad problem. */
 int edg_krylov_one_launch(const edg_krylov_problem* p);

@@ -282,3 +282,44 @@ def test_krylov_status_names_both_waits():
     ev.status = Status()
     with pytest.raises(_lib.EdgError, match="grid-wide wait"):
         ev.check_status()
+
+
+@pytest.mark.parametrize("vec,total", [(2, 2_000_000), (3, 3_000_000)])
+def test_krylov_one_launch_form_is_for_few_entries(vec, total):
+    """The lines of the form on the entries: in all, and a CTA (one up to 256
+    rows, then one for every 128)."""
+    from edgpu import _lib
+
+    p = _lib.KrylovProblem()
+    p.vec_dtype, p.mat_dtype, p.m = vec, vec - 2, 30
+    p.rowptr = p.diag = p.cols = p.vals = p.status = 16
+    for n, most in ((1, 27000), (256, 27000), (257, 3 * 27000), (1000, 8 * 27000), (100000, total),
+                    (1024 * 148, total)):
+        p.n_rows, p.nnz = n, most
+        assert _lib.lib.edg_krylov_one_launch(ctypes.byref(p)) == 1
+        p.nnz = most + 1
+        assert _lib.lib.edg_krylov_one_launch(ctypes.byref(p)) == 0
+
+
+@pytest.mark.parametrize("dtype,total,per_cta", [(0, 4_500_000, 100_000), (1, 3_500_000, 60_000)])
+def test_lanczos_one_launch_form_is_for_few_rows_and_entries(dtype, total, per_cta):
+    from edgpu import _lib
+
+    one = lambda: _lib.lib.edg_lanczos_one_launch(ctypes.byref(p))  # noqa: E731
+    p = _lib.LanczosProblem()
+    p.dtype, p.nvec, p.k, p.max_iter, p.tol, p.check_every = dtype, 1, 1, 50, 1e-8, 5
+    p.rowptr = p.diag = p.cols = p.vals = 16
+    rows = _lib.lib.edg_lanczos_small_rows()
+    for n, most in ((1, per_cta), (256, per_cta), (257, 3 * per_cta), (100000, total), (rows, total)):
+        p.n_rows, p.nnz = n, most
+        assert one() == 1
+        p.nnz = most + 1
+        assert one() == 0
+    p.n_rows, p.nnz = rows + 1, 10
+    assert one() == 0
+    p.n_rows = 1000
+    assert one() == 1
+    p.nvec = 2
+    assert one() == 0
+    p.nvec, p.k = 1, 99
+    assert one() == -1

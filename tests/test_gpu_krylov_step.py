@@ -132,3 +132,36 @@ def test_step_with_and_without_a_status_word(n, precision, status, want_error):
     assert e is None or 0.0 <= e < 1e-10
     err = float(torch.linalg.vector_norm(got.to(torch.complex128) - want) / torch.linalg.vector_norm(want))
     assert err < (5e-6 if precision == "c64" else 1e-12), err
+
+
+@pytest.mark.parametrize("per_row", [60, 80])
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+def test_both_sides_of_the_line_on_the_entries(per_row, precision):
+    """At 700 rows a step of up to 162,000 entries is one launch."""
+    import ctypes
+
+    import torch
+
+    from edgpu._lib import lib
+    from edgpu.dynamics import KrylovEvolver
+    from edgpu.modeling.assembly import DeviceMatrix
+
+    n, rng = 700, np.random.default_rng(per_row)
+    h = np.triu(np.where(rng.random((n, n)) < 3.6 * per_row / n, rng.choice([0.5, -0.25, 0.125], (n, n)), 0.0), 1)
+    h = h + h.T
+    r, c = np.nonzero(h)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    d = rng.uniform(-2, 2, n)
+    mat = DeviceMatrix(n, up(np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))])), up(c.astype(np.int32)),
+                       up(h[r, c]), up(d), None, False)
+    ev = KrylovEvolver(mat, m=60, precision=precision, matvec="csr")
+    assert lib.edg_krylov_one_launch(ctypes.byref(ev.p)) == (len(r) <= 6 * 27000) == (per_row == 60)
+    psi = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    e, u = np.linalg.eigh(h + np.diag(d))
+    dt = 10.0 / np.abs(e).max()
+    want = u @ (np.exp(-1j * dt * e) * (u.T @ psi))
+    got = up(psi).to(ev.vdtype)
+    ev.step(got, dt)
+    ev.check_status()
+    err = np.linalg.norm(got.cpu().numpy() - want) / np.linalg.norm(want)
+    assert err < (5e-6 if precision == "c64" else 1e-12), err
