@@ -20,7 +20,8 @@
 //
 // When both operators are diagonal and real (densities, Casimirs: the usual
 // case) corr = sum_r |psi_r|^2 a(r) b(r)^T is a contraction over the rows, and
-// up to 32 sites it runs on the f64 tensor instruction (twobody_mma_k); the
+// up to 32 sites it runs on the f64 tensor instruction (twobody_mma_k) where the
+// sector has enough rows for one more launch; the
 // transition-table kernel then returns at once, and the other way round.
 #include "digits.cuh"
 #include "lookup.cuh"
@@ -307,6 +308,11 @@ __global__ void __launch_bounds__(kThreads, 3) twobody_k(const Args a) {
 // Only the blocks that hold a listed pair are multiplied.
 // ---------------------------------------------------------------------------
 constexpr int kMmaTableCap = 32 * 1024;
+// Rows from which it runs: below, the launch more costs what the rows save (a
+// call at 8,953 rows of SU(2) L = 10 88 us without it, 94 with; 70,755 rows of
+// QED L = 20 136 and 139, 73,789 of SU(2) L = 12 104 and 101, 616,227 of L = 14
+// 163 and 123, 745,889 of QED L = 24 462 and 217).
+constexpr int64_t kMmaRows = 65536;
 __host__ __device__ inline int mma_pitch(int nb) { return 16 * nb + 4; }
 template <int NB>
 struct MmaSmem {
@@ -522,7 +528,7 @@ extern "C" int edg_twobody_expval(const edg_lookup_table* sector, const uint64_t
   const int64_t smem = layout(n_sites, dmax, a.tables_in_smem, a.diag_in_smem).total;
   // real diagonal operators: the tensor kernel's limits, and the same limit as
   // the real diagonal table of the other kernel, which decides it skips them
-  a.mma = a.diag_in_smem && mma_fits(n_sites, dmax);
+  a.mma = a.diag_in_smem && mma_fits(n_sites, dmax) && sector->n >= kMmaRows;
   if (a.mma) {
     switch (psi_dtype) {
       case 0: e = launch_mma_nb<0>(a, stream); break;

@@ -70,3 +70,29 @@ def test_two_body_correlators(n_sites, n, dtype, subset):
     for i, j in pairs or [(i, j) for i in range(n_sites) for j in range(i + 1, n_sites)]:
         ref[i, j] = ref[j, i] = full[i, j]
     assert np.max(np.abs(got - ref)) < 1e-12
+
+
+@pytest.mark.parametrize("n_sites", [16, 17, 24, 25, 32, 33])
+@pytest.mark.parametrize("n", [65535, 65536, 70001])
+@pytest.mark.parametrize("dtype", ["float64", "float32", "complex128", "complex64"])
+def test_two_body_correlators_on_both_sides_of_the_row_line(n_sites, n, dtype):
+    """Sectors just below and above the rows from which real diagonal operators
+    go to the tensor instruction, with a pair listed either way round."""
+    from edgpu.models.quantum_model import twobody_corr_device
+    from edgpu.symmetries import Sector
+
+    sec, cfg, dims, rng = _sector(n_sites, 100000, 300 * n_sites, d_hi=3)
+    assert len(cfg) >= n
+    sec, cfg = Sector(sec.keys[:n].clone(), dims), cfg[:n]
+    a, b = _operator(n_sites, dims, rng), _operator(n_sites, dims, rng)
+    psi, p = _state(n, dtype, rng)
+    pairs = [(i, j) for i in range(n_sites) for j in range(i + 1, n_sites) if (i, j) != (1, n_sites - 1)]
+    pairs.append((n_sites - 1, 1))
+    got = twobody_corr_device(sec, a, b, psi, pairs).cpu().numpy()
+    va = np.stack([np.real(a[s, cfg[:, s], cfg[:, s]]) for s in range(n_sites)])
+    vb = np.stack([np.real(b[s, cfg[:, s], cfg[:, s]]) for s in range(n_sites)])
+    full = (va * p) @ vb.T
+    ref = np.zeros((n_sites, n_sites))
+    for i, j in pairs:
+        ref[i, j] = ref[j, i] = full[i, j]
+    assert np.max(np.abs(got - ref)) < 1e-12

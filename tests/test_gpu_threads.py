@@ -100,7 +100,7 @@ def _twobody(large):
     from edgpu._lib import lib, ptr
 
     n_sites, dmax = 26, 32 if large else 2
-    sec, rng = _sector(n_sites, 2, 256), np.random.default_rng(3)
+    sec, rng = _sector(n_sites, 2, 70000), np.random.default_rng(3)
     count = np.ones((2, n_sites, dmax))
     ket = np.zeros((2, n_sites, dmax, dmax))
     ket[..., 0] = np.arange(dmax)
