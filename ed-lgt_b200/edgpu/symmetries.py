@@ -435,9 +435,12 @@ class Sector:
 
 
 # Prefixes a level may have inside the one-launch enumeration (two buffers of
-# keys and sums: 100 MB for one-word keys and one global symmetry).  Larger
-# levels go through one pair of launches each, with a host read of their size.
+# keys and sums: 100 MB for one-word keys and one global symmetry; where the
+# device has no room for them, LEVELS_LOW prefixes, 6 MB).  Larger levels go
+# through one pair of launches each, with a host read of their size.  (A first
+# try of LEVELS_LOW everywhere made the set-up of the L = 14 ring 5 % slower.)
 LEVELS_CAP = 1 << 22
+LEVELS_LOW = 1 << 18
 
 
 def enumerate_sector(spec: SectorSpec, device=None) -> Sector:
@@ -452,9 +455,17 @@ def enumerate_sector(spec: SectorSpec, device=None) -> Sector:
     ng = spec.glob_val.shape[0]
     kshape = (lambda m: (m, 2)) if spec.key_words == 2 else (lambda m: (m,))
     space = int(np.prod(np.asarray(spec.loc_dims).astype(object)))
+
+    def buffers(n):
+        return ([torch.empty(kshape(n), dtype=torch.int64, device=device) for _ in range(2)],
+                [torch.empty(max(n * ng, 1), dtype=torch.int32, device=device) for _ in range(2)])
+
     cap = max(1, min(LEVELS_CAP, space, int(lib.edg_sector_levels_cap(C_ref(tables.struct)))))
-    keys = [torch.empty(kshape(cap), dtype=torch.int64, device=device) for _ in range(2)]
-    sums = [torch.empty(max(cap * ng, 1), dtype=torch.int32, device=device) for _ in range(2)]
+    try:
+        keys, sums = buffers(cap)
+    except torch.OutOfMemoryError:
+        cap = min(cap, LEVELS_LOW)
+        keys, sums = buffers(cap)
     work = torch.empty(int(lib.edg_sector_levels_work_elems()), dtype=torch.int64, device=device)
     check(lib.edg_sector_levels(C_ref(tables.struct), ptr(keys[0]), ptr(keys[1]), ptr(sums[0]), ptr(sums[1]), cap,
                                 ptr(work), st), "edg_sector_levels")

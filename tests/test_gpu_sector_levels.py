@@ -80,3 +80,26 @@ def test_levels_match_the_filtered_product_space(dims, frozen, glob, links, nbod
             assert np.array_equal(sec.configs, ref), cap
         assert sizes is None or sec.level_sizes == sizes
         sizes = sec.level_sizes
+
+
+def test_little_free_memory():
+    """With 60 MB left the enumeration works with fewer prefixes a level."""
+    import torch
+
+    from edgpu.symmetries import SectorSpec, enumerate_sector, get_symmetry_sector_generators
+
+    op = np.zeros((14, 4, 4))
+    op[:, np.arange(4), np.arange(4)] = np.arange(4)
+    op[6:, 1:, 1:] = 9.0  # the last sites keep their first state: 4^6 states pass
+    gens = get_symmetry_sector_generators([op], "global")
+    spec = SectorSpec(loc_dims=np.full(14, 4), glob_op_diags=gens, glob_sectors=[9], sym_type_flag="U")
+    want = enumerate_sector(spec)
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    room = torch.cuda.memory_reserved() + 60 * 2**20
+    torch.cuda.set_per_process_memory_fraction(room / total)
+    try:
+        got = enumerate_sector(spec)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert len(want) > 100 and torch.equal(got.keys, want.keys) and got.level_sizes == want.level_sizes
