@@ -994,11 +994,11 @@ struct CoopArgs {
   const int64_t* rowptr;
   const int32_t* cols;
   const T* vals;
-  const T* diag;  // [n][NV]
-  const T* v0;    // [n][NV] or NULL
-  T* V;           // [m_max + 1][NV][n_pad], written and read by this launch
-  double* partial;  // [2 (m_max + 1) NV][G]
-  double* npart;    // [2][NV][G]
+  const T* diag;
+  const T* v0;  // or NULL
+  T* V;         // [m_max + 1][n_pad], written and read by this launch
+  double* partial;  // [2 (m_max + 1)][G]
+  double* npart;    // [2][G]
   double *tri_eval, *tri_vec, *tri_work;
   DevState* st;
   unsigned* bar;
@@ -1011,33 +1011,31 @@ struct CoopArgs {
 
 // Bytes of the fixed part of a CTA's shared memory: u, w | row offsets | alpha,
 // beta | totals.
-__host__ __device__ inline int64_t coop_fixed(int rows, int nv, int m_max) {
-  return (int64_t)rows * nv * 16 + (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)) +
-         (int64_t)nv * (m_max + 2) * 16 + (int64_t)nv * 2 * (m_max + 2) * 8;
+__host__ __device__ inline int64_t coop_fixed(int rows, int m_max) {
+  return (int64_t)rows * 16 + (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)) + (int64_t)(m_max + 2) * 32;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs<T> A) {
-  constexpr int NV = 1;  // problems (batches of small ones have their own solver)
   // vectors and rows of a lane in flight in the dots (an f32 basis is mostly in
   // shared memory, where a second vector only costs: 73,789 rows mixed 0.85 ms
   // a solve against 1.34; f64 1.78 against 1.83 with one)
   constexpr int kVecs = sizeof(T) == 8 ? 2 : 1, kRowsAhead = sizeof(T) == 8 ? 8 : 12;
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double red[NV][kCoopWarps];
-  __shared__ double total_s[NV], coef[NV][4];
+  __shared__ double red[kCoopWarps];
+  __shared__ double total_s, coef[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = (int)gridDim.x, m_max = A.m_max;
   const int64_t r0 = A.n_pad * blockIdx.x / G, r1 = A.n_pad * (blockIdx.x + 1) / G;
   const int rows = (int)(r1 - r0);
-  double* const u = reinterpret_cast<double*>(sm);  // [NV][rows]
-  double* const w = u + (int64_t)rows * NV;
-  int32_t* const rp = reinterpret_cast<int32_t*>(w + (int64_t)rows * NV);
+  double* const u = reinterpret_cast<double*>(sm);  // [rows]
+  double* const w = u + rows;
+  int32_t* const rp = reinterpret_cast<int32_t*>(w + rows);
   double* const al = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(rp) +
-                                               (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)));  // [NV][m_max + 2]
-  double* const be = al + (int64_t)NV * (m_max + 2);
-  double* const tot = be + (int64_t)NV * (m_max + 2);  // [NV][2 (m_max + 2)]
-  int64_t off = coop_fixed(rows, NV, m_max);
+                                               (((int64_t)(rows + 1) * 4 + 15) & ~int64_t(15)));  // [m_max + 2]
+  double* const be = al + (m_max + 2);
+  double* const tot = be + (m_max + 2);  // [2 (m_max + 2)]
+  int64_t off = coop_fixed(rows, m_max);
   // the matrix rows (rows past n are empty)
   const int64_t e0 = A.rowptr[r0 < A.n ? r0 : A.n], ne = A.rowptr[r1 < A.n ? r1 : A.n] - e0;
   for (int r = tid; r <= rows; r += kCoopThreads) rp[r] = (int32_t)(A.rowptr[r0 + r < A.n ? r0 + r : A.n] - e0);
@@ -1054,76 +1052,64 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     cols = sc;
     off = (off + ne * (int64_t)(sizeof(T) + 4) + 15) & ~int64_t(15);
   }
-  T* own = A.V + r0;  // this CTA's rows of the basis: vector stride ld_i, problem stride ld_v
-  int64_t ld_v = A.n_pad;
-  const bool basis_here = off + (int64_t)rows * NV * (m_max + 1) * (int64_t)sizeof(T) <= kCoopSmem;
+  T* own = A.V + r0;  // this CTA's rows of the basis and their vector stride
+  int64_t ld_i = A.n_pad;
+  const bool basis_here = off + (int64_t)rows * (m_max + 1) * (int64_t)sizeof(T) <= kCoopSmem;
   if (basis_here) {
     own = reinterpret_cast<T*>(sm + off);
-    ld_v = rows;
+    ld_i = rows;
   }
-  const int64_t ld_i = ld_v * NV;
   edg::GridSync gs{A.bar, A.err};
   constexpr int kPer = (edg::kSmCount + 31) / 32;  // partials of a lane (one CTA an SM)
   unsigned waits = 0;
-  // totals over the grid of NV values per thread (in total_s); false when a
-  // wait ran out
-  auto grid_sum = [&](double (&a)[NV]) -> bool {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a[v] += __shfl_xor_sync(0xffffffffu, a[v], o);
-      if (lane == 0) red[v][warp] = a[v];
-    }
+  // total over the grid of a value per thread (in total_s); false when a wait
+  // ran out
+  auto grid_sum = [&](double a) -> bool {
+    a = edg::warp_sum(a);
+    if (lane == 0) red[warp] = a;
     __syncthreads();
-    double* part = A.npart + (int64_t)(waits & 1) * NV * G;
+    double* part = A.npart + (int64_t)(waits & 1) * G;
     ++waits;
-    if (tid < NV) {
+    if (tid == 0) {
       double t = 0.0;
-      for (int q = 0; q < kCoopWarps; ++q) t += red[tid][q];
-      part[(int64_t)tid * G + blockIdx.x] = t;
+      for (int q = 0; q < kCoopWarps; ++q) t += red[q];
+      part[blockIdx.x] = t;
     }
     if (!gs.wait()) return false;
-    if (warp < NV) {
-      const double t = edg::warp_sum(edg::lane_share<kPer>(part + (int64_t)warp * G, 1, G));
-      if (lane == 0) total_s[warp] = t;
+    if (warp == 0) {
+      const double t = edg::warp_sum(edg::lane_share<kPer>(part, 1, G));
+      if (lane == 0) total_s = t;
     }
     __syncthreads();
     return true;
   };
   // writes the candidate u_j (already rounded to T) to the basis
-  auto put = [&](int64_t i, int v, int r, double x) {
-    A.V[(i * NV + v) * A.n_pad + r0 + r] = (T)x;
-    if (basis_here) own[i * ld_i + v * ld_v + r] = (T)x;
+  auto put = [&](int64_t i, int r, double x) {
+    A.V[i * A.n_pad + r0 + r] = (T)x;
+    if (basis_here) own[i * ld_i + r] = (T)x;
   };
   // ---- start vector ----
-  double nrm[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    nrm[v] = 0.0;
-    for (int r = tid; r < rows; r += kCoopThreads) {
-      double x = 0.0;
-      if (r0 + r < A.n) {
-        if (A.v0) {
-          x = (double)A.v0[(r0 + r) * NV + v];
-        } else {
-          const uint64_t z = splitmix64(A.seed ^ splitmix64((uint64_t)((r0 + r) * NV + v)));
-          x = ((double)(z >> 11) * (1.0 / 9007199254740992.0)) * 2.0 - 1.0;
-        }
+  double nrm = 0.0;
+  for (int r = tid; r < rows; r += kCoopThreads) {
+    double x = 0.0;
+    if (r0 + r < A.n) {
+      if (A.v0) {
+        x = (double)A.v0[r0 + r];
+      } else {
+        const uint64_t z = splitmix64(A.seed ^ splitmix64((uint64_t)(r0 + r)));
+        x = ((double)(z >> 11) * (1.0 / 9007199254740992.0)) * 2.0 - 1.0;
       }
-      w[v * rows + r] = x;
-      nrm[v] = fma(x, x, nrm[v]);
     }
+    w[r] = x;
+    nrm = fma(x, x, nrm);
   }
-  for (int i = tid; i < NV * (m_max + 2); i += kCoopThreads) al[i] = be[i] = 0.0;
+  for (int i = tid; i < m_max + 2; i += kCoopThreads) al[i] = be[i] = 0.0;
   if (!grid_sum(nrm)) return;
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const double nb = sqrt(total_s[v]), inv = nb > 0.0 ? 1.0 / nb : 0.0;
-    for (int r = tid; r < rows; r += kCoopThreads) {
-      const double x = (double)(T)(w[v * rows + r] * inv);
-      u[v * rows + r] = x;
-      put(0, v, r, x);
-    }
+  const double nb = sqrt(total_s), inv = nb > 0.0 ? 1.0 / nb : 0.0;
+  for (int r = tid; r < rows; r += kCoopThreads) {
+    const double x = (double)(T)(w[r] * inv);
+    u[r] = x;
+    put(0, r, x);
   }
   if (!gs.wait()) return;
   int next_check = A.first_check;
@@ -1132,58 +1118,46 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     const int n_vec = j + 1 - lo;
     // ---- w = H u on this CTA's rows ----
     {
-      const T* x = A.V + (int64_t)j * NV * A.n_pad;
+      const T* x = A.V + (int64_t)j * A.n_pad;
       const int part = tid & (kCoopLanes - 1);
       const int n_it = (rows + kCoopThreads / kCoopLanes - 1) / (kCoopThreads / kCoopLanes);
       for (int it = 0; it < n_it; ++it) {
         const int r = it * (kCoopThreads / kCoopLanes) + tid / kCoopLanes;
-        double acc[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+        double acc = 0.0;
         if (r < rows) {
           constexpr int U = 4;  // gathers in flight per lane
           const int end = rp[r + 1];
           for (int p0 = rp[r] + part; p0 < end; p0 += U * kCoopLanes) {
-            T xv[U][NV], a[U];
+            T xv[U], a[U];
 #pragma unroll
             for (int q = 0; q < U; ++q)
               if (p0 + q * kCoopLanes < end) {
-                const int c = cols[p0 + q * kCoopLanes];
                 a[q] = vals[p0 + q * kCoopLanes];
-#pragma unroll
-                for (int v = 0; v < NV; ++v) xv[q][v] = x[(int64_t)v * A.n_pad + c];
+                xv[q] = x[cols[p0 + q * kCoopLanes]];
               }
 #pragma unroll
             for (int q = 0; q < U; ++q)
-              if (p0 + q * kCoopLanes < end)
-#pragma unroll
-                for (int v = 0; v < NV; ++v) acc[v] = fma((double)a[q], (double)xv[q][v], acc[v]);
+              if (p0 + q * kCoopLanes < end) acc = fma((double)a[q], (double)xv[q], acc);
           }
         }
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-#pragma unroll
-          for (int o = kCoopLanes / 2; o > 0; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o, kCoopLanes);
-          if (r < rows && part == 0) {
-            const int64_t gr = r0 + r;
-            const double d = gr < A.n ? (double)__ldg(A.diag + gr * NV + v) : 0.0;
-            w[v * rows + r] = fma(d, u[v * rows + r], acc[v]);
-          }
+        for (int o = kCoopLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, kCoopLanes);
+        if (r < rows && part == 0) {
+          const double d = r0 + r < A.n ? (double)__ldg(A.diag + r0 + r) : 0.0;
+          w[r] = fma(d, u[r], acc);
         }
       }
     }
     __syncthreads();
-    // ---- dots of this CTA's rows: a warp per vector and problem ----
-    for (int e0 = warp; e0 < n_vec * NV; e0 += kVecs * kCoopWarps) {
+    // ---- dots of this CTA's rows: a warp per vector ----
+    for (int e0 = warp; e0 < n_vec; e0 += kVecs * kCoopWarps) {
       double s[kVecs], z[kVecs];
       const T* b[kVecs];
 #pragma unroll
       for (int h = 0; h < kVecs; ++h) {
-        const int e = e0 + h * kCoopWarps, t = e / NV, v = e - t * NV;
-        b[h] = own + (int64_t)(lo + t) * ld_i + v * ld_v;
+        b[h] = own + (int64_t)(lo + e0 + h * kCoopWarps) * ld_i;
         s[h] = z[h] = 0.0;
       }
-      static_assert(NV == 1, "u and w are one problem's");
       for (int r = lane; r < rows; r += 32 * kRowsAhead) {
         T x[kVecs][kRowsAhead];
 #pragma unroll
@@ -1215,14 +1189,14 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     }
     if (!gs.wait()) return;
     // ---- totals and coefficients ----
-    for (int e0 = warp; e0 < 2 * n_vec * NV; e0 += 4 * kCoopWarps) {
+    for (int e0 = warp; e0 < 2 * n_vec; e0 += 4 * kCoopWarps) {
       double p[4][kPer];  // four sums' partials in flight
 #pragma unroll
       for (int h = 0; h < 4; ++h)
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
           const int e = e0 + h * kCoopWarps, b = lane + 32 * k;
-          p[h][k] = e < 2 * n_vec * NV && b < G ? __ldcg(A.partial + (int64_t)e * G + b) : 0.0;
+          p[h][k] = e < 2 * n_vec && b < G ? __ldcg(A.partial + (int64_t)e * G + b) : 0.0;
         }
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
@@ -1231,23 +1205,18 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
         for (int k = 0; k < kPer; ++k) a += p[h][k];
         a = edg::warp_sum(a);
         const int e = e0 + h * kCoopWarps;
-        if (lane == 0 && e < 2 * n_vec * NV) {
-          const int t = (e >> 1) / NV, v = (e >> 1) - t * NV;
-          tot[(int64_t)v * 2 * (m_max + 2) + 2 * t + (e & 1)] = a;
-        }
+        if (lane == 0 && e < 2 * n_vec) tot[e] = a;
       }
     }
     __syncthreads();
-    if (warp < NV) {
+    if (warp == 0) {
       double out[4];
-      double* alv = al + (int64_t)warp * (m_max + 2);
-      double* bev = be + (int64_t)warp * (m_max + 2);
-      coef_small(lo, j, tot + (int64_t)warp * 2 * (m_max + 2), alv, bev, out);
+      coef_small(lo, j, tot, al, be, out);
       __syncwarp();
       if (lane == 0) {
-        for (int q = 0; q < 4; ++q) coef[warp][q] = out[q];
-        alv[j] = out[2];
-        if (j > lo) bev[j] = out[3];
+        for (int q = 0; q < 4; ++q) coef[q] = out[q];
+        al[j] = out[2];
+        if (j > lo) be[j] = out[3];
       }
     }
     __syncthreads();
@@ -1255,70 +1224,57 @@ __global__ void __launch_bounds__(kCoopThreads, 1) lanczos_coop_k(const CoopArgs
     const int lpr = rows * 2 <= kCoopThreads ? 2 : 1;  // lanes per row
     const int part = tid & (lpr - 1);
     const int n_it = (rows * lpr + kCoopThreads - 1) / kCoopThreads;
+    const double ri = coef[0], c = coef[1];
+    nrm = 0.0;
+    for (int it = 0; it < n_it; ++it) {
+      const int r = (it * kCoopThreads + tid) / lpr;
+      double su = 0.0, sw = 0.0;
+      if (r < rows) {
+        const T* b = own + (int64_t)lo * ld_i + r;
+        for (int t = part; t < n_vec - 1; t += kAhead * lpr) {
+          T x[kAhead];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double ri = coef[v][0], c = coef[v][1];
-      const double* tv = tot + (int64_t)v * 2 * (m_max + 2);
-      nrm[v] = 0.0;
-      for (int it = 0; it < n_it; ++it) {
-        const int r = (it * kCoopThreads + tid) / lpr;
-        double su = 0.0, sw = 0.0;
-        if (r < rows) {
-          const T* b = own + (int64_t)lo * ld_i + v * ld_v + r;
-          for (int t = part; t < n_vec - 1; t += kAhead * lpr) {
-            T x[kAhead];
+          for (int q = 0; q < kAhead; ++q) x[q] = t + q * lpr < n_vec - 1 ? b[(int64_t)(t + q * lpr) * ld_i] : T(0);
 #pragma unroll
-            for (int q = 0; q < kAhead; ++q) x[q] = t + q * lpr < n_vec - 1 ? b[(int64_t)(t + q * lpr) * ld_i] : T(0);
-#pragma unroll
-            for (int q = 0; q < kAhead; ++q)
-              if (t + q * lpr < n_vec - 1) {
-                su = fma((double)x[q], tv[2 * (t + q * lpr)], su);
-                sw = fma((double)x[q], tv[2 * (t + q * lpr) + 1], sw);
-              }
-          }
+          for (int q = 0; q < kAhead; ++q)
+            if (t + q * lpr < n_vec - 1) {
+              su = fma((double)x[q], tot[2 * (t + q * lpr)], su);
+              sw = fma((double)x[q], tot[2 * (t + q * lpr) + 1], sw);
+            }
         }
-        if (lpr == 2) {
-          su += __shfl_xor_sync(0xffffffffu, su, 1);
-          sw += __shfl_xor_sync(0xffffffffu, sw, 1);
-        }
-        if (r < rows && part == 0) {
-          const double q = (double)(T)((u[v * rows + r] - su) * ri);
-          double y = (w[v * rows + r] - sw) - q * c;
-          nrm[v] = fma(y, y, nrm[v]);
-          y = (double)(T)(y * ri);
-          u[v * rows + r] = y;
-          put(j, v, r, q);
-          put(j + 1, v, r, y);
-        }
+      }
+      if (lpr == 2) {
+        su += __shfl_xor_sync(0xffffffffu, su, 1);
+        sw += __shfl_xor_sync(0xffffffffu, sw, 1);
+      }
+      if (r < rows && part == 0) {
+        const double q = (double)(T)((u[r] - su) * ri);
+        double y = (w[r] - sw) - q * c;
+        nrm = fma(y, y, nrm);
+        y = (double)(T)(y * ri);
+        u[r] = y;
+        put(j, r, q);
+        put(j + 1, r, y);
       }
     }
     if (!grid_sum(nrm)) return;
-    if (tid < NV) be[(int64_t)tid * (m_max + 2) + j + 1] = sqrt(total_s[tid]) * coef[tid][0];
+    if (tid == 0) be[j + 1] = sqrt(total_s) * coef[0];
     __syncthreads();
     // ---- convergence ----
     const int m = j + 1;
     if (m >= next_check || m >= m_max || (int64_t)m >= A.n) {
       volatile DevState* vst = A.st;
       if (blockIdx.x == 0) {
-        for (int v = 0; v < NV; ++v) {
-          if (vst->m_conv[v] != 0) continue;
-          const double* alv = al + (int64_t)v * (m_max + 2);
-          const double* bev = be + (int64_t)v * (m_max + 2);
-          double* S = A.tri_vec + (int64_t)v * kMaxK * A.ld_s;
-          bool ends;
-          const int mv = edg::ritz_dimension<kCoopThreads>(alv, bev, m, &ends), kk = A.k < mv ? A.k : mv;
-          const bool exact = ends || (int64_t)m == A.n;
-          for (int e = tid; e < kMaxK * A.ld_s; e += kCoopThreads) S[e] = 0.0;
-          __syncthreads();
-          tridiag_body<kCoopThreads>(alv, bev, mv, kk, A.tri_eval + (int64_t)v * kMaxK, S, A.ld_s,
-                                     A.tri_work + (int64_t)v * 6 * A.ld_s);
-          __syncthreads();
-          if (tid == 0)
-            judge(vst, v, mv, kk, A.k, exact, A.tol, A.tri_eval + (int64_t)v * kMaxK, bev[mv], S, A.ld_s);
-          __syncthreads();
-        }
+        bool ends;
+        const int mv = edg::ritz_dimension<kCoopThreads>(al, be, m, &ends), kk = A.k < mv ? A.k : mv;
+        const bool exact = ends || (int64_t)m == A.n;
+        for (int e = tid; e < kMaxK * A.ld_s; e += kCoopThreads) A.tri_vec[e] = 0.0;
+        __syncthreads();
+        tridiag_body<kCoopThreads>(al, be, mv, kk, A.tri_eval, A.tri_vec, A.ld_s, A.tri_work);
+        __syncthreads();
         if (tid == 0) {
-          const int done = after_check(vst, NV, m, m_max, A.n, A.tol, A.check_every);
+          judge(vst, 0, mv, kk, A.k, exact, A.tol, A.tri_eval, be[mv], A.tri_vec, A.ld_s);
+          const int done = after_check(vst, 1, m, m_max, A.n, A.tol, A.check_every);
           vst->checks = vst->checks + 1;
           vst->j = m;
           vst->done = done;
@@ -1458,7 +1414,7 @@ int run_lanczos(const edg_lanczos_problem* p, char* ws, double* evals, void* eve
     if (e != cudaSuccess) return edg::cuda_status(e, "edg_lanczos: set-up");
     const int64_t g = edg::coop_ctas(n_pad, n_sm);
     const int rows = (int)((n_pad + g - 1) / g);
-    if (coop && occ >= 1 && rows <= kCoopRows && coop_fixed(rows, NV, L.m_max) <= kCoopSmem) {
+    if (coop && occ >= 1 && rows <= kCoopRows && coop_fixed(rows, L.m_max) <= kCoopSmem) {
       state_init_k<<<1, 32, 0, s>>>(st, first_check, p->reorth_window);
       if ((e = cudaMemsetAsync(tickets, 0, 8 * sizeof(int), s)) != cudaSuccess)
         return edg::cuda_status(e, "edg_lanczos: tickets");
