@@ -246,8 +246,7 @@ class QMB_hamiltonian:
         sec = self.sector
         n = len(sec)
         dims = _lib.SiteDims()
-        for s in range(sec.n_sites):
-            dims.d[s] = int(sec.loc_dims[s])
+        dims.d[: sec.n_sites] = sec.loc_dims.tolist()
         out = torch.empty(n, dtype=torch.complex128, device=sec.device)
         code = 0 if psi is None else _PSI_CODES[psi.dtype]
         stride = 1 if psi is None else max(int(psi.stride(0)), 1)
