@@ -19,7 +19,7 @@
 // needs the updated w written in f64 and a further pass that reads it back
 // (40 B a row of a complex64 basis).
 //
-// Two forms, chosen by the number of rows (coop_fits):
+// Two forms, chosen by the number of rows and entries (one_launch):
 //   * large sectors: matvec, dots, coefficients, update as launches over all
 //     rows; for the local recurrence on the packed layout the dots are summed
 //     in the matvec's epilogue (packed.cu) and a step is two launches;

@@ -453,7 +453,7 @@ typedef struct {
                           /* [5] check ms (CUDA events on the stream)       */
   int32_t* host_progress; /* optional PINNED host memory, >= 4 int32: the   */
                           /* device writes [0] steps done, [1] done flag;   */
-                          /* NULL = the host synchronises once per replay   */
+                          /* NULL = the host synchronises once per group    */
   const int32_t* sell_perm;   /* optional SELL layout of the off-diagonal   */
   const int32_t* sell_width;  /* matrix (edg_sell_*), used by the f32 path  */
   const int64_t* sell_off;    /* when sell_entries is not NULL              */
@@ -478,7 +478,7 @@ int64_t edg_lanczos_small_rows(void);
 int edg_lanczos_one_launch(const edg_lanczos_problem* p);
 /* Bytes of device workspace edg_lanczos needs. */
 int64_t edg_lanczos_workspace_bytes(const edg_lanczos_problem* p);
-/* Runs to convergence (synchronizes every check_every steps).  Outputs:
+/* Runs to convergence (returns when the results are on the host).  Outputs:
  * evals [nvec][k] (f64), evecs [k][n_rows][nvec] in the problem dtype (may be
  * NULL), iters_out [nvec] steps used, resid_out [nvec][k] residual bounds. */
 int edg_lanczos(const edg_lanczos_problem* p, void* workspace,
