@@ -26,6 +26,11 @@ from ._lib import check, lib, ptr, stream_handle
 __all__ = ["MomentumBasis", "translation_sources", "krylov_evolve", "DENSE_MAX"]
 
 DENSE_MAX = 4096
+# Sector rows up to which the projector's host arrays are narrowed on the host: a
+# small basis pays more for a few device operations than for its bytes (host_arrays
+# at 282 rows 0.10 ms so, 0.18 to 0.27 with them; 2,214 rows 0.13, 0.19 to 0.25;
+# 17,906 rows 0.29 to 0.32, 0.23 to 0.32; 147,578 rows 1.6 to 1.9, 0.53 to 0.74)
+HOST_ROWS = 1 << 14
 
 
 def translation_sources(lvals, unit_cell):
@@ -152,18 +157,28 @@ class MomentumBasis:
     # ------------------------------------------------------------ host view
     def host_arrays(self) -> dict:
         """The reference's momentum_basis dict (CSC and CSR of B, host)."""
-        # narrowed on the device: half the bytes to copy, no pass over them here
-        has = self.row_col[: self.n_rows] >= 0
-        r_ptr = torch.zeros(self.n_rows + 1, dtype=torch.int32, device=self.device)
-        torch.cumsum(has, 0, dtype=torch.int32, out=r_ptr[1:])
+        cp, ri = self.col_ptr, self.row_idx[: self.nnz]
         dv, rv, rc = self.data[: self.nnz], self.row_val[: self.n_rows], self.row_col[: self.n_rows]
-        if self.nnz < self.n_rows:
-            rv, rc = rv[has], rc[has]
-        if self.zero_k:
-            dv, rv = dv.real, rv.real
-        cp, ri, dv, r_ptr, rc, rv = (x.cpu().numpy() for x in (
-            self.col_ptr.to(torch.int32), self.row_idx[: self.nnz], dv.contiguous(), r_ptr, rc.to(torch.int32),
-            rv.contiguous()))
+        if self.n_rows <= HOST_ROWS:
+            cp, ri, dv, rv, rc = (x.cpu().numpy() for x in (cp, ri, dv, rv, rc))
+            has = rc >= 0
+            r_ptr = np.zeros(self.n_rows + 1, dtype=np.int32)
+            np.cumsum(has, out=r_ptr[1:])
+            rv, rc = rv[has], rc[has].astype(np.int32)
+            if self.zero_k:
+                dv, rv = dv.real.copy(), rv.real.copy()
+            cp, ri = cp.astype(np.int32), ri.astype(np.int32, copy=False)
+        else:
+            # narrowed on the device: half the bytes to copy, no pass over them here
+            has = rc >= 0
+            r_ptr = torch.zeros(self.n_rows + 1, dtype=torch.int32, device=self.device)
+            torch.cumsum(has, 0, dtype=torch.int32, out=r_ptr[1:])
+            if self.nnz < self.n_rows:
+                rv, rc = rv[has], rc[has]
+            if self.zero_k:
+                dv, rv = dv.real, rv.real
+            cp, ri, dv, r_ptr, rc, rv = (x.cpu().numpy() for x in (
+                cp.to(torch.int32), ri, dv.contiguous(), r_ptr, rc.to(torch.int32), rv.contiguous()))
         return {"pair_mode": False, "n_rows": self.n_rows, "n_cols": self.n_cols, "L_col_ptr": cp,
                 "L_row_idx": ri, "L_data": dv, "R_row_ptr": r_ptr, "R_col_idx": rc, "R_data": rv}
 

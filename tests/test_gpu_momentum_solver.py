@@ -78,3 +78,25 @@ def test_reduce_column_lengths(n_cols):
     ref = np.array([np.sum(data[a:b].conj() * w[rows[a:b]]) for a, b in zip(col_ptr[:-1], col_ptr[1:])])
     out = y.cpu().numpy()
     assert np.max(np.abs(out[:n_cols] - ref)) <= 1e-13 * 33 and out[n_cols] == 7.0
+
+
+@pytest.mark.parametrize("name", ["su2_1d_L6_pbc", "su2_1d_L8_pbc_uc2", "qed1d_L6_pbc_uc2", "su2_1d_L8_pbc_tc"])
+def test_host_arrays_narrowed_on_either_side(name, monkeypatch):
+    """The projector's host arrays are the same, types included, whichever side
+    narrows them."""
+    from cases import build_momentum_case
+    from edgpu import momentum
+
+    model, g, m, ucs, ks = build_momentum_case(name, device="cuda")
+    for k in ks:
+        got = []
+        for rows in (0, 1 << 30):
+            monkeypatch.setattr(momentum, "HOST_ROWS", rows)
+            model.set_momentum_sector(ucs, k, TC_symmetry=name.endswith("_tc"))
+            got.append(model.momentum_basis)
+        assert got[0].keys() == got[1].keys()
+        for key, a in got[0].items():
+            b = got[1][key]
+            assert np.array_equal(a, b)
+            if isinstance(a, np.ndarray):
+                assert a.dtype == b.dtype and a.flags["C_CONTIGUOUS"] and b.flags["C_CONTIGUOUS"], key
